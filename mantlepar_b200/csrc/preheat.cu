@@ -157,8 +157,8 @@ __device__ __forceinline__ EdgeGeo edge_geo(const StageHot& t, int nx, int ny, l
         g.L = g.reverse ? (long long)(j - 1) * nx + i : (long long)j * nx + i;
         if (!g.boundary) g.R = (long long)(j - 1) * nx + i;
         else g.wall = j == 0 ? 0 : 1;
-        g.lfix = g.reverse ? t.Y : -t.Y;
-        g.rfix = t.Y;
+        g.lfix = g.reverse ? 1.0 : -1.0;
+        g.rfix = 1.0;
     } else {
         const unsigned k = (unsigned)(e - nI);
         const int i = (int)(k % (unsigned)(nx + 1)), j = (int)(k / (unsigned)(nx + 1));
@@ -168,8 +168,8 @@ __device__ __forceinline__ EdgeGeo edge_geo(const StageHot& t, int nx, int ny, l
         g.L = g.reverse ? (long long)j * nx : (long long)j * nx + (i - 1);
         if (!g.boundary) g.R = (long long)j * nx + i;
         else g.wall = i == 0 ? 2 : 3;
-        g.lfix = g.reverse ? -t.X : t.X;
-        g.rfix = -t.X;
+        g.lfix = g.reverse ? -1.0 : 1.0;
+        g.rfix = -1.0;
     }
     return g;
 }
@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(128) pre_recon_kernel(int nx, int ny, const do
         }
     const int ci = i == 0 ? 0 : (i == nx - 1 ? 2 : 1), cj = j == 0 ? 0 : (j == ny - 1 ? 2 : 1);
     double D[9];
-    const int st = reconstruct(t, ci, cj, u, D);
+    const int st = ci == 1 && cj == 1 ? reconstruct<true>(t, 31u, u, D)
+                                      : reconstruct<false>(t, candidate_mask(ci, cj), u, D);
 #pragma unroll
     for (int m = 0; m < 9; ++m) rec[(size_t)m * N + cell] = D[m];
     if (st) record_error(status, PART_UPDATE, cell, st);
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(128, 8) pre_face_kernel(int nx, int ny, const 
 #pragma unroll
     for (int q = 0; q < kNQ; ++q) {
         const int cq = g.reverse ? kNQ - 1 - q : q;
-        const double at = g.horizontal ? t.gx[cq] : t.gy[cq];
+        const double at = t.g[cq];
         const double v = sgn * __ldg(vn + e * kNQ + cq);
         const double uL = mL + quad(l0, l1, l2, at);
         if (!isfinite(v) || !isfinite(uL)) st = st ? st : E_OUTOFRANGE;
@@ -462,19 +463,19 @@ __global__ void __launch_bounds__(128) pre_diag_kernel(int nx, int ny, const dou
                 u[dj][di] = __ldg(F + (size_t)jj * nx + ii);
             }
         m[f] = u[1][1];
-        const int s = reconstruct(t, ci, cj, u, D[f]);
+        const int s = reconstruct<false>(t, candidate_mask(ci, cj), u, D[f]);
         st = st ? st : s;
     }
     if (st) { record_error(status, PART_UPDATE, cell, st); return; }
     double Ts = 0.0, Ps = 0.0;
     for (int b = 0; b < kNQ; ++b) {
         double h0, h1, h2, c0, c1, c2;
-        const double y = t.gy[b];
+        const double y = t.g[b];
         q2_row(D[0], y, h0, h1, h2);
         q2_row(D[1], y, c0, c1, c2);
         const double tep = tep_at(ph, height(t, j, y));
         for (int q = 0; q < kNQ; ++q) {
-            const double x = t.gx[q];
+            const double x = t.g[q];
             PhaseLean pl;
             const int s = phase_stage_lean(ph.sk, m[0] + quad(h0, h1, h2, x), m[1] + quad(c0, c1, c2, x), tep, pl);
             if (s) { st = st ? st : s; continue; }

@@ -247,11 +247,15 @@ __device__ __forceinline__ int reconstruct_quad(const QuadDev& q, size_t N, long
             if (sg[f][k + 1] < 0.0) st[f] = MP_ERR_FP;
     }
     double w[F][5];
+    const double ie = 1.0 / eA;
+    const unsigned mask = candidate_mask(ci, cj);
 #pragma unroll
-    for (int f = 0; f < F; ++f) weights(sg[f], on, eA, w[f]);
+    for (int f = 0; f < F; ++f) {
+        double s[5];
 #pragma unroll
-    for (int f = 0; f < F; ++f)
-        if (!isfinite(w[f][0] + w[f][1] + w[f][2] + w[f][3] + w[f][4])) st[f] = MP_ERR_FP;
+        for (int k = 0; k < 5; ++k) s[k] = fma(sg[f][k], ie, 1.0);
+        if (weno_weights<false>(s, mask, eA * eA, w[f])) st[f] = MP_ERR_FP;
+    }
 #pragma unroll
     for (int f = 0; f < F; ++f)
 #pragma unroll

@@ -28,7 +28,7 @@ struct ParamTables {
     StageHot d;
 };
 
-inline void make_param_tables(const StageTables& t, ParamTables& p) { p.d = static_cast<const StageHot&>(t); }
+inline void make_param_tables(const StageTables& t, ParamTables& p) { p.d = t; }
 
 template <class R> struct Tab;
 // Tab pointing at the parameter-space copy (inside a kernel taking a
@@ -36,24 +36,34 @@ template <class R> struct Tab;
 template <class R> __device__ __forceinline__ Tab<R> param_tab(const ParamTables& p);
 template <> struct Tab<double> {
     const StageHot* t;
-    __device__ double C9(int c, int m) const { return t->C9[c][m]; }
-    __device__ double S9(int r, int c) const { return t->S9[r][c]; }
-    __device__ double C4(int c, int m) const { return t->C4[c][m]; }
-    __device__ double S4(int k, int r, int c) const { return t->S4[k][r][c]; }
-    __device__ double SF9(int k) const { return t->SF9[k]; }
-    __device__ double SF4(int p, int k) const { return t->SF4[p][k]; }
-    __device__ double X() const { return t->X; }
-    __device__ double Y() const { return t->Y; }
-    __device__ double epsA() const { return t->epsA; }
-    __device__ double gx(int q) const { return t->gx[q]; }
-    __device__ double gy(int q) const { return t->gy[q]; }
-    __device__ double line_c(int l) const { return t->line_c[l]; }
 };
 
 template <> __device__ __forceinline__ Tab<double> param_tab<double>(const ParamTables& p) { return Tab<double>{&p.d}; }
 
 template <class R> __device__ __forceinline__ R eps_of();
 template <> __device__ __forceinline__ double eps_of<double>() { return 2.220446049250313e-16; }
+
+// 1/x for normal x with a normal reciprocal: the hardware's approximation
+// (relative error e below 2^-19.9) and one third-order Newton step
+// y (1 + e + e^2). Rounds to another double than 1.0 / x for 3 in 10^4
+// arguments, by one ulp; three FP64 operations, no branch and no call, where
+// the division's range tests and slow path end a basic block.
+__device__ __forceinline__ double rcp(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double e = fma(-x, y, 1.0);
+    e = fma(e, e, e);
+    return fma(y, e, y);
+}
+// a/b through rcp with the remainder's correction (Markstein's final step).
+__device__ __forceinline__ double div_normal(double a, double b) {
+    const double y = rcp(b), q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+// Magnitude within [2^-960, 2^960]: rcp and div_normal apply.
+__device__ __forceinline__ bool rcp_range(double x) {
+    return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x03f00000u <= 0x78000000u;
+}
 
 // Row / column coefficients of a Q2 polynomial (coefficient m = j*3 + i of
 // xi^i eta^j): along the row eta = y, p(xi) = a0 + xi*(a1 + xi*a2).
@@ -105,139 +115,136 @@ __device__ __forceinline__ R smoothness(GF&& SF, G&& S, const R* diff) {
     return exact > R(0) ? exact : R(0);
 }
 
-// Nonlinear weights alpha_k = (sigma_k + eps*A)^-(s*r_k + eta(r_k)): 7 for
-// the 3x3 order-2 candidate, 5 for the 2x2 order-1 candidates
-// (reconstruction.cpp:43-54,212-265). Written as ratios r = epsA/(sigma+epsA)
-// in (0,1] with the common factor (epsA)^-7 divided out, so nothing
-// overflows; normalised to sum 1.
-__device__ __forceinline__ void weights(const double* sig, const bool* on, double eA, double* w) {
-    // The five reciprocals 1/(sigma_k + epsA) from one division: prefix
-    // and suffix products of s_k = sigma_k + epsA (s_k >= epsA > 0).
-    double sk[5], pre[5], suf[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) sk[k] = sig[k] + eA;
-    pre[0] = 1.0;
-#pragma unroll
-    for (int k = 1; k < 5; ++k) pre[k] = pre[k - 1] * sk[k - 1];
-    suf[4] = 1.0;
-#pragma unroll
-    for (int k = 3; k >= 0; --k) suf[k] = suf[k + 1] * sk[k + 1];
-    const double P = pre[4] * sk[4];
-    double inv_s[5];
-    if (P > 1e-290 && P < 1e290) {
-        const double invP = 1.0 / P;
-#pragma unroll
-        for (int k = 0; k < 5; ++k) inv_s[k] = (pre[k] * suf[k]) * invP;
-    } else {
-#pragma unroll
-        for (int k = 0; k < 5; ++k) inv_s[k] = 1.0 / sk[k];
-    }
-    double alpha[5];
-    const double scale = on[0] ? eA * eA : 1.0;
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        const double r = eA * inv_s[k];
-        const double r2 = r * r;
-        alpha[k] = !on[k] ? 0.0 : (k == 0 ? r2 * r2 * r2 * r : scale * (r2 * r2 * r));
-    }
+// Nonlinear weights alpha_k = (sigma_k + epsA)^-(s*r_k + eta(r_k)): exponent
+// 7 for the 3x3 order-2 candidate, 5 for the 2x2 order-1 candidates
+// (reconstruction.cpp:43-54,212-265), normalised to sum 1, from
+// s_k = 1 + sigma_k / epsA >= 1 (s_k = 1 for a candidate that is off).
+// Multiplying every alpha by epsA^7 s_0^7 (s_1 s_2 s_3 s_4)^5 leaves products
+// only: w_0 ~ (s_1 s_2 s_3 s_4)^5 and w_k ~ epsA^2 s_0^7 (the other three)^5,
+// one reciprocal for the five weights. Q = s_0^2 s_1 s_2 s_3 s_4 < 1e59 keeps
+// every product below 1e296 (s_0^7 t^5 <= Q^5 as s_0 >= 1); it is false for a
+// non-finite s_k, so only the general form below has to test for one.
+static __device__ __noinline__ int weights_general(const double* s, unsigned on, double epsA2, double* w) {
+    // Ratios r = epsA/(sigma + epsA) = 1/s in (0, 1]: nothing overflows.
     double sum = 0;
+    int st = 0;
+    for (int k = 0; k < 5; ++k) {
+        if (!((on >> k) & 1u)) { w[k] = 0; continue; }
+        if (!(s[k] < INFINITY)) st = MP_ERR_FP;
+        const double r = 1.0 / s[k], r2 = r * r;
+        w[k] = k == 0 ? r2 * r2 * r2 * r : ((on & 1u) ? epsA2 : 1.0) * (r2 * r2 * r);
+        sum += w[k];
+    }
+    for (int k = 0; k < 5; ++k) w[k] /= sum;
+    if (!isfinite(w[0] + w[1] + w[2] + w[3] + w[4])) st = MP_ERR_FP;
+    return st;
+}
+// kAll: every candidate is on (on is not read).
+template <bool kAll>
+__device__ __forceinline__ int weno_weights(const double (&s)[5], unsigned on, double epsA2, double (&w)[5]) {
+    const double s12 = s[1] * s[2], s34 = s[3] * s[4], P = s12 * s34, s02 = s[0] * s[0];
+    if (!(P * s02 < 1e59)) {
+        // Copies, so that the arrays of the common path stay in registers.
+        double sc[5], wc[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) sum += alpha[k];
-    const double inv = 1.0 / sum;
+        for (int k = 0; k < 5; ++k) sc[k] = s[k];
+        const int st = weights_general(sc, kAll ? 31u : on, epsA2, wc);
 #pragma unroll
-    for (int k = 0; k < 5; ++k) w[k] = alpha[k] * inv;
+        for (int k = 0; k < 5; ++k) w[k] = wc[k];
+        return st;
+    }
+    auto p5 = [](double x) { const double x2 = x * x; return x2 * x2 * x; };
+    const double f = (kAll || (on & 1u) ? epsA2 : 1.0) * (s02 * s02 * (s02 * s[0]));
+    w[0] = p5(P);
+    w[1] = f * p5(s[2] * s34);
+    w[2] = f * p5(s[1] * s34);
+    w[3] = f * p5(s12 * s[4]);
+    w[4] = f * p5(s12 * s[3]);
+    if (!kAll) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) w[k] = (on >> k) & 1u ? w[k] : 0.0;
+    }
+    const double sum = (w[0] + (w[1] + w[2])) + (w[3] + w[4]);
+    const double inv = rcp_range(sum) ? rcp(sum) : 1.0 / sum;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) w[k] *= inv;
+    return 0;
 }
 
-// Build D (9 coefficients, FP64) for one field from the 3x3 neighbourhood
-// u[dj][di] (index 1,1 = target). Candidate mask by boundary class (ci, cj):
-// stencils that leave the domain are dropped (reconstruction.cpp:150-153).
-// Returns a nonzero PETSC_ERR_FP-class status when a smoothness form is
-// negative beyond roundoff or the weights cannot be normalised.
-__device__ __forceinline__ int reconstruct(const StageHot& td, int ci, int cj, const double (&u)[3][3],
-                                           double (&D)[9]) {
-    using R = double;
-    const Tab<double> t{&td};
-    double d[3][3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) d[a][b] = u[a][b] - u[1][1];
-    // Candidate order: 3x3 at (-1,-1); 2x2 at (0,-1), (0,0), (-1,-1), (-1,0).
-    const int offi[4] = {0, 0, -1, -1}, offj[4] = {-1, 0, -1, 0};
-    bool on[5];
-    on[0] = (ci == 1 && cj == 1);
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        on[k + 1] = !((offi[k] == 0 && ci == 2) || (offi[k] == -1 && ci == 0) || (offj[k] == 0 && cj == 2) ||
-                      (offj[k] == -1 && cj == 0));
-    R sig[5];
-    int st = 0;
-    // Pass 1: smoothness of every active candidate.
-    if (on[0]) {
-        R diff[8];
-#pragma unroll
-        for (int c = 1; c < 9; ++c) diff[c - 1] = (R)(d[c / 3][c % 3] - d[0][0]);
-        sig[0] = smoothness<R, 8>([&](int k) { return t.SF9(k); }, [&](int r, int c) { return t.S9(r, c); }, diff);
-        if (sig[0] < R(0)) st = MP_ERR_FP;
-    } else {
-        sig[0] = 0;
+// Candidates kept at a boundary class (ci, cj): stencils that leave the
+// domain are dropped (reconstruction.cpp:150-153). Bit 0: the 3x3 stencil;
+// bits 1-4: the 2x2 stencils with lower-left cell (0,-1), (0,0), (-1,-1),
+// (-1,0) relative to the target, i.e. towards SE, NE, SW, NW.
+__device__ __forceinline__ unsigned candidate_mask(int ci, int cj) {
+    const bool e = ci != 2, w = ci != 0, n = cj != 2, s = cj != 0;
+    return (e && w && n && s ? 1u : 0u) | (e && s ? 2u : 0u) | (e && n ? 4u : 0u) | (w && s ? 8u : 0u) |
+           (w && n ? 16u : 0u);
+}
+
+// Build D (9 coefficients) for one field from the 3x3 neighbourhood
+// u[dj][di] (index 1,1 = target) on a uniform mesh. In the cell's frame the
+// candidates have closed forms: with d the differences to the target,
+//   order 1 towards NE: dE/2 xi + dN/2 eta + (dNE - dE - dN)/4 xi eta
+// (mean over the target zero), and the order-2 candidate is the tensor
+// product of the 1D averages' inverse (a1 = (u+ - u-)/4, a2 = (u+ - 2 u0 +
+// u-)/8, a0 = u0 - a2/3). Their smoothness forms are sums of squares
+// (tables.hpp), so no sigma is negative. The kernel is bound by the FP64
+// pipe (one warp instruction per two cycles): with the general basis and
+// smoothness matrices of the mesh (64 + 44 FMAs and 4 x 21 per field) and the
+// limiter scan line by line it issued 1680 FP64 instructions per warp and took
+// 160 us at 640x1280; with these forms and scan_interior 1121 and 89 us.
+// kAll: an interior cell. Returns MP_ERR_FP when the weights cannot be
+// normalised (non-finite data).
+template <bool kAll>
+__device__ __forceinline__ int reconstruct(const StageHot& t, unsigned on, const double (&u)[3][3], double (&D)[9]) {
+    const double c = u[1][1];
+    const double dSW = u[0][0] - c, dS = u[0][1] - c, dSE = u[0][2] - c, dW = u[1][0] - c, dE = u[1][2] - c,
+                 dNW = u[2][0] - c, dN = u[2][1] - c, dNE = u[2][2] - c;
+    // Order 2: x differences of each row (A first, B second), then along y.
+    const double AS = dSE - dSW, A0 = dE - dW, AN = dNE - dNW;
+    const double BS = fma(-2.0, dS, dSE + dSW), B0 = dE + dW, BN = fma(-2.0, dN, dNE + dNW);
+    const double q11 = (AN - AS) * 0.0625, q12 = fma(-2.0, A0, AN + AS) * 0.03125;
+    const double q21 = (BN - BS) * 0.03125, q22 = fma(-2.0, B0, BN + BS) * 0.015625;
+    const double q10 = fma(-1.0 / 3.0, q12, 0.25 * A0), q01 = fma(-1.0 / 3.0, q21, 0.25 * (dN - dS));
+    const double q20 = fma(-1.0 / 3.0, q22, 0.125 * B0), q02 = fma(-1.0 / 3.0, q22, 0.125 * (dN + dS));
+    const double q00 = fma(-1.0 / 3.0, q20 + q02, (-1.0 / 9.0) * q22);
+    double s[5];
+    {
+        const double t1 = fma(t.cy, q12, q10), t2 = fma(t.cx, q21, q01), t3 = fma(t.cy, q22, q20),
+                     t4 = fma(t.cx, q22, q02);
+        const double a = fma(t.sg[0] * t1, t1, 1.0), b = (t.sg[1] * t2) * t2;
+        double x = fma(t.sg[2] * t3, t3, a), y = fma(t.sg[3] * t4, t4, b);
+        x = fma(t.sg[4] * q11, q11, x);
+        y = fma(t.sg[5] * q12, q12, y);
+        x = fma(t.sg[6] * q21, q21, x);
+        y = fma(t.sg[7] * q22, q22, y);
+        s[0] = x + y;
     }
+    // Order 1: mixed differences and sigma of the four quadrants.
+    const double bSE = (dSE - dE) - dS, bNE = (dNE - dE) - dN, bSW = (dSW - dW) - dS, bNW = (dNW - dW) - dN;
+    {
+        const double e = fma(t.gx2 * dE, dE, 1.0), w = fma(t.gx2 * dW, dW, 1.0);
+        const double n = (t.gy2 * dN) * dN, o = (t.gy2 * dS) * dS;
+        s[1] = fma(t.gb * bSE, bSE, e + o);
+        s[2] = fma(t.gb * bNE, bNE, e + n);
+        s[3] = fma(t.gb * bSW, bSW, w + o);
+        s[4] = fma(t.gb * bNW, bNW, w + n);
+    }
+    if (!kAll) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (!on[k + 1]) { sig[k + 1] = 0; continue; }
-        const int oi = offi[k], oj = offj[k];
-        const double a0 = d[1 + oj][1 + oi];
-        R diff[3];
-#pragma unroll
-        for (int c = 1; c < 4; ++c) diff[c - 1] = (R)(d[1 + oj + c / 2][1 + oi + c % 2] - a0);
-        const int tpos = (-oj) * 2 + (-oi);
-        sig[k + 1] = smoothness<R, 3>([&](int q) { return t.SF4(tpos, q); }, [&](int r, int c) { return t.S4(tpos, r, c); },
-                                      diff);
-        if (sig[k + 1] < R(0)) st = MP_ERR_FP;
+        for (int k = 0; k < 5; ++k) s[k] = (on >> k) & 1u ? s[k] : 1.0;
     }
     double w[5];
-    weights(sig, on, t.epsA(), w);
-    if (!isfinite(w[0] + w[1] + w[2] + w[3] + w[4])) st = MP_ERR_FP;
-    // Pass 2: weighted coefficients accumulated into D (FP64).
-#pragma unroll
-    for (int m = 0; m < 9; ++m) D[m] = 0;
-    if (on[0]) {
-        double diff[8];
-#pragma unroll
-        for (int c = 1; c < 9; ++c) diff[c - 1] = d[c / 3][c % 3] - d[0][0];
-#pragma unroll
-        for (int m = 0; m < 9; ++m) {
-            double v = m == 0 ? d[0][0] : 0.0;
-#pragma unroll
-            for (int c = 1; c < 9; ++c) v += diff[c - 1] * td.C9[c][m];
-            D[m] = w[0] * v;
-        }
-    }
-    const double X = td.X, Y = td.Y;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (!on[k + 1]) continue;
-        const int oi = offi[k], oj = offj[k];
-        const double a0 = d[1 + oj][1 + oi];
-        double diff[3];
-#pragma unroll
-        for (int c = 1; c < 4; ++c) diff[c - 1] = d[1 + oj + c / 2][1 + oi + c % 2] - a0;
-        double b[4];
-#pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            double v = m == 0 ? a0 : 0.0;
-#pragma unroll
-            for (int c = 1; c < 4; ++c) v += diff[c - 1] * td.C4[c][m];
-            b[m] = v;
-        }
-        // Re-expand about the target centre: zeta = xi - delta, delta = ((2oi+1)X, (2oj+1)Y).
-        const double dx = (double)(2 * oi + 1) * X, dy = (double)(2 * oj + 1) * Y;
-        const double wk = w[k + 1];
-        D[0] += wk * (b[0] - b[1] * dx - b[2] * dy + b[3] * dx * dy);
-        D[1] += wk * (b[1] - b[3] * dy);
-        D[3] += wk * (b[2] - b[3] * dx);
-        D[4] += wk * b[3];
-    }
+    const int st = weno_weights<kAll>(s, on, t.epsA2, w);
+    D[0] = w[0] * q00;
+    D[1] = fma(w[0], q10, 0.5 * fma(w[1] + w[2], dE, -((w[3] + w[4]) * dW)));
+    D[2] = w[0] * q20;
+    D[3] = fma(w[0], q01, 0.5 * fma(w[2] + w[4], dN, -((w[1] + w[3]) * dS)));
+    D[4] = fma(w[0], q11, 0.25 * (fma(w[2], bNE, -(w[1] * bSE)) + fma(w[3], bSW, -(w[4] * bNW))));
+    D[5] = w[0] * q21;
+    D[6] = w[0] * q02;
+    D[7] = w[0] * q12;
+    D[8] = w[0] * q22;
     return st;
 }
 

@@ -145,19 +145,18 @@ struct ReconArgs {
 };
 
 // Max/min of the deviation polynomial over the class's limiter points by
-// exact per-point evaluation in FP64, with the finiteness check of every
-// value. Used when the coefficients are too large for the fast scan's bound.
+// per-point evaluation with the finiteness check of every value. Used when
+// the data are so large that a value could overflow.
 __device__ __noinline__ void scan_lines_exact(const StageHot& t, int l0, int l1, const double* D, double& mx,
                                               double& mn, bool& bad) {
     double rmx = D[0], rmn = D[0];
     bad = bad || !isfinite(D[0]);
     for (int l = l0; l < l1; ++l) {
         double a0, a1, a2;
-        const bool row = t.line_dir[l] == 0;
-        if (row) q2_row(D, t.line_c[l], a0, a1, a2);
+        if (t.line_dir[l] == 0) q2_row(D, t.line_c[l], a0, a1, a2);
         else q2_col(D, t.line_c[l], a0, a1, a2);
         for (int q = 0; q < kNQ; ++q) {
-            const double v = quad(a0, a1, a2, row ? t.gx[q] : t.gy[q]);
+            const double v = quad(a0, a1, a2, t.g[q]);
             rmx = fmax(rmx, v); rmn = fmin(rmn, v);
             bad = bad || !isfinite(v);
         }
@@ -165,48 +164,69 @@ __device__ __noinline__ void scan_lines_exact(const StageHot& t, int l0, int l1,
     mx = rmx; mn = rmn;
 }
 
-// Candidates of one limiter line: its centre p0 = a0 and the larger (p1, p2)
-// and smaller (m1, m2) value of each Gauss pair, v(+-s_k) = e_k +- a1 s_k.
-template <class R>
-__device__ __forceinline__ void line_candidates(const StageHot& t, const Tab<R>& tb, int l, const R* D, R sx1, R sx2,
-                                                R sy1, R sy2, R qx1, R qx2, R qy1, R qy2, R& p0, R& p1, R& p2, R& m1,
-                                                R& m2) {
-    const R c = tb.line_c(l);
-    R a0, a1, a2;
-    const bool row = t.line_dir[l] == 0;
-    if (row) q2_row(D, c, a0, a1, a2);
-    else q2_col(D, c, a0, a1, a2);
-    const R s1 = row ? sx1 : sy1, s2 = row ? sx2 : sy2;
-    const R e1 = fma(a2, row ? qx1 : qy1, a0), e2 = fma(a2, row ? qx2 : qy2, a0);
-    const R b = fabs(a1);
-    const R d1 = b * s1, d2 = b * s2;
-    p0 = a0; p1 = e1 + d1; p2 = e2 + d2; m1 = e1 - d1; m2 = e2 - d2;
+// The nonnegative 5-point Gauss nodes on [-1, 1].
+constexpr double kG1 = 0.538469310105683091036314420700, kG2 = 0.906179845938663992797626878299;
+
+// Running extremes of the limiter scan.
+struct Extremes {
+    double mx, mn;
+    __device__ __forceinline__ void up(double v) { mx = v > mx ? v : mx; }
+    __device__ __forceinline__ void down(double v) { mn = v < mn ? v : mn; }
+    // The two Gauss pairs s = +-g1, +-g2 of a line a0 + s (a1 + s a2): the
+    // larger of a pair is (a0 + a2 s^2) + |a1| s, the smaller with the minus.
+    __device__ __forceinline__ void pairs(double a0, double a1, double a2) {
+        const double e1 = fma(a2, kG1 * kG1, a0), e2 = fma(a2, kG2 * kG2, a0), b = fabs(a1);
+        up(fma(b, kG1, e1)); up(fma(b, kG2, e2));
+        down(fma(-b, kG1, e1)); down(fma(-b, kG2, e2));
+    }
+    // The lines at +c and -c of the coefficient rows (p0 + c p1 + c^2 p2) of
+    // the three powers along the line; the two centres again as a pair.
+    __device__ __forceinline__ void line_pair(double c, const double (&p0)[3], const double (&p1)[3],
+                                              const double (&p2)[3]) {
+        double e[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) e[k] = fma(p2[k], c * c, p0[k]);
+        up(fma(fabs(p1[0]), c, e[0]));
+        down(fma(-fabs(p1[0]), c, e[0]));
+        pairs(fma(p1[0], c, e[0]), fma(p1[1], c, e[1]), fma(p1[2], c, e[2]));
+        pairs(fma(p1[0], -c, e[0]), fma(p1[1], -c, e[1]), fma(p1[2], -c, e[2]));
+    }
+};
+
+// The 86 limiter points of an interior cell (state_reconstruction.cpp:
+// 152-168): on the rows eta = 0, +-g1, +-g2 (cell quadrature), +-1 (edges),
+// +-0.4, +-0.8 (diffusion samples: 0.3 and 0.9 cell sizes from each edge) and
+// the columns xi = +-1, +-0.4, +-0.8, five Gauss points each. The lines come
+// in symmetric pairs and their points in symmetric pairs, so 85 points take
+// 274 FP64 operations, 84 of them comparisons.
+__device__ __forceinline__ void scan_interior(const double (&D)[9], double& mx, double& mn) {
+    Extremes x{D[0], D[0]};
+    x.pairs(D[0], D[1], D[2]);
+    const double r0[3] = {D[0], D[1], D[2]}, r1[3] = {D[3], D[4], D[5]}, r2[3] = {D[6], D[7], D[8]};
+    x.line_pair(kG1, r0, r1, r2);
+    x.line_pair(kG2, r0, r1, r2);
+    x.line_pair(0.4, r0, r1, r2);
+    x.line_pair(0.8, r0, r1, r2);
+    x.line_pair(1.0, r0, r1, r2);
+    const double c0[3] = {D[0], D[3], D[6]}, c1[3] = {D[1], D[4], D[7]}, c2[3] = {D[2], D[5], D[8]};
+    x.line_pair(0.4, c0, c1, c2);
+    x.line_pair(0.8, c0, c1, c2);
+    x.line_pair(1.0, c0, c1, c2);
+    mx = x.mx; mn = x.mn;
 }
 
-// Max/min of the deviation polynomial over the class's limiter points. Each
-// line holds its centre (s = 0) and the symmetric Gauss pairs s = +-s_k
-// (g = 0, +-g1, +-g2), so along a line v(+-s_k) = (a0 + a2 s_k^2) +- a1 s_k
-// and the larger of a pair is e_k + |a1| s_k: three candidates per line for
-// the maximum and three for the minimum. With every |D_m| below scan_guard
-// no value can overflow, so no per-point finiteness test is needed;
-// otherwise the exact scan runs.
-template <class R>
-__device__ __forceinline__ void scan_lines(const StageHot& t, const Tab<R>& tb, int l0, int l1, const double* D,
-                                           double& mx, double& mn, bool& bad) {
-    bool small = true;
-#pragma unroll
-    for (int m = 0; m < 9; ++m) small = small && fabs(D[m]) < t.scan_guard;
-    if (!small) { scan_lines_exact(t, l0, l1, D, mx, mn, bad); return; }
-    const double sx1 = tb.gx(3), sx2 = tb.gx(4), sy1 = tb.gy(3), sy2 = tb.gy(4);
-    const double qx1 = sx1 * sx1, qx2 = sx2 * sx2, qy1 = sy1 * sy1, qy2 = sy2 * sy2;
-    double rmx = D[0], rmn = D[0];   // cell centre
+// The limiter points of a boundary class, line by line from the tables.
+__device__ __forceinline__ void scan_lines(const StageHot& t, int l0, int l1, const double (&D)[9], double& mx,
+                                           double& mn) {
+    Extremes x{D[0], D[0]};
     for (int l = l0; l < l1; ++l) {
-        double p0, p1, p2, m1, m2;
-        line_candidates<double>(t, tb, l, D, sx1, sx2, sy1, sy2, qx1, qx2, qy1, qy2, p0, p1, p2, m1, m2);
-        rmx = p0 > rmx ? p0 : rmx; rmx = p1 > rmx ? p1 : rmx; rmx = p2 > rmx ? p2 : rmx;
-        rmn = p0 < rmn ? p0 : rmn; rmn = m1 < rmn ? m1 : rmn; rmn = m2 < rmn ? m2 : rmn;
+        double a0, a1, a2;
+        if (t.line_dir[l] == 0) q2_row(D, t.line_c[l], a0, a1, a2);
+        else q2_col(D, t.line_c[l], a0, a1, a2);
+        x.up(a0); x.down(a0);
+        x.pairs(a0, a1, a2);
     }
-    mx = rmx; mn = rmn;
+    mx = x.mx; mn = x.mn;
 }
 
 // theta of one field: min over points of (bound - mean)/(v - mean) for v
@@ -214,74 +234,98 @@ __device__ __forceinline__ void scan_lines(const StageHot& t, const Tab<R>& tb, 
 // rounding monotone, the minimum is reached at the extreme D, so one
 // division per bound gives the reference's value.
 __device__ __forceinline__ double theta_of(double m, double lo, double hi, double dmax, double dmin) {
+    auto ratio = [](double a, double b) { return rcp_range(b) ? div_normal(a, b) : a / b; };
     double th = 1.0;
     const double vmax = m + dmax, vmin = m + dmin;
-    if (vmax > hi) th = fmin(th, (hi - m) / (vmax - m));
-    if (vmin < lo) th = fmin(th, (lo - m) / (vmin - m));
+    if (vmax > hi) th = fmin(th, ratio(hi - m, vmax - m));
+    if (vmin < lo) th = fmin(th, ratio(lo - m, vmin - m));
     return th < 1.0 ? fmax(0.0, th * (1.0 - 1e-13)) : 1.0;
 }
 
-template <class R>
-__device__ __forceinline__ void recon_cell(const ReconArgs<R>& a, const Physics& ph, int i, int j) {
-    if (i >= a.nx || j >= a.ny) return;
+// Averages of this magnitude or more: a limiter value could overflow.
+constexpr double kScanGuard = 1e30;
+
+// One field of one cell: gather, neighbour bounds, reconstruction, limiter
+// factor th and the unlimited D. kInterior: the cell has all eight
+// neighbours (no candidate is dropped, the limiter points are the fixed set).
+// top: the field's upper bound (Xe for the composition).
+template <bool kInterior>
+__device__ __forceinline__ void recon_field(const StageHot& t, const double* __restrict__ F, const unsigned (&at)[3][3],
+                                            unsigned on, int cls, double top, double (&D)[9], double& mean, double& lo,
+                                            double& hi, double& th, int& st, bool& bad) {
+    double u[3][3];
+#pragma unroll
+    for (int dj = 0; dj < 3; ++dj)
+#pragma unroll
+        for (int di = 0; di < 3; ++di) u[dj][di] = __ldg(F + at[dj][di]);
+    // 3x3 neighbour bounds (state_reconstruction.cpp:189-196); the clamped
+    // gather repeats in-domain values, which leaves min/max unchanged.
+    mean = lo = hi = u[1][1];
+#pragma unroll
+    for (int dj = 0; dj < 3; ++dj)
+#pragma unroll
+        for (int di = 0; di < 3; ++di) {
+            const double v = u[dj][di];
+            lo = v < lo ? v : lo;
+            hi = v > hi ? v : hi;
+        }
+    const bool small = lo > -kScanGuard && hi < kScanGuard;
+    lo = fmax(0.0, lo);
+    hi = top < hi ? top : hi;
+    const int s1 = reconstruct<kInterior>(t, on, u, D);
+    st = st ? st : s1;
+    double mx, mn;
+    if (!small) {
+        // Copies, so that the arrays of the common path stay in registers.
+        double Dc[9], x, n;
+        bool b = false;
+#pragma unroll
+        for (int m = 0; m < 9; ++m) Dc[m] = D[m];
+        scan_lines_exact(t, t.line_off[cls], t.line_off[cls + 1], Dc, x, n, b);
+        mx = x; mn = n;
+        bad = bad || b;
+    } else if (kInterior) scan_interior(D, mx, mn);
+    else scan_lines(t, t.line_off[cls], t.line_off[cls + 1], D, mx, mn);
+    th = theta_of(mean, lo, hi, mx, mn);
+}
+
+// Reconstruction and limiter of both fields, one field after the other
+// through the same code (18 limited coefficients live one field at a time).
+template <bool kInterior, class R>
+__device__ __forceinline__ void recon_cell_t(const ReconArgs<R>& a, const Physics& ph, int i, int j, int ci, int cj) {
     const StageHot& t = *a.tab.t;
     const int nx = a.nx, ny = a.ny;
     const long long cell = (long long)j * nx + i;
     const size_t N = (size_t)nx * ny;
-    MP_CHECK_INDEX(a.status, cell, N);
-    const int ci = i == 0 ? 0 : (i == nx - 1 ? 2 : 1);
-    const int gj = a.gj0 + j, gny = global_ny(a);
-    const int cj = gj == 0 ? 0 : (gj == gny - 1 ? 2 : 1);
+    const int gj = a.gj0 + j;
     const long long key = cell + (long long)a.gj0 * nx;
-    int st_lim = 0;
-
-    double u[3][3];
-    double DH[9], DC[9];
-    double mH, mC, loH, hiH, loC, hiC;
-    int st = 0;
-    // Enthalpy, then composition: one 3x3 gather at a time keeps registers low.
+    // Cells stay below 2^31 (checked on create).
+    unsigned at[3][3];
 #pragma unroll
-    for (int f = 0; f < 2; ++f) {
-        const double* F = f ? a.C : a.H;
+    for (int dj = 0; dj < 3; ++dj)
 #pragma unroll
-        for (int dj = 0; dj < 3; ++dj)
-#pragma unroll
-            for (int di = 0; di < 3; ++di) {
-                const int ii = min(max(i + di - 1, 0), nx - 1), jj = min(max(j + dj - 1, 0), ny - 1);
-                MP_CHECK_INDEX(a.status, (long long)jj * nx + ii, N);
-                u[dj][di] = __ldg(F + (size_t)jj * nx + ii);
-            }
-        // 3x3 neighbour bounds (state_reconstruction.cpp:189-196); the clamped
-        // gather repeats in-domain values, which leaves min/max unchanged.
-        double lo = u[1][1], hi = u[1][1];
-#pragma unroll
-        for (int dj = 0; dj < 3; ++dj)
-#pragma unroll
-            for (int di = 0; di < 3; ++di) { lo = fmin(lo, u[dj][di]); hi = fmax(hi, u[dj][di]); }
-        if (f == 0) {
-            mH = u[1][1]; loH = fmax(0.0, lo); hiH = hi;
-            const int s1 = reconstruct(t, ci, cj, u, DH);
-            st = st ? st : s1;
-        } else {
-            mC = u[1][1]; loC = fmax(0.0, lo); hiC = fmin(ph.k.Xe, hi);
-            const int s1 = reconstruct(t, ci, cj, u, DC);
-            st = st ? st : s1;
+        for (int di = 0; di < 3; ++di) {
+            const int ii = min(max(i + di - 1, 0), nx - 1), jj = min(max(j + dj - 1, 0), ny - 1);
+            MP_CHECK_INDEX(a.status, (long long)jj * nx + ii, N);
+            at[dj][di] = (unsigned)jj * (unsigned)nx + (unsigned)ii;
         }
-    }
-    // state_reconstruction.cpp:187-188: admissible means.
-    if (!(isfinite(mH) && mH >= 0.0 && isfinite(mC) && mC >= 0.0 && mC <= ph.k.Xe)) st_lim = E_OUTOFRANGE;
-
-    // Limiter over the class's points, evaluated line by line.
+    const unsigned on = candidate_mask(ci, cj);
     const int cls = cj * 3 + ci;
-    const int l0 = t.line_off[cls], l1 = t.line_off[cls + 1];
-    double hmx, hmn, cmx, cmn;
-    bool bad = false;
-    scan_lines<R>(t, a.tab, l0, l1, DH, hmx, hmn, bad);
-    scan_lines<R>(t, a.tab, l0, l1, DC, cmx, cmn, bad);
-    if (bad) st_lim = st_lim ? st_lim : E_FP;
-    const double thH = theta_of(mH, loH, hiH, hmx, hmn);
-    const double thC = theta_of(mC, loC, hiC, cmx, cmn);
-    if (a.theta) { a.theta[cell] = thH; a.theta[N + cell] = thC; }
+    int st = 0;
+    bool bad = false, means = true;
+    double hiH = 0, hiC = 0;
+#pragma unroll 1
+    for (int f = 0; f < 2; ++f) {
+        double D[9], mean, lo, hi, th;
+        recon_field<kInterior>(t, f ? a.C : a.H, at, on, cls, f ? ph.k.Xe : INFINITY, D, mean, lo, hi, th, st, bad);
+        // state_reconstruction.cpp:187-188: admissible means.
+        means = means && isfinite(mean) && mean >= 0.0 && (f == 0 || mean <= ph.k.Xe);
+        if (f) hiC = hi; else hiH = hi;
+        if (a.theta) a.theta[f * N + cell] = th;
+#pragma unroll
+        for (int m = 0; m < 9; ++m) a.rec[(size_t)(m + 9 * f) * N + cell] = D[m] * th;
+    }
+    const int st_lim = !means ? (int)E_OUTOFRANGE : (bad ? (int)E_FP : 0);
     // Diffusion samples (zero diffusivity: kept for their admissibility
     // check). Limited values at limiter points stay in [lo, hi], so the
     // samples are admissible when hi_H is below the liquidus at hi_C and
@@ -290,14 +334,19 @@ __device__ __forceinline__ void recon_cell(const ReconArgs<R>& a, const Physics&
     const double tep = ph.litho ? fmin(tep_at(ph, t.y0 + gj * t.dy), tep_at(ph, t.y0 + (gj + 1) * t.dy)) : ph.Tep;
     const double Hliq = tep + (1.0 - hiC / ph.k.Xe) + ph.k.LD;
     const bool safe = tep >= 0.0 && hiH + 1e-12 * (1.0 + fabs(hiH)) < Hliq;
-#pragma unroll
-    for (int m = 0; m < 9; ++m) {
-        a.rec[(size_t)m * N + cell] = DH[m] * thH;
-        a.rec[(size_t)(m + 9) * N + cell] = DC[m] * thC;
-    }
     a.flags[cell] = safe ? 0 : FLAG_CHECK;
     if (st) record_error(a.status, PART_UPDATE, key, st);
     if (st_lim) record_error(a.status, PART_LIMIT, key, st_lim);
+}
+
+template <class R>
+__device__ __forceinline__ void recon_cell(const ReconArgs<R>& a, const Physics& ph, int i, int j) {
+    if (i >= a.nx || j >= a.ny) return;
+    MP_CHECK_INDEX(a.status, (long long)j * a.nx + i, (size_t)a.nx * a.ny);
+    const int gj = a.gj0 + j, gny = global_ny(a);
+    const int ci = i == 0 ? 0 : (i == a.nx - 1 ? 2 : 1), cj = gj == 0 ? 0 : (gj == gny - 1 ? 2 : 1);
+    if (ci == 1 && cj == 1) recon_cell_t<true>(a, ph, i, j, ci, cj);
+    else recon_cell_t<false>(a, ph, i, j, ci, cj);
 }
 
 // ---------------------------------------------------------- cell phase kernel
@@ -352,13 +401,13 @@ __device__ __forceinline__ void cellphase_cell(const CellPhaseArgs<R>& a, const 
     const int gjc = a.gj0 + (int)(cell / a.nx);
     for (int b = 0; b < kNQ; ++b) {
         double h0, h1, h2, c0, c1, c2;
-        const double y = t.gy[b];
+        const double y = t.g[b];
         q2_row(DH, y, h0, h1, h2);
         q2_row(DC, y, c0, c1, c2);
         const double tep = (kExt && ph.litho) ? tep_at(ph, height(t, gjc, y)) : ph.Tep;
 #pragma unroll
         for (int q = 0; q < kNQ; ++q) {
-            const double x = t.gx[q];
+            const double x = t.g[q];
             const double h = mH + quad(h0, h1, h2, x);
             const double c = mC + quad(c0, c1, c2, x);
             PhaseLean pl;
@@ -396,10 +445,10 @@ __device__ __forceinline__ void cellphase_cell(const CellPhaseArgs<R>& a, const 
             if (row) { q2_row(DH, lc, h0, h1, h2); q2_row(DC, lc, c0, c1, c2); }
             else { q2_col(DH, lc, h0, h1, h2); q2_col(DC, lc, c0, c1, c2); }
             for (int q = 0; q < kNQ; ++q) {
-                const double s_ = row ? t.gx[q] : t.gy[q];
+                const double s_ = t.g[q];
                 const double h = mH + quad(h0, h1, h2, s_);
                 const double c = mC + quad(c0, c1, c2, s_);
-                const double tep = (kExt && ph.litho) ? tep_at(ph, height(t, j, row ? lc : t.gy[q])) : ph.Tep;
+                const double tep = (kExt && ph.litho) ? tep_at(ph, height(t, j, row ? lc : t.g[q])) : ph.Tep;
                 PhaseLean pl;
                 const int s = phase_stage_lean(ph.sk, h, c, tep, pl);
                 if (s) { st_face = st_face ? st_face : s; continue; }
@@ -542,7 +591,7 @@ __device__ __forceinline__ void face_edge(const FaceArgs<R>& a, const Physics& p
     int erow;                // local row of the edge (horizontal) or of its cells (vertical)
     long long L, Rc = -1;
     double len;
-    double lfix, rfix;   // the edge's fixed normalised coordinate in the left / right cell frame
+    double lfix, rfix;   // the edge's fixed coordinate in the left / right cell frame
     // Left/right cells and orientation as the reference's Build (evolve.cpp:230-251).
     if (e < nI) {
         horizontal = true;
@@ -554,8 +603,8 @@ __device__ __forceinline__ void face_edge(const FaceArgs<R>& a, const Physics& p
         reverse = (gj == gny);
         L = reverse ? (long long)(j - 1) * nx + i : (long long)j * nx + i;
         if (!boundary) Rc = (long long)(j - 1) * nx + i;
-        lfix = reverse ? t.Y : -t.Y;
-        rfix = t.Y;
+        lfix = reverse ? 1.0 : -1.0;
+        rfix = 1.0;
         len = t.len_h;
     } else {
         horizontal = false;
@@ -566,8 +615,8 @@ __device__ __forceinline__ void face_edge(const FaceArgs<R>& a, const Physics& p
         reverse = (i == 0);
         L = reverse ? (long long)j * nx : (long long)j * nx + (i - 1);
         if (!boundary) Rc = (long long)j * nx + i;
-        lfix = reverse ? -t.X : t.X;
-        rfix = -t.X;
+        lfix = reverse ? -1.0 : 1.0;
+        rfix = -1.0;
         len = t.len_v;
     }
     MP_CHECK_INDEX(a.status, L, N);
@@ -582,7 +631,7 @@ __device__ __forceinline__ void face_edge(const FaceArgs<R>& a, const Physics& p
     int st = 0;
     for (int q = 0; q < kNQ; ++q) {
         const int cq = reverse ? kNQ - 1 - q : q;
-        const double at = horizontal ? t.gx[cq] : t.gy[cq];
+        const double at = t.g[cq];
         const double vs = sgn * __ldg(a.vsn + e * kNQ + cq);
         const double ud = sgn * __ldg(a.udn + e * kNQ + cq);
         double hL, cL, hR, cR;
@@ -723,7 +772,7 @@ __device__ __forceinline__ void diffusion_edge(const FaceArgs<R>& a, const Physi
         const double w = t.dif_w[o][q];
         if (boundary && type == 2) { integral += w * ph.wall_value[wall]; continue; }
         const int cq = reverse ? kNQ - 1 - q : q;
-        const double at = horizontal ? t.gx[cq] : t.gy[cq];
+        const double at = t.g[cq];
         const int count = boundary ? 5 : 4;
         double v[5];
         // Temperatures at the samples: limited H, C on the line across the edge

@@ -32,7 +32,7 @@ struct Grid {
 // Normal-line samples of a uniform rectangular mesh (diffusiveflux.cpp:255-334,
 // numberOfSamples 4, extentFraction 0.9): the available ray distance across
 // an edge is the cell size normal to it.
-void fill_diffusion(StageHot& t, double dx, double dy, double h, const std::vector<double>& gw) {
+void fill_diffusion(StageHot& t, double dx, double dy, const std::vector<double>& gw) {
     typedef long double ld;
     const int N = 4;
     const ld frac = 0.9L;
@@ -45,23 +45,23 @@ void fill_diffusion(StageHot& t, double dx, double dy, double h, const std::vect
         t.dif_ds[o][1] = (double)(frac * size[o] * (1.0L / N));
         for (int q = 0; q < kNQ; ++q) t.dif_w[o][q] = (double)((ld)len[o] * gw[q] / 2);
     }
-    const double Y = t.Y, X = t.X;
     // Interior: offsets (k - 1.5) ds along the edge normal, which points from
     // the left cell into the right one: down for horizontal edges (left cell
     // above), +x for vertical edges (left cell at smaller x).
+    const double hx = 0.5 * dx, hy = 0.5 * dy;
     for (int k = 0; k < N; ++k) {
         const ld off = (ld)k - (N - 1) / 2.0L;
-        const double sh = (double)(off * t.dif_ds[0][0] / h), sv = (double)(off * t.dif_ds[1][0] / h);
-        t.dif_pos_int[0][k] = k < N / 2 ? -Y - sh : Y - sh;
-        t.dif_pos_int[1][k] = k < N / 2 ? X + sv : -X + sv;
+        const double sh = (double)(off * t.dif_ds[0][0] / hy), sv = (double)(off * t.dif_ds[1][0] / hx);
+        t.dif_pos_int[0][k] = k < N / 2 ? -1.0 - sh : 1.0 - sh;
+        t.dif_pos_int[1][k] = k < N / 2 ? 1.0 + sv : -1.0 + sv;
     }
     // Walls: interior samples at (N - k) ds inside, farthest first.
     for (int k = 0; k < N; ++k) {
-        const double dh = (double)((ld)(N - k) * t.dif_ds[0][1] / h), dv = (double)((ld)(N - k) * t.dif_ds[1][1] / h);
-        t.dif_pos_bnd[0][k] = -Y + dh;   // bottom wall: the cell above it
-        t.dif_pos_bnd[1][k] = Y - dh;    // top wall: the cell below it
-        t.dif_pos_bnd[2][k] = -X + dv;   // left wall
-        t.dif_pos_bnd[3][k] = X - dv;    // right wall
+        const double dh = (double)((ld)(N - k) * t.dif_ds[0][1] / hy), dv = (double)((ld)(N - k) * t.dif_ds[1][1] / hx);
+        t.dif_pos_bnd[0][k] = -1.0 + dh;   // bottom wall: the cell above it
+        t.dif_pos_bnd[1][k] = 1.0 - dh;    // top wall: the cell below it
+        t.dif_pos_bnd[2][k] = -1.0 + dv;   // left wall
+        t.dif_pos_bnd[3][k] = 1.0 - dv;    // right wall
     }
 }
 
@@ -77,54 +77,40 @@ int build_stage_tables(int nx, int ny, double x0, double x1, double y0, double y
     gauss_legendre(1, p1, w1);
     gauss_legendre(kNQ, gp, gw);
     const double area = cell_integral(target, p1, w1, [](V2) { return 1.0; });
-    const double h = std::sqrt(area);
     const V2 c{0.5 * dx, 0.5 * dy};   // target centre = centre of the 3x3 stencil
-
-    StencilBuild big;
-    if (!big.build(g, -1, -1, 3, 2, h, -1, -1)) return MP_ERR_ARG_WRONG;
-    for (int r = 0; r < 9; ++r) for (int m = 0; m < 9; ++m) t.C9[r][m] = big.coef[(size_t)r * 9 + m];
-    for (int r = 1; r < 9; ++r) for (int s = 1; s < 9; ++s) t.S9[r - 1][s - 1] = big.sigma[(size_t)r * 9 + s];
-    for (int tpos = 0; tpos < 4; ++tpos) {
-        StencilBuild small;
-        if (!small.build(g, 0, 0, 2, 1, h, tpos % 2, tpos / 2)) return MP_ERR_ARG_WRONG;
-        if (tpos == 0) for (int r = 0; r < 4; ++r) for (int m = 0; m < 4; ++m) t.C4[r][m] = small.coef[(size_t)r * 4 + m];
-        for (int r = 1; r < 4; ++r) for (int s = 1; s < 4; ++s) t.S4[tpos][r - 1][s - 1] = small.target[(size_t)r * 4 + s];
-    }
-    {
-        int k = 0;
-        for (int r = 0; r < 8; ++r)
-            for (int c = r; c < 8; ++c) t.SF9[k++] = c == r ? t.S9[r][r] : 2.0 * t.S9[r][c];
-        for (int tpos = 0; tpos < 4; ++tpos) {
-            k = 0;
-            for (int r = 0; r < 3; ++r)
-                for (int c = r; c < 3; ++c) t.SF4[tpos][k++] = c == r ? t.S4[tpos][r][r] : 2.0 * t.S4[tpos][r][c];
-        }
-    }
-    t.X = 0.5 * dx / h;
-    t.Y = 0.5 * dy / h;
-    t.scan_guard = 1e36 / (16.0 * std::max(1.0, t.X * t.X) * std::max(1.0, t.Y * t.Y));
-    fill_diffusion(t, dx, dy, h, gw);
-    t.y0 = y0; t.dy = dy; t.hn = h;
+    // iX2 = 1/Xh^2 = 4 dy/dx, iY2 = 1/Yh^2 = 4 dx/dy (see tables.hpp).
     t.epsA = 1e-2 * area;
+    t.epsA2 = t.epsA * t.epsA;
+    const double iX2 = 4.0 * (dy / dx), iY2 = 4.0 * (dx / dy), ie = 1.0 / t.epsA;
+    if (!(area > 0) || !std::isfinite(iX2 * iX2 * ie) || !std::isfinite(iY2 * iY2 * ie)) return MP_ERR_ARG_WRONG;
+    t.cx = iX2 / 12.0;
+    t.cy = iY2 / 12.0;
+    const double sg[8] = {iX2, iY2, (13.0 / 3.0) * iX2 * iX2, (13.0 / 3.0) * iY2 * iY2, (7.0 / 6.0) * 16.0,
+                          0.7 * 16.0 * iY2, 0.7 * 16.0 * iX2, (43.0 / 270.0) * 256.0};
+    for (int k = 0; k < 8; ++k) t.sg[k] = sg[k] * ie;
+    // Order-1 candidates: slopes dE/2, dN/2 and mixed coefficient b/4.
+    t.gx2 = 0.25 * iX2 * ie;
+    t.gy2 = 0.25 * iY2 * ie;
+    t.gb = (1.0 / iX2 + 1.0 / iY2) / 3.0 * ie;
+    fill_diffusion(t, dx, dy, gw);
+    t.y0 = y0; t.dy = dy; t.hn = 0.5 * dy;
     t.area = area;
     t.len_h = dx;
     t.len_v = dy;
-    for (int q = 0; q < kNQ; ++q) { t.gq[q] = gp[q]; t.gw[q] = gw[q]; }
+    for (int q = 0; q < kNQ; ++q) { t.g[q] = gp[q]; t.gw[q] = gw[q]; }
     for (int b = 0; b < kNQ; ++b)
         for (int a = 0; a < kNQ; ++a) {
             const V2 r{gp[a], gp[b]};
             t.cw[b * kNQ + a] = gw[a] * gw[b] * jacobian(r, target) / area;
             t.cwp[b * kNQ + a] = gw[a] * gw[b] * jacobian(r, target);
         }
-    for (int q = 0; q < kNQ; ++q) { t.gx[q] = t.X * gp[q]; t.gy[q] = t.Y * gp[q]; }
     // Limiter points per class: class = cj*3 + ci, ci in {0: left wall, 1, 2: right wall}.
-    int at = 0, nl = 0;
+    int nl = 0;
     for (int cls = 0; cls < 9; ++cls) {
-        t.pt_off[cls] = at;
         const int ci = cls % 3, cj = cls / 3;
         std::vector<V2> pts;
         std::vector<unsigned char> kind;
-        auto add = [&](V2 p, unsigned char k) { pts.push_back(V2{(p.x - c.x) / h, (p.y - c.y) / h}); kind.push_back(k); };
+        auto add = [&](V2 p, unsigned char k) { pts.push_back(V2{(p.x - c.x) / (0.5 * dx), (p.y - c.y) / (0.5 * dy)}); kind.push_back(k); };
         add(bilinear(V2{0, 0}, target), 0);
         for (double a : gp) for (double b : gp) add(bilinear(V2{a, b}, target), 0);
         for (int e = 0; e < 4; ++e) {
@@ -137,12 +123,10 @@ int build_stage_tables(int nx, int ny, double x0, double x1, double y0, double y
             else { const Quad other = g.cell(ni, nj); left_samples(a, b, target, &other, gp, s); }
             for (const V2& q : s) add(q, 1);
         }
-        if (at + (int)pts.size() > kMaxPoints) return MP_ERR_ARG_SIZ;
-        for (size_t k = 0; k < pts.size(); ++k) { t.pt_x[at] = pts[k].x; t.pt_y[at] = pts[k].y; t.pt_kind[at] = kind[k]; ++at; }
         // Group the points after the centre into 5-point lines. Each group of
         // 5 consecutive points (a Gauss row, an edge, or one sample depth of
         // an edge) shares one normalised coordinate; its other coordinate is
-        // X*g_q or Y*g_q up to the rounding of the bilinear map.
+        // g_q up to the rounding of the bilinear map.
         t.line_off[cls] = nl;
         std::vector<std::array<double, 3>> lines;  // dir, fixed coordinate, kind
         // 5x5 Gauss points were added with a outer (x), b inner (y): regroup into rows.
@@ -173,7 +157,6 @@ int build_stage_tables(int nx, int ny, double x0, double x1, double y0, double y
         if (nl + (int)lines.size() > kMaxLines) return MP_ERR_ARG_SIZ;
         for (const auto& l : lines) { t.line_dir[nl] = (unsigned char)l[0]; t.line_c[nl] = l[1]; t.line_kind[nl] = (unsigned char)l[2]; ++nl; }
     }
-    t.pt_off[9] = at;
     t.line_off[9] = nl;
     return MP_OK;
 }

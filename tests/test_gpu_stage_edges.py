@@ -1,0 +1,62 @@
+"""The stage kernels at the sizes and data where their fast forms meet their
+general ones: tile edges and remainders of the 32x4-cell blocks, meshes
+without an interior cell, and a domain so small that the smoothness
+indicators leave the range of the product form of the weights. Oracle: the
+restated CPU driver on the same inputs.
+
+Tolerances. Per-cell |x - ref| / max(|ref|, 1e-3 max|ref|). Limiter factors
+1e-11: a factor is a ratio of differences of averages, and two roundings of
+the stencil tables move the worst of 3.3 million such cells by 1e-11. Stage
+T 1e-12, RHS 1e-12 of its largest value (the bars of the golden stages)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from mantlepar_b200 import synthetic as sy
+
+pytestmark = pytest.mark.gpu
+
+
+def per_cell(x, ref):
+    x, ref = np.asarray(x).reshape(-1), np.asarray(ref).reshape(-1)
+    return np.max(np.abs(x - ref) / np.maximum(np.abs(ref), 1e-3 * np.max(np.abs(ref))))
+
+
+def pair(w, **config):
+    """The GPU instance and the oracle's with the same inputs."""
+    from mantlepar_b200.transport import Transport, TransportConfig
+    from oracle import pyoracle as po
+    o = po.TransportOracle(sy.material_s(), w, lib=po.restated(), integrator=w.integrator, **config)
+    t = Transport(w, TransportConfig(cfl=w.cfl, integrator=w.integrator, **config))
+    H, C = sy.initial_state(w)
+    vs, ud = sy.face_velocity(w)
+    for x in (o, t):
+        x.set_face_velocity(vs, ud)
+        x.set_state(H, C)
+    return t, o
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e-6])
+@pytest.mark.parametrize("nx,ny", [(2, 2), (2, 7), (3, 3), (31, 4), (33, 5), (65, 9)])
+def test_reconstruction_and_limiter(nx, ny, scale):
+    # scale 1e-6: epsilon * area is 1e-12 smaller, sigma / (epsilon * area) up
+    # to 1e15, beyond the product form of the weights.
+    w = sy.Workload(nx=nx, ny=ny, x1=0.5 * scale, y1=scale, seed=nx + ny, noise_H=0.05 * scale if scale < 1 else 0.05)
+    if scale < 1:
+        # Keep the enthalpy of the unit domain: 1 - y needs its own height.
+        H = (1.0 - (np.arange(nx * ny) // nx + 0.5) / ny) + 0.05 * sy.unit_noise(w.seed, 0, np.arange(nx * ny, dtype=np.uint64))
+        C = sy.initial_state(w)[1]
+    t, o = pair(w)
+    if scale < 1:
+        t.set_state(H, C)
+        o.set_state(H, C)
+    code, *factors = o.limiter()
+    assert code == 0
+    for g, r in zip(t.limiter(), factors):
+        assert np.max(np.abs(g - r)) <= 1e-11
+    got, (code, ref) = t.rhs(), o.rhs()
+    assert code == 0
+    assert per_cell(got["T"], ref["T"]) <= 1e-12
+    for k in ("rhsH", "rhsC"):
+        assert np.max(np.abs(got[k] - ref[k])) <= 1e-12 * np.max(np.abs(ref[k]))
