@@ -42,11 +42,10 @@ namespace {
 enum : int { KIND_P = 0, KIND_B = 1, KIND_C = 2, NKIND = 3 };
 
 // Per-instance records of one stage kind, read by the batched kernels.
-template <class R>
 struct InstArgs {
-    ReconArgs<R> recon;
-    CellPhaseArgs<R> phase;
-    FaceArgs<R> face;
+    ReconArgs recon;
+    CellPhaseArgs phase;
+    FaceArgs face;
     SumArgs sum;
 };
 
@@ -75,41 +74,38 @@ struct Tuning { int bx = 32, by = 4, cpt = 1; };
 
 // ------------------------------------------------------------ batched kernels
 
-template <class R>
-__global__ void __launch_bounds__(128) batch_recon_kernel(const InstArgs<R>* args, const Work* work, const int* active,
-                                                          Physics ph, int cpt) {
+__global__ void __launch_bounds__(128) batch_recon_kernel(const InstArgs* args, const Work* work, const int* active,
+                                                          const __grid_constant__ Physics ph, int cpt) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
-    const ReconArgs<R>& a = args[w.inst].recon;
+    const ReconArgs& a = args[w.inst].recon;
     const int j = w.b + threadIdx.y;
-    for (int c = 0; c < cpt; ++c) recon_cell(a, ph, w.a + c * blockDim.x + threadIdx.x, j);
+    for (int c = 0; c < cpt; ++c) recon_cell(*a.tab, a, ph, w.a + c * blockDim.x + threadIdx.x, j);
 }
 
 // kExt: the adiabatic source (alpha0 != 0) is compiled in.
-template <class R, bool kExt>
-__global__ void __launch_bounds__(128, 8) batch_phase_kernel(const InstArgs<R>* args, const Work* work, const int* active,
+template <bool kExt>
+__global__ void __launch_bounds__(128, 8) batch_phase_kernel(const InstArgs* args, const Work* work, const int* active,
                                                           Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
-    cellphase_cell<R, kExt>(args[w.inst].phase, ph, (long long)w.a + threadIdx.x);
+    cellphase_cell<kExt>(*args[w.inst].phase.tab, args[w.inst].phase, ph, (long long)w.a + threadIdx.x);
 }
 
-template <class R>
-__global__ void __launch_bounds__(128, 5) batch_face_kernel(const InstArgs<R>* args, const Work* work, const int* active,
+__global__ void __launch_bounds__(128, 5) batch_face_kernel(const InstArgs* args, const Work* work, const int* active,
                                                          Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const long long e = (long long)w.a + threadIdx.x;
-    if (e < w.b) face_edge(args[w.inst].face, ph, e);
+    if (e < w.b) face_edge<false>(*args[w.inst].face.tab, args[w.inst].face, ph, e);
 }
 
-template <class R>
-__global__ void __launch_bounds__(128) batch_diffusion_kernel(const InstArgs<R>* args, const Work* work, const int* active,
+__global__ void __launch_bounds__(128) batch_diffusion_kernel(const InstArgs* args, const Work* work, const int* active,
                                                               Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const long long e = (long long)w.a + threadIdx.x;
-    if (e < w.b) diffusion_edge(args[w.inst].face, ph, e);
+    if (e < w.b) diffusion_edge(*args[w.inst].face.tab, args[w.inst].face, ph, e);
 }
 
 // General quad meshes: the per-element bodies of the single-mesh quad
@@ -159,8 +155,8 @@ __global__ void __launch_bounds__(128) batch_quad_diffusion_kernel(const QuadSta
 
 // kSrc: the adiabatic source terms are added. An instance with per-cell
 // areas (a general quad mesh) takes them.
-template <class R, bool kSrc>
-__global__ void __launch_bounds__(kRedBlock) batch_sum_kernel(const InstArgs<R>* args, const Work* work, const int* active) {
+template <bool kSrc>
+__global__ void __launch_bounds__(kRedBlock) batch_sum_kernel(const InstArgs* args, const Work* work, const int* active) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const SumArgs& a = args[w.inst].sum;
@@ -466,9 +462,8 @@ mp_status grow(T** p, int& cap, int need, cudaStream_t s, bool* grown) {
 }
 
 // Rebuild per-instance argument records, work maps and partial offsets.
-template <class R>
 mp_status rebuild_args(mp_batch* b, int slots) {
-    std::vector<InstArgs<R>> args[NKIND];
+    std::vector<InstArgs> args[NKIND];
     for (int k = 0; k < NKIND; ++k) args[k].resize(slots);
     std::vector<QuadStageArgs> qargs[NKIND];
     for (int k = 0; k < NKIND; ++k) qargs[k].resize(slots);
@@ -482,8 +477,6 @@ mp_status rebuild_args(mp_batch* b, int slots) {
     for (int i = 0; i < slots; ++i) {
         MPInstance& in = b->inst[i];
         if (!in.used) continue;
-        Tab<R> tb;
-        tb.t = in.tab;
         const double area = in.quad ? 1.0 : in.host_tab.area;   // a quad mesh: per-cell areas
         const int nsum = (int)((in.N + kSumCells - 1) / kSumCells);
         part_off[i] = parts; part_cnt[i] = nsum;
@@ -494,11 +487,11 @@ mp_status rebuild_args(mp_batch* b, int slots) {
             const double* inC = k == KIND_P ? in.C : (k == KIND_B ? in.S1C : in.S2C);
             double* outH = k == KIND_P ? in.LH : (k == KIND_B ? in.S2H : in.S1H);
             double* outC = k == KIND_P ? in.LC : (k == KIND_B ? in.S2C : in.S1C);
-            InstArgs<R>& a = args[k][i];
-            a.recon = ReconArgs<R>{in.nx, in.ny, tb, inH, inC, in.rec, in.flags, b->d_status + i, nullptr};
-            a.phase = CellPhaseArgs<R>{in.nx, in.ny, tb, inH, inC, in.rec, in.flags, in.T, in.phi, b->d_status + i,
+            InstArgs& a = args[k][i];
+            a.recon = ReconArgs{in.nx, in.ny, in.tab, inH, inC, in.rec, in.flags, b->d_status + i, nullptr};
+            a.phase = CellPhaseArgs{in.nx, in.ny, in.tab, inH, inC, in.rec, in.flags, in.T, in.phi, b->d_status + i,
                                        0, 0, in.cvs_y, in.cud_y, in.srcH, in.srcR, in.srcS};
-            a.face = FaceArgs<R>{in.nx, in.ny, tb, inH, inC, in.rec, in.flags, in.vsn, in.udn, in.face, b->d_status + i};
+            a.face = FaceArgs{in.nx, in.ny, in.tab, inH, inC, in.rec, in.flags, in.vsn, in.udn, in.face, b->d_status + i};
             const bool rk3 = b->opts.integrator == MP_SSPRK3;
             const double a0 = k == KIND_B ? (rk3 ? 0.75 : 0.5) : (1.0 / 3.0);
             const double a1 = k == KIND_B ? (rk3 ? 0.25 : 0.5) : (2.0 / 3.0);
@@ -544,7 +537,7 @@ mp_status rebuild_args(mp_batch* b, int slots) {
     part_off.resize(cap, 0);
     part_cnt.resize(cap, 0);
     for (int k = 0; k < NKIND; ++k)
-        MP_CUDA(cudaMemcpyAsync(b->d_args[k], args[k].data(), cap * sizeof(InstArgs<R>), cudaMemcpyHostToDevice, s));
+        MP_CUDA(cudaMemcpyAsync(b->d_args[k], args[k].data(), cap * sizeof(InstArgs), cudaMemcpyHostToDevice, s));
     for (int k = 0; k < NKIND; ++k)
         MP_CUDA(cudaMemcpyAsync(b->d_qargs[k], qargs[k].data(), cap * sizeof(QuadStageArgs), cudaMemcpyHostToDevice, s));
     MP_CUDA(cudaMemcpyAsync(b->d_axpy, ax.data(), cap * sizeof(AxpyArgs), cudaMemcpyHostToDevice, s));
@@ -605,7 +598,7 @@ mp_status rebuild(mp_batch* b) {
         MP_CUDA(cudaMallocAsync((void**)&b->d_dt, cap * sizeof(double), s));
         MP_CUDA(cudaMallocAsync((void**)&b->d_axpy, cap * sizeof(AxpyArgs), s));
         MP_CUDA(cudaMallocAsync((void**)&b->d_commit, cap * sizeof(CommitArgs), s));
-        for (int k = 0; k < NKIND; ++k) MP_CUDA(cudaMallocAsync(&b->d_args[k], cap * sizeof(InstArgs<double>), s));
+        for (int k = 0; k < NKIND; ++k) MP_CUDA(cudaMallocAsync(&b->d_args[k], cap * sizeof(InstArgs), s));
         for (int k = 0; k < NKIND; ++k) MP_CUDA(cudaMallocAsync(&b->d_qargs[k], cap * sizeof(QuadStageArgs), s));
         MP_CUDA(cudaMallocHost((void**)&b->h_tot, cap * sizeof(Totals)));
         MP_CUDA(cudaMallocHost((void**)&b->h_status, cap * sizeof(unsigned long long)));
@@ -624,7 +617,7 @@ mp_status rebuild(mp_batch* b) {
         b->partial_cap = n;
         b->gen += 1;
     }
-    MP_TRY(rebuild_args<double>(b, slots));
+    MP_TRY(rebuild_args(b, slots));
     b->dirty = false;
     return MP_OK;
 }
@@ -636,18 +629,17 @@ mp_status set_active(mp_batch* b, const std::vector<int>& act) {
     return MP_OK;
 }
 
-template <class R>
 void launch_kind(mp_batch* b, int kind) {
     cudaStream_t s = b->stream;
-    const InstArgs<R>* args = static_cast<const InstArgs<R>*>(b->d_args[kind]);
+    const InstArgs* args = static_cast<const InstArgs*>(b->d_args[kind]);
     const Tuning tu = b->tune;
     // Grids cover the work lists' capacities (padded items exit at once).
-    timed(b, 0, [&] { batch_recon_kernel<R><<<b->cap_wrecon, dim3(tu.bx, tu.by), 0, s>>>(args, b->d_wrecon, b->d_active, b->ph, tu.cpt); });
-    if (b->ph.source) timed(b, 1, [&] { batch_phase_kernel<R, true><<<b->cap_wphase, 128, 0, s>>>(args, b->d_wphase, b->d_active, b->ph); });
-    else timed(b, 1, [&] { batch_phase_kernel<R, false><<<b->cap_wphase, 128, 0, s>>>(args, b->d_wphase, b->d_active, b->ph); });
-    timed(b, 2, [&] { batch_face_kernel<R><<<b->cap_wface, 128, 0, s>>>(args, b->d_wface, b->d_active, b->ph); });
+    timed(b, 0, [&] { batch_recon_kernel<<<b->cap_wrecon, dim3(tu.bx, tu.by), 0, s>>>(args, b->d_wrecon, b->d_active, b->ph, tu.cpt); });
+    if (b->ph.source) timed(b, 1, [&] { batch_phase_kernel<true><<<b->cap_wphase, 128, 0, s>>>(args, b->d_wphase, b->d_active, b->ph); });
+    else timed(b, 1, [&] { batch_phase_kernel<false><<<b->cap_wphase, 128, 0, s>>>(args, b->d_wphase, b->d_active, b->ph); });
+    timed(b, 2, [&] { batch_face_kernel<<<b->cap_wface, 128, 0, s>>>(args, b->d_wface, b->d_active, b->ph); });
     if (b->ph.diffusion)
-        timed(b, 2, [&] { batch_diffusion_kernel<R><<<b->cap_wface, 128, 0, s>>>(args, b->d_wface, b->d_active, b->ph); });
+        timed(b, 2, [&] { batch_diffusion_kernel<<<b->cap_wface, 128, 0, s>>>(args, b->d_wface, b->d_active, b->ph); });
     if (b->has_quads) {
         // General quad meshes: reconstruction, limiter, cell phase (the wet
         // flags the faces read), faces; the sums below cover every instance.
@@ -660,8 +652,8 @@ void launch_kind(mp_batch* b, int kind) {
             timed(b, 2, [&] { batch_quad_diffusion_kernel<<<b->cap_wqface, 128, 0, s>>>(qa, b->d_wqface, b->d_active, b->ph); });
         count_launch(b->ph.diffusion ? 5 : 4);
     }
-    if (b->ph.source) timed(b, 3, [&] { batch_sum_kernel<R, true><<<b->cap_wsum, kRedBlock, 0, s>>>(args, b->d_wsum, b->d_active); });
-    else timed(b, 3, [&] { batch_sum_kernel<R, false><<<b->cap_wsum, kRedBlock, 0, s>>>(args, b->d_wsum, b->d_active); });
+    if (b->ph.source) timed(b, 3, [&] { batch_sum_kernel<true><<<b->cap_wsum, kRedBlock, 0, s>>>(args, b->d_wsum, b->d_active); });
+    else timed(b, 3, [&] { batch_sum_kernel<false><<<b->cap_wsum, kRedBlock, 0, s>>>(args, b->d_wsum, b->d_active); });
     timed(b, 4, [&] { batch_reduce_kernel<<<b->slots, 1024, 0, s>>>(b->d_partial, b->d_part_off, b->d_part_cnt, b->d_active, b->d_tot); });
     count_launch(5);
 }
@@ -672,7 +664,7 @@ mp_status run_stage(mp_batch* b, int kind, const std::vector<int>& act) {
     MP_TRY(set_active(b, act));
     const int slots = (int)b->inst.size();
     MP_CUDA(cudaMemsetAsync(b->d_status, 0xff, slots * sizeof(unsigned long long), b->stream));
-    launch_kind<double>(b, kind);
+    launch_kind(b, kind);
     MP_CUDA(cudaGetLastError());
     MP_CUDA(cudaMemcpyAsync(b->h_tot, b->d_tot, slots * sizeof(Totals), cudaMemcpyDeviceToHost, b->stream));
     MP_CUDA(cudaMemcpyAsync(b->h_status, b->d_status, slots * sizeof(unsigned long long), cudaMemcpyDeviceToHost, b->stream));
@@ -875,9 +867,9 @@ mp_status autotune(mp_batch* b, int reps, double* best_ms) {
         b->dirty = true;
         MP_TRY(rebuild(b));
         MP_TRY(set_active(b, act));
-        launch_kind<double>(b, KIND_P);   // warm-up
+        launch_kind(b, KIND_P);   // warm-up
         cudaEventRecord(e0, b->stream);
-        for (int r = 0; r < reps; ++r) launch_kind<double>(b, KIND_P);
+        for (int r = 0; r < reps; ++r) launch_kind(b, KIND_P);
         cudaEventRecord(e1, b->stream);
         MP_CUDA(cudaEventSynchronize(e1));
         float ms = 0.f;
@@ -936,7 +928,6 @@ mp_status add_while(cudaGraph_t g, const std::vector<cudaGraphNode_t>& deps, cud
 //   WHILE run:  begin -> WHILE attempt: {attempt, axpy, reduce, gate,
 //               stage B, control [, stage C, control]} -> commit, copy,
 //               stage P (L(U^{n+1})), control (run condition).
-template <class R>
 mp_status capture_graph(mp_batch* b, cudaGraph_t* out) {
     cudaStream_t s = b->stream;
     const int slots = b->slots;          // control records of every slot of the capacity
@@ -966,11 +957,11 @@ mp_status capture_graph(mp_batch* b, cudaGraph_t* out) {
     batch_axpy_kernel<<<b->cap_wsum, kRedBlock, 0, s>>>(b->d_axpy, b->d_wsum, b->d_active);
     batch_reduce_kernel<<<b->slots, 1024, 0, s>>>(b->d_partial, b->d_part_off, b->d_part_cnt, b->d_active, b->d_tot);
     ctl_after_axpy_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_tot, b->d_status, b->d_active);
-    launch_kind<R>(b, KIND_B);
+    launch_kind(b, KIND_B);
     ctl_after_stage_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_tot, b->d_status, b->d_active, 2,
                                                       rk3 ? 0 : 1, b->d_hdr, attempt);
     if (rk3) {
-        launch_kind<R>(b, KIND_C);
+        launch_kind(b, KIND_C);
         ctl_after_stage_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_tot, b->d_status, b->d_active, 3, 1,
                                                           b->d_hdr, attempt);
     }
@@ -979,7 +970,7 @@ mp_status capture_graph(mp_batch* b, cudaGraph_t* out) {
     MP_CUDA(cudaStreamBeginCaptureToGraph(s, step_body, &attempt_node, nullptr, 1, mode));
     ctl_commit_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_hdr, b->d_rep, b->d_status, b->d_active);
     batch_commit_kernel<<<b->cap_wsum, kRedBlock, 0, s>>>(b->d_commit, b->d_wsum, b->d_active);
-    launch_kind<R>(b, KIND_P);
+    launch_kind(b, KIND_P);
     ctl_after_rhs_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_tot, b->d_status, b->d_rep, b->d_hdr, 0,
                                                     run);
     MP_CUDA(cudaStreamEndCapture(s, &tmp));
@@ -1020,7 +1011,7 @@ mp_status ensure_graph(mp_batch* b) {
     cudaStream_t user = b->stream;
     b->stream = cap;
     g_capturing = true;
-    const mp_status st = capture_graph<double>(b, &b->graph);
+    const mp_status st = capture_graph(b, &b->graph);
     g_capturing = false;
     cudaStreamCaptureStatus cs;
     if (cudaStreamIsCapturing(cap, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) {

@@ -236,6 +236,8 @@ MP_HD int phase_lean(const PhaseConst& k, double H, double C, const Bounds& b, P
 // Constants of the stage kernels' phase evaluation (precomputed reciprocals).
 struct StageConst {
     double Xe, LD, invXe, invLD, halfInvLD, fourLD, LDoverXe;
+    double fourLDoverXe, halfXe;
+    int ordinary;           // scales for which phase_plain's products stay in range
 };
 
 MP_HD StageConst stage_const(const PhaseConst& k) {
@@ -243,6 +245,8 @@ MP_HD StageConst stage_const(const PhaseConst& k) {
     c.Xe = k.Xe; c.LD = k.LD;
     c.invXe = 1.0 / k.Xe; c.invLD = 1.0 / k.LD; c.halfInvLD = 0.5 / k.LD;
     c.fourLD = 4.0 * k.LD; c.LDoverXe = k.LD / k.Xe;
+    c.fourLDoverXe = c.fourLD / k.Xe; c.halfXe = 0.5 * k.Xe;
+    c.ordinary = k.LD > 1e-30 && k.LD < 1e30 && k.Xe > 1e-30;
     return c;
 }
 

@@ -30,16 +30,6 @@ struct ParamTables {
 
 inline void make_param_tables(const StageTables& t, ParamTables& p) { p.d = t; }
 
-template <class R> struct Tab;
-// Tab pointing at the parameter-space copy (inside a kernel taking a
-// __grid_constant__ ParamTables).
-template <class R> __device__ __forceinline__ Tab<R> param_tab(const ParamTables& p);
-template <> struct Tab<double> {
-    const StageHot* t;
-};
-
-template <> __device__ __forceinline__ Tab<double> param_tab<double>(const ParamTables& p) { return Tab<double>{&p.d}; }
-
 template <class R> __device__ __forceinline__ R eps_of();
 template <> __device__ __forceinline__ double eps_of<double>() { return 2.220446049250313e-16; }
 
@@ -63,6 +53,65 @@ __device__ __forceinline__ double div_normal(double a, double b) {
 // Magnitude within [2^-960, 2^960]: rcp and div_normal apply.
 __device__ __forceinline__ bool rcp_range(double x) {
     return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x03f00000u <= 0x78000000u;
+}
+
+// Square root of a normal q in rcp's range and, with kInverse, its
+// reciprocal: the hardware's reciprocal square root (relative error below
+// 2^-19) and two Newton steps on the residual q - s^2, exact as an FMA, and
+// one third-order step for the reciprocal. Off by at most one ulp (4 in 10^4
+// arguments), six and three FP64 operations, no branch and no call.
+template <bool kInverse>
+__device__ __forceinline__ double sqrt_normal(double q, double& inv) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
+    const double h = 0.5 * y;
+    double s = q * y;
+    s = fma(fma(-s, s, q), h, s);
+    s = fma(fma(-s, s, q), h, s);
+    if (kInverse) {
+        double e = fma(-s, y, 1.0);
+        e = fma(e, e, e);
+        inv = fma(y, e, y);
+    }
+    return s;
+}
+
+// The phase evaluation of phase_stage_t for a point known to be plain: H in
+// [0, Hliq) and C in [1e-100, Xe] with a margin, Tep in [1e-9, 1e100] and
+// ordinary scales (the flag a cell's neighbour bounds give it, plain_cell
+// below). Every admissibility test of phase_stage_t then holds, and the
+// solid + liquid quadratic LD melt^2 - a melt - C/Xe = 0 needs one square
+// root and one reciprocal for both roots: with disc = sqrt(a^2 + 4 LD C/Xe),
+// big = disc + |a| and small = disc - |a| = (4 LD C/Xe) / big, melt is the
+// one of its sign over 2 LD, the other (oth) gives T = Tmp - oth/2 and
+// cl = C/melt = Xe oth/2. No division, no call, no clip.
+template <bool kFull>
+__device__ __forceinline__ void phase_plain(const StageConst& k, double H, double C, double Tep, PhaseLean& s) {
+    if (H <= Tep) {
+        s.T = H; s.phil = 0.0;
+        if (kFull) { s.cl = 0.0; s.cs = C; s.dTdC = 0.0; }
+        return;
+    }
+    if (H <= fma(C, k.LDoverXe, Tep)) {
+        const double r = C * k.invXe, m = (H - Tep) * k.invLD, melt = r < m ? r : m;
+        s.T = Tep; s.phil = melt;
+        if (kFull) {
+            const double second = fma(-melt, k.Xe, C);
+            s.cl = k.Xe;
+            s.cs = second > 0.0 ? second * rcp(1.0 - melt) : 0.0;
+            s.dTdC = 0.0;
+        }
+        return;
+    }
+    const double Tmp = Tep + 1.0, a = H - Tmp, b = C * k.fourLDoverXe;
+    double inv;
+    const double disc = sqrt_normal<kFull>(fma(a, a, b), inv);
+    const double big = disc + fabs(a), small = b * rcp(big);
+    const bool below = a < 0.0;
+    const double same = below ? small : big, oth = below ? big : small;
+    s.phil = same * k.halfInvLD;
+    s.T = fma(-0.5, oth, Tmp);
+    if (kFull) { s.cl = k.halfXe * oth; s.cs = 0.0; s.dTdC = -k.LDoverXe * inv; }
 }
 
 // Row / column coefficients of a Q2 polynomial (coefficient m = j*3 + i of

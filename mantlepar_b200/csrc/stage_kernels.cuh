@@ -127,13 +127,28 @@ __device__ __forceinline__ void record_error(unsigned long long* status, int par
 // ------------------------------------------------------- reconstruction kernel
 
 // Cell flags byte: bit 0 wet (porosity sampling), bit 1 exact diffusion-sample
-// check needed (the cheap bound could not prove admissibility).
-enum : unsigned char { FLAG_WET = 1, FLAG_CHECK = 2 };
+// check needed (the cheap bound could not prove admissibility), bit 2 plain:
+// every limited value of the cell is a plain phase point (phase_plain).
+enum : unsigned char { FLAG_WET = 1, FLAG_CHECK = 2, FLAG_PLAIN = 4 };
 
-template <class R>
+// The flag byte of a cell from its neighbour bounds: the limiter keeps every
+// limited value at the cell's points (cell and edge Gauss points, diffusion
+// samples) within [lo, hi] up to roundoff, and Hliq at (hi_C, lowest tep) is
+// the lowest liquidus, so bounds that keep a margin of 1e-12 prove each
+// point's admissibility: the samples' (cell flagged otherwise: they are
+// checked one by one), and for a plain cell all of them.
+__device__ __forceinline__ unsigned char cell_flags(const Physics& ph, double tep_lo, double tep_hi, double loH, double hiH,
+                                                    double loC, double hiC) {
+    const double Hliq = tep_lo + (1.0 - hiC * ph.sk.invXe) + ph.k.LD;
+    const double slack = 1e-12 * (1.0 + fabs(hiH));
+    if (!(tep_lo >= 0.0 && hiH + slack < Hliq)) return FLAG_CHECK;
+    return ph.sk.ordinary && tep_lo >= 1e-9 && tep_hi <= 1e100 && loH >= slack && loC >= 1e-90 &&
+           hiC <= ph.k.Xe * (1.0 - 1e-12) ? FLAG_PLAIN : 0;
+}
+
 struct ReconArgs {
     int nx, ny;
-    Tab<R> tab;
+    const StageHot* tab;   // batched instances: their tables in device memory
     const double* H;
     const double* C;
     double* rec;           // 18 * ncell, SoA: rec[m*N + cell], m < 9 for H
@@ -291,9 +306,8 @@ __device__ __forceinline__ void recon_field(const StageHot& t, const double* __r
 
 // Reconstruction and limiter of both fields, one field after the other
 // through the same code (18 limited coefficients live one field at a time).
-template <bool kInterior, class R>
-__device__ __forceinline__ void recon_cell_t(const ReconArgs<R>& a, const Physics& ph, int i, int j, int ci, int cj) {
-    const StageHot& t = *a.tab.t;
+template <bool kInterior>
+__device__ __forceinline__ void recon_cell_t(const StageHot& t, const ReconArgs& a, const Physics& ph, int i, int j, int ci, int cj) {
     const int nx = a.nx, ny = a.ny;
     const long long cell = (long long)j * nx + i;
     const size_t N = (size_t)nx * ny;
@@ -313,48 +327,46 @@ __device__ __forceinline__ void recon_cell_t(const ReconArgs<R>& a, const Physic
     const int cls = cj * 3 + ci;
     int st = 0;
     bool bad = false, means = true;
-    double hiH = 0, hiC = 0;
+    double loH = 0, hiH = 0, loC = 0, hiC = 0;
 #pragma unroll 1
     for (int f = 0; f < 2; ++f) {
         double D[9], mean, lo, hi, th;
         recon_field<kInterior>(t, f ? a.C : a.H, at, on, cls, f ? ph.k.Xe : INFINITY, D, mean, lo, hi, th, st, bad);
         // state_reconstruction.cpp:187-188: admissible means.
         means = means && isfinite(mean) && mean >= 0.0 && (f == 0 || mean <= ph.k.Xe);
-        if (f) hiC = hi; else hiH = hi;
+        if (f) { loC = lo; hiC = hi; }
+        else { loH = lo; hiH = hi; }
         if (a.theta) a.theta[f * N + cell] = th;
 #pragma unroll
         for (int m = 0; m < 9; ++m) a.rec[(size_t)(m + 9 * f) * N + cell] = D[m] * th;
     }
     const int st_lim = !means ? (int)E_OUTOFRANGE : (bad ? (int)E_FP : 0);
-    // Diffusion samples (zero diffusivity: kept for their admissibility
-    // check). Limited values at limiter points stay in [lo, hi], so the
-    // samples are admissible when hi_H is below the liquidus at hi_C and
-    // Tep >= 0; otherwise the phase kernel checks each sample exactly.
-    // (With a lithostatic pressure the lower Tep over the cell's height bounds it.)
-    const double tep = ph.litho ? fmin(tep_at(ph, t.y0 + gj * t.dy), tep_at(ph, t.y0 + (gj + 1) * t.dy)) : ph.Tep;
-    const double Hliq = tep + (1.0 - hiC / ph.k.Xe) + ph.k.LD;
-    const bool safe = tep >= 0.0 && hiH + 1e-12 * (1.0 + fabs(hiH)) < Hliq;
-    a.flags[cell] = safe ? 0 : FLAG_CHECK;
+    // With a lithostatic pressure Tep is monotone over the cell's height.
+    double t0 = ph.Tep, t1 = t0;
+    if (ph.litho) {
+        t0 = tep_at(ph, t.y0 + gj * t.dy);
+        t1 = tep_at(ph, t.y0 + (gj + 1) * t.dy);
+    }
+    a.flags[cell] = st || st_lim ? (unsigned char)FLAG_CHECK
+                                 : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), loH, hiH, loC, hiC);
     if (st) record_error(a.status, PART_UPDATE, key, st);
     if (st_lim) record_error(a.status, PART_LIMIT, key, st_lim);
 }
 
-template <class R>
-__device__ __forceinline__ void recon_cell(const ReconArgs<R>& a, const Physics& ph, int i, int j) {
+__device__ __forceinline__ void recon_cell(const StageHot& t, const ReconArgs& a, const Physics& ph, int i, int j) {
     if (i >= a.nx || j >= a.ny) return;
     MP_CHECK_INDEX(a.status, (long long)j * a.nx + i, (size_t)a.nx * a.ny);
     const int gj = a.gj0 + j, gny = global_ny(a);
     const int ci = i == 0 ? 0 : (i == a.nx - 1 ? 2 : 1), cj = gj == 0 ? 0 : (gj == gny - 1 ? 2 : 1);
-    if (ci == 1 && cj == 1) recon_cell_t<true>(a, ph, i, j, ci, cj);
-    else recon_cell_t<false>(a, ph, i, j, ci, cj);
+    if (ci == 1 && cj == 1) recon_cell_t<true>(t, a, ph, i, j, ci, cj);
+    else recon_cell_t<false>(t, a, ph, i, j, ci, cj);
 }
 
 // ---------------------------------------------------------- cell phase kernel
 
-template <class R>
 struct CellPhaseArgs {
     int nx, ny;
-    Tab<R> tab;
+    const StageHot* tab;   // batched instances: their tables in device memory
     const double* H;
     const double* C;
     const double* rec;
@@ -383,15 +395,16 @@ __device__ __forceinline__ void load_rec(const double* rec, size_t N, long long 
 }
 
 // Cell quadrature of T and phi (evolve.cpp:359-376) and the wet flag of the
-// porosity sampling (initial_flow.cpp:56-67) on the same 5x5 points.
+// porosity sampling (initial_flow.cpp:56-67) on the same 5x5 points, with
+// every point's admissibility test and the exact check of the diffusion
+// samples. Out of line: cells that are not plain.
 // kExt: the lithostatic pressure and the adiabatic source are compiled in
 // (a launch picks the variant; the default path carries none of their code).
-template <class R, bool kExt = false>
-__device__ __forceinline__ void cellphase_cell(const CellPhaseArgs<R>& a, const Physics& ph, long long cell) {
+template <bool kExt>
+__device__ __noinline__ void cellphase_general(const StageHot& t, const CellPhaseArgs& a, const Physics& ph, long long cell) {
     const long long N = (long long)a.nx * a.ny;
     if (cell >= N) return;
     MP_CHECK_INDEX(a.status, cell, N);
-    const StageHot& t = *a.tab.t;
     const double mH = __ldg(a.H + cell), mC = __ldg(a.C + cell);
     double DH[9], DC[9];
     load_rec(a.rec, (size_t)N, cell, DH, DC);
@@ -466,12 +479,61 @@ __device__ __forceinline__ void cellphase_cell(const CellPhaseArgs<R>& a, const 
     if (kExt && ph.source) { a.srcH[cell] = Ssum; a.srcR[cell] = Rsum; a.srcS[cell] = Wsum; }
 }
 
+// The same quadrature of a plain cell: no tests, no failure. Bound by the
+// FP64 pipe; with the tests, clips and library divisions of every point
+// (1239 FP64 and 3187 instructions per warp) it took 100 us at 640x1280, so
+// (641 and 1223) 54 us.
+template <bool kExt>
+__device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhaseArgs& a, const Physics& ph, long long cell) {
+    const long long N = (long long)a.nx * a.ny;
+    if (cell >= N) return;
+    MP_CHECK_INDEX(a.status, cell, N);
+    const unsigned char fl = a.flags[cell];
+    if (!(fl & FLAG_PLAIN)) { cellphase_general<kExt>(t, a, ph, cell); return; }
+    double DH[9], DC[9];
+    load_rec(a.rec, (size_t)N, cell, DH, DC);
+    DH[0] += __ldg(a.H + cell);
+    DC[0] += __ldg(a.C + cell);
+    const int gj = a.gj0 + (int)((unsigned)cell / (unsigned)a.nx);
+    double Tsum = 0.0, Psum = 0.0, Ssum = 0.0, Rsum = 0.0, Wsum = 0.0;
+#pragma unroll 1
+    for (int b = 0; b < kNQ; ++b) {
+        const double y = t.g[b];
+        double h0, h1, h2, c0, c1, c2;
+        q2_row(DH, y, h0, h1, h2);
+        q2_row(DC, y, c0, c1, c2);
+        const double tep = (kExt && ph.litho) ? tep_at(ph, height(t, gj, y)) : ph.Tep;
+#pragma unroll
+        for (int q = 0; q < kNQ; ++q) {
+            const double x = t.g[q];
+            PhaseLean pl;
+            phase_plain<false>(ph.sk, quad(h0, h1, h2, x), quad(c0, c1, c2, x), tep, pl);
+            const double w = t.cw[b * kNQ + q];
+            Tsum = fma(w, pl.T, Tsum);
+            Psum = fma(w, pl.phil, Psum);
+            if (kExt && ph.source) {
+                const long long at = cell * (kNQ * kNQ) + b * kNQ + q;
+                const double factor = pl.phil == 0.0 ? 0.0 : (ph.theta == 0.0 ? pl.phil : pow(pl.phil, 1.0 + ph.theta));
+                const double vy = __ldg(a.cvs_y + at) + factor * __ldg(a.cud_y + at);
+                const double src = -ph.cooling * pl.T * vy;
+                Ssum += w * src;
+                Rsum += w * ph.cooling * fabs(vy);
+                Wsum += t.cwp[b * kNQ + q] * src;
+            }
+        }
+    }
+    // Porosities are not negative: the cell is wet where their mean is not 0.
+    a.flags[cell] = (unsigned char)(fl | (Psum > 0.0 ? FLAG_WET : 0));
+    a.T[cell] = Tsum;
+    a.phi[cell] = Psum;
+    if (kExt && ph.source) { a.srcH[cell] = Ssum; a.srcR[cell] = Rsum; a.srcS[cell] = Wsum; }
+}
+
 // ---------------------------------------------------------------- face kernel
 
-template <class R>
 struct FaceArgs {
     int nx, ny;
-    Tab<R> tab;
+    const StageHot* tab;   // batched instances: their tables in device memory
     const double* H;
     const double* C;
     const double* rec;
@@ -490,8 +552,7 @@ struct SideLine {
     double h0, h1, h2, c0, c1, c2;
 };
 
-template <class R>
-__device__ __forceinline__ void side_line(const FaceArgs<R>& a, size_t N, long long cell, bool row, double fixed,
+__device__ __forceinline__ void side_line(const FaceArgs& a, size_t N, long long cell, bool row, double fixed,
                                           SideLine& s) {
     double DH[9], DC[9];
     load_rec(a.rec, N, cell, DH, DC);
@@ -579,13 +640,12 @@ __device__ __forceinline__ PointFlux face_point(const Physics& ph, const PhaseLe
 }
 
 // kExt: the lithostatic pressure is compiled in.
-template <class R, bool kExt = false>
-__device__ __forceinline__ void face_edge(const FaceArgs<R>& a, const Physics& ph, long long e) {
+template <bool kExt>
+__device__ __forceinline__ void face_edge(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
     const int nx = a.nx, ny = a.ny;
     const long long nI = (long long)nx * (ny + 1);
     const long long nE = nI + (long long)(nx + 1) * ny;
     if (e >= nE) return;
-    const StageHot& t = *a.tab.t;
     const size_t N = (size_t)nx * ny;
     bool boundary, reverse, horizontal;
     int erow;                // local row of the edge (horizontal) or of its cells (vertical)
@@ -719,13 +779,11 @@ __device__ __forceinline__ void face_edge(const FaceArgs<R>& a, const Physics& p
 // wall value), gradient sum_k c_k (T_k - T_last) / ds, flux -= w kappa grad,
 // and |d flux / d T_k| added to the rate sample by sample. Added to the face
 // results after the advective part, as the reference adds them.
-template <class R>
-__device__ __forceinline__ void diffusion_edge(const FaceArgs<R>& a, const Physics& ph, long long e) {
+__device__ __forceinline__ void diffusion_edge(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
     const int nx = a.nx, ny = a.ny;
     const long long nI = (long long)nx * (ny + 1);
     const long long nE = nI + (long long)(nx + 1) * ny;
     if (e >= nE) return;
-    const StageHot& t = *a.tab.t;
     const size_t N = (size_t)nx * ny;
     bool boundary, reverse, horizontal;
     long long L, Rc = -1;

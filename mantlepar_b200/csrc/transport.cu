@@ -64,51 +64,48 @@ struct SourceBufs {
 // blocks per SM (register caps) as measured fastest on B200: cell phase 8,
 // faces 5; the reconstruction keeps its natural register count.
 // Rows [jlo, jhi) are reconstructed (all rows, or a slab's owned rows +- 1).
-template <class R>
-__global__ void __launch_bounds__(128) recon_kernel(ReconArgs<R> a, Physics ph, const __grid_constant__ ParamTables p,
-                                                    int jlo, int jhi) {
+__global__ void __launch_bounds__(128) recon_kernel(const __grid_constant__ ReconArgs a,
+                                                    const __grid_constant__ Physics ph,
+                                                    const __grid_constant__ ParamTables p, int jlo, int jhi) {
     if (gated_off(a.gate)) return;
-    ReconArgs<R> b = a;
-    b.tab = param_tab<R>(p);
     const int j = jlo + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    if (j < jhi) recon_cell(b, ph, blockIdx.x * blockDim.x + threadIdx.x, j);
+    if (j < jhi) recon_cell(p.d, a, ph, blockIdx.x * blockDim.x + threadIdx.x, j);
 }
-template <class R, bool kExt>
-__global__ void __launch_bounds__(128, 8) cellphase_kernel(CellPhaseArgs<R> a, Physics ph,
-                                                        const __grid_constant__ ParamTables p, long long c0, long long c1) {
+template <bool kExt>
+__global__ void __launch_bounds__(128, 8) cellphase_kernel(const __grid_constant__ CellPhaseArgs a,
+                                                           const __grid_constant__ Physics ph,
+                                                           const __grid_constant__ ParamTables p, long long c0,
+                                                           long long c1) {
     if (gated_off(a.gate)) return;
-    CellPhaseArgs<R> b = a;
-    b.tab = param_tab<R>(p);
     const long long cell = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (cell < c1) cellphase_cell<R, kExt>(b, ph, cell);
+    if (cell < c1) cellphase_cell<kExt>(p.d, a, ph, cell);
 }
 // Edges [h0, h0 + nh) (horizontal) then [v0, v0 + nv) (vertical): every edge
 // of the mesh, or of a slab's owned cells.
 // kRange: the edges of a slab's owned rows (two ranges); otherwise every
 // edge of the mesh with the plain linear mapping (measurably faster).
-template <class R, bool kExt, bool kRange>
-__global__ void __launch_bounds__(128, 5) face_kernel(FaceArgs<R> a, Physics ph, const __grid_constant__ ParamTables p,
-                                                      long long h0, long long nh, long long v0, long long nv) {
+template <bool kExt, bool kRange>
+__global__ void __launch_bounds__(128, 5) face_kernel(const __grid_constant__ FaceArgs a,
+                                                      const __grid_constant__ Physics ph,
+                                                      const __grid_constant__ ParamTables p, long long h0, long long nh,
+                                                      long long v0, long long nv) {
     if (gated_off(a.gate)) return;
-    FaceArgs<R> b = a;
-    b.tab = param_tab<R>(p);
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if constexpr (kRange) {
         // One call site: the edge body is inlined once.
-        if (k < nh + nv) face_edge<R, kExt>(b, ph, k < nh ? h0 + k : v0 + (k - nh));
+        if (k < nh + nv) face_edge<kExt>(p.d, a, ph, k < nh ? h0 + k : v0 + (k - nh));
     } else {
-        face_edge<R, kExt>(b, ph, k);
+        face_edge<kExt>(p.d, a, ph, k);
     }
 }
 // The diffusive part of the same edges (only launched when diffusion is on).
-template <class R>
-__global__ void __launch_bounds__(128) diffusion_kernel(FaceArgs<R> a, Physics ph, const __grid_constant__ ParamTables p,
-                                                        long long h0, long long nh, long long v0, long long nv) {
+__global__ void __launch_bounds__(128) diffusion_kernel(const __grid_constant__ FaceArgs a,
+                                                        const __grid_constant__ Physics ph,
+                                                        const __grid_constant__ ParamTables p, long long h0,
+                                                        long long nh, long long v0, long long nv) {
     if (gated_off(a.gate)) return;
-    FaceArgs<R> b = a;
-    b.tab = param_tab<R>(p);
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < nh + nv) diffusion_edge(b, ph, k < nh ? h0 + k : v0 + (k - nh));
+    if (k < nh + nv) diffusion_edge(p.d, a, ph, k < nh ? h0 + k : v0 + (k - nh));
 }
 
 template <bool kSrc, bool kArea = false>
@@ -303,8 +300,7 @@ mp_status check_status(mp_transport* t, const char* where) {
     return (mp_status)code;
 }
 
-// Launch the stage kernels of state (H, C) in arithmetic type R.
-template <class R>
+// Launch the stage kernels of state (H, C).
 void launch_stage_kernels(int nx, int ny, const StageRange& rg, const ParamTables& pt, const Physics& ph, const double* H, const double* C, double* rec,
                           unsigned char* flags, double* T, double* phi, const double* vsn, const double* udn,
                           double* face, unsigned long long* status, double* theta, cudaStream_t s,
@@ -312,20 +308,20 @@ void launch_stage_kernels(int nx, int ny, const StageRange& rg, const ParamTable
     const size_t NE = (size_t)nx * (ny + 1) + (size_t)(nx + 1) * ny;
     auto run = [&](int kind, auto&& f) { if (prof) timed(prof, kind, f); else f(); };
     {
-        ReconArgs<R> a{nx, ny, Tab<R>{}, H, C, rec, flags, status, theta, rg.gj0, rg.gny, gate};
+        ReconArgs a{nx, ny, nullptr, H, C, rec, flags, status, theta, rg.gj0, rg.gny, gate};
         dim3 blk(32, 4), grd((nx + 31) / 32, (rg.rec1 - rg.rec0 + 3) / 4);
-        run(0, [&] { recon_kernel<R><<<grd, blk, 0, s>>>(a, ph, pt, rg.rec0, rg.rec1); });
+        run(0, [&] { recon_kernel<<<grd, blk, 0, s>>>(a, ph, pt, rg.rec0, rg.rec1); });
     }
     {
-        CellPhaseArgs<R> a{nx, ny, Tab<R>{}, H, C, rec, flags, T, phi, status, rg.gj0, rg.gny,
+        CellPhaseArgs a{nx, ny, nullptr, H, C, rec, flags, T, phi, status, rg.gj0, rg.gny,
                            src.cvs_y, src.cud_y, src.srcH, src.srcR, src.srcS, gate};
         const long long c0 = (long long)rg.rec0 * nx, c1 = (long long)rg.rec1 * nx;
         const unsigned g = (unsigned)((c1 - c0 + 127) / 128);
-        if (ph.litho || ph.source) run(1, [&] { cellphase_kernel<R, true><<<g, 128, 0, s>>>(a, ph, pt, c0, c1); });
-        else run(1, [&] { cellphase_kernel<R, false><<<g, 128, 0, s>>>(a, ph, pt, c0, c1); });
+        if (ph.litho || ph.source) run(1, [&] { cellphase_kernel<true><<<g, 128, 0, s>>>(a, ph, pt, c0, c1); });
+        else run(1, [&] { cellphase_kernel<false><<<g, 128, 0, s>>>(a, ph, pt, c0, c1); });
     }
     {
-        FaceArgs<R> a{nx, ny, Tab<R>{}, H, C, rec, flags, vsn, udn, face, status, rg.gj0, rg.gny, gate};
+        FaceArgs a{nx, ny, nullptr, H, C, rec, flags, vsn, udn, face, status, rg.gj0, rg.gny, gate};
         const long long nI = (long long)nx * (ny + 1);
         const long long h0 = (long long)rg.own0 * nx, nh = (long long)(rg.own1 - rg.own0 + 1) * nx;
         const long long v0 = nI + (long long)rg.own0 * (nx + 1), nv = (long long)(rg.own1 - rg.own0) * (nx + 1);
@@ -333,14 +329,14 @@ void launch_stage_kernels(int nx, int ny, const StageRange& rg, const ParamTable
         const unsigned g = (unsigned)((nh + nv + 127) / 128);
         const bool ranged = !(rg.own0 == 0 && rg.own1 == ny);
         if (ranged) {
-            if (ph.litho) run(2, [&] { face_kernel<R, true, true><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
-            else run(2, [&] { face_kernel<R, false, true><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
+            if (ph.litho) run(2, [&] { face_kernel<true, true><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
+            else run(2, [&] { face_kernel<false, true><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
         } else {
-            if (ph.litho) run(2, [&] { face_kernel<R, true, false><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
-            else run(2, [&] { face_kernel<R, false, false><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
+            if (ph.litho) run(2, [&] { face_kernel<true, false><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
+            else run(2, [&] { face_kernel<false, false><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
         }
         if (ph.diffusion)
-            run(2, [&] { diffusion_kernel<R><<<(unsigned)((nh + nv + 127) / 128), 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
+            run(2, [&] { diffusion_kernel<<<(unsigned)((nh + nv + 127) / 128), 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
     }
 }
 
@@ -381,7 +377,7 @@ mp_status launch_stage(mp_transport* t, const double* H, const double* C, int mo
                               t->d_status, theta, SourcePtrs{sb.cvs_y, sb.cud_y, sb.srcH, sb.srcR, sb.srcS}, s, gate);
         });
     } else {
-        launch_stage_kernels<double>(t->nx, t->ny, t->range, t->ptab, t->ph, H, C, static_cast<double*>(t->rec), t->flags, t->T,
+        launch_stage_kernels(t->nx, t->ny, t->range, t->ptab, t->ph, H, C, static_cast<double*>(t->rec), t->flags, t->T,
                                      t->phi, t->vsn, t->udn, t->face, t->d_status, theta, s, prof, sb, gate);
     }
     {
@@ -1259,7 +1255,7 @@ mp_status stage_rhs_raw(int nx, int ny, const mp_transport_opts& o, const double
     (void)NE;
     ParamTables pt;
     make_param_tables(tab, pt);
-    launch_stage_kernels<double>(nx, ny, whole(ny), pt, ph, H, C, rec, wet, T, phi, vsn, udn, face, status, nullptr, s,
+    launch_stage_kernels(nx, ny, whole(ny), pt, ph, H, C, rec, wet, T, phi, vsn, udn, face, status, nullptr, s,
                                  nullptr);
     {
         SumArgs a{nx, ny, tab.area, 1.0 / tab.area, face, H, C, H, C, rhsH, rhsC, rate, SUM_STORE_L, 0.0, 0.0, 0.0, part};
