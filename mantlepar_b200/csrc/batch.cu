@@ -85,23 +85,24 @@ __global__ void __launch_bounds__(128) batch_recon_kernel(const InstArgs* args, 
 
 // kExt: the adiabatic source (alpha0 != 0) is compiled in.
 template <bool kExt>
-__global__ void __launch_bounds__(128, 8) batch_phase_kernel(const InstArgs* args, const Work* work, const int* active,
-                                                          Physics ph) {
+__global__ void __launch_bounds__(128, 6) batch_phase_kernel(const InstArgs* args, const Work* work, const int* active,
+                                                          const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     cellphase_cell<kExt>(*args[w.inst].phase.tab, args[w.inst].phase, ph, (long long)w.a + threadIdx.x);
 }
 
 __global__ void __launch_bounds__(128, 5) batch_face_kernel(const InstArgs* args, const Work* work, const int* active,
-                                                         Physics ph) {
+                                                         const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
-    const long long e = (long long)w.a + threadIdx.x;
-    if (e < w.b) face_edge<false>(*args[w.inst].face.tab, args[w.inst].face, ph, e);
+    const long long k = (long long)w.a + threadIdx.x;
+    const FaceArgs& a = args[w.inst].face;
+    if (k < w.b) face_edge<false>(*a.tab, a, ph, edge_by_kind(a.nx, a.ny, k));
 }
 
 __global__ void __launch_bounds__(128) batch_diffusion_kernel(const InstArgs* args, const Work* work, const int* active,
-                                                              Physics ph) {
+                                                              const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const long long e = (long long)w.a + threadIdx.x;
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(128, 3) batch_quad_weno_kernel(const QuadStage
 }
 
 __global__ void __launch_bounds__(128, 4) batch_quad_limit_kernel(const QuadStageArgs* args, const Work* work,
-                                                                  const int* active, Physics ph) {
+                                                                  const int* active, const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const QuadStageArgs& a = args[w.inst];
@@ -129,7 +130,7 @@ __global__ void __launch_bounds__(128, 4) batch_quad_limit_kernel(const QuadStag
 }
 
 __global__ void __launch_bounds__(128, 4) batch_quad_phase_kernel(const QuadStageArgs* args, const Work* work,
-                                                                  const int* active, Physics ph) {
+                                                                  const int* active, const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const QuadStageArgs& a = args[w.inst];
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(128, 4) batch_quad_phase_kernel(const QuadStag
 }
 
 __global__ void __launch_bounds__(128, 4) batch_quad_face_kernel(const QuadStageArgs* args, const Work* work,
-                                                                 const int* active, Physics ph) {
+                                                                 const int* active, const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const long long e = (long long)w.a + threadIdx.x;
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(128, 4) batch_quad_face_kernel(const QuadStage
 }
 
 __global__ void __launch_bounds__(128) batch_quad_diffusion_kernel(const QuadStageArgs* args, const Work* work,
-                                                                   const int* active, Physics ph) {
+                                                                   const int* active, const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const long long e = (long long)w.a + threadIdx.x;

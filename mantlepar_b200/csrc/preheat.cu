@@ -201,8 +201,7 @@ __global__ void __launch_bounds__(128) pre_recon_kernel(int nx, int ny, const do
         }
     const int ci = i == 0 ? 0 : (i == nx - 1 ? 2 : 1), cj = j == 0 ? 0 : (j == ny - 1 ? 2 : 1);
     double D[9];
-    const int st = ci == 1 && cj == 1 ? reconstruct<true>(t, 31u, u, D)
-                                      : reconstruct<false>(t, candidate_mask(ci, cj), u, D);
+    const int st = reconstruct(t, candidate_mask(ci, cj), u, D);
 #pragma unroll
     for (int m = 0; m < 9; ++m) rec[(size_t)m * N + cell] = D[m];
     if (st) record_error(status, PART_UPDATE, cell, st);
@@ -463,7 +462,7 @@ __global__ void __launch_bounds__(128) pre_diag_kernel(int nx, int ny, const dou
                 u[dj][di] = __ldg(F + (size_t)jj * nx + ii);
             }
         m[f] = u[1][1];
-        const int s = reconstruct<false>(t, candidate_mask(ci, cj), u, D[f]);
+        const int s = reconstruct(t, candidate_mask(ci, cj), u, D[f]);
         st = st ? st : s;
     }
     if (st) { record_error(status, PART_UPDATE, cell, st); return; }

@@ -254,7 +254,7 @@ __device__ __forceinline__ int reconstruct_quad(const QuadDev& q, size_t N, long
         double s[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) s[k] = fma(sg[f][k], ie, 1.0);
-        if (weno_weights<false>(s, mask, eA * eA, w[f])) st[f] = MP_ERR_FP;
+        if (weno_weights(s, mask, eA * eA, w[f])) st[f] = MP_ERR_FP;
     }
 #pragma unroll
     for (int f = 0; f < F; ++f)

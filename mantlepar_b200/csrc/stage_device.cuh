@@ -188,8 +188,6 @@ static __device__ __noinline__ int weights_general(const double* s, unsigned on,
     if (!isfinite(w[0] + w[1] + w[2] + w[3] + w[4])) st = MP_ERR_FP;
     return st;
 }
-// kAll: every candidate is on (on is not read).
-template <bool kAll>
 __device__ __forceinline__ int weno_weights(const double (&s)[5], unsigned on, double epsA2, double (&w)[5]) {
     const double s12 = s[1] * s[2], s34 = s[3] * s[4], P = s12 * s34, s02 = s[0] * s[0];
     if (!(P * s02 < 1e59)) {
@@ -197,19 +195,19 @@ __device__ __forceinline__ int weno_weights(const double (&s)[5], unsigned on, d
         double sc[5], wc[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) sc[k] = s[k];
-        const int st = weights_general(sc, kAll ? 31u : on, epsA2, wc);
+        const int st = weights_general(sc, on, epsA2, wc);
 #pragma unroll
         for (int k = 0; k < 5; ++k) w[k] = wc[k];
         return st;
     }
     auto p5 = [](double x) { const double x2 = x * x; return x2 * x2 * x; };
-    const double f = (kAll || (on & 1u) ? epsA2 : 1.0) * (s02 * s02 * (s02 * s[0]));
+    const double f = (on & 1u ? epsA2 : 1.0) * (s02 * s02 * (s02 * s[0]));
     w[0] = p5(P);
     w[1] = f * p5(s[2] * s34);
     w[2] = f * p5(s[1] * s34);
     w[3] = f * p5(s12 * s[4]);
     w[4] = f * p5(s12 * s[3]);
-    if (!kAll) {
+    if (on != 31u) {
 #pragma unroll
         for (int k = 0; k < 5; ++k) w[k] = (on >> k) & 1u ? w[k] : 0.0;
     }
@@ -241,10 +239,9 @@ __device__ __forceinline__ unsigned candidate_mask(int ci, int cj) {
 // pipe (one warp instruction per two cycles): with the general basis and
 // smoothness matrices of the mesh (64 + 44 FMAs and 4 x 21 per field) and the
 // limiter scan line by line it issued 1680 FP64 instructions per warp and took
-// 160 us at 640x1280; with these forms and scan_interior 1121 and 89 us.
-// kAll: an interior cell. Returns MP_ERR_FP when the weights cannot be
-// normalised (non-finite data).
-template <bool kAll>
+// 160 us at 640x1280; with these forms and scan_cell 1121 and 89 us.
+// on: candidate_mask of the cell. Returns MP_ERR_FP when the weights cannot
+// be normalised (non-finite data).
 __device__ __forceinline__ int reconstruct(const StageHot& t, unsigned on, const double (&u)[3][3], double (&D)[9]) {
     const double c = u[1][1];
     const double dSW = u[0][0] - c, dS = u[0][1] - c, dSE = u[0][2] - c, dW = u[1][0] - c, dE = u[1][2] - c,
@@ -279,12 +276,12 @@ __device__ __forceinline__ int reconstruct(const StageHot& t, unsigned on, const
         s[3] = fma(t.gb * bSW, bSW, w + o);
         s[4] = fma(t.gb * bNW, bNW, w + n);
     }
-    if (!kAll) {
+    if (on != 31u) {
 #pragma unroll
         for (int k = 0; k < 5; ++k) s[k] = (on >> k) & 1u ? s[k] : 1.0;
     }
     double w[5];
-    const int st = weno_weights<kAll>(s, on, t.epsA2, w);
+    const int st = weno_weights(s, on, t.epsA2, w);
     D[0] = w[0] * q00;
     D[1] = fma(w[0], q10, 0.5 * fma(w[1] + w[2], dE, -((w[3] + w[4]) * dW)));
     D[2] = w[0] * q20;

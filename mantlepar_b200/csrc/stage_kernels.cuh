@@ -194,6 +194,11 @@ struct Extremes {
         up(fma(b, kG1, e1)); up(fma(b, kG2, e2));
         down(fma(-b, kG1, e1)); down(fma(-b, kG2, e2));
     }
+    // A line and its centre.
+    __device__ __forceinline__ void line(double a0, double a1, double a2) {
+        up(a0); down(a0);
+        pairs(a0, a1, a2);
+    }
     // The lines at +c and -c of the coefficient rows (p0 + c p1 + c^2 p2) of
     // the three powers along the line; the two centres again as a pair.
     __device__ __forceinline__ void line_pair(double c, const double (&p0)[3], const double (&p1)[3],
@@ -208,39 +213,34 @@ struct Extremes {
     }
 };
 
-// The 86 limiter points of an interior cell (state_reconstruction.cpp:
-// 152-168): on the rows eta = 0, +-g1, +-g2 (cell quadrature), +-1 (edges),
-// +-0.4, +-0.8 (diffusion samples: 0.3 and 0.9 cell sizes from each edge) and
-// the columns xi = +-1, +-0.4, +-0.8, five Gauss points each. The lines come
-// in symmetric pairs and their points in symmetric pairs, so 85 points take
-// 274 FP64 operations, 84 of them comparisons.
-__device__ __forceinline__ void scan_interior(const double (&D)[9], double& mx, double& mn) {
+// The limiter points of a cell of boundary class (ci, cj)
+// (state_reconstruction.cpp:152-168), five Gauss points on each of: the rows
+// eta = 0, +-g1, +-g2 (cell quadrature) and +-1 (edges), the columns xi = +-1,
+// and the diffusion samples' lines, 0.9 and 0.3 cell sizes from an interior
+// edge (+-0.8, +-0.4) and 0.9, 0.675, 0.45 and 0.225 from a wall: there the
+// 0.3 line gives way to three. The lines common to every cell are scanned as
+// symmetric pairs and their points as symmetric pairs (85 points in 280 FP64
+// operations, 84 of them comparisons); a wall adds its lines, so that a cell
+// takes the same operations whatever its neighbours in the warp are.
+__device__ __forceinline__ void scan_cell(const double (&D)[9], int ci, int cj, double& mx, double& mn) {
     Extremes x{D[0], D[0]};
     x.pairs(D[0], D[1], D[2]);
     const double r0[3] = {D[0], D[1], D[2]}, r1[3] = {D[3], D[4], D[5]}, r2[3] = {D[6], D[7], D[8]};
     x.line_pair(kG1, r0, r1, r2);
     x.line_pair(kG2, r0, r1, r2);
-    x.line_pair(0.4, r0, r1, r2);
     x.line_pair(0.8, r0, r1, r2);
     x.line_pair(1.0, r0, r1, r2);
     const double c0[3] = {D[0], D[3], D[6]}, c1[3] = {D[1], D[4], D[7]}, c2[3] = {D[2], D[5], D[8]};
-    x.line_pair(0.4, c0, c1, c2);
     x.line_pair(0.8, c0, c1, c2);
     x.line_pair(1.0, c0, c1, c2);
-    mx = x.mx; mn = x.mn;
-}
-
-// The limiter points of a boundary class, line by line from the tables.
-__device__ __forceinline__ void scan_lines(const StageHot& t, int l0, int l1, const double (&D)[9], double& mx,
-                                           double& mn) {
-    Extremes x{D[0], D[0]};
-    for (int l = l0; l < l1; ++l) {
-        double a0, a1, a2;
-        if (t.line_dir[l] == 0) q2_row(D, t.line_c[l], a0, a1, a2);
-        else q2_col(D, t.line_c[l], a0, a1, a2);
-        x.up(a0); x.down(a0);
-        x.pairs(a0, a1, a2);
-    }
+    auto row = [&](double c) { double a0, a1, a2; q2_row(D, c, a0, a1, a2); x.line(a0, a1, a2); };
+    auto col = [&](double c) { double a0, a1, a2; q2_col(D, c, a0, a1, a2); x.line(a0, a1, a2); };
+    row(cj == 0 ? 0.35 : -0.4);
+    row(cj == 2 ? -0.35 : 0.4);
+    col(ci == 0 ? 0.35 : -0.4);
+    col(ci == 2 ? -0.35 : 0.4);
+    if (cj != 1) { const double s = cj == 0 ? 1.0 : -1.0; row(-0.1 * s); row(-0.55 * s); }
+    if (ci != 1) { const double s = ci == 0 ? 1.0 : -1.0; col(-0.1 * s); col(-0.55 * s); }
     mx = x.mx; mn = x.mn;
 }
 
@@ -261,12 +261,10 @@ __device__ __forceinline__ double theta_of(double m, double lo, double hi, doubl
 constexpr double kScanGuard = 1e30;
 
 // One field of one cell: gather, neighbour bounds, reconstruction, limiter
-// factor th and the unlimited D. kInterior: the cell has all eight
-// neighbours (no candidate is dropped, the limiter points are the fixed set).
-// top: the field's upper bound (Xe for the composition).
-template <bool kInterior>
+// factor th and the unlimited D. top: the field's upper bound (Xe for the
+// composition).
 __device__ __forceinline__ void recon_field(const StageHot& t, const double* __restrict__ F, const unsigned (&at)[3][3],
-                                            unsigned on, int cls, double top, double (&D)[9], double& mean, double& lo,
+                                            int ci, int cj, double top, double (&D)[9], double& mean, double& lo,
                                             double& hi, double& th, int& st, bool& bad) {
     double u[3][3];
 #pragma unroll
@@ -287,7 +285,7 @@ __device__ __forceinline__ void recon_field(const StageHot& t, const double* __r
     const bool small = lo > -kScanGuard && hi < kScanGuard;
     lo = fmax(0.0, lo);
     hi = top < hi ? top : hi;
-    const int s1 = reconstruct<kInterior>(t, on, u, D);
+    const int s1 = reconstruct(t, candidate_mask(ci, cj), u, D);
     st = st ? st : s1;
     double mx, mn;
     if (!small) {
@@ -296,22 +294,25 @@ __device__ __forceinline__ void recon_field(const StageHot& t, const double* __r
         bool b = false;
 #pragma unroll
         for (int m = 0; m < 9; ++m) Dc[m] = D[m];
-        scan_lines_exact(t, t.line_off[cls], t.line_off[cls + 1], Dc, x, n, b);
+        scan_lines_exact(t, t.line_off[cj * 3 + ci], t.line_off[cj * 3 + ci + 1], Dc, x, n, b);
         mx = x; mn = n;
         bad = bad || b;
-    } else if (kInterior) scan_interior(D, mx, mn);
-    else scan_lines(t, t.line_off[cls], t.line_off[cls + 1], D, mx, mn);
+    } else {
+        scan_cell(D, ci, cj, mx, mn);
+    }
     th = theta_of(mean, lo, hi, mx, mn);
 }
 
 // Reconstruction and limiter of both fields, one field after the other
 // through the same code (18 limited coefficients live one field at a time).
-template <bool kInterior>
-__device__ __forceinline__ void recon_cell_t(const StageHot& t, const ReconArgs& a, const Physics& ph, int i, int j, int ci, int cj) {
+__device__ __forceinline__ void recon_cell(const StageHot& t, const ReconArgs& a, const Physics& ph, int i, int j) {
+    if (i >= a.nx || j >= a.ny) return;
     const int nx = a.nx, ny = a.ny;
     const long long cell = (long long)j * nx + i;
     const size_t N = (size_t)nx * ny;
-    const int gj = a.gj0 + j;
+    MP_CHECK_INDEX(a.status, cell, N);
+    const int gj = a.gj0 + j, gny = global_ny(a);
+    const int ci = i == 0 ? 0 : (i == nx - 1 ? 2 : 1), cj = gj == 0 ? 0 : (gj == gny - 1 ? 2 : 1);
     const long long key = cell + (long long)a.gj0 * nx;
     // Cells stay below 2^31 (checked on create).
     unsigned at[3][3];
@@ -323,15 +324,13 @@ __device__ __forceinline__ void recon_cell_t(const StageHot& t, const ReconArgs&
             MP_CHECK_INDEX(a.status, (long long)jj * nx + ii, N);
             at[dj][di] = (unsigned)jj * (unsigned)nx + (unsigned)ii;
         }
-    const unsigned on = candidate_mask(ci, cj);
-    const int cls = cj * 3 + ci;
     int st = 0;
     bool bad = false, means = true;
     double loH = 0, hiH = 0, loC = 0, hiC = 0;
 #pragma unroll 1
     for (int f = 0; f < 2; ++f) {
         double D[9], mean, lo, hi, th;
-        recon_field<kInterior>(t, f ? a.C : a.H, at, on, cls, f ? ph.k.Xe : INFINITY, D, mean, lo, hi, th, st, bad);
+        recon_field(t, f ? a.C : a.H, at, ci, cj, f ? ph.k.Xe : INFINITY, D, mean, lo, hi, th, st, bad);
         // state_reconstruction.cpp:187-188: admissible means.
         means = means && isfinite(mean) && mean >= 0.0 && (f == 0 || mean <= ph.k.Xe);
         if (f) { loC = lo; hiC = hi; }
@@ -351,15 +350,6 @@ __device__ __forceinline__ void recon_cell_t(const StageHot& t, const ReconArgs&
                                  : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), loH, hiH, loC, hiC);
     if (st) record_error(a.status, PART_UPDATE, key, st);
     if (st_lim) record_error(a.status, PART_LIMIT, key, st_lim);
-}
-
-__device__ __forceinline__ void recon_cell(const StageHot& t, const ReconArgs& a, const Physics& ph, int i, int j) {
-    if (i >= a.nx || j >= a.ny) return;
-    MP_CHECK_INDEX(a.status, (long long)j * a.nx + i, (size_t)a.nx * a.ny);
-    const int gj = a.gj0 + j, gny = global_ny(a);
-    const int ci = i == 0 ? 0 : (i == a.nx - 1 ? 2 : 1), cj = gj == 0 ? 0 : (gj == gny - 1 ? 2 : 1);
-    if (ci == 1 && cj == 1) recon_cell_t<true>(t, a, ph, i, j, ci, cj);
-    else recon_cell_t<false>(t, a, ph, i, j, ci, cj);
 }
 
 // ---------------------------------------------------------- cell phase kernel
@@ -576,9 +566,6 @@ __device__ __forceinline__ int side_phase(const Physics& ph, const SideLine& s, 
 // edge porosity, transport velocities, Lax-Friedrichs fluxes or the boundary
 // policy (evolve.cpp:36-52,292-329; initial_flow.cpp:94-117), and the point's
 // CFL rate term before its quadrature weight; st keeps the first failure.
-// Used by the general-quad face kernel. face_edge below carries the same
-// statements inline: called from there, this function changes the uniform
-// face kernel's register allocation (12 more bytes of spills, 2% slower).
 struct PointFlux {
     double fh, fc, vn, speed;   // speed: (aC + aH + 2 |vs|) * sens
 };
@@ -639,58 +626,166 @@ __device__ __forceinline__ PointFlux face_point(const Physics& ph, const PhaseLe
     return PointFlux{fh, fc, vn, (aC + aH + 2.0 * fabs(vs)) * sens};
 }
 
+// A phase point checked to be plain here, else through the tested form.
+__device__ __forceinline__ int inflow_temperature(const Physics& ph, double H, double C, double tep, double& T) {
+    PhaseLean p;
+    const double slack = 1e-12 * (1.0 + fabs(H));
+    int st = 0;
+    if (ph.sk.ordinary && tep >= 1e-9 && tep <= 1e100 && H >= slack && H + slack < tep + (1.0 - C * ph.sk.invXe) + ph.k.LD &&
+        C >= 1e-90 && C <= ph.k.Xe * (1.0 - 1e-12))
+        phase_plain<false>(ph.sk, H, C, tep, p);
+    else
+        st = phase_stage(ph.sk, H, C, tep, p);
+    T = p.T;
+    return st;
+}
+
+// Transport velocities of an edge point between plain phase states
+// (face_point's, without a division): the edge porosity, the mixture velocity
+// vn and the composition velocity ve.
+__device__ __forceinline__ void plain_velocities(const Physics& ph, const PhaseLean& A, const PhaseLean& B, bool wet,
+                                                 double vs, double ud, double& ephi, double& vn, double& ve) {
+    ephi = 0.0;
+    vn = ve = vs;
+    const double P2 = 2.0 * A.phil * B.phil;
+    if (!(wet && P2 > 0.0)) return;
+    // ephi = P2/S and cl/bulk = cl S/Q as face_point forms them.
+    const double S = A.phil + B.phil, cl = 0.5 * (A.cl + B.cl), cs = 0.5 * (A.cs + B.cs);
+    const double Q = fma(P2, cl - cs, cs * S), SQ = S * Q;
+    double clb;
+    if (rcp_range(SQ)) {
+        const double x = rcp(SQ);
+        ephi = P2 * (Q * x);
+        clb = cl * (S * (S * x));
+    } else {
+        ephi = P2 / S;
+        const double bulk = ephi * cl + (1.0 - ephi) * cs;
+        clb = bulk > 0.0 ? cl / bulk : 0.0;
+    }
+    const double flux = (ph.theta == 0.0 || ephi == 0.0 ? ephi : pow(ephi, 1.0 + ph.theta)) * ud;
+    vn = vs + flux;
+    ve = fma(clb, flux, vs);
+}
+
+// face_point of an interior edge between two plain cells. With local speeds
+// the Lax-Friedrichs flux is the upwind one.
+__device__ __forceinline__ PointFlux face_point_plain(const Physics& ph, const PhaseLean& A, const PhaseLean& B, double cL,
+                                                      double cR, bool wet, double vs, double ud, int& st) {
+    double ephi, vn, ve, fh, fc;
+    plain_velocities(ph, A, B, wet, vs, ud, ephi, vn, ve);
+    const double latent = ph.k.LD * (1.0 - ephi) * vs;
+    double aH = fabs(vn), aC = fabs(ve);
+    if (ph.lf_global) {
+        if (!(ph.lf_speed + 1e-14 >= aH && ph.lf_speed + 1e-14 >= aC)) st = st ? st : E_OUTOFRANGE;
+        aH = aC = ph.lf_speed;
+        fh = 0.5 * (vn * (A.T + B.T) - aH * (B.T - A.T)) - latent;
+        fc = 0.5 * (ve * (cL + cR) - aC * (cR - cL));
+    } else {
+        fh = fma(vn, vn >= 0.0 ? A.T : B.T, -latent);
+        fc = ve * (ve >= 0.0 ? cL : cR);
+    }
+    const double dA = fabs(A.dTdC), dB = fabs(B.dTdC);
+    return PointFlux{fh, fc, vn, (aC + aH + 2.0 * fabs(vs)) * (1.0 + (dA > dB ? dA : dB))};
+}
+
+// face_point at the wall of a plain cell: EvaluateAdvectionBoundary
+// (initialization.cpp:469-489) per field.
+__device__ __forceinline__ PointFlux wall_point_plain(const Physics& ph, const PhaseLean& A, double c, bool wet, double vs,
+                                                      double ud, double tep, int& st) {
+    double ephi, vn, ve;
+    plain_velocities(ph, A, A, wet, vs, ud, ephi, vn, ve);
+    double aH = fabs(vn), aC = fabs(ve);
+    if (ph.lf_global) {
+        if (!(ph.lf_speed + 1e-14 >= aH && ph.lf_speed + 1e-14 >= aC)) st = st ? st : E_OUTOFRANGE;
+        aH = aC = ph.lf_speed;
+    }
+    const bool inH = vn < 0.0 && ph.Hpol != MP_BC_ZERO_FLUX, inC = ve < 0.0 && ph.Cpol != MP_BC_ZERO_FLUX;
+    if ((inH && ph.Hpol != MP_BC_INFLOW_OUTFLOW) || (inC && ph.Cpol != MP_BC_INFLOW_OUTFLOW)) st = st ? st : E_OUTOFRANGE;
+    const double cb = inC ? ph.inflowC : c;
+    double Tb = A.T;
+    if (inH) {
+        const int s = inflow_temperature(ph, ph.inflowH, cb, tep, Tb);
+        st = st ? st : s;
+    }
+    const double fh = ph.Hpol == MP_BC_ZERO_FLUX || vn == 0.0 ? 0.0 : fma(vn, Tb, -(ph.k.LD * (1.0 - ephi) * vs));
+    const double fc = ph.Cpol == MP_BC_ZERO_FLUX ? 0.0 : ve * cb;
+    return PointFlux{fh, fc, vn, (aC + aH + 2.0 * fabs(vs)) * (1.0 + fabs(A.dTdC))};
+}
+
+// An edge of the mesh: the edge along i (horizontal) or j at (i, j).
+struct EdgeAt {
+    bool horizontal;
+    int i, j;
+};
+// Edge k in id order (slabs, and the out-of-line forms below).
+__device__ __forceinline__ EdgeAt edge_by_id(int nx, int ny, long long e) {
+    const long long nI = (long long)nx * (ny + 1);
+    if (e < nI) return EdgeAt{true, (int)((unsigned)e % (unsigned)nx), (int)((unsigned)e / (unsigned)nx)};
+    const unsigned k = (unsigned)(e - nI), w = (unsigned)nx + 1u;
+    return EdgeAt{false, (int)(k % w), (int)(k / w)};
+}
+// Edge k of a whole mesh in the order interior horizontal, interior vertical,
+// walls: the walls' boundary policy runs in warps of its own instead of in
+// one or two lanes of every row's first and last warp.
+__device__ __forceinline__ EdgeAt edge_by_kind(int nx, int ny, long long kk) {
+    unsigned k = (unsigned)kk;
+    const unsigned nh = (unsigned)nx * (unsigned)(ny - 1), w = (unsigned)nx - 1u, nv = w * (unsigned)ny;
+    if (k < nh) return EdgeAt{true, (int)(k % (unsigned)nx), (int)(k / (unsigned)nx) + 1};
+    k -= nh;
+    if (k < nv) return EdgeAt{false, (int)(k % w) + 1, (int)(k / w)};
+    k -= nv;
+    if (k < 2u * (unsigned)nx) return EdgeAt{true, (int)(k < (unsigned)nx ? k : k - nx), k < (unsigned)nx ? 0 : ny};
+    k -= 2u * (unsigned)nx;
+    return EdgeAt{false, k < (unsigned)ny ? 0 : nx, (int)(k < (unsigned)ny ? k : k - ny)};
+}
+
+// Left/right cells and orientation as the reference's Build (evolve.cpp:230-251).
+struct EdgeCells {
+    long long e, L, R;
+    bool boundary, reverse;
+};
+__device__ __forceinline__ EdgeCells edge_cells(const FaceArgs& a, const EdgeAt& g) {
+    const int nx = a.nx;
+    EdgeCells c;
+    if (g.horizontal) {
+        const int gj = a.gj0 + g.j, gny = global_ny(a);
+        c.e = (long long)g.j * nx + g.i;
+        c.boundary = gj == 0 || gj == gny;
+        c.reverse = gj == gny;
+        c.L = c.reverse ? c.e - nx : c.e;
+        c.R = c.boundary ? -1 : c.e - nx;
+    } else {
+        c.e = (long long)nx * (a.ny + 1) + (long long)g.j * (nx + 1) + g.i;
+        c.boundary = g.i == 0 || g.i == nx;
+        c.reverse = g.i == 0;
+        const long long row = (long long)g.j * nx;
+        c.L = c.reverse ? row : row + g.i - 1;
+        c.R = c.boundary ? -1 : row + g.i;
+    }
+    return c;
+}
+
+// An edge of any cells, every point with its admissibility tests. Out of
+// line: edges with a cell that is not plain.
 // kExt: the lithostatic pressure is compiled in.
 template <bool kExt>
-__device__ __forceinline__ void face_edge(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
-    const int nx = a.nx, ny = a.ny;
-    const long long nI = (long long)nx * (ny + 1);
-    const long long nE = nI + (long long)(nx + 1) * ny;
-    if (e >= nE) return;
-    const size_t N = (size_t)nx * ny;
-    bool boundary, reverse, horizontal;
-    int erow;                // local row of the edge (horizontal) or of its cells (vertical)
-    long long L, Rc = -1;
-    double len;
-    double lfix, rfix;   // the edge's fixed coordinate in the left / right cell frame
-    // Left/right cells and orientation as the reference's Build (evolve.cpp:230-251).
-    if (e < nI) {
-        horizontal = true;
-        const unsigned ue = (unsigned)e;   // edge counts stay below 2^31 (checked on create)
-        const int i = (int)(ue % (unsigned)nx), j = (int)(ue / (unsigned)nx);
-        const int gj = a.gj0 + j, gny = global_ny(a);
-        erow = j;
-        boundary = (gj == 0 || gj == gny);
-        reverse = (gj == gny);
-        L = reverse ? (long long)(j - 1) * nx + i : (long long)j * nx + i;
-        if (!boundary) Rc = (long long)(j - 1) * nx + i;
-        lfix = reverse ? 1.0 : -1.0;
-        rfix = 1.0;
-        len = t.len_h;
-    } else {
-        horizontal = false;
-        const unsigned k = (unsigned)(e - nI);
-        const int i = (int)(k % (unsigned)(nx + 1)), j = (int)(k / (unsigned)(nx + 1));
-        erow = j;
-        boundary = (i == 0 || i == nx);
-        reverse = (i == 0);
-        L = reverse ? (long long)j * nx : (long long)j * nx + (i - 1);
-        if (!boundary) Rc = (long long)j * nx + i;
-        lfix = reverse ? -1.0 : 1.0;
-        rfix = -1.0;
-        len = t.len_v;
-    }
-    MP_CHECK_INDEX(a.status, L, N);
-    if (!boundary) MP_CHECK_INDEX(a.status, Rc, N);
+__device__ __noinline__ void face_general(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
+    const long long nE = (long long)a.nx * (a.ny + 1) + (long long)(a.nx + 1) * a.ny;
+    const size_t N = (size_t)a.nx * a.ny;
+    const EdgeAt at_ = edge_by_id(a.nx, a.ny, e);
+    const EdgeCells g = edge_cells(a, at_);
+    const double len = at_.horizontal ? t.len_h : t.len_v;
+    // The edge's fixed coordinate in the left / right cell frame.
+    const double lfix = at_.horizontal == g.reverse ? 1.0 : -1.0, rfix = at_.horizontal ? 1.0 : -1.0;
     SideLine sl, sr;
-    side_line(a, N, L, horizontal, lfix, sl);
-    if (!boundary) side_line(a, N, Rc, horizontal, rfix, sr);
-    const bool wetL = (a.flags[L] & FLAG_WET) != 0, wetR = boundary ? true : (a.flags[Rc] & FLAG_WET) != 0;
-    const double sgn = reverse ? -1.0 : 1.0;
-    const double LD = ph.k.LD;
+    side_line(a, N, g.L, at_.horizontal, lfix, sl);
+    if (!g.boundary) side_line(a, N, g.R, at_.horizontal, rfix, sr);
+    const bool wetL = (a.flags[g.L] & FLAG_WET) != 0, wetR = g.boundary ? true : (a.flags[g.R] & FLAG_WET) != 0;
+    const double sgn = g.reverse ? -1.0 : 1.0;
     double fluxH = 0.0, fluxC = 0.0, fluxMix = 0.0, rate = 0.0;
     int st = 0;
     for (int q = 0; q < kNQ; ++q) {
-        const int cq = reverse ? kNQ - 1 - q : q;
+        const int cq = g.reverse ? kNQ - 1 - q : q;
         const double at = t.g[cq];
         const double vs = sgn * __ldg(a.vsn + e * kNQ + cq);
         const double ud = sgn * __ldg(a.udn + e * kNQ + cq);
@@ -698,76 +793,136 @@ __device__ __forceinline__ void face_edge(const StageHot& t, const FaceArgs& a, 
         PhaseLean A, B;
         // Height of this Gauss point: the edge row for horizontal edges.
         const double tep = !(kExt && ph.litho) ? ph.Tep
-                         : tep_at(ph, horizontal ? t.y0 + (a.gj0 + erow) * t.dy : height(t, a.gj0 + erow, at));
+                         : tep_at(ph, at_.horizontal ? t.y0 + (a.gj0 + at_.j) * t.dy : height(t, a.gj0 + at_.j, at));
         int s = side_phase(ph, sl, at, tep, hL, cL, A);
-        if (boundary) { B = A; hR = hL; cR = cL; }
+        if (g.boundary) { B = A; hR = hL; cR = cL; }
         else {
             const int s2 = side_phase(ph, sr, at, tep, hR, cR, B);
             s = s ? s : s2;
         }
         if (s) { st = st ? st : s; continue; }
-        // Edge porosity: harmonic mean of both sides, zero next to a dry cell
-        // (initial_flow.cpp:94-117). PhaseTransportVelocities (evolve.cpp:36-52)
-        // on normal components: bulk = ephi cl + (1 - ephi) cs, and the
-        // composition velocity adds cl/bulk times the Darcy flux. With
-        // S = phil_A + phil_B and Q = S bulk, ephi = 2 phil_A phil_B / S and
-        // cl/bulk = cl S / Q come from one division 1/(S Q) where it is in range.
-        const double cl = 0.5 * (A.cl + B.cl), cs = 0.5 * (A.cs + B.cs);
-        const double S = A.phil + B.phil;
-        double ephi = 0.0, clb = 0.0;   // clb = cl/bulk where bulk > 0, else 0
-        if (wetL && wetR && S > 0.0) {
-            const double P2 = 2.0 * A.phil * B.phil;
-            const double Q = P2 * (cl - cs) + cs * S;
-            const double SQ = S * Q;
-            if (SQ > 1e-290 && SQ < 1e290) {
-                const double x = 1.0 / SQ;
-                ephi = P2 * (Q * x);
-                clb = cl * (S * (S * x));
-            } else {
-                ephi = P2 / S;
-                const double bulk = ephi * cl + (1.0 - ephi) * cs;
-                clb = bulk > 0.0 ? cl / bulk : 0.0;
-            }
-        }
-        const double factor = ephi == 0.0 ? 0.0 : (ph.theta == 0.0 ? ephi : pow(ephi, 1.0 + ph.theta));
-        const double flux = factor * ud;
-        const double vn = vs + flux;
-        const double ve = vs + clb * flux;
-        const double aH = ph.lf_global ? ph.lf_speed : fabs(vn);
-        const double aC = ph.lf_global ? ph.lf_speed : fabs(ve);
-        if (ph.lf_global && !(aH + 1e-14 >= fabs(vn) && aC + 1e-14 >= fabs(ve))) st = st ? st : E_OUTOFRANGE;
-        double fh = 0.5 * (vn * (A.T + B.T) - aH * (B.T - A.T)) - LD * (1.0 - ephi) * vs;
-        double fc = 0.5 * (ve * (cL + cR) - aC * (cR - cL));
-        if (boundary) {
-            // EvaluateAdvectionBoundary (initialization.cpp:469-489) per field.
-            const int kh = (ph.Hpol == MP_BC_ZERO_FLUX || vn == 0.0) ? 2 : (vn < 0.0 ? 0 : 1);
-            const int kc = (ph.Cpol == MP_BC_ZERO_FLUX || ve == 0.0) ? 2 : (ve < 0.0 ? 0 : 1);
-            if ((kh == 0 && ph.Hpol != MP_BC_INFLOW_OUTFLOW) || (kc == 0 && ph.Cpol != MP_BC_INFLOW_OUTFLOW))
-                st = st ? st : E_OUTOFRANGE;
-            const double inC = kc == 0 ? ph.inflowC : cL;
-            double Tb = A.T;
-            if (kh == 0) {
-                PhaseLean pin;
-                const int s3 = phase_stage(ph.sk, ph.inflowH, inC, tep, pin);
-                if (s3) st = st ? st : s3;
-                Tb = pin.T;
-            }
-            fh = kh == 2 ? 0.0 : vn * Tb - LD * (1.0 - ephi) * vs;
-            fc = kc == 2 ? 0.0 : ve * (kc == 0 ? ph.inflowC : cL);
-        }
+        const PointFlux pf = face_point(ph, A, B, cL, cR, wetL, wetR, g.boundary, vs, ud, tep, ph.k.LD, st);
         const double w = 0.5 * len * t.gw[q];
-        fluxH += w * fh;
-        fluxC += w * fc;
-        fluxMix += w * vn;
-        const double sens = 1.0 + fmax(fabs(A.dTdC), fabs(B.dTdC));
-        if (!isfinite(sens)) st = st ? st : E_FP;
-        rate += w * (aC + aH + 2.0 * fabs(vs)) * sens;
+        fluxH += w * pf.fh;
+        fluxC += w * pf.fc;
+        fluxMix += w * pf.vn;
+        rate += w * pf.speed;
     }
-    if (st) record_error(a.status, PART_FACES, L + (long long)a.gj0 * nx, st);
+    if (st) record_error(a.status, PART_FACES, g.L + (long long)a.gj0 * a.nx, st);
     a.face[e] = fluxH;
     a.face[nE + e] = fluxC;
     a.face[2 * nE + e] = rate;
     a.face[3 * nE + e] = fluxMix;
+}
+
+// Limited H and C of one side along an edge of a uniform mesh: the cell's
+// polynomial at xi or eta = s = +-1, mean included.
+__device__ __forceinline__ void edge_line(const FaceArgs& a, size_t N, long long cell, bool horizontal, double s,
+                                          double (&h)[3], double (&c)[3]) {
+    double DH[9], DC[9];
+    load_rec(a.rec, N, cell, DH, DC);
+    DH[0] += __ldg(a.H + cell);
+    DC[0] += __ldg(a.C + cell);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (horizontal) {
+            h[k] = fma(s, DH[k + 3], DH[k] + DH[k + 6]);
+            c[k] = fma(s, DC[k + 3], DC[k] + DC[k + 6]);
+        } else {
+            h[k] = fma(s, DH[3 * k + 1], DH[3 * k] + DH[3 * k + 2]);
+            c[k] = fma(s, DC[3 * k + 1], DC[3 * k] + DC[3 * k + 2]);
+        }
+    }
+}
+
+__device__ __forceinline__ void store_face(const FaceArgs& a, long long e, double half, double fluxH, double fluxC,
+                                           double rate, double fluxMix) {
+    const long long nE = (long long)a.nx * (a.ny + 1) + (long long)(a.nx + 1) * a.ny;
+    a.face[e] = half * fluxH;
+    a.face[nE + e] = half * fluxC;
+    a.face[2 * nE + e] = half * rate;
+    a.face[3 * nE + e] = half * fluxMix;
+}
+
+// A wall edge of a plain cell (in warps of their own, edge_by_kind). Out of
+// line: its branches in the interior edges' loop cost that loop registers
+// (147 us against 130 at 640x1280).
+template <bool kExt>
+__device__ __noinline__ void face_wall(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
+    const EdgeAt at = edge_by_id(a.nx, a.ny, e);
+    const EdgeCells g = edge_cells(a, at);
+    double h[3], c[3];
+    edge_line(a, (size_t)a.nx * a.ny, g.L, at.horizontal, at.horizontal == g.reverse ? 1.0 : -1.0, h, c);
+    const bool wet = (a.flags[g.L] & FLAG_WET) != 0;
+    const double sgn = g.reverse ? -1.0 : 1.0;
+    double fluxH = 0.0, fluxC = 0.0, fluxMix = 0.0, rate = 0.0;
+    int st = 0;
+    for (int q = 0; q < kNQ; ++q) {
+        const double x = t.g[q], w = t.gw[q];
+        const double vs = sgn * __ldg(a.vsn + e * kNQ + q), ud = sgn * __ldg(a.udn + e * kNQ + q);
+        const double tep = !(kExt && ph.litho) ? ph.Tep
+                         : tep_at(ph, at.horizontal ? t.y0 + (a.gj0 + at.j) * t.dy : height(t, a.gj0 + at.j, x));
+        const double cx = quad(c[0], c[1], c[2], x);
+        PhaseLean A;
+        phase_plain<true>(ph.sk, quad(h[0], h[1], h[2], x), cx, tep, A);
+        const PointFlux pf = wall_point_plain(ph, A, cx, wet, vs, ud, tep, st);
+        fluxH = fma(w, pf.fh, fluxH);
+        fluxC = fma(w, pf.fc, fluxC);
+        fluxMix = fma(w, pf.vn, fluxMix);
+        rate = fma(w, pf.speed, rate);
+    }
+    if (st) record_error(a.status, PART_FACES, g.L + (long long)a.gj0 * a.nx, st);
+    store_face(a, e, 0.5 * (at.horizontal ? t.len_h : t.len_v), fluxH, fluxC, rate, fluxMix);
+}
+
+// Fluxes and rate of one edge. The Gauss points are taken as the centre and
+// two symmetric pairs, whose values share their even part. With every point
+// tested, clipped and divided through the library, in a loop that carried the
+// boundary policy, the kernel issued 2909 instructions per warp, 969 of them
+// FP64, and took 219 us at 640x1280; so 1201, 474 and 125 us. Bound by the
+// latency of the phase evaluation's chain and the records' loads together
+// (issue 48 %, FP64 pipe 38 %, DRAM 3.6 TB/s).
+template <bool kExt>
+__device__ __forceinline__ void face_edge(const StageHot& t, const FaceArgs& a, const Physics& ph, const EdgeAt& at) {
+    const EdgeCells g = edge_cells(a, at);
+    const size_t N = (size_t)a.nx * a.ny;
+    MP_CHECK_INDEX(a.status, g.L, N);
+    if (!g.boundary) MP_CHECK_INDEX(a.status, g.R, N);
+    const unsigned char fl = a.flags[g.L] & (g.boundary ? 0xff : a.flags[g.R]);
+    if (!(fl & FLAG_PLAIN)) { face_general<kExt>(t, a, ph, g.e); return; }
+    if (g.boundary) { face_wall<kExt>(t, a, ph, g.e); return; }
+    const bool wet = (fl & FLAG_WET) != 0;
+    double hL[3], cL[3], hR[3], cR[3];
+    edge_line(a, N, g.L, at.horizontal, at.horizontal ? -1.0 : 1.0, hL, cL);
+    edge_line(a, N, g.R, at.horizontal, at.horizontal ? 1.0 : -1.0, hR, cR);
+    double fluxH = 0.0, fluxC = 0.0, fluxMix = 0.0, rate = 0.0;
+    int st = 0;
+#pragma unroll 1
+    for (int p = 0; p < 3; ++p) {
+        const double x = t.g[2 + p], x2 = x * x, w = t.gw[2 + p];
+        const double eHL = fma(hL[2], x2, hL[0]), eCL = fma(cL[2], x2, cL[0]);
+        const double eHR = fma(hR[2], x2, hR[0]), eCR = fma(cR[2], x2, cR[0]);
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            if (m == 1 && p == 0) break;
+            const double s = m ? -x : x;
+            const long long v = g.e * kNQ + (m ? 2 - p : 2 + p);
+            const double vs = __ldg(a.vsn + v), ud = __ldg(a.udn + v);
+            const double tep = !(kExt && ph.litho) ? ph.Tep
+                             : tep_at(ph, at.horizontal ? t.y0 + (a.gj0 + at.j) * t.dy : height(t, a.gj0 + at.j, s));
+            const double cl = fma(cL[1], s, eCL), cr = fma(cR[1], s, eCR);
+            PhaseLean A, B;
+            phase_plain<true>(ph.sk, fma(hL[1], s, eHL), cl, tep, A);
+            phase_plain<true>(ph.sk, fma(hR[1], s, eHR), cr, tep, B);
+            const PointFlux pf = face_point_plain(ph, A, B, cl, cr, wet, vs, ud, st);
+            fluxH = fma(w, pf.fh, fluxH);
+            fluxC = fma(w, pf.fc, fluxC);
+            fluxMix = fma(w, pf.vn, fluxMix);
+            rate = fma(w, pf.speed, rate);
+        }
+    }
+    if (st) record_error(a.status, PART_FACES, g.L + (long long)a.gj0 * a.nx, st);
+    store_face(a, g.e, 0.5 * (at.horizontal ? t.len_h : t.len_v), fluxH, fluxC, rate, fluxMix);
 }
 
 // ------------------------------------------------------------- diffusion

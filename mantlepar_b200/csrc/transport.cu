@@ -61,8 +61,10 @@ struct SourceBufs {
 // Single-instance kernels: one thread per cell / edge.
 // The stage tables arrive by value as a __grid_constant__ parameter, so the
 // unrolled table coefficients are constant-bank operands. Minimum resident
-// blocks per SM (register caps) as measured fastest on B200: cell phase 8,
-// faces 5; the reconstruction keeps its natural register count.
+// blocks per SM (register caps) as measured fastest on B200: cell phase 6
+// (48 us at 640x1280; 8: 55, 5: 51),
+// faces 5 (127; 4: 133, 6: 129); the reconstruction keeps its natural register
+// count (87 us; 5 and 6 blocks the same).
 // Rows [jlo, jhi) are reconstructed (all rows, or a slab's owned rows +- 1).
 __global__ void __launch_bounds__(128) recon_kernel(const __grid_constant__ ReconArgs a,
                                                     const __grid_constant__ Physics ph,
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(128) recon_kernel(const __grid_constant__ Reco
     if (j < jhi) recon_cell(p.d, a, ph, blockIdx.x * blockDim.x + threadIdx.x, j);
 }
 template <bool kExt>
-__global__ void __launch_bounds__(128, 8) cellphase_kernel(const __grid_constant__ CellPhaseArgs a,
+__global__ void __launch_bounds__(128, 6) cellphase_kernel(const __grid_constant__ CellPhaseArgs a,
                                                            const __grid_constant__ Physics ph,
                                                            const __grid_constant__ ParamTables p, long long c0,
                                                            long long c1) {
@@ -82,8 +84,8 @@ __global__ void __launch_bounds__(128, 8) cellphase_kernel(const __grid_constant
 }
 // Edges [h0, h0 + nh) (horizontal) then [v0, v0 + nv) (vertical): every edge
 // of the mesh, or of a slab's owned cells.
-// kRange: the edges of a slab's owned rows (two ranges); otherwise every
-// edge of the mesh with the plain linear mapping (measurably faster).
+// kRange: the edges of a slab's owned rows (two ranges, in id order);
+// otherwise every edge of the mesh, the walls last.
 template <bool kExt, bool kRange>
 __global__ void __launch_bounds__(128, 5) face_kernel(const __grid_constant__ FaceArgs a,
                                                       const __grid_constant__ Physics ph,
@@ -91,12 +93,10 @@ __global__ void __launch_bounds__(128, 5) face_kernel(const __grid_constant__ Fa
                                                       long long v0, long long nv) {
     if (gated_off(a.gate)) return;
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if constexpr (kRange) {
-        // One call site: the edge body is inlined once.
-        if (k < nh + nv) face_edge<kExt>(p.d, a, ph, k < nh ? h0 + k : v0 + (k - nh));
-    } else {
-        face_edge<kExt>(p.d, a, ph, k);
-    }
+    if (k >= nh + nv) return;
+    // One call site: the edge body is inlined once.
+    face_edge<kExt>(p.d, a, ph, kRange ? edge_by_id(a.nx, a.ny, k < nh ? h0 + k : v0 + (k - nh))
+                                       : edge_by_kind(a.nx, a.ny, k));
 }
 // The diffusive part of the same edges (only launched when diffusion is on).
 __global__ void __launch_bounds__(128) diffusion_kernel(const __grid_constant__ FaceArgs a,

@@ -60,3 +60,35 @@ def test_reconstruction_and_limiter(nx, ny, scale):
     assert per_cell(got["T"], ref["T"]) <= 1e-12
     for k in ("rhsH", "rhsC"):
         assert np.max(np.abs(got[k] - ref[k])) <= 1e-12 * np.max(np.abs(ref[k]))
+
+
+def patchy_state(w):
+    """Columns of pure component (C = 0), of eutectic composition (C = Xe) and
+    ordinary ones, two-solid to solid + liquid: cells that take the tested
+    phase evaluation beside cells that do not need it, and the edges between."""
+    i = np.arange(w.cells) % w.nx
+    band = (3 * i) // w.nx
+    C = np.where(band == 0, 0.0, np.where(band == 1, 0.3 + 0.02 * sy.unit_noise(w.seed, 1, np.arange(w.cells, dtype=np.uint64)), 0.5))
+    H = 0.05 + 0.6 * (np.arange(w.cells) // w.nx + 0.5) / w.ny + 0.03 * sy.unit_noise(w.seed, 0, np.arange(w.cells, dtype=np.uint64))
+    return H, C
+
+
+@pytest.mark.parametrize("config", [{}, {"theta": 2.0}, {"lf_global": 1, "lf_global_speed": 1.0}, {"C_policy": 2}, {"H_policy": 2}],
+                         ids=["plain", "darcy_exponent", "global_lf", "zero_flux_C", "zero_flux_H"])
+@pytest.mark.parametrize("nx,ny", [(4, 3), (37, 11)])
+def test_faces_of_mixed_cells_and_walls(nx, ny, config):
+    w = sy.Workload(nx=nx, ny=ny, seed=7)
+    t, o = pair(w, inflow_H=0.6, inflow_C=0.31, **config)
+    H, C = patchy_state(w)
+    vs, ud = sy.face_velocity(w)
+    vs = vs.copy()
+    vs[: nx * (ny + 1)] += 0.05            # through-flow: inflow at one wall, outflow at the other
+    for x in (t, o):
+        x.set_state(H, C)
+        x.set_face_velocity(vs, ud)
+    got, (code, ref) = t.rhs(), o.rhs()
+    assert code == 0
+    assert per_cell(got["T"], ref["T"]) <= 1e-12
+    assert per_cell(got["phi"], ref["phi"]) <= 1e-12
+    for k in ("rhsH", "rhsC", "rate"):
+        assert np.max(np.abs(got[k] - ref[k])) <= 1e-12 * np.max(np.abs(ref[k]))
