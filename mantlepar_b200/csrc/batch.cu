@@ -138,12 +138,13 @@ __global__ void __launch_bounds__(128, 4) batch_quad_phase_kernel(const QuadStag
     if (cell < (long long)a.nx * a.ny) quad_cellphase_cell(a, ph, cell);
 }
 
-__global__ void __launch_bounds__(128, 4) batch_quad_face_kernel(const QuadStageArgs* args, const Work* work,
+__global__ void __launch_bounds__(128, 5) batch_quad_face_kernel(const QuadStageArgs* args, const Work* work,
                                                                  const int* active, const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
-    const long long e = (long long)w.a + threadIdx.x;
-    if (e < w.b) quad_face_edge(args[w.inst], ph, e);
+    const long long k = (long long)w.a + threadIdx.x;
+    const QuadStageArgs& a = args[w.inst];
+    if (k < w.b) quad_face_edge(a, ph, edge_by_kind(a.nx, a.ny, k));
 }
 
 __global__ void __launch_bounds__(128) batch_quad_diffusion_kernel(const QuadStageArgs* args, const Work* work,

@@ -71,6 +71,27 @@ __device__ __forceinline__ CellFrame cell_frame(const QuadDev& q, int nx, size_t
     return f;
 }
 
+// The bilinear map of a cell in its own frame: x(r, s) = m + b r + c s + d r s.
+struct NormalCell {
+    P2 n[4];               // corners
+    P2 m, b, c, d;
+};
+__device__ __forceinline__ NormalCell normal_cell(const CellFrame& f) {
+    NormalCell k;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) k.n[v] = P2{(f.c[v].x - f.cx) * f.inv_h, (f.c[v].y - f.cy) * f.inv_h};
+    auto quarter = [&](double s1, double s2, double s3) {
+        return P2{0.25 * (k.n[0].x + s1 * k.n[1].x + s2 * k.n[2].x + s3 * k.n[3].x),
+                  0.25 * (k.n[0].y + s1 * k.n[1].y + s2 * k.n[2].y + s3 * k.n[3].y)};
+    };
+    k.m = quarter(1.0, 1.0, 1.0);
+    k.d = quarter(-1.0, 1.0, -1.0);
+    const P2 b = quarter(-1.0, -1.0, 1.0), c = quarter(1.0, -1.0, -1.0);
+    k.b = P2{-b.x, -b.y};
+    k.c = P2{-c.x, -c.y};
+    return k;
+}
+
 // Edge e of cell (i, j) in counter-clockwise order (0 bottom, 1 right, 2 top,
 // 3 left): its local edge id, whether it is a wall, and whether the cell's
 // point order runs against the canonical one. Local rows j of a mesh whose
@@ -317,40 +338,46 @@ __device__ __forceinline__ int reconstruct_quad(const QuadDev& q, size_t N, long
 // Left/right cells and oriented vertices of edge e (evolve.cpp:230-251).
 struct QuadEdge {
     bool horizontal, boundary, reverse;
-    long long L, R;
+    long long e, L, R;
     int wall;
     P2 a, b;
 };
-__device__ __forceinline__ QuadEdge quad_edge(const QuadDev& q, int nx, int ny, int gj0, int gny, long long e) {
-    const long long nI = (long long)nx * (ny + 1);
+__device__ __forceinline__ QuadEdge quad_edge(const QuadDev& q, int nx, int ny, int gj0, int gny, bool horizontal, int i,
+                                              int j) {
     QuadEdge g;
     g.R = -1;
     g.wall = -1;
+    g.horizontal = horizontal;
     P2 v0, v1;
-    if (e < nI) {
-        const int i = (int)(e % nx), j = (int)(e / nx);
+    if (horizontal) {
         const int gj = gj0 + j;
-        g.horizontal = true;
+        g.e = (long long)j * nx + i;
         g.boundary = gj == 0 || gj == gny;
         g.reverse = gj == gny;
-        g.L = g.reverse ? (long long)(j - 1) * nx + i : (long long)j * nx + i;
-        if (!g.boundary) g.R = (long long)(j - 1) * nx + i;
+        g.L = g.reverse ? g.e - nx : g.e;
+        if (!g.boundary) g.R = g.e - nx;
         else g.wall = gj == 0 ? 0 : 1;
         v0 = vtx(q, nx, i, j); v1 = vtx(q, nx, i + 1, j);
     } else {
-        const long long k = e - nI;
-        const int i = (int)(k % (nx + 1)), j = (int)(k / (nx + 1));
-        g.horizontal = false;
+        const long long row = (long long)j * nx;
+        g.e = (long long)nx * (ny + 1) + row + j + i;
         g.boundary = i == 0 || i == nx;
         g.reverse = i == 0;
-        g.L = g.reverse ? (long long)j * nx : (long long)j * nx + (i - 1);
-        if (!g.boundary) g.R = (long long)j * nx + i;
+        g.L = g.reverse ? row : row + (i - 1);
+        if (!g.boundary) g.R = row + i;
         else g.wall = i == 0 ? 2 : 3;
         v0 = vtx(q, nx, i, j); v1 = vtx(q, nx, i, j + 1);
     }
     g.a = g.reverse ? v1 : v0;
     g.b = g.reverse ? v0 : v1;
     return g;
+}
+// Edge e in id order.
+__device__ __forceinline__ QuadEdge quad_edge(const QuadDev& q, int nx, int ny, int gj0, int gny, long long e) {
+    const long long nI = (long long)nx * (ny + 1);
+    const bool horizontal = e < nI;
+    const unsigned k = (unsigned)(horizontal ? e : e - nI), w = (unsigned)(horizontal ? nx : nx + 1);
+    return quad_edge(q, nx, ny, gj0, gny, horizontal, (int)(k % w), (int)(k / w));
 }
 
 }  // namespace

@@ -92,3 +92,34 @@ def test_faces_of_mixed_cells_and_walls(nx, ny, config):
     assert per_cell(got["phi"], ref["phi"]) <= 1e-12
     for k in ("rhsH", "rhsC", "rate"):
         assert np.max(np.abs(got[k] - ref[k])) <= 1e-12 * np.max(np.abs(ref[k]))
+
+
+@pytest.mark.parametrize("family", [1, 2], ids=["perturbed", "stretched"])
+@pytest.mark.parametrize("config", [{}, {"theta": 2.0}, {"lf_global": 1, "lf_global_speed": 1.0}, {"H_policy": 2}],
+                         ids=["plain", "darcy_exponent", "global_lf", "zero_flux_H"])
+@pytest.mark.parametrize("nx,ny", [(2, 3), (35, 9)])
+def test_quad_mesh_of_mixed_cells_and_walls(nx, ny, config, family):
+    from mantlepar_b200.transport import Transport, TransportConfig
+    from oracle import pyoracle as po
+    w = sy.Workload(nx=nx, ny=ny, seed=7)
+    bc = dict(inflow_H=0.6, inflow_C=0.31, **config)
+    o = po.TransportOracle(sy.material_s(), w, lib=po.restated(), integrator=3, mesh_family=family, perturbation=0.2,
+                           mesh_seed=11, **bc)
+    xy = o.vertices()
+    t = Transport(w, TransportConfig(cfl=w.cfl, integrator=3, **bc), vertices=xy)
+    vs, ud = sy.face_velocity_quads(w, xy)
+    vs = vs + 0.05 * (ud / w.darcy)
+    H, C = patchy_state(w)
+    for x in (t, o):
+        x.set_state(H, C)
+        x.set_face_velocity(vs, ud)
+    got, (code, ref) = t.rhs(), o.rhs()
+    assert code == 0
+    assert per_cell(got["T"], ref["T"]) <= 1e-12
+    assert per_cell(got["phi"], ref["phi"]) <= 1e-12
+    for k in ("rhsH", "rhsC", "rate"):
+        assert np.max(np.abs(got[k] - ref[k])) <= 1e-12 * np.max(np.abs(ref[k]))
+    code, *factors = o.limiter()
+    assert code == 0
+    for g, r in zip(t.limiter(), factors):
+        assert np.max(np.abs(g - r)) <= 1e-11
