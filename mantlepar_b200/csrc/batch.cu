@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(128) batch_diffusion_kernel(const InstArgs* ar
 
 // General quad meshes: the per-element bodies of the single-mesh quad
 // kernels (quad_kernels.cuh) over the quad instances' work lists.
-__global__ void __launch_bounds__(128, 3) batch_quad_weno_kernel(const QuadStageArgs* args, const Work* work,
+__global__ void __launch_bounds__(128, 2) batch_quad_weno_kernel(const QuadStageArgs* args, const Work* work,
                                                                  const int* active) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
@@ -426,7 +426,7 @@ mp_status alloc_quad_instance(mp_batch* b, MPInstance& in, const mp_mesh_desc& m
         }
         return cuda_status(ce, "mp_batch_add_quads");
     }
-    in.qbytes = ((size_t)(kQG0 + kQS9 + kQT4 + kQS4 + kQGeo) * N + qt.xy.size() + qt.spacing.size()) * sizeof(double);
+    in.qbytes = ((size_t)(kQG0 + kQT4 + kQMom + kQGeo) * N + qt.xy.size() + qt.spacing.size()) * sizeof(double);
     in.cell_area = in.qdev.geo + 3 * N;
     in.quad = true;
     in.used = true;

@@ -132,30 +132,20 @@ __device__ __forceinline__ void visit_samples(const QuadDev& q, int nx, int ny, 
     }
 }
 
-// Folded smoothness row offsets: entry (r, c >= r) of an n x n form.
-__device__ __forceinline__ int fold_at(int n, int r, int c) { return r * n - (r * (r - 1)) / 2 + (c - r); }
-
-// smoothness<>'s decision for a chain that failed its range test (roundoff
-// at sigma ~ 0, or bad data), out of line: form n x n, folded entries at
-// base[k * stride].
-template <int NN>
-__device__ __noinline__ double smoothness_out_of_line(const double* base, size_t stride, const double* diff) {
-    auto SF = [&](int k) { return __ldg(base + (size_t)k * stride); };
-    auto S = [&](int r, int c) { const double v = SF(fold_at(NN, r, c)); return r == c ? v : 0.5 * v; };
-    return smoothness<double, NN>(SF, S, diff);
-}
-
 // The deviation polynomials D[f] of F fields from their 3x3 neighbourhoods
-// u[f] with the cell's own tables (same candidate set, weights and clipping
-// as reconstruct() of the uniform path). The fields share the cell's
-// stencils and so its tables: every table entry is read once and applied to
-// each field, and per field the operations run in the same order whatever F
-// is, so a field's result does not depend on the fields reconstructed with
-// it. For F > 1 smoothness<>'s FMA chains are formed here for all fields at
-// once, and a chain that fails its range test is decided by smoothness<> out
-// of line (it forms the same chain again, then the term-by-term sum), so
-// that the rare path does not cost the multi-field form registers; F = 1
-// calls smoothness<> inline. Returns the first failure in field order.
+// u[f] with the cell's own tables (same candidate set and weights as
+// reconstruct() of the uniform path). The fields share the cell's stencils
+// and so its tables: every entry is read once and applied to each field, and
+// per field the operations run in the same order whatever F is, so a field's
+// result does not depend on the fields reconstructed with it. The kernel is
+// bound by the bytes of the tables: the coefficients of each candidate are
+// formed once, the smoothness indicators as sums of squares from them and the
+// cell's six moments (quad_tables.hpp; 115 doubles per cell), and a 2x2
+// candidate's constant from its zero mean over the target; reading the folded
+// smoothness matrices and the constants as well (181 doubles) took 278 us at
+// 640x1280, so it takes 155 (two resident blocks of 255 registers, every
+// table load of a cell in flight; three blocks 176, four 228). Tables of candidates that are off are zero. Returns the first
+// failure in field order.
 template <int F>
 __device__ __forceinline__ int reconstruct_quad(const QuadDev& q, size_t N, long long cell, int ci, int cj,
                                                 double eA, const double (&u)[F][3][3], double (&D)[F][9]) {
@@ -166,173 +156,111 @@ __device__ __forceinline__ int reconstruct_quad(const QuadDev& q, size_t N, long
         for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int b = 0; b < 3; ++b) d[f][a][b] = u[f][a][b] - u[f][1][1];
-    const int offi[4] = {0, 0, -1, -1}, offj[4] = {-1, 0, -1, 0};
-    bool on[5];
-    on[0] = (ci == 1 && cj == 1);
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        on[k + 1] = !((offi[k] == 0 && ci == 2) || (offi[k] == -1 && ci == 0) || (offj[k] == 0 && cj == 2) ||
-                      (offj[k] == -1 && cj == 0));
-    double sg[F][5];
-    int st[F];
-#pragma unroll
-    for (int f = 0; f < F; ++f) st[f] = 0;
-    auto fast_ok = [](double v) { return v >= 0.0 && v < INFINITY; };
-    if (on[0]) {
-        double fd[F][8];
-#pragma unroll
-        for (int f = 0; f < F; ++f)
-#pragma unroll
-            for (int c = 1; c < 9; ++c) fd[f][c - 1] = d[f][c / 3][c % 3] - d[f][0][0];
-        auto SF = [&](int k) { return __ldg(q.S9 + (size_t)k * N + cell); };
-        auto S = [&](int r, int c) { const double v = SF(fold_at(8, r, c)); return r == c ? v : 0.5 * v; };
-        if constexpr (F == 1) {
-            sg[0][0] = smoothness<double, 8>(SF, S, fd[0]);
-        } else {
-            double sum[F];
-#pragma unroll
-            for (int f = 0; f < F; ++f) sum[f] = 0;
-            int k = 0;
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const double s0 = SF(k++);
-                double t[F];
-#pragma unroll
-                for (int f = 0; f < F; ++f) t[f] = s0 * fd[f][r];
-#pragma unroll
-                for (int c = r + 1; c < 8; ++c) {
-                    const double sv = SF(k++);
-#pragma unroll
-                    for (int f = 0; f < F; ++f) t[f] = fma(sv, fd[f][c], t[f]);
-                }
-#pragma unroll
-                for (int f = 0; f < F; ++f) sum[f] = fma(fd[f][r], t[f], sum[f]);
-            }
-#pragma unroll
-            for (int f = 0; f < F; ++f)
-                sg[f][0] = fast_ok(sum[f]) ? sum[f] : smoothness_out_of_line<8>(q.S9 + cell, N, fd[f]);
-        }
-#pragma unroll
-        for (int f = 0; f < F; ++f)
-            if (sg[f][0] < 0.0) st[f] = MP_ERR_FP;
-    } else {
-#pragma unroll
-        for (int f = 0; f < F; ++f) sg[f][0] = 0;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (!on[k + 1]) {
-#pragma unroll
-            for (int f = 0; f < F; ++f) sg[f][k + 1] = 0;
-            continue;
-        }
-        const int oi = offi[k], oj = offj[k];
-        double fd[F][3];
-#pragma unroll
-        for (int f = 0; f < F; ++f) {
-            const double a0 = d[f][1 + oj][1 + oi];
-#pragma unroll
-            for (int c = 1; c < 4; ++c) fd[f][c - 1] = d[f][1 + oj + c / 2][1 + oi + c % 2] - a0;
-        }
-        auto SF = [&](int m) { return __ldg(q.S4 + (size_t)(k * 6 + m) * N + cell); };
-        auto S = [&](int r, int c) { const double v = SF(fold_at(3, r, c)); return r == c ? v : 0.5 * v; };
-        if constexpr (F == 1) {
-            sg[0][k + 1] = smoothness<double, 3>(SF, S, fd[0]);
-        } else {
-            double sum[F];
-#pragma unroll
-            for (int f = 0; f < F; ++f) sum[f] = 0;
-            int m = 0;
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                const double s0 = SF(m++);
-                double t[F];
-#pragma unroll
-                for (int f = 0; f < F; ++f) t[f] = s0 * fd[f][r];
-#pragma unroll
-                for (int c = r + 1; c < 3; ++c) {
-                    const double sv = SF(m++);
-#pragma unroll
-                    for (int f = 0; f < F; ++f) t[f] = fma(sv, fd[f][c], t[f]);
-                }
-#pragma unroll
-                for (int f = 0; f < F; ++f) sum[f] = fma(fd[f][r], t[f], sum[f]);
-            }
-#pragma unroll
-            for (int f = 0; f < F; ++f)
-                sg[f][k + 1] = fast_ok(sum[f]) ? sum[f]
-                                               : smoothness_out_of_line<3>(q.S4 + (size_t)k * 6 * N + cell, N, fd[f]);
-        }
-#pragma unroll
-        for (int f = 0; f < F; ++f)
-            if (sg[f][k + 1] < 0.0) st[f] = MP_ERR_FP;
-    }
-    double w[F][5];
+    auto mom = [&](int k) { return __ldg(q.mom + (size_t)k * N + cell); };
+    const unsigned on = candidate_mask(ci, cj);
     const double ie = 1.0 / eA;
-    const unsigned mask = candidate_mask(ci, cj);
+    // 3x3 candidate in the target's frame.
 #pragma unroll
     for (int f = 0; f < F; ++f) {
-        double s[5];
+        D[f][0] = d[f][0][0];
 #pragma unroll
-        for (int k = 0; k < 5; ++k) s[k] = fma(sg[f][k], ie, 1.0);
-        if (weno_weights(s, mask, eA * eA, w[f])) st[f] = MP_ERR_FP;
+        for (int m = 1; m < 9; ++m) D[f][m] = 0.0;
     }
 #pragma unroll
-    for (int f = 0; f < F; ++f)
+    for (int c = 1; c < 9; ++c) {
+        double x[F];
 #pragma unroll
-        for (int mm = 0; mm < 9; ++mm) D[f][mm] = 0;
-    if (on[0]) {
-        double fd[F][8];
+        for (int f = 0; f < F; ++f) x[f] = d[f][c / 3][c % 3] - d[f][0][0];
+#pragma unroll
+        for (int m = 0; m < 9; ++m) {
+            const double g = __ldg(q.G0 + (size_t)((c - 1) * 9 + m) * N + cell);
+#pragma unroll
+            for (int f = 0; f < F; ++f) D[f][m] = fma(x[f], g, D[f][m]);
+        }
+    }
+    double s[F][5];
+    {
+        // Its sigma over the unit square of the stencil's frame, whose
+        // coordinates are the target's plus (dx, dy): the coefficients moved
+        // back (monomial j*3 + i; the constant is not needed), then the
+        // closed form of tables.hpp with Xh = Yh = 1.
+        const double dx = mom(0), dy = mom(1);
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+            const double* p = D[f];
+            // Along x: c1 = p1 - 2 dx p2, c0 = p0 - dx p1 + dx^2 p2.
+            const double r01 = fma(-2.0 * dx, p[2], p[1]);
+            const double r11 = fma(-2.0 * dx, p[5], p[4]), r10 = fma(-dx, fma(-dx, p[5], p[4]), p[3]);
+            const double r21 = fma(-2.0 * dx, p[8], p[7]), r20 = fma(-dx, fma(-dx, p[8], p[7]), p[6]);
+            // Along y, per power of x.
+            const double q01 = fma(-2.0 * dy, r20, r10), q02 = r20;
+            const double q10 = fma(-dy, fma(-dy, r21, r11), r01), q11 = fma(-2.0 * dy, r21, r11), q12 = r21;
+            const double q20 = fma(-dy, fma(-dy, p[8], p[5]), p[2]), q21 = fma(-2.0 * dy, p[8], p[5]), q22 = p[8];
+            const double c = 1.0 / 12.0;
+            const double t1 = fma(c, q12, q10), t2 = fma(c, q21, q01), t3 = fma(c, q22, q20), t4 = fma(c, q22, q02);
+            double a = t1 * t1, b = t2 * t2;
+            a = fma((13.0 / 3.0) * t3, t3, a);
+            b = fma((13.0 / 3.0) * t4, t4, b);
+            a = fma((7.0 / 6.0) * q11, q11, a);
+            b = fma(0.7 * q12, q12, b);
+            a = fma(0.7 * q21, q21, a);
+            b = fma((43.0 / 270.0) * q22, q22, b);
+            s[f][0] = fma(a + b, ie, 1.0);
+        }
+    }
+    // 2x2 candidates: slopes b1, b2 and mixed coefficient b3; sigma is the
+    // mean over the target of (b1 + b3 y)^2 + (b2 + b3 x)^2.
+    const double mx = mom(2), my = mom(3), mxy = mom(4), var = mom(5);
+    const int offi[4] = {0, 0, -1, -1}, offj[4] = {-1, 0, -1, 0};
+    double b[F][4][3];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int oi = offi[k], oj = offj[k];
 #pragma unroll
         for (int f = 0; f < F; ++f)
 #pragma unroll
-            for (int c = 1; c < 9; ++c) fd[f][c - 1] = d[f][c / 3][c % 3] - d[f][0][0];
+            for (int m = 0; m < 3; ++m) b[f][k][m] = 0.0;
 #pragma unroll
-        for (int mm = 0; mm < 9; ++mm) {
-            double v[F];
+        for (int c = 1; c < 4; ++c) {
+            double x[F];
 #pragma unroll
-            for (int f = 0; f < F; ++f) v[f] = mm == 0 ? d[f][0][0] : 0.0;
+            for (int f = 0; f < F; ++f) x[f] = d[f][1 + oj + c / 2][1 + oi + c % 2] - d[f][1 + oj][1 + oi];
 #pragma unroll
-            for (int c = 1; c < 9; ++c) {
-                const double g = __ldg(q.G0 + (size_t)((c - 1) * 9 + mm) * N + cell);
+            for (int m = 0; m < 3; ++m) {
+                const double tv = __ldg(q.T4 + (size_t)(k * 12 + (c - 1) * 4 + m + 1) * N + cell);
 #pragma unroll
-                for (int f = 0; f < F; ++f) v[f] += fd[f][c - 1] * g;
+                for (int f = 0; f < F; ++f) b[f][k][m] = fma(x[f], tv, b[f][k][m]);
             }
-#pragma unroll
-            for (int f = 0; f < F; ++f) D[f][mm] = w[f][0] * v[f];
         }
-    }
-    const int slot[4] = {0, 1, 3, 4};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (!on[k + 1]) continue;
-        const int oi = offi[k], oj = offj[k];
-        double a0[F], fd[F][3];
 #pragma unroll
         for (int f = 0; f < F; ++f) {
-            a0[f] = d[f][1 + oj][1 + oi];
-#pragma unroll
-            for (int c = 1; c < 4; ++c) fd[f][c - 1] = d[f][1 + oj + c / 2][1 + oi + c % 2] - a0[f];
-        }
-#pragma unroll
-        for (int mm = 0; mm < 4; ++mm) {
-            double v[F];
-#pragma unroll
-            for (int f = 0; f < F; ++f) v[f] = mm == 0 ? a0[f] : 0.0;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const double tv = __ldg(q.T4 + (size_t)(k * 12 + c * 4 + mm) * N + cell);
-#pragma unroll
-                for (int f = 0; f < F; ++f) v[f] += fd[f][c] * tv;
-            }
-#pragma unroll
-            for (int f = 0; f < F; ++f) D[f][slot[mm]] += w[f][k + 1] * v[f];
+            const double gx = fma(b[f][k][2], my, b[f][k][0]), gy = fma(b[f][k][2], mx, b[f][k][1]);
+            s[f][k + 1] = fma(fma(var * b[f][k][2], b[f][k][2], fma(gy, gy, gx * gx)), ie, 1.0);
         }
     }
+    int st = 0;
 #pragma unroll
-    for (int f = 0; f < F; ++f)
-        if (st[f]) return st[f];
-    return 0;
+    for (int f = 0; f < F; ++f) {
+        if (on != 31u) {
+#pragma unroll
+            for (int k = 0; k < 5; ++k) s[f][k] = (on >> k) & 1u ? s[f][k] : 1.0;
+        }
+        double w[5];
+        const int s1 = weno_weights(s[f], on, eA * eA, w);
+        st = st ? st : s1;
+#pragma unroll
+        for (int m = 0; m < 9; ++m) D[f][m] = on & 1u ? D[f][m] * w[0] : 0.0;
+        double g[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int m = 0; m < 3; ++m) g[m] = fma(w[k + 1], b[f][k][m], g[m]);
+        D[f][0] -= fma(g[0], mx, fma(g[1], my, g[2] * mxy));
+        D[f][1] += g[0];
+        D[f][3] += g[1];
+        D[f][4] += g[2];
+    }
+    return st;
 }
 
 // Left/right cells and oriented vertices of edge e (evolve.cpp:230-251).

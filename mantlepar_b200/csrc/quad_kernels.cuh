@@ -3,7 +3,7 @@
 // stencil geometry (src/core/mesh.cpp:27-55; src/mlweno/reconstruction.cpp:
 // 109-210). Same stage as the uniform kernels (src/couple/evolve.cpp:279-384),
 // with
-//   * per-cell candidate matrices and smoothness forms read from HBM
+//   * per-cell candidate matrices and cell moments read from HBM
 //     (quad_tables.hpp) instead of one table set in the kernel parameters;
 //   * every evaluation point mapped from the cell's corners (bilinear map,
 //     edge interpolation, normal-line samples with per-edge spacing) into the
@@ -93,7 +93,7 @@ __device__ __forceinline__ void quad_weno_cell(const QuadStageArgs& a, int i, in
     }
     if (st) record_error(status, PART_UPDATE, cell + (long long)gj0 * nx, st);
 }
-__global__ void __launch_bounds__(128, 3) quad_weno_kernel(const __grid_constant__ QuadStageArgs a, int jlo, int jhi,
+__global__ void __launch_bounds__(128, 2) quad_weno_kernel(const __grid_constant__ QuadStageArgs a, int jlo, int jhi,
                                                            const int* gate) {
     if (gated_off(gate)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x, j = jlo + (int)(blockIdx.y * blockDim.y + threadIdx.y);

@@ -143,7 +143,8 @@ __device__ void smoothness(const DV2* nc, const Rules& R, int order, const doubl
 
 // Basis coefficients coef[cell*n + m] of the S x S stencil with lower-left
 // cell (I0, J0), normalised by h, its centre, and (ti >= 0) the smoothness
-// form on its cell (ti, tj); without a target cell, on the reference square.
+// form on its cell (ti, tj); without a target cell, on the reference square
+// (form null: neither).
 template <int S>
 __device__ bool stencil(const double* xy, int nx, int I0, int J0, int order, double h, int ti, int tj, const Rules& R,
                         double* coef, double* form, DV2& center) {
@@ -167,6 +168,7 @@ __device__ bool stencil(const double* xy, int nx, int I0, int J0, int order, dou
     if (!solve_identity(n, M, X)) return false;
     for (int c = 0; c < n; ++c)
         for (int m = 0; m < n; ++m) coef[c * n + m] = X[m * n + c];
+    if (!form) return true;
     if (ti < 0) {
         const DV2 ref[4] = {DV2{-0.5, -0.5}, DV2{0.5, -0.5}, DV2{0.5, 0.5}, DV2{-0.5, 0.5}};
         smoothness<S>(ref, R, order, coef, form);
@@ -201,7 +203,7 @@ __global__ void __launch_bounds__(64) quad_table_kernel(int nx, int ny, const do
     if (ci == 1 && cj == 1) {
         double coef[81], sigma[81];
         DV2 center;
-        if (!stencil<3>(xy, nx, i - 1, j - 1, 2, h, -1, -1, R, coef, sigma, center)) { atomicExch(failed, 1); return; }
+        if (!stencil<3>(xy, nx, i - 1, j - 1, 2, h, -1, -1, R, coef, S9 ? sigma : nullptr, center)) { atomicExch(failed, 1); return; }
         const double dx = (c.x - center.x) / h, dy = (c.y - center.y) / h;
         // Binomial re-expansion of each basis polynomial into the cell's frame.
         const double bin[3][3] = {{1, 0, 0}, {1, 1, 0}, {1, 2, 1}};
@@ -218,7 +220,7 @@ __global__ void __launch_bounds__(64) quad_table_kernel(int nx, int ny, const do
                 }
         }
         int q = 0;
-        for (int r = 1; r < 9; ++r)
+        for (int r = 1; S9 && r < 9; ++r)
             for (int cc = r; cc < 9; ++cc) S9[(size_t)(q++) * N + cell] = cc == r ? sigma[r * 9 + r] : 2.0 * sigma[r * 9 + cc];
     }
     const int offi[4] = {0, 0, -1, -1}, offj[4] = {-1, 0, -1, 0};
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(64) quad_table_kernel(int nx, int ny, const do
         if (!on) continue;
         double coef[16], form[16];
         DV2 center;
-        if (!stencil<2>(xy, nx, i + oi, j + oj, 1, h, -oi, -oj, R, coef, form, center)) { atomicExch(failed, 1); return; }
+        if (!stencil<2>(xy, nx, i + oi, j + oj, 1, h, -oi, -oj, R, coef, S4 ? form : nullptr, center)) { atomicExch(failed, 1); return; }
         const double dx = (c.x - center.x) / h, dy = (c.y - center.y) / h;
         for (int s = 1; s < 4; ++s) {
             const double* a = coef + s * 4;
@@ -236,24 +238,75 @@ __global__ void __launch_bounds__(64) quad_table_kernel(int nx, int ny, const do
             for (int mm = 0; mm < 4; ++mm) T4[(size_t)(kk * 12 + (s - 1) * 4 + mm) * N + cell] = v[mm];
         }
         int q = 0;
-        for (int r = 1; r < 4; ++r)
+        for (int r = 1; S4 && r < 4; ++r)
             for (int cc = r; cc < 4; ++cc) S4[(size_t)(kk * 6 + q++) * N + cell] = cc == r ? form[r * 4 + r] : 2.0 * form[r * 4 + cc];
     }
 }
 
+// The moments of one cell (quad_tables.hpp). The 3-point rule is exact for
+// them: the integrands have degree 3 at most in each reference coordinate.
+__global__ void __launch_bounds__(128) quad_moment_kernel(int nx, int ny, const double* __restrict__ xy, int row0,
+                                                          int rows, Rules R, double* mom) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t N = (size_t)nx * rows, cell = (size_t)k;
+    if (k >= (long long)N) return;
+    const int i = (int)(k % nx), j = row0 + (int)(k / nx);
+    DV2 t[4];
+    cell_quad(xy, nx, i, j, t);
+    const double p[1] = {R.p1}, w[1] = {R.w1};
+    const double h = sqrt(cell_area(t, p, w, 1));
+    double off[2] = {0, 0};
+    for (int v = 0; v < 4; ++v) { off[0] += (t[v].x - t[0].x) / 4; off[1] += (t[v].y - t[0].y) / 4; }
+    const DV2 c{t[0].x + off[0], t[0].y + off[1]};
+    for (int v = 0; v < 4; ++v) t[v] = DV2{(t[v].x - c.x) / h, (t[v].y - c.y) / h};
+    double dx = 0, dy = 0;
+    if (i > 0 && i < nx - 1 && j > 0 && j < ny - 1) {
+        // Centre of the 3x3 stencil: the mean of its four outer corners.
+        const DV2 o[4] = {vtx(xy, nx, i - 1, j - 1), vtx(xy, nx, i + 2, j - 1), vtx(xy, nx, i + 2, j + 2), vtx(xy, nx, i - 1, j + 2)};
+        double oc[2] = {0, 0};
+        for (int v = 0; v < 4; ++v) { oc[0] += (o[v].x - o[0].x) / 4; oc[1] += (o[v].y - o[0].y) / 4; }
+        dx = (c.x - (o[0].x + oc[0])) / h;
+        dy = (c.y - (o[0].y + oc[1])) / h;
+    }
+    const double area = cell_area(t, R.p3, R.w3, 3);
+    const double mx = cell_moment(t, R.p3, R.w3, 3, 1, 0) / area, my = cell_moment(t, R.p3, R.w3, 3, 0, 1) / area;
+    const double mxy = cell_moment(t, R.p3, R.w3, 3, 1, 1) / area;
+    double var = 0;
+    for (int b = 0; b < 3; ++b)
+        for (int a = 0; a < 3; ++a) {
+            const DV2 x = bilinear(R.p3[a], R.p3[b], t);
+            var += R.w3[a] * R.w3[b] * jacobian(R.p3[a], R.p3[b], t) * ((x.x - mx) * (x.x - mx) + (x.y - my) * (x.y - my));
+        }
+    const double v[kQMom] = {dx, dy, mx, my, mxy, var / area};
+    for (int q = 0; q < kQMom; ++q) mom[(size_t)q * N + cell] = v[q];
+}
+
+Rules rules_of(const double* gq3, const double* gw3, double gq1, double gw1) {
+    Rules R;
+    for (int k = 0; k < 3; ++k) { R.p3[k] = gq3[k]; R.w3[k] = gw3[k]; }
+    R.p1 = gq1; R.w1 = gw1;
+    return R;
+}
+
 }  // namespace
+
+int build_quad_moments_gpu(int nx, int ny, const double* d_xy, int row0, int rows, const double* gq3, const double* gw3,
+                           double gq1, double gw1, double* mom, cudaStream_t stream) {
+    const size_t N = (size_t)nx * rows;
+    quad_moment_kernel<<<(unsigned)((N + 127) / 128), 128, 0, stream>>>(nx, ny, d_xy, row0, rows,
+                                                                        rules_of(gq3, gw3, gq1, gw1), mom);
+    return cudaGetLastError() == cudaSuccess ? MP_OK : MP_ERR_CUDA;
+}
 
 int build_quad_cell_tables_gpu(int nx, int ny, const double* d_xy, int row0, int rows, const double* gq3,
                                const double* gw3, double gq1, double gw1, double* G0, double* S9, double* T4,
                                double* S4, double* geo, int* d_failed, cudaStream_t stream) {
-    Rules R;
-    for (int k = 0; k < 3; ++k) { R.p3[k] = gq3[k]; R.w3[k] = gw3[k]; }
-    R.p1 = gq1; R.w1 = gw1;
+    const Rules R = rules_of(gq3, gw3, gq1, gw1);
     const size_t N = (size_t)nx * rows;
     const size_t counts[4] = {kQG0 * N, kQS9 * N, kQT4 * N, kQS4 * N};
     double* zero_ptrs[4] = {G0, S9, T4, S4};
     for (int k = 0; k < 4; ++k)
-        if (cudaMemsetAsync(zero_ptrs[k], 0, counts[k] * sizeof(double), stream) != cudaSuccess) return MP_ERR_CUDA;
+        if (zero_ptrs[k] && cudaMemsetAsync(zero_ptrs[k], 0, counts[k] * sizeof(double), stream) != cudaSuccess) return MP_ERR_CUDA;
     if (cudaMemsetAsync(d_failed, 0, sizeof(int), stream) != cudaSuccess) return MP_ERR_CUDA;
     quad_table_kernel<<<(unsigned)((N + 63) / 64), 64, 0, stream>>>(nx, ny, d_xy, row0, rows, R, G0, S9, T4, S4, geo,
                                                                    d_failed);
@@ -270,7 +323,7 @@ int upload_quad_tables(int nx, int ny, const double* xy, const QuadTables& qt, i
     *buf = nullptr;
     const size_t N = (size_t)nx * rows;
     const size_t V = qt.xy.size(), NEq = qt.spacing.size();
-    const size_t total = V + (size_t)(kQG0 + kQS9 + kQT4 + kQS4 + kQGeo) * N + NEq;
+    const size_t total = V + (size_t)(kQG0 + kQT4 + kQMom + kQGeo) * N + NEq;
     e = cudaMalloc((void**)buf, total * sizeof(double));
     if (e != cudaSuccess) *buf = nullptr;
     double* at = *buf;
@@ -280,12 +333,11 @@ int upload_quad_tables(int nx, int ny, const double* xy, const QuadTables& qt, i
         at += n;
         return p;
     };
-    double *G0, *S9, *T4, *S4, *geo;
+    double *G0, *T4, *mom, *geo;
     q.xy = put(&qt.xy, V);
     q.G0 = G0 = put(nullptr, (size_t)kQG0 * N);
-    q.S9 = S9 = put(nullptr, (size_t)kQS9 * N);
     q.T4 = T4 = put(nullptr, (size_t)kQT4 * N);
-    q.S4 = S4 = put(nullptr, (size_t)kQS4 * N);
+    q.mom = mom = put(nullptr, (size_t)kQMom * N);
     q.geo = geo = put(nullptr, (size_t)kQGeo * N);
     q.sp = put(&qt.spacing, NEq);
     for (int k = 0; k < 5; ++k) { q.gq[k] = qt.gq[k]; q.gw[k] = qt.gw[k]; q.dif_c_bnd[k] = qt.dif_c_bnd[k]; }
@@ -304,8 +356,10 @@ int upload_quad_tables(int nx, int ny, const double* xy, const QuadTables& qt, i
     }
     int gs = MP_OK;
     if (e == cudaSuccess)
-        gs = build_quad_cell_tables_gpu(nx, ny, d_all, row0, rows, qt.gq3, qt.gw3, qt.gq1, qt.gw1, G0, S9, T4, S4, geo,
-                                        d_failed, stream);
+        gs = build_quad_moments_gpu(nx, ny, d_all, row0, rows, qt.gq3, qt.gw3, qt.gq1, qt.gw1, mom, stream);
+    if (e == cudaSuccess && gs == MP_OK)
+        gs = build_quad_cell_tables_gpu(nx, ny, d_all, row0, rows, qt.gq3, qt.gw3, qt.gq1, qt.gw1, G0, nullptr, T4,
+                                        nullptr, geo, d_failed, stream);
     if (gs == MP_ERR_CUDA) {
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaErrorUnknown;

@@ -3,9 +3,8 @@
 // (TensorStencilPoly::Initialize, src/mlweno/tensorstencilpoly.cpp:146-231;
 // SetTargetSmoothness :383-398; Reconstruction::Initialize,
 // src/mlweno/reconstruction.cpp:109-210), so on a perturbed or stretched mesh
-// each cell carries its own candidate matrices. They are built once on the
-// host and kept in HBM as structure-of-arrays (entry k of cell c at
-// k*ncell + c).
+// each cell carries its own candidate matrices. They are built once and kept
+// in HBM as structure-of-arrays (entry k of cell c at k*ncell + c).
 //
 // Every candidate polynomial is re-expanded into the cell's own frame
 // xi = (x - c_t)/h, c_t the average of the cell's corners, h = sqrt(area), so
@@ -13,8 +12,14 @@
 // m = j*3 + i of xi^i eta^j:
 //   3x3 candidate  D[m] = d00 [m == 0] + sum_{c=1..8} (d_c - d_0) G0[c-1][m]
 //   2x2 candidate k  D[{0,1,3,4}][mm] += a0 [mm == 0] + sum_{c=1..3} (d_c - d_0) T4[k][c-1][mm]
-// with d the stencil values minus the target value, and the smoothness forms
-// folded to their upper triangles (entry (r, r) = S_rr, (r, c > r) = 2 S_rc).
+// with d the stencil values minus the target value. The smoothness forms of
+// both (sigma over the reference square of the 3x3 stencil's frame, over the
+// target cell for a 2x2 candidate) follow from the coefficients and six
+// numbers per cell, the moments `mom`: the target centre in the 3x3 stencil's
+// frame, and over the target cell in its own frame the means of x, y and xy
+// and the sum of the variances of x and y. The host builder also forms the
+// smoothness matrices, folded to their upper triangles (entry (r, r) = S_rr,
+// (r, c > r) = 2 S_rc).
 #ifndef MP_QUAD_TABLES_HPP
 #define MP_QUAD_TABLES_HPP
 
@@ -29,6 +34,7 @@ constexpr int kQS9 = 36;   // folded 8x8
 constexpr int kQT4 = 48;   // 4 candidates x 3 differences x 4 monomials
 constexpr int kQS4 = 24;   // 4 candidates x folded 3x3
 constexpr int kQGeo = 4;   // c_x, c_y, h, area
+constexpr int kQMom = 6;   // stencil-frame centre (2), means of x, y, xy, variance sum
 
 struct QuadTables {
     int nx = 0, ny = 0;
@@ -47,9 +53,8 @@ struct QuadTables {
 struct QuadDev {
     const double* xy;
     const double* G0;
-    const double* S9;
     const double* T4;
-    const double* S4;
+    const double* mom;
     const double* geo;
     const double* sp;
     double gq[5], gw[5];
@@ -76,9 +81,15 @@ int validate_quads(int nx, int ny, const double* xy, long long* bad);
 int build_quad_tables(int nx, int ny, const double* xy, int threads, QuadTables& t, int row0 = 0, int rows = -1,
                       bool cell_tables = true);
 
+// The moments `mom` (kQMom arrays of ncell = nx * rows cells) of the local
+// rows on the GPU, from the whole mesh's vertices. 0 or MP_ERR_CUDA.
+int build_quad_moments_gpu(int nx, int ny, const double* d_xy, int row0, int rows, const double* gq3, const double* gw3,
+                           double gq1, double gw1, double* mom, cudaStream_t stream);
+
 // The per-cell arrays of the same tables (identical values: the host
 // builder's arithmetic without FMA contraction) on the GPU, written into the
-// device arrays of ncell = nx * rows cells (layout as QuadTables); d_xy holds
+// device arrays of ncell = nx * rows cells (layout as QuadTables; S9 and S4
+// may be null: the smoothness matrices are not formed); d_xy holds
 // the whole mesh's vertices; d_failed is one device int of scratch.
 // Synchronous on `stream`. Returns 0, MP_ERR_ARG_WRONG (a singular stencil
 // or a cell without positive area) or MP_ERR_CUDA.

@@ -30,9 +30,6 @@ struct ParamTables {
 
 inline void make_param_tables(const StageTables& t, ParamTables& p) { p.d = t; }
 
-template <class R> __device__ __forceinline__ R eps_of();
-template <> __device__ __forceinline__ double eps_of<double>() { return 2.220446049250313e-16; }
-
 // 1/x for normal x with a normal reciprocal: the hardware's approximation
 // (relative error e below 2^-19.9) and one third-order Newton step
 // y (1 + e + e^2). Rounds to another double than 1.0 / x for 3 in 10^4
@@ -131,38 +128,6 @@ __device__ __forceinline__ void q2_col(const R* D, R x, R& b0, R& b1, R& b2) {
 }
 template <class R>
 __device__ __forceinline__ R quad(R c0, R c1, R c2, R s) { return c0 + s * (c1 + s * c2); }
-
-// sigma = d^T S d on differences to stencil cell 0, formed as one FMA chain
-// per row of the folded upper triangle SF. A negative or non-finite chain
-// (roundoff at sigma ~ 0, or bad data) is decided as the reference does:
-// the term-by-term sum with its roundoff clip (tensorstencilpoly.cpp:424-430).
-// Returns -1 on failure.
-template <class R, int N, class GF, class G>
-__device__ __forceinline__ R smoothness(GF&& SF, G&& S, const R* diff) {
-    R sum = 0;
-    int k = 0;
-#pragma unroll
-    for (int r = 0; r < N; ++r) {
-        R tr = SF(k++) * diff[r];
-#pragma unroll
-        for (int c = r + 1; c < N; ++c) tr = fma(SF(k++), diff[c], tr);
-        sum = fma(diff[r], tr, sum);
-    }
-    if (sum >= R(0) && sum < R(INFINITY)) return sum;
-    R exact = 0, mag = 0;
-#pragma unroll
-    for (int r = 0; r < N; ++r) {
-        const R sr = S(r, r) * diff[r] * diff[r];
-        exact += sr; mag += fabs(sr);
-#pragma unroll
-        for (int c = r + 1; c < N; ++c) {
-            const R term = R(2) * (S(r, c) * diff[r]) * diff[c];
-            exact += term; mag += fabs(term);
-        }
-    }
-    if (!isfinite(exact) || exact < -R(64) * eps_of<R>() * mag) return R(-1);
-    return exact > R(0) ? exact : R(0);
-}
 
 // Nonlinear weights alpha_k = (sigma_k + epsA)^-(s*r_k + eta(r_k)): exponent
 // 7 for the 3x3 order-2 candidate, 5 for the 2x2 order-1 candidates

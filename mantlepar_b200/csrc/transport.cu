@@ -920,7 +920,7 @@ extern "C" size_t mp_transport_instance_bytes(const mp_mesh_desc* mesh, int quad
         // Per-cell tables and geometry, vertices and edge spacing in one
         // allocation; the builder's copy of the vertices is held while the
         // tables are built.
-        b += pages(((size_t)(kQG0 + kQS9 + kQT4 + kQS4 + kQGeo) * N + V + NE * kNQ) * sizeof(double)) +
+        b += pages(((size_t)(kQG0 + kQT4 + kQMom + kQGeo) * N + V + NE * kNQ) * sizeof(double)) +
              pages(V * sizeof(double) + sizeof(int));
     }
     return b;
