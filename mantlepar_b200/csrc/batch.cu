@@ -320,7 +320,7 @@ size_t instance_bytes(int nx, int ny) {
     const size_t N = (size_t)nx * ny, NE = (size_t)nx * (ny + 1) + (size_t)(nx + 1) * ny;
     size_t b = 0;
     b += 11 * align256(N * sizeof(double));      // H C S1H S1C S2H S2C LH LC T phi rate
-    b += align256(18 * N * sizeof(double));      // rec
+    b += align256(rec_doubles(N) * sizeof(double)); // rec
     b += align256(N);                            // flags
     b += 2 * align256(NE * kNQ * sizeof(double));// vsn udn
     b += align256(4 * NE * sizeof(double));      // face
@@ -365,7 +365,7 @@ mp_status alloc_instance(mp_batch* b, MPInstance& in, const mp_mesh_desc& m) {
     const size_t N = in.N, NE = in.NE;
     double** dbl[] = {&in.H, &in.C, &in.S1H, &in.S1C, &in.S2H, &in.S2C, &in.LH, &in.LC, &in.T, &in.phi, &in.rate};
     for (double** q : dbl) *q = static_cast<double*>(take(N * sizeof(double)));
-    in.rec = static_cast<double*>(take(18 * N * sizeof(double)));
+    in.rec = static_cast<double*>(take(rec_doubles(N) * sizeof(double)));
     in.flags = static_cast<unsigned char*>(take(N));
     in.vsn = static_cast<double*>(take(NE * kNQ * sizeof(double)));
     in.udn = static_cast<double*>(take(NE * kNQ * sizeof(double)));
@@ -405,7 +405,7 @@ mp_status alloc_quad_instance(mp_batch* b, MPInstance& in, const mp_mesh_desc& m
     const size_t N = in.N, NE = in.NE;
     double** dbl[] = {&in.H, &in.C, &in.S1H, &in.S1C, &in.S2H, &in.S2C, &in.LH, &in.LC, &in.T, &in.phi, &in.rate};
     for (double** q : dbl) *q = static_cast<double*>(take(N * sizeof(double)));
-    in.rec = static_cast<double*>(take(18 * N * sizeof(double)));
+    in.rec = static_cast<double*>(take(rec_doubles(N) * sizeof(double)));
     in.flags = static_cast<unsigned char*>(take(N));
     in.vsn = static_cast<double*>(take(NE * kNQ * sizeof(double)));
     in.udn = static_cast<double*>(take(NE * kNQ * sizeof(double)));

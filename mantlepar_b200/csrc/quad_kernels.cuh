@@ -41,7 +41,7 @@ struct QuadStageArgs {
     int nx = 0, ny = 0, gj0 = 0, gny = 0;   // local rows; local row 0 is global row gj0 of gny
     const double* H = nullptr;              // stage input
     const double* C = nullptr;
-    double* rec = nullptr;                  // 18 * ncell deviation coefficients
+    double* rec = nullptr;                  // deviation coefficients (rec_at)
     unsigned char* flags = nullptr;
     double* T = nullptr;
     double* phi = nullptr;
@@ -86,10 +86,11 @@ __device__ __forceinline__ void quad_weno_cell(const QuadStageArgs& a, int i, in
         }
     double D[2][9];
     const int st = reconstruct_quad<2>(q, N, cell, ci, cj, eA, u, D);
+    double* r = rec + rec_at(cell);
 #pragma unroll
     for (int m = 0; m < 9; ++m) {
-        rec[(size_t)m * N + cell] = D[0][m];
-        rec[(size_t)(m + 9) * N + cell] = D[1][m];
+        r[m * kRecStride] = D[0][m];
+        r[(m + 9) * kRecStride] = D[1][m];
     }
     if (st) record_error(status, PART_UPDATE, cell + (long long)gj0 * nx, st);
 }
@@ -198,7 +199,7 @@ __device__ __forceinline__ void quad_limit_cell(const QuadStageArgs& a, const Ph
     MP_CHECK_INDEX(status, cell, N);
     const CellFrame f = cell_frame(q, nx, N, cell);
     double DH[9], DC[9];
-    load_rec(rec, N, cell, DH, DC);
+    load_rec(rec, cell, DH, DC);
     // 3x3 neighbour bounds of the averages (state_reconstruction.cpp:189-196).
     double lo[2], hi[2], m[2];
 #pragma unroll
@@ -244,10 +245,11 @@ __device__ __forceinline__ void quad_limit_cell(const QuadStageArgs& a, const Ph
 #pragma unroll
     for (int k = 1; k < 4; ++k) { ylo = fmin(ylo, f.c[k].y); yhi = fmax(yhi, f.c[k].y); }
     const double t0 = ph.litho ? tep_at(ph, ylo) : ph.Tep, t1 = ph.litho ? tep_at(ph, yhi) : ph.Tep;
+    double* r = rec + rec_at(cell);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-        rec[(size_t)k * N + cell] = DH[k] * thH;
-        rec[(size_t)(k + 9) * N + cell] = DC[k] * thC;
+        r[k * kRecStride] = DH[k] * thH;
+        r[(k + 9) * kRecStride] = DC[k] * thC;
     }
     flags[cell] = st_lim ? (unsigned char)FLAG_CHECK
                          : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), loH, hiH, loC, hiC);
@@ -282,7 +284,7 @@ __device__ __noinline__ void quad_cellphase_general(const QuadStageArgs& a, cons
     const CellFrame f = cell_frame(q, nx, (size_t)N, cell);
     const double mH = __ldg(H + cell), mC = __ldg(C + cell);
     double DH[9], DC[9];
-    load_rec(rec, (size_t)N, cell, DH, DC);
+    load_rec(rec, cell, DH, DC);
     int st_por = 0, st_cell = 0, st_face = 0;
     double Tsum = 0.0, Psum = 0.0, Ssum = 0.0, Rsum = 0.0, Wsum = 0.0;
     bool wet = false;
@@ -345,7 +347,7 @@ __device__ __forceinline__ void quad_cellphase_cell(const QuadStageArgs& a, cons
     const CellFrame f = cell_frame(q, nx, N, cell);
     const NormalCell k = normal_cell(f);
     double DH[9], DC[9];
-    load_rec(a.rec, N, cell, DH, DC);
+    load_rec(a.rec, cell, DH, DC);
     DH[0] += __ldg(a.H + cell);
     DC[0] += __ldg(a.C + cell);
     const double j0 = k.b.x * k.c.y - k.b.y * k.c.x, jr = k.b.x * k.d.y - k.b.y * k.d.x,
@@ -400,7 +402,7 @@ __device__ __forceinline__ void load_side(const QuadDev& q, size_t N, const doub
     s.inv_h = 1.0 / __ldg(q.geo + 2 * N + cell);
     s.mH = __ldg(H + cell);
     s.mC = __ldg(C + cell);
-    load_rec(rec, N, cell, s.DH, s.DC);
+    load_rec(rec, cell, s.DH, s.DC);
 }
 __device__ __forceinline__ void side_values(const Side& s, P2 p, double& h, double& c) {
     const double x = (p.x - s.cx) * s.inv_h, y = (p.y - s.cy) * s.inv_h;
@@ -477,7 +479,7 @@ __device__ __forceinline__ void quad_edge_values(const QuadStageArgs& a, size_t 
     const QuadDev& q = a.q;
     const double cx = __ldg(q.geo + cell), cy = __ldg(q.geo + N + cell), inv_h = 1.0 / __ldg(q.geo + 2 * N + cell);
     double DH[9], DC[9];
-    load_rec(a.rec, N, cell, DH, DC);
+    load_rec(a.rec, cell, DH, DC);
     DH[0] += __ldg(a.H + cell);
     DC[0] += __ldg(a.C + cell);
     const P2 u = P2{(ea.x - cx) * inv_h, (ea.y - cy) * inv_h}, v = P2{(eb.x - cx) * inv_h, (eb.y - cy) * inv_h};

@@ -17,6 +17,14 @@ namespace mp {
 namespace {
 
 constexpr int kRec = 18;          // limited deviation coefficients: 9 for H, 9 for C
+// Records lie in groups of 32 cells, coefficient by coefficient: the 18 loads
+// of a cell are one address and constant offsets, and a warp's record is one
+// stretch of 4.6 KB.
+constexpr int kRecStride = 32;
+__host__ __device__ __forceinline__ size_t rec_doubles(size_t cells) { return (cells + 31) / 32 * (32 * kRec); }
+__device__ __forceinline__ size_t rec_at(long long cell) {
+    return (size_t)((unsigned)cell >> 5) * (32 * kRec) + ((unsigned)cell & 31u);
+}
 constexpr int kRedBlock = 256;
 // The accumulation and axpy kernels give each thread kSumPer cells (strided
 // by the block size, so loads stay coalesced) before one block reduction.
@@ -151,7 +159,7 @@ struct ReconArgs {
     const StageHot* tab;   // batched instances: their tables in device memory
     const double* H;
     const double* C;
-    double* rec;           // 18 * ncell, SoA: rec[m*N + cell], m < 9 for H
+    double* rec;           // coefficient m of a cell at rec_at(cell) + m * kRecStride, m < 9 for H
     unsigned char* flags;
     unsigned long long* status;
     double* theta;         // optional (2 * ncell): limiter factors for H, C
@@ -336,8 +344,9 @@ __device__ __forceinline__ void recon_cell(const StageHot& t, const ReconArgs& a
         if (f) { loC = lo; hiC = hi; }
         else { loH = lo; hiH = hi; }
         if (a.theta) a.theta[f * N + cell] = th;
+        double* r = a.rec + rec_at(cell) + f * 9 * kRecStride;
 #pragma unroll
-        for (int m = 0; m < 9; ++m) a.rec[(size_t)(m + 9 * f) * N + cell] = D[m] * th;
+        for (int m = 0; m < 9; ++m) r[m * kRecStride] = D[m] * th;
     }
     const int st_lim = !means ? (int)E_OUTOFRANGE : (bad ? (int)E_FP : 0);
     // With a lithostatic pressure Tep is monotone over the cell's height.
@@ -376,11 +385,12 @@ struct CellPhaseArgs {
     const int* gate = nullptr;   // device flag: the launch does nothing while it is 0
 };
 
-__device__ __forceinline__ void load_rec(const double* rec, size_t N, long long cell, double* DH, double* DC) {
+__device__ __forceinline__ void load_rec(const double* rec, long long cell, double* DH, double* DC) {
+    const double* r = rec + rec_at(cell);
 #pragma unroll
     for (int m = 0; m < 9; ++m) {
-        DH[m] = __ldg(rec + (size_t)m * N + cell);
-        DC[m] = __ldg(rec + (size_t)(m + 9) * N + cell);
+        DH[m] = __ldg(r + m * kRecStride);
+        DC[m] = __ldg(r + (m + 9) * kRecStride);
     }
 }
 
@@ -397,7 +407,7 @@ __device__ __noinline__ void cellphase_general(const StageHot& t, const CellPhas
     MP_CHECK_INDEX(a.status, cell, N);
     const double mH = __ldg(a.H + cell), mC = __ldg(a.C + cell);
     double DH[9], DC[9];
-    load_rec(a.rec, (size_t)N, cell, DH, DC);
+    load_rec(a.rec, cell, DH, DC);
     int st_por = 0, st_cell = 0, st_face = 0;
     double Tsum = 0.0, Psum = 0.0, Ssum = 0.0, Rsum = 0.0, Wsum = 0.0;
     bool wet = false;
@@ -481,7 +491,7 @@ __device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhas
     const unsigned char fl = a.flags[cell];
     if (!(fl & FLAG_PLAIN)) { cellphase_general<kExt>(t, a, ph, cell); return; }
     double DH[9], DC[9];
-    load_rec(a.rec, (size_t)N, cell, DH, DC);
+    load_rec(a.rec, cell, DH, DC);
     DH[0] += __ldg(a.H + cell);
     DC[0] += __ldg(a.C + cell);
     const int gj = a.gj0 + (int)((unsigned)cell / (unsigned)a.nx);
@@ -542,10 +552,10 @@ struct SideLine {
     double h0, h1, h2, c0, c1, c2;
 };
 
-__device__ __forceinline__ void side_line(const FaceArgs& a, size_t N, long long cell, bool row, double fixed,
+__device__ __forceinline__ void side_line(const FaceArgs& a, long long cell, bool row, double fixed,
                                           SideLine& s) {
     double DH[9], DC[9];
-    load_rec(a.rec, N, cell, DH, DC);
+    load_rec(a.rec, cell, DH, DC);
     s.mH = __ldg(a.H + cell);
     s.mC = __ldg(a.C + cell);
     if (row) { q2_row(DH, fixed, s.h0, s.h1, s.h2); q2_row(DC, fixed, s.c0, s.c1, s.c2); }
@@ -778,8 +788,8 @@ __device__ __noinline__ void face_general(const StageHot& t, const FaceArgs& a, 
     // The edge's fixed coordinate in the left / right cell frame.
     const double lfix = at_.horizontal == g.reverse ? 1.0 : -1.0, rfix = at_.horizontal ? 1.0 : -1.0;
     SideLine sl, sr;
-    side_line(a, N, g.L, at_.horizontal, lfix, sl);
-    if (!g.boundary) side_line(a, N, g.R, at_.horizontal, rfix, sr);
+    side_line(a, g.L, at_.horizontal, lfix, sl);
+    if (!g.boundary) side_line(a, g.R, at_.horizontal, rfix, sr);
     const bool wetL = (a.flags[g.L] & FLAG_WET) != 0, wetR = g.boundary ? true : (a.flags[g.R] & FLAG_WET) != 0;
     const double sgn = g.reverse ? -1.0 : 1.0;
     double fluxH = 0.0, fluxC = 0.0, fluxMix = 0.0, rate = 0.0;
@@ -817,10 +827,10 @@ __device__ __noinline__ void face_general(const StageHot& t, const FaceArgs& a, 
 
 // Limited H and C of one side along an edge of a uniform mesh: the cell's
 // polynomial at xi or eta = s = +-1, mean included.
-__device__ __forceinline__ void edge_line(const FaceArgs& a, size_t N, long long cell, bool horizontal, double s,
+__device__ __forceinline__ void edge_line(const FaceArgs& a, long long cell, bool horizontal, double s,
                                           double (&h)[3], double (&c)[3]) {
     double DH[9], DC[9];
-    load_rec(a.rec, N, cell, DH, DC);
+    load_rec(a.rec, cell, DH, DC);
     DH[0] += __ldg(a.H + cell);
     DC[0] += __ldg(a.C + cell);
 #pragma unroll
@@ -852,7 +862,7 @@ __device__ __noinline__ void face_wall(const StageHot& t, const FaceArgs& a, con
     const EdgeAt at = edge_by_id(a.nx, a.ny, e);
     const EdgeCells g = edge_cells(a, at);
     double h[3], c[3];
-    edge_line(a, (size_t)a.nx * a.ny, g.L, at.horizontal, at.horizontal == g.reverse ? 1.0 : -1.0, h, c);
+    edge_line(a, g.L, at.horizontal, at.horizontal == g.reverse ? 1.0 : -1.0, h, c);
     const bool wet = (a.flags[g.L] & FLAG_WET) != 0;
     const double sgn = g.reverse ? -1.0 : 1.0;
     double fluxH = 0.0, fluxC = 0.0, fluxMix = 0.0, rate = 0.0;
@@ -893,8 +903,8 @@ __device__ __forceinline__ void face_edge(const StageHot& t, const FaceArgs& a, 
     if (g.boundary) { face_wall<kExt>(t, a, ph, g.e); return; }
     const bool wet = (fl & FLAG_WET) != 0;
     double hL[3], cL[3], hR[3], cR[3];
-    edge_line(a, N, g.L, at.horizontal, at.horizontal ? -1.0 : 1.0, hL, cL);
-    edge_line(a, N, g.R, at.horizontal, at.horizontal ? 1.0 : -1.0, hR, cR);
+    edge_line(a, g.L, at.horizontal, at.horizontal ? -1.0 : 1.0, hL, cL);
+    edge_line(a, g.R, at.horizontal, at.horizontal ? 1.0 : -1.0, hR, cR);
     double fluxH = 0.0, fluxC = 0.0, fluxMix = 0.0, rate = 0.0;
     int st = 0;
 #pragma unroll 1
@@ -971,10 +981,10 @@ __device__ __forceinline__ void diffusion_edge(const StageHot& t, const FaceArgs
     double DL[9], CL[9], DR[9], CR[9];
     double mHL = 0, mCL = 0, mHR = 0, mCR = 0;
     if (type == 1) {
-        load_rec(a.rec, N, L, DL, CL);
+        load_rec(a.rec, L, DL, CL);
         mHL = __ldg(a.H + L); mCL = __ldg(a.C + L);
         if (!boundary) {
-            load_rec(a.rec, N, Rc, DR, CR);
+            load_rec(a.rec, Rc, DR, CR);
             mHR = __ldg(a.H + Rc); mCR = __ldg(a.C + Rc);
         }
     }

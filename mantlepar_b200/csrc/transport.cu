@@ -858,7 +858,7 @@ mp_status create_impl(const mp_mesh_desc* mesh, bool slab, int row_begin, int ro
     auto alloc = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes); };
     for (double** p : {&t->H, &t->C, &t->S1H, &t->S1C, &t->S2H, &t->S2C, &t->LH, &t->LC, &t->T, &t->phi, &t->rate})
         alloc((void**)p, N * sizeof(double));
-    alloc((void**)&t->rec, (size_t)kRec * N * sizeof(double));
+    alloc((void**)&t->rec, rec_doubles(N) * sizeof(double));
     alloc((void**)&t->flags, N);
     alloc((void**)&t->vsn, NE * kNQ * sizeof(double));
     alloc((void**)&t->udn, NE * kNQ * sizeof(double));
@@ -912,7 +912,7 @@ extern "C" size_t mp_transport_instance_bytes(const mp_mesh_desc* mesh, int quad
     const size_t page = (size_t)2 << 20;
     auto pages = [&](size_t bytes) { return (bytes + page - 1) / page * page; };
     size_t b = 11 * pages(N * sizeof(double))                   // state, stage buffers, L, T, phi, rate
-             + pages((size_t)kRec * N * sizeof(double)) + pages(N)   // records, flags
+             + pages(rec_doubles(N) * sizeof(double)) + pages(N)   // records, flags
              + 2 * pages(NE * kNQ * sizeof(double)) + pages(4 * NE * sizeof(double))   // velocities, face values
              + pages(((N + kSumCells - 1) / kSumCells) * sizeof(Partial)) + page;
     if (quads) {
@@ -1227,7 +1227,8 @@ size_t raw_partial_bytes(size_t ncell) { return ((ncell + kSumCells - 1) / kSumC
 size_t raw_totals_bytes() { return sizeof(Totals); }
 
 // One stage evaluation L(U) (STORE_L mode) on buffers the caller provides:
-// tab (host StageTables, passed to the kernels by value), rec (18*ncell doubles), wet (ncell bytes), face
+// tab (host StageTables, passed to the kernels by value), rec (18 doubles per
+// cell, cells rounded up to 32), wet (ncell bytes), face
 // (4*nedge doubles), partial (raw_partial_bytes), totals (raw_totals_bytes),
 // status (one unsigned long long). Used by entry points that cannot allocate.
 mp_status stage_rhs_raw(int nx, int ny, const mp_transport_opts& o, const double* H, const double* C,
