@@ -85,11 +85,16 @@ __global__ void __launch_bounds__(128) batch_recon_kernel(const InstArgs* args, 
 
 // kExt: the adiabatic source (alpha0 != 0) is compiled in.
 template <bool kExt>
-__global__ void __launch_bounds__(128, 6) batch_phase_kernel(const InstArgs* args, const Work* work, const int* active,
+__global__ void __launch_bounds__(128, kExt ? 4 : 6) batch_phase_kernel(const InstArgs* args, const Work* work, const int* active,
                                                           const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
-    cellphase_cell<kExt>(*args[w.inst].phase.tab, args[w.inst].phase, ph, (long long)w.a + threadIdx.x);
+    const CellPhaseArgs& a = args[w.inst].phase;
+    extern __shared__ double source_buf[];
+    double* vy = kExt ? source_buf + (threadIdx.x >> 5) * (2 * 32 * kCellPoints) : nullptr;
+    const long long N = (long long)a.nx * a.ny, cell = (long long)w.a + threadIdx.x, first = cell - (threadIdx.x & 31);
+    if (kExt && ph.source && first < N) stage_source(a, first, N, vy);
+    cellphase_cell<kExt>(*a.tab, a, ph, cell, N, vy);
 }
 
 __global__ void __launch_bounds__(128, 5) batch_face_kernel(const InstArgs* args, const Work* work, const int* active,
@@ -101,12 +106,13 @@ __global__ void __launch_bounds__(128, 5) batch_face_kernel(const InstArgs* args
     if (k < w.b) face_edge<false>(*a.tab, a, ph, edge_by_kind(a.nx, a.ny, k));
 }
 
-__global__ void __launch_bounds__(128) batch_diffusion_kernel(const InstArgs* args, const Work* work, const int* active,
+__global__ void __launch_bounds__(128, 4) batch_diffusion_kernel(const InstArgs* args, const Work* work, const int* active,
                                                               const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
-    const long long e = (long long)w.a + threadIdx.x;
-    if (e < w.b) diffusion_edge(*args[w.inst].face.tab, args[w.inst].face, ph, e);
+    const long long k = (long long)w.a + threadIdx.x;
+    const FaceArgs& a = args[w.inst].face;
+    if (k < w.b) diffusion_edge(*a.tab, a, ph, edge_by_kind(a.nx, a.ny, k));
 }
 
 // General quad meshes: the per-element bodies of the single-mesh quad
@@ -637,7 +643,7 @@ void launch_kind(mp_batch* b, int kind) {
     const Tuning tu = b->tune;
     // Grids cover the work lists' capacities (padded items exit at once).
     timed(b, 0, [&] { batch_recon_kernel<<<b->cap_wrecon, dim3(tu.bx, tu.by), 0, s>>>(args, b->d_wrecon, b->d_active, b->ph, tu.cpt); });
-    if (b->ph.source) timed(b, 1, [&] { batch_phase_kernel<true><<<b->cap_wphase, 128, 0, s>>>(args, b->d_wphase, b->d_active, b->ph); });
+    if (b->ph.source) timed(b, 1, [&] { batch_phase_kernel<true><<<b->cap_wphase, 128, kSourceBufBytes, s>>>(args, b->d_wphase, b->d_active, b->ph); });
     else timed(b, 1, [&] { batch_phase_kernel<false><<<b->cap_wphase, 128, 0, s>>>(args, b->d_wphase, b->d_active, b->ph); });
     timed(b, 2, [&] { batch_face_kernel<<<b->cap_wface, 128, 0, s>>>(args, b->d_wface, b->d_active, b->ph); });
     if (b->ph.diffusion)
@@ -1109,6 +1115,11 @@ extern "C" mp_status mp_batch_create(const mp_mesh_desc* meshes, int count, cons
     b->ph.litho = 0; b->ph.tep_a = b->ph.tep_b = b->ph.surface = 0.0;
     b->ph.source = opts->material.alpha0 != 0.0;
     b->ph.cooling = opts->material.alpha0 * der.l0 * opts->material.g / opts->material.cp;
+    if (b->ph.source) {
+        const cudaError_t e = cudaFuncSetAttribute(batch_phase_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)kSourceBufBytes);
+        if (e != cudaSuccess) { delete b; return cuda_status(e, "mp_batch_create"); }
+    }
     b->inst.resize(count);
     for (int i = 0; i < count; ++i) {
         if (meshes[i].nx < 2 || meshes[i].ny < 2) { set_error("instance %d: at least 2x2 cells", i); mp_batch_destroy(b); return MP_ERR_ARG_SIZ; }

@@ -8,6 +8,8 @@
 #ifndef MP_STAGE_KERNELS_CUH
 #define MP_STAGE_KERNELS_CUH
 
+#include <cuda_pipeline.h>
+
 #include "common.hpp"
 #include "phase_math.cuh"
 #include "stage_device.cuh"
@@ -483,19 +485,47 @@ __device__ __noinline__ void cellphase_general(const StageHot& t, const CellPhas
 // FP64 pipe; with the tests, clips and library divisions of every point
 // (1239 FP64 and 3187 instructions per warp) it took 100 us at 640x1280, so
 // (641 and 1223) 54 us.
+//
+// The adiabatic source's two velocities at 25 points lie cell by cell (200
+// bytes apart from lane to lane): a warp first copies its cells' stretch to
+// shared memory, lane by lane, where the stride of 25 doubles has no bank
+// conflict. Read in place they took 938 L1 wavefronts per warp and 188 us at
+// 640x1280. vy: the warp's buffer of 2 x 32 x 25 doubles (kExt, source on).
+constexpr int kCellPoints = kNQ * kNQ;
+constexpr size_t kSourceBufBytes = 4 * 2 * 32 * kCellPoints * sizeof(double);   // four warps
+
+__device__ __forceinline__ void stage_source(const CellPhaseArgs& a, long long first, long long end, double* vy) {
+    const int lane = threadIdx.x & 31;
+    const int n = (int)min(32LL, end - first) * kCellPoints;
+    const double* vs = a.cvs_y + first * kCellPoints;
+    const double* ud = a.cud_y + first * kCellPoints;
+    for (int k = lane; k < n; k += 32) {
+        __pipeline_memcpy_async(vy + k, vs + k, sizeof(double));
+        __pipeline_memcpy_async(vy + 32 * kCellPoints + k, ud + k, sizeof(double));
+    }
+    __pipeline_commit();
+}
+// The cell of this lane, [0, end) (every lane of a warp calls).
 template <bool kExt>
-__device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhaseArgs& a, const Physics& ph, long long cell) {
-    const long long N = (long long)a.nx * a.ny;
-    if (cell >= N) return;
-    MP_CHECK_INDEX(a.status, cell, N);
-    const unsigned char fl = a.flags[cell];
-    if (!(fl & FLAG_PLAIN)) { cellphase_general<kExt>(t, a, ph, cell); return; }
+__device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhaseArgs& a, const Physics& ph, long long cell,
+                                               long long end, const double* vy = nullptr) {
+    const bool valid = cell < end;
+    const unsigned char fl = valid ? a.flags[cell] : 0;
     double DH[9], DC[9];
-    load_rec(a.rec, cell, DH, DC);
-    DH[0] += __ldg(a.H + cell);
-    DC[0] += __ldg(a.C + cell);
+    if (fl & FLAG_PLAIN) {
+        load_rec(a.rec, cell, DH, DC);
+        DH[0] += __ldg(a.H + cell);
+        DC[0] += __ldg(a.C + cell);
+    }
+    if (kExt && ph.source) {
+        __pipeline_wait_prior(0);
+        __syncwarp();
+    }
+    if (!valid) return;
+    MP_CHECK_INDEX(a.status, cell, (long long)a.nx * a.ny);
+    if (!(fl & FLAG_PLAIN)) { cellphase_general<kExt>(t, a, ph, cell); return; }
     const int gj = a.gj0 + (int)((unsigned)cell / (unsigned)a.nx);
-    double Tsum = 0.0, Psum = 0.0, Ssum = 0.0, Rsum = 0.0, Wsum = 0.0;
+    double Tsum = 0.0, Psum = 0.0, Ssum = 0.0, Rsum = 0.0;
 #pragma unroll 1
     for (int b = 0; b < kNQ; ++b) {
         const double y = t.g[b];
@@ -512,13 +542,12 @@ __device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhas
             Tsum = fma(w, pl.T, Tsum);
             Psum = fma(w, pl.phil, Psum);
             if (kExt && ph.source) {
-                const long long at = cell * (kNQ * kNQ) + b * kNQ + q;
+                const int at = (int)(threadIdx.x & 31) * kCellPoints + b * kNQ + q;
                 const double factor = pl.phil == 0.0 ? 0.0 : (ph.theta == 0.0 ? pl.phil : pow(pl.phil, 1.0 + ph.theta));
-                const double vy = __ldg(a.cvs_y + at) + factor * __ldg(a.cud_y + at);
-                const double src = -ph.cooling * pl.T * vy;
-                Ssum += w * src;
-                Rsum += w * ph.cooling * fabs(vy);
-                Wsum += t.cwp[b * kNQ + q] * src;
+                const double v = fma(factor, vy[32 * kCellPoints + at], vy[at]);
+                const double wv = w * v;
+                Ssum = fma(wv, pl.T, Ssum);
+                Rsum += fabs(wv);
             }
         }
     }
@@ -526,7 +555,11 @@ __device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhas
     a.flags[cell] = (unsigned char)(fl | (Psum > 0.0 ? FLAG_WET : 0));
     a.T[cell] = Tsum;
     a.phi[cell] = Psum;
-    if (kExt && ph.source) { a.srcH[cell] = Ssum; a.srcR[cell] = Rsum; a.srcS[cell] = Wsum; }
+    if (kExt && ph.source) {
+        // The quadrature weights are per area here and absolute in srcS.
+        const double heat = -ph.cooling * Ssum;
+        a.srcH[cell] = heat; a.srcR[cell] = ph.cooling * Rsum; a.srcS[cell] = heat * t.area;
+    }
 }
 
 // ---------------------------------------------------------------- face kernel
@@ -944,7 +977,8 @@ __device__ __forceinline__ void face_edge(const StageHot& t, const FaceArgs& a, 
 // wall value), gradient sum_k c_k (T_k - T_last) / ds, flux -= w kappa grad,
 // and |d flux / d T_k| added to the rate sample by sample. Added to the face
 // results after the advective part, as the reference adds them.
-__device__ __forceinline__ void diffusion_edge(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
+// Out of line: edges with a cell that is not plain.
+__device__ __noinline__ void diffusion_general(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
     const int nx = a.nx, ny = a.ny;
     const long long nI = (long long)nx * (ny + 1);
     const long long nE = nI + (long long)(nx + 1) * ny;
@@ -1040,6 +1074,101 @@ __device__ __forceinline__ void diffusion_edge(const StageHot& t, const FaceArgs
     if (st) record_error(a.status, PART_FACES, L + (long long)a.gj0 * nx, st);
     a.face[e] += integral;
     a.face[2 * nE + e] = rate;
+}
+
+// The same part of an interior edge between plain cells or (kWall) of a plain
+// cell at a wall of prescribed temperature: on each Gauss point's normal line
+// the limited states are one quadratic per side, whose coefficients are taken
+// for the centre and the two symmetric pairs of points. The rate's share is a
+// constant of the edge. 1204 instructions and 151 us at 640x1280; with every
+// sample tested and its derivative added to the rate one by one 4591 and 441.
+// The derivative
+// weights are [1/24, -9/8, 9/8, -1/24] and [1/4, -4/3, 3, -4, 25/12].
+template <bool kWall>
+__device__ __forceinline__ void diffusion_plain(const StageHot& t, const FaceArgs& a, const Physics& ph, const EdgeAt& at,
+                                                const EdgeCells& g, int wall) {
+    const int o = at.horizontal ? 0 : 1;
+    // Coefficients of each side by power across the edge [k] and along it [j].
+    struct SideD { double h[3][3], c[3][3]; } s[kWall ? 1 : 2];
+#pragma unroll
+    for (int n = 0; n < (kWall ? 1 : 2); ++n) {
+        const long long cell = n ? g.R : g.L;
+        double DH[9], DC[9];
+        load_rec(a.rec, cell, DH, DC);
+        DH[0] += __ldg(a.H + cell);
+        DC[0] += __ldg(a.C + cell);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                s[n].h[k][j] = at.horizontal ? DH[3 * k + j] : DH[3 * j + k];
+                s[n].c[k][j] = at.horizontal ? DC[3 * k + j] : DC[3 * j + k];
+            }
+    }
+    double sum = 0.0;
+#pragma unroll 1
+    for (int p = 0; p < 3; ++p) {
+        const double x = t.g[2 + p], x2 = x * x, w = t.gw[2 + p];
+#pragma unroll 1
+        for (int m = 0; m < (p ? 2 : 1); ++m) {
+            const double xs = m ? -x : x;
+            double v[4];
+#pragma unroll
+            for (int n = 0; n < (kWall ? 1 : 2); ++n) {
+                double h[3], c[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    h[k] = fma(s[n].h[k][1], xs, fma(s[n].h[k][2], x2, s[n].h[k][0]));
+                    c[k] = fma(s[n].c[k][1], xs, fma(s[n].c[k][2], x2, s[n].c[k][0]));
+                }
+                const int row = a.gj0 + (at.horizontal ? (g.reverse || n ? at.j - 1 : at.j) : at.j);
+#pragma unroll
+                for (int q = 0; q < (kWall ? 4 : 2); ++q) {
+                    const double y = kWall ? t.dif_pos_bnd[wall][q] : t.dif_pos_int[o][2 * n + q];
+                    const double tep = !ph.litho ? ph.Tep : tep_at(ph, height(t, row, at.horizontal ? y : xs));
+                    PhaseLean pl;
+                    phase_plain<false>(ph.sk, quad(h[0], h[1], h[2], y), quad(c[0], c[1], c[2], y), tep, pl);
+                    v[2 * n + q] = pl.T;
+                }
+            }
+            if (kWall) {
+                const double last = ph.wall_value[wall];
+                double grad = 0.0;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) grad = fma(t.dif_c_bnd[q], v[q] - last, grad);
+                sum = fma(w, grad, sum);
+            } else {
+                sum = fma(w, fma(t.dif_c_int[0], v[0] - v[3], t.dif_c_int[2] * (v[2] - v[1])), sum);
+            }
+        }
+    }
+    // flux -= sum_q (len w_q / 2) kappa grad_q / ds; the rate gets the same
+    // sum of |d flux / d T_k|, whose Gauss weights add up to 2.
+    const double len = at.horizontal ? t.len_h : t.len_v;
+    const double scale = 0.5 * len * ph.kappa / t.dif_ds[o][kWall ? 1 : 0];
+    double weights = 0.0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) weights += fabs(kWall ? t.dif_c_bnd[q] : t.dif_c_int[q]);
+    const long long nE = (long long)a.nx * (a.ny + 1) + (long long)(a.nx + 1) * a.ny;
+    a.face[g.e] = fma(-scale, sum, a.face[g.e]);
+    a.face[2 * nE + g.e] = fma(2.0 * scale, weights, a.face[2 * nE + g.e]);
+}
+__device__ __noinline__ void diffusion_wall(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e, int wall) {
+    const EdgeAt at = edge_by_id(a.nx, a.ny, e);
+    diffusion_plain<true>(t, a, ph, at, edge_cells(a, at), wall);
+}
+
+__device__ __forceinline__ void diffusion_edge(const StageHot& t, const FaceArgs& a, const Physics& ph, const EdgeAt& at) {
+    const EdgeCells g = edge_cells(a, at);
+    const size_t N = (size_t)a.nx * a.ny;
+    const int wall = at.horizontal ? (g.reverse ? 1 : 0) : (g.reverse ? 2 : 3);
+    if (g.boundary && ph.wall_type[wall] == MP_THERMAL_ZERO_FLUX) return;
+    MP_CHECK_INDEX(a.status, g.L, N);
+    if (!g.boundary) MP_CHECK_INDEX(a.status, g.R, N);
+    const unsigned char fl = a.flags[g.L] & (g.boundary ? 0xff : a.flags[g.R]);
+    if (!(fl & FLAG_PLAIN) || (g.boundary && ph.wall_type[wall] == MP_THERMAL_FLUX)) diffusion_general(t, a, ph, g.e);
+    else if (g.boundary) diffusion_wall(t, a, ph, g.e, wall);
+    else diffusion_plain<false>(t, a, ph, at, g, 0);
 }
 
 // ----------------------------------------------------------------- sum kernel

@@ -62,7 +62,8 @@ struct SourceBufs {
 // The stage tables arrive by value as a __grid_constant__ parameter, so the
 // unrolled table coefficients are constant-bank operands. Minimum resident
 // blocks per SM (register caps) as measured fastest on B200: cell phase 6
-// (48 us at 640x1280; 8: 55, 5: 51),
+// (48 us at 640x1280; 8: 55, 5: 51; with the source's buffers 4: 118, 5: 135,
+// 6: 139),
 // faces 5 (127; 4: 133, 6: 129); the reconstruction keeps its natural register
 // count (87 us; 5 and 6 blocks the same).
 // Rows [jlo, jhi) are reconstructed (all rows, or a slab's owned rows +- 1).
@@ -74,13 +75,17 @@ __global__ void __launch_bounds__(128) recon_kernel(const __grid_constant__ Reco
     if (j < jhi) recon_cell(p.d, a, ph, blockIdx.x * blockDim.x + threadIdx.x, j);
 }
 template <bool kExt>
-__global__ void __launch_bounds__(128, 6) cellphase_kernel(const __grid_constant__ CellPhaseArgs a,
+__global__ void __launch_bounds__(128, kExt ? 4 : 6) cellphase_kernel(const __grid_constant__ CellPhaseArgs a,
                                                            const __grid_constant__ Physics ph,
                                                            const __grid_constant__ ParamTables p, long long c0,
                                                            long long c1) {
     if (gated_off(a.gate)) return;
     const long long cell = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (cell < c1) cellphase_cell<kExt>(p.d, a, ph, cell);
+    extern __shared__ double source_buf[];
+    double* vy = kExt ? source_buf + (threadIdx.x >> 5) * (2 * 32 * kCellPoints) : nullptr;
+    const long long first = cell - (threadIdx.x & 31);
+    if (kExt && ph.source && first < c1) stage_source(a, first, c1, vy);
+    cellphase_cell<kExt>(p.d, a, ph, cell, c1, vy);
 }
 // Edges [h0, h0 + nh) (horizontal) then [v0, v0 + nv) (vertical): every edge
 // of the mesh, or of a slab's owned cells.
@@ -99,13 +104,16 @@ __global__ void __launch_bounds__(128, 5) face_kernel(const __grid_constant__ Fa
                                        : edge_by_kind(a.nx, a.ny, k));
 }
 // The diffusive part of the same edges (only launched when diffusion is on).
-__global__ void __launch_bounds__(128) diffusion_kernel(const __grid_constant__ FaceArgs a,
+// 4 resident blocks: 151 us at 640x1280 (5: 152; 3, unbounded: 171).
+__global__ void __launch_bounds__(128, 4) diffusion_kernel(const __grid_constant__ FaceArgs a,
                                                         const __grid_constant__ Physics ph,
                                                         const __grid_constant__ ParamTables p, long long h0,
                                                         long long nh, long long v0, long long nv) {
     if (gated_off(a.gate)) return;
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < nh + nv) diffusion_edge(p.d, a, ph, k < nh ? h0 + k : v0 + (k - nh));
+    if (k >= nh + nv) return;
+    const bool all = nh == (long long)a.nx * (a.ny + 1) && nv == (long long)(a.nx + 1) * a.ny;
+    diffusion_edge(p.d, a, ph, all ? edge_by_kind(a.nx, a.ny, k) : edge_by_id(a.nx, a.ny, k < nh ? h0 + k : v0 + (k - nh)));
 }
 
 template <bool kSrc, bool kArea = false>
@@ -317,7 +325,7 @@ void launch_stage_kernels(int nx, int ny, const StageRange& rg, const ParamTable
                            src.cvs_y, src.cud_y, src.srcH, src.srcR, src.srcS, gate};
         const long long c0 = (long long)rg.rec0 * nx, c1 = (long long)rg.rec1 * nx;
         const unsigned g = (unsigned)((c1 - c0 + 127) / 128);
-        if (ph.litho || ph.source) run(1, [&] { cellphase_kernel<true><<<g, 128, 0, s>>>(a, ph, pt, c0, c1); });
+        if (ph.litho || ph.source) run(1, [&] { cellphase_kernel<true><<<g, 128, ph.source ? kSourceBufBytes : 0, s>>>(a, ph, pt, c0, c1); });
         else run(1, [&] { cellphase_kernel<false><<<g, 128, 0, s>>>(a, ph, pt, c0, c1); });
     }
     {
@@ -855,6 +863,8 @@ mp_status create_impl(const mp_mesh_desc* mesh, bool slab, int row_begin, int ro
     t->sum_blocks = (int)((own_count(t) + kSumCells - 1) / kSumCells);
     const size_t N = t->N, NE = t->NE;
     cudaError_t e = cudaSuccess;
+    if (t->ph.source)
+        e = cudaFuncSetAttribute(cellphase_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSourceBufBytes);
     auto alloc = [&](void** p, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(p, bytes); };
     for (double** p : {&t->H, &t->C, &t->S1H, &t->S1C, &t->S2H, &t->S2C, &t->LH, &t->LC, &t->T, &t->phi, &t->rate})
         alloc((void**)p, N * sizeof(double));

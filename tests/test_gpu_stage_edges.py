@@ -123,3 +123,35 @@ def test_quad_mesh_of_mixed_cells_and_walls(nx, ny, config, family):
     assert code == 0
     for g, r in zip(t.limiter(), factors):
         assert np.max(np.abs(g - r)) <= 1e-11
+
+
+@pytest.mark.parametrize("types,values", [((1, 2, 0, 1), (0.9, -0.02, 0.0, 0.4)), ((1, 1, 1, 1), (0.9, 0.2, 0.5, 0.5)),
+                                          ((2, 0, 1, 2), (0.01, 0.0, 0.6, -0.03))], ids=["mixed", "temperature", "flux"])
+@pytest.mark.parametrize("nx,ny,patchy", [(2, 2, False), (33, 6, False), (37, 11, True)])
+def test_diffusion_and_source(nx, ny, patchy, types, values):
+    # Diffusion with every kind of wall, lithostatic pressure and the
+    # adiabatic source, whose cell velocities a warp stages 32 cells at a
+    # time (66 and 407 cells: last warps of 2 and 23 cells).
+    import dataclasses
+    from mantlepar_b200.transport import Transport, TransportConfig
+    from oracle import pyoracle as po
+    w = sy.Workload(nx=nx, ny=ny, seed=5)
+    mat = dataclasses.replace(sy.material_s(), rho=100.0, alpha0=3e-5)
+    o = po.TransportOracle(mat, w, lib=po.restated(), integrator=2, theta=2.0)
+    t = Transport(w, TransportConfig(material=mat, cfl=w.cfl, integrator=2, theta=2.0, diffusivity=0.02))
+    assert o.set_diffusion(0.02, types, values) == 0
+    t.set_thermal_bc(types, values)
+    assert o.set_pressure_model(1, 1.1) in (0, None)
+    t.set_pressure_model(t.LITHOSTATIC, 1.1)
+    H, C = patchy_state(w) if patchy else sy.initial_state(w)
+    vs, ud = sy.face_velocity(w)
+    for x in (t, o):
+        x.set_cell_velocity(*sy.cell_velocity(w))
+        x.set_face_velocity(vs, ud)
+        x.set_state(H, C)
+    got, (code, ref) = t.rhs(), o.rhs()
+    assert code == 0
+    assert per_cell(got["T"], ref["T"]) <= 1e-12
+    assert per_cell(got["phi"], ref["phi"]) <= 1e-12
+    for k in ("rhsH", "rhsC", "rate"):
+        assert np.max(np.abs(got[k] - ref[k])) <= 1e-12 * np.max(np.abs(ref[k]))
