@@ -55,7 +55,7 @@ struct AxpyArgs {
     double *H1, *C1;
     const double* dtp;
     double area;
-    Partial* partial;
+    Shares shares;
     const double* cell_area;   // per-cell areas (general quad mesh), else null
 };
 
@@ -168,8 +168,8 @@ __global__ void __launch_bounds__(kRedBlock) batch_sum_kernel(const InstArgs* ar
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const SumArgs& a = args[w.inst].sum;
-    const Partial v = a.cell_area ? sum_cells<kSrc, true>(a, w.a) : sum_cells<kSrc>(a, w.a);
-    block_reduce_write(v, a.partial + w.part);
+    const Partial v = a.cell_area ? sum_cells<kSrc, true>(a, w.a, a.dtp) : sum_cells<kSrc>(a, w.a, a.dtp);
+    finish_block(v, a.shares, w.part);
 }
 
 __global__ void __launch_bounds__(kRedBlock) batch_axpy_kernel(const AxpyArgs* args, const Work* work, const int* active) {
@@ -177,39 +177,23 @@ __global__ void __launch_bounds__(kRedBlock) batch_axpy_kernel(const AxpyArgs* a
     if (!active[w.inst]) return;
     const AxpyArgs& a = args[w.inst];
     const Partial v = axpy_cells(a.n, a.H0, a.C0, a.LH, a.LC, *a.dtp, a.area, a.H1, a.C1, w.a, a.cell_area);
-    block_reduce_write(v, a.partial + w.part);
+    finish_block(v, a.shares, w.part);
 }
 
 // Copy of U^{n+1} into U^n for the instances that accepted their step (the
-// accumulation work list: kSumCells cells per block).
+// accumulation work list).
 __global__ void __launch_bounds__(kRedBlock) batch_commit_kernel(const CommitArgs* args, const Work* work,
                                                                  const int* active) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const CommitArgs& a = args[w.inst];
+    const int per = sum_per(a.n);
 #pragma unroll
     for (int q = 0; q < kSumPer; ++q) {
+        if (q >= per) break;
         const long long k = (long long)w.a + q * kRedBlock + threadIdx.x;
         if (k < a.n) { a.dstH[k] = a.srcH[k]; a.dstC[k] = a.srcC[k]; }
     }
-}
-
-// One block per instance: fixed-order reduction of its block partials (the
-// same thread/tree shape as the single-instance reduction, so totals agree
-// bit for bit).
-__global__ void __launch_bounds__(1024) batch_reduce_kernel(const Partial* partial, const int* part_off,
-                                                           const int* part_cnt, const int* active, Totals* out) {
-    const int inst = blockIdx.x;
-    if (!active[inst]) return;
-    const int off = part_off[inst], cnt = part_cnt[inst];
-    Partial v = partial_identity();
-    for (int b = threadIdx.x; b < cnt; b += blockDim.x) fold_partial(v, partial[off + b]);
-    __shared__ Partial result;
-    block_reduce_write(v, &result);
-    __syncthreads();
-    if (threadIdx.x == 0)
-        out[inst] = Totals{result.maxRate, result.divergence, result.bH, result.bC, result.HI, result.CI,
-                           result.Hmin, result.Cmin, result.Cmax, result.nonfinite, result.sH};
 }
 
 }  // namespace
@@ -280,7 +264,8 @@ struct mp_batch {
     mp::Work *d_wqrec = nullptr, *d_wqphase = nullptr, *d_wqface = nullptr;
     int n_wqrec = 0, n_wqphase = 0, n_wqface = 0;
     int cap_wqrec = 0, cap_wqphase = 0, cap_wqface = 0;
-    int *d_active = nullptr, *d_part_off = nullptr, *d_part_cnt = nullptr;
+    int* d_active = nullptr;
+    unsigned* d_ticket = nullptr;      // finished blocks of each slot's running reduction
     mp::Partial* d_partial = nullptr;
     int partial_cap = 0;
     mp::Totals* d_tot = nullptr;
@@ -321,6 +306,12 @@ namespace mp {
 namespace {
 
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
+
+// Blocks of the accumulation of an instance.
+int sum_blocks_of(size_t cells) {
+    const size_t per = (size_t)sum_cells_per_block((long long)cells);
+    return (int)((cells + per - 1) / per);
+}
 
 size_t instance_bytes(int nx, int ny) {
     const size_t N = (size_t)nx * ny, NE = (size_t)nx * (ny + 1) + (size_t)(nx + 1) * ny;
@@ -478,7 +469,6 @@ mp_status rebuild_args(mp_batch* b, int slots) {
     std::vector<Work> wqr, wqp, wqf;
     std::vector<AxpyArgs> ax(slots);
     std::vector<CommitArgs> cm(slots);
-    std::vector<int> part_off(slots, 0), part_cnt(slots, 0);
     std::vector<Work> wr, wp, wf, ws;
     int parts = 0;
     const Tuning tu = b->tune;
@@ -486,10 +476,8 @@ mp_status rebuild_args(mp_batch* b, int slots) {
         MPInstance& in = b->inst[i];
         if (!in.used) continue;
         const double area = in.quad ? 1.0 : in.host_tab.area;   // a quad mesh: per-cell areas
-        const int nsum = (int)((in.N + kSumCells - 1) / kSumCells);
-        part_off[i] = parts; part_cnt[i] = nsum;
-        Partial* pp = nullptr;  // fixed below once the partial array exists
-        (void)pp;
+        const int nsum = sum_blocks_of(in.N);
+        const Shares shares{b->d_partial + parts, b->d_tot + i, b->d_ticket + i, nsum};
         for (int k = 0; k < NKIND; ++k) {
             const double* inH = k == KIND_P ? in.H : (k == KIND_B ? in.S1H : in.S2H);
             const double* inC = k == KIND_P ? in.C : (k == KIND_B ? in.S1C : in.S2C);
@@ -504,8 +492,8 @@ mp_status rebuild_args(mp_batch* b, int slots) {
             const double a0 = k == KIND_B ? (rk3 ? 0.75 : 0.5) : (1.0 / 3.0);
             const double a1 = k == KIND_B ? (rk3 ? 0.25 : 0.5) : (2.0 / 3.0);
             a.sum = SumArgs{in.nx, in.ny, area, 1.0 / area, in.face, inH, inC, in.H, in.C, outH, outC, in.rate,
-                            k == KIND_P ? (int)SUM_STORE_L : (int)SUM_RK, a0, a1, 0.0, b->d_partial + parts,
-                            b->d_dt + i, 0, 0, 0, -1, in.srcH, in.srcR, in.srcS, in.cell_area, nullptr, b->d_status + i};
+                            k == KIND_P ? (int)SUM_STORE_L : (int)SUM_RK, a0, a1, 0.0, shares,
+                            b->d_dt + i, 0, 0, 0, (long long)in.N, in.srcH, in.srcR, in.srcS, in.cell_area, nullptr, b->d_status + i};
             if (in.quad) {
                 QuadStageArgs& q = qargs[k][i];
                 q.nx = in.nx; q.ny = in.ny; q.gj0 = 0; q.gny = in.ny;
@@ -516,7 +504,7 @@ mp_status rebuild_args(mp_batch* b, int slots) {
             }
         }
         ax[i] = AxpyArgs{(int)in.N, in.H, in.C, in.LH, in.LC, in.S1H, in.S1C, b->d_dt + i, area,
-                         b->d_partial + parts, in.cell_area};
+                         shares, in.cell_area};
         const bool rk3 = b->opts.integrator == MP_SSPRK3;
         cm[i] = CommitArgs{(int)in.N, rk3 ? in.S1H : in.S2H, rk3 ? in.S1C : in.S2C, in.H, in.C};
         if (in.quad) {
@@ -531,7 +519,7 @@ mp_status rebuild_args(mp_batch* b, int slots) {
             for (size_t c = 0; c < in.N; c += 128) wp.push_back(Work{i, (int)c, 0, 0});
             for (size_t e = 0; e < in.NE; e += 128) wf.push_back(Work{i, (int)e, (int)std::min(in.NE, e + 128), 0});
         }
-        for (int s = 0; s < nsum; ++s) ws.push_back(Work{i, s * kSumCells, 0, s});
+        for (int s = 0; s < nsum; ++s) ws.push_back(Work{i, s * sum_cells_per_block((long long)in.N), 0, s});
         parts += nsum;
     }
     (void)parts;
@@ -542,16 +530,12 @@ mp_status rebuild_args(mp_batch* b, int slots) {
     for (int k = 0; k < NKIND; ++k) qargs[k].resize(cap);
     ax.resize(cap);
     cm.resize(cap);
-    part_off.resize(cap, 0);
-    part_cnt.resize(cap, 0);
     for (int k = 0; k < NKIND; ++k)
         MP_CUDA(cudaMemcpyAsync(b->d_args[k], args[k].data(), cap * sizeof(InstArgs), cudaMemcpyHostToDevice, s));
     for (int k = 0; k < NKIND; ++k)
         MP_CUDA(cudaMemcpyAsync(b->d_qargs[k], qargs[k].data(), cap * sizeof(QuadStageArgs), cudaMemcpyHostToDevice, s));
     MP_CUDA(cudaMemcpyAsync(b->d_axpy, ax.data(), cap * sizeof(AxpyArgs), cudaMemcpyHostToDevice, s));
     MP_CUDA(cudaMemcpyAsync(b->d_commit, cm.data(), cap * sizeof(CommitArgs), cudaMemcpyHostToDevice, s));
-    MP_CUDA(cudaMemcpyAsync(b->d_part_off, part_off.data(), cap * sizeof(int), cudaMemcpyHostToDevice, s));
-    MP_CUDA(cudaMemcpyAsync(b->d_part_cnt, part_cnt.data(), cap * sizeof(int), cudaMemcpyHostToDevice, s));
     // Work lists, padded to their capacity with the sentinel slot.
     bool grown = false;
     b->n_wrecon = (int)wr.size(); b->n_wphase = (int)wp.size(); b->n_wface = (int)wf.size(); b->n_wsum = (int)ws.size();
@@ -587,7 +571,7 @@ mp_status rebuild(mp_batch* b) {
     // Per-slot arrays, with headroom; d_active has one more entry, the
     // sentinel slot named by padded work items, which stays 0.
     if (slots > b->slots || b->slots == 0) {
-        for (void* p : {(void*)b->d_active, (void*)b->d_part_off, (void*)b->d_part_cnt, (void*)b->d_tot,
+        for (void* p : {(void*)b->d_active, (void*)b->d_ticket, (void*)b->d_tot,
                         (void*)b->d_status, (void*)b->d_dt, (void*)b->d_axpy, (void*)b->d_commit, b->d_args[0],
                         b->d_args[1], b->d_args[2], b->d_qargs[0], b->d_qargs[1], b->d_qargs[2]})
             if (p) cudaFreeAsync(p, s);
@@ -598,8 +582,8 @@ mp_status rebuild(mp_batch* b) {
         const int cap = std::max(slots + slots / 2, 8);
         MP_CUDA(cudaMallocAsync((void**)&b->d_active, (cap + 1) * sizeof(int), s));
         MP_CUDA(cudaMemsetAsync(b->d_active, 0, (cap + 1) * sizeof(int), s));
-        MP_CUDA(cudaMallocAsync((void**)&b->d_part_off, cap * sizeof(int), s));
-        MP_CUDA(cudaMallocAsync((void**)&b->d_part_cnt, cap * sizeof(int), s));
+        MP_CUDA(cudaMallocAsync((void**)&b->d_ticket, cap * sizeof(unsigned), s));
+        MP_CUDA(cudaMemsetAsync(b->d_ticket, 0, cap * sizeof(unsigned), s));
         MP_CUDA(cudaMallocAsync((void**)&b->d_tot, cap * sizeof(Totals), s));
         MP_CUDA(cudaMallocAsync((void**)&b->d_status, cap * sizeof(unsigned long long), s));
         MP_CUDA(cudaMemsetAsync(b->d_status, 0xff, cap * sizeof(unsigned long long), s));
@@ -617,7 +601,7 @@ mp_status rebuild(mp_batch* b) {
         b->gen += 1;
     }
     int parts = 0;
-    for (const MPInstance& in : b->inst) if (in.used) parts += (int)((in.N + kSumCells - 1) / kSumCells);
+    for (const MPInstance& in : b->inst) if (in.used) parts += sum_blocks_of(in.N);
     if (parts > b->partial_cap) {
         if (b->d_partial) cudaFreeAsync(b->d_partial, s);
         const int n = std::max(parts + parts / 2, 64);
@@ -662,8 +646,7 @@ void launch_kind(mp_batch* b, int kind) {
     }
     if (b->ph.source) timed(b, 3, [&] { batch_sum_kernel<true><<<b->cap_wsum, kRedBlock, 0, s>>>(args, b->d_wsum, b->d_active); });
     else timed(b, 3, [&] { batch_sum_kernel<false><<<b->cap_wsum, kRedBlock, 0, s>>>(args, b->d_wsum, b->d_active); });
-    timed(b, 4, [&] { batch_reduce_kernel<<<b->slots, 1024, 0, s>>>(b->d_partial, b->d_part_off, b->d_part_cnt, b->d_active, b->d_tot); });
-    count_launch(5);
+    count_launch(4);
 }
 
 // Stage of one kind on the active instances; totals and status to the host.
@@ -688,8 +671,7 @@ mp_status run_axpy(mp_batch* b, const std::vector<int>& act) {
     cudaStream_t s = b->stream;
     MP_CUDA(cudaMemcpyAsync(b->d_dt, b->h_dt, slots * sizeof(double), cudaMemcpyHostToDevice, s));
     timed(b, 4, [&] { batch_axpy_kernel<<<b->cap_wsum, kRedBlock, 0, s>>>(b->d_axpy, b->d_wsum, b->d_active); });
-    timed(b, 4, [&] { batch_reduce_kernel<<<b->slots, 1024, 0, s>>>(b->d_partial, b->d_part_off, b->d_part_cnt, b->d_active, b->d_tot); });
-    count_launch(2);
+    count_launch();
     MP_CUDA(cudaGetLastError());
     MP_CUDA(cudaMemcpyAsync(b->h_tot, b->d_tot, slots * sizeof(Totals), cudaMemcpyDeviceToHost, s));
     MP_CUDA(cudaStreamSynchronize(s));
@@ -963,7 +945,6 @@ mp_status capture_graph(mp_batch* b, cudaGraph_t* out) {
     MP_CUDA(cudaStreamBeginCaptureToGraph(s, attempt_body, nullptr, nullptr, 0, mode));
     ctl_attempt_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_hdr, b->d_active, b->d_dt);
     batch_axpy_kernel<<<b->cap_wsum, kRedBlock, 0, s>>>(b->d_axpy, b->d_wsum, b->d_active);
-    batch_reduce_kernel<<<b->slots, 1024, 0, s>>>(b->d_partial, b->d_part_off, b->d_part_cnt, b->d_active, b->d_tot);
     ctl_after_axpy_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_tot, b->d_status, b->d_active);
     launch_kind(b, KIND_B);
     ctl_after_stage_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_tot, b->d_status, b->d_active, 2,
@@ -1011,7 +992,7 @@ mp_status ensure_graph(mp_batch* b) {
     }
     if (b->graph_exec && b->graph_gen == b->gen) return MP_OK;
     release_graph(b);
-    b->stage_kernels = 5 + (b->ph.diffusion ? 1 : 0) + (b->has_quads ? (b->ph.diffusion ? 5 : 4) : 0);
+    b->stage_kernels = 4 + (b->ph.diffusion ? 1 : 0) + (b->has_quads ? (b->ph.diffusion ? 5 : 4) : 0);
     // Capture on a private stream (the caller's may be the legacy default
     // stream, which cannot be captured); the graph runs on the caller's.
     cudaStream_t cap = nullptr;
@@ -1145,7 +1126,7 @@ extern "C" void mp_batch_destroy(mp_batch* b) {
     for (int k = 0; k < mp::NKIND; ++k) if (b->d_qargs[k]) cudaFreeAsync(b->d_qargs[k], b->stream);
     for (void* p : {(void*)b->d_wqrec, (void*)b->d_wqphase, (void*)b->d_wqface}) if (p) cudaFreeAsync(p, b->stream);
     for (void* p : {(void*)b->d_axpy, (void*)b->d_wrecon, (void*)b->d_wphase, (void*)b->d_wface, (void*)b->d_wsum,
-                    (void*)b->d_active, (void*)b->d_part_off, (void*)b->d_part_cnt, (void*)b->d_partial,
+                    (void*)b->d_active, (void*)b->d_ticket, (void*)b->d_partial,
                     (void*)b->d_tot, (void*)b->d_status, (void*)b->d_dt})
         if (p) cudaFreeAsync(p, b->stream);
     cudaStreamSynchronize(b->stream);

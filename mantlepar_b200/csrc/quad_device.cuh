@@ -42,16 +42,13 @@ __device__ __forceinline__ void edge_geometry(P2 a, P2 b, double& len, P2& n) {
     const double dx = b.x - a.x, dy = b.y - a.y;
     const double scale = fmax(fabs(dx), fabs(dy));
     const double ux = dx / scale, uy = dy / scale;
-    const double norm = sqrt(ux * ux + uy * uy);
+    const double norm = sqrt(fma(ux, ux, __dmul_rn(uy, uy)));
     len = scale * norm;
     n = P2{uy / norm, -ux / norm};
 }
 // Full Q2 form, monomial m = j*3 + i of xi^i eta^j.
 __device__ __forceinline__ double q2v(const double* D, double x, double y) {
-    const double r0 = D[0] + x * (D[1] + x * D[2]);
-    const double r1 = D[3] + x * (D[4] + x * D[5]);
-    const double r2 = D[6] + x * (D[7] + x * D[8]);
-    return r0 + y * (r1 + y * r2);
+    return quad(quad(D[0], D[1], D[2], x), quad(D[3], D[4], D[5], x), quad(D[6], D[7], D[8], x), y);
 }
 
 // The cell's frame: centre, 1/h, and corners.
@@ -71,15 +68,23 @@ __device__ __forceinline__ CellFrame cell_frame(const QuadDev& q, int nx, size_t
     return f;
 }
 
+// A point in a cell's frame. Rounded products (no contraction with what
+// follows), so that every kernel forms the same point.
+__device__ __forceinline__ P2 normalised(P2 p, double cx, double cy, double inv_h) {
+    return P2{__dmul_rn(p.x - cx, inv_h), __dmul_rn(p.y - cy, inv_h)};
+}
+
 // The bilinear map of a cell in its own frame: x(r, s) = m + b r + c s + d r s.
 struct NormalCell {
     P2 n[4];               // corners
     P2 m, b, c, d;
+    // Jacobian j0 + jr r + js s of the map (d x d vanishes).
+    __device__ __forceinline__ static double cross(P2 u, P2 v) { return fma(u.x, v.y, -__dmul_rn(u.y, v.x)); }
 };
 __device__ __forceinline__ NormalCell normal_cell(const CellFrame& f) {
     NormalCell k;
 #pragma unroll
-    for (int v = 0; v < 4; ++v) k.n[v] = P2{(f.c[v].x - f.cx) * f.inv_h, (f.c[v].y - f.cy) * f.inv_h};
+    for (int v = 0; v < 4; ++v) k.n[v] = normalised(f.c[v], f.cx, f.cy, f.inv_h);
     auto quarter = [&](double s1, double s2, double s3) {
         return P2{0.25 * (k.n[0].x + s1 * k.n[1].x + s2 * k.n[2].x + s3 * k.n[3].x),
                   0.25 * (k.n[0].y + s1 * k.n[1].y + s2 * k.n[2].y + s3 * k.n[3].y)};

@@ -63,11 +63,11 @@ struct QuadStageArgs {
 // registers (the table reads need many warps in flight).
 __device__ __forceinline__ void quad_weno_cell(const QuadStageArgs& a, int i, int j) {
     const int nx = a.nx, ny = a.ny, gj0 = a.gj0, gny = a.gny;
-    const double* __restrict__ H = a.H;
-    const double* __restrict__ C = a.C;
+    const double* H = a.H;
+    const double* C = a.C;
     unsigned long long* status = a.status;
     const QuadDev& q = a.q;
-    double* __restrict__ rec = a.rec;
+    double* rec = a.rec;
     const long long cell = (long long)j * nx + i;
     const size_t N = (size_t)nx * ny;
     MP_CHECK_INDEX(status, cell, N);
@@ -81,8 +81,8 @@ __device__ __forceinline__ void quad_weno_cell(const QuadStageArgs& a, int i, in
         for (int di = 0; di < 3; ++di) {
             const int ii = min(max(i + di - 1, 0), nx - 1), jj = min(max(j + dj - 1, 0), ny - 1);
             MP_CHECK_INDEX(status, (long long)jj * nx + ii, N);
-            u[0][dj][di] = __ldg(H + (size_t)jj * nx + ii);
-            u[1][dj][di] = __ldg(C + (size_t)jj * nx + ii);
+            u[0][dj][di] = MP_LD(H + (size_t)jj * nx + ii);
+            u[1][dj][di] = MP_LD(C + (size_t)jj * nx + ii);
         }
     double D[2][9];
     const int st = reconstruct_quad<2>(q, N, cell, ci, cj, eA, u, D);
@@ -187,12 +187,12 @@ __device__ __forceinline__ void quad_scan(const QuadStageArgs& a, int i, int j, 
 // are scaled in place.
 __device__ __forceinline__ void quad_limit_cell(const QuadStageArgs& a, const Physics& ph, int i, int j) {
     const int nx = a.nx, ny = a.ny, gj0 = a.gj0, gny = a.gny;
-    const double* __restrict__ H = a.H;
-    const double* __restrict__ C = a.C;
+    const double* H = a.H;
+    const double* C = a.C;
     unsigned long long* status = a.status;
     const QuadDev& q = a.q;
-    double* __restrict__ rec = a.rec;
-    unsigned char* __restrict__ flags = a.flags;
+    double* rec = a.rec;
+    unsigned char* flags = a.flags;
     double* theta = a.theta;
     const long long cell = (long long)j * nx + i;
     const size_t N = (size_t)nx * ny;
@@ -205,7 +205,7 @@ __device__ __forceinline__ void quad_limit_cell(const QuadStageArgs& a, const Ph
 #pragma unroll
     for (int fi = 0; fi < 2; ++fi) {
         const double* F = fi ? C : H;
-        m[fi] = __ldg(F + cell);
+        m[fi] = MP_LD(F + cell);
         lo[fi] = m[fi]; hi[fi] = m[fi];
 #pragma unroll
         for (int dj = -1; dj <= 1; ++dj)
@@ -213,7 +213,7 @@ __device__ __forceinline__ void quad_limit_cell(const QuadStageArgs& a, const Ph
             for (int di = -1; di <= 1; ++di) {
                 const int ii = min(max(i + di, 0), nx - 1), jj = min(max(j + dj, 0), ny - 1);
                 MP_CHECK_INDEX(status, (long long)jj * nx + ii, N);
-                const double v = __ldg(F + (size_t)jj * nx + ii);
+                const double v = MP_LD(F + (size_t)jj * nx + ii);
                 lo[fi] = fmin(lo[fi], v); hi[fi] = fmax(hi[fi], v);
             }
     }
@@ -269,20 +269,20 @@ __global__ void __launch_bounds__(128, 4) quad_limit_kernel(const __grid_constan
 // point with its admissibility test. Out of line: cells that are not plain.
 __device__ __noinline__ void quad_cellphase_general(const QuadStageArgs& a, const Physics& ph, long long cell) {
     const int nx = a.nx, ny = a.ny, gj0 = a.gj0, gny = a.gny;
-    const double* __restrict__ H = a.H;
-    const double* __restrict__ C = a.C;
+    const double* H = a.H;
+    const double* C = a.C;
     unsigned long long* status = a.status;
     const QuadDev& q = a.q;
-    const double* __restrict__ rec = a.rec;
-    unsigned char* __restrict__ flags = a.flags;
-    double* __restrict__ T = a.T;
-    double* __restrict__ phi = a.phi;
+    const double* rec = a.rec;
+    unsigned char* flags = a.flags;
+    double* T = a.T;
+    double* phi = a.phi;
     const SourcePtrs& src = a.src;
     const long long N = (long long)nx * ny;
     MP_CHECK_INDEX(status, cell, N);
     const int i = (int)(cell % nx), j = (int)(cell / nx);
     const CellFrame f = cell_frame(q, nx, (size_t)N, cell);
-    const double mH = __ldg(H + cell), mC = __ldg(C + cell);
+    const double mH = MP_LD(H + cell), mC = MP_LD(C + cell);
     double DH[9], DC[9];
     load_rec(rec, cell, DH, DC);
     int st_por = 0, st_cell = 0, st_face = 0;
@@ -348,16 +348,16 @@ __device__ __forceinline__ void quad_cellphase_cell(const QuadStageArgs& a, cons
     const NormalCell k = normal_cell(f);
     double DH[9], DC[9];
     load_rec(a.rec, cell, DH, DC);
-    DH[0] += __ldg(a.H + cell);
-    DC[0] += __ldg(a.C + cell);
-    const double j0 = k.b.x * k.c.y - k.b.y * k.c.x, jr = k.b.x * k.d.y - k.b.y * k.d.x,
-                 js = k.d.x * k.c.y - k.d.y * k.c.x;
+    DH[0] += MP_LD(a.H + cell);
+    DC[0] += MP_LD(a.C + cell);
+    const double j0 = k.cross(k.b, k.c), jr = k.cross(k.b, k.d), js = k.cross(k.d, k.c);
     double Tsum = 0.0, Psum = 0.0, Ssum = 0.0, Rsum = 0.0;
 #pragma unroll 1
     for (int b = 0; b < kNQ; ++b) {
         const double s = q.gq[b], ws = q.gw[b], js0 = fma(js, s, j0);
         const double x0 = fma(k.c.x, s, k.m.x), y0 = fma(k.c.y, s, k.m.y);
         const double x1 = fma(k.d.x, s, k.b.x), y1 = fma(k.d.y, s, k.b.y);
+        double Trow = 0.0, Prow = 0.0;   // by row, as the split form adds them
 #pragma unroll
         for (int r = 0; r < kNQ; ++r) {
             const double x = fma(x1, q.gq[r], x0), y = fma(y1, q.gq[r], y0);
@@ -365,8 +365,8 @@ __device__ __forceinline__ void quad_cellphase_cell(const QuadStageArgs& a, cons
             const double tep = ph.litho ? tep_at(ph, fma(y, 1.0 / f.inv_h, f.cy)) : ph.Tep;
             PhaseLean pl;
             phase_plain<false>(ph.sk, q2v(DH, x, y), q2v(DC, x, y), tep, pl);
-            Tsum = fma(w, pl.T, Tsum);
-            Psum = fma(w, pl.phil, Psum);
+            Trow = fma(w, pl.T, Trow);
+            Prow = fma(w, pl.phil, Prow);
             if (ph.source) {
                 const long long at = cell * (kNQ * kNQ) + b * kNQ + r;
                 const double factor = pl.phil == 0.0 ? 0.0 : (ph.theta == 0.0 ? pl.phil : pow(pl.phil, 1.0 + ph.theta));
@@ -375,6 +375,8 @@ __device__ __forceinline__ void quad_cellphase_cell(const QuadStageArgs& a, cons
                 Rsum += w * ph.cooling * fabs(vy);
             }
         }
+        Tsum += Trow;
+        Psum += Prow;
     }
     // Porosities are not negative: the cell is wet where their mean is not 0.
     a.flags[cell] = (unsigned char)(fl | (Psum > 0.0 ? FLAG_WET : 0));
@@ -400,8 +402,8 @@ __device__ __forceinline__ void load_side(const QuadDev& q, size_t N, const doub
     s.cx = __ldg(q.geo + cell);
     s.cy = __ldg(q.geo + N + cell);
     s.inv_h = 1.0 / __ldg(q.geo + 2 * N + cell);
-    s.mH = __ldg(H + cell);
-    s.mC = __ldg(C + cell);
+    s.mH = MP_LD(H + cell);
+    s.mC = MP_LD(C + cell);
     load_rec(rec, cell, s.DH, s.DC);
 }
 __device__ __forceinline__ void side_values(const Side& s, P2 p, double& h, double& c) {
@@ -415,15 +417,15 @@ __device__ __forceinline__ void side_values(const Side& s, P2 p, double& h, doub
 // that is not plain.
 __device__ __noinline__ void quad_face_general(const QuadStageArgs& a, const Physics& ph, long long e) {
     const int nx = a.nx, ny = a.ny, gj0 = a.gj0, gny = a.gny;
-    const double* __restrict__ H = a.H;
-    const double* __restrict__ C = a.C;
+    const double* H = a.H;
+    const double* C = a.C;
     unsigned long long* status = a.status;
     const QuadDev& q = a.q;
-    const double* __restrict__ rec = a.rec;
-    const unsigned char* __restrict__ flags = a.flags;
-    const double* __restrict__ vsn = a.vsn;
-    const double* __restrict__ udn = a.udn;
-    double* __restrict__ face = a.face;
+    const double* rec = a.rec;
+    const unsigned char* flags = a.flags;
+    const double* vsn = a.vsn;
+    const double* udn = a.udn;
+    double* face = a.face;
     const long long nE = (long long)nx * (ny + 1) + (long long)(nx + 1) * ny;
     const size_t N = (size_t)nx * ny;
     MP_CHECK_INDEX(status, e, nE);
@@ -480,9 +482,9 @@ __device__ __forceinline__ void quad_edge_values(const QuadStageArgs& a, size_t 
     const double cx = __ldg(q.geo + cell), cy = __ldg(q.geo + N + cell), inv_h = 1.0 / __ldg(q.geo + 2 * N + cell);
     double DH[9], DC[9];
     load_rec(a.rec, cell, DH, DC);
-    DH[0] += __ldg(a.H + cell);
-    DC[0] += __ldg(a.C + cell);
-    const P2 u = P2{(ea.x - cx) * inv_h, (ea.y - cy) * inv_h}, v = P2{(eb.x - cx) * inv_h, (eb.y - cy) * inv_h};
+    DH[0] += MP_LD(a.H + cell);
+    DC[0] += MP_LD(a.C + cell);
+    const P2 u = normalised(ea, cx, cy, inv_h), v = normalised(eb, cx, cy, inv_h);
     const P2 mid = P2{0.5 * (u.x + v.x), 0.5 * (u.y + v.y)}, half = P2{0.5 * (v.x - u.x), 0.5 * (v.y - u.y)};
 #pragma unroll
     for (int k = 0; k < kNQ; ++k) {
@@ -569,12 +571,12 @@ __global__ void __launch_bounds__(128, 5) quad_face_kernel(const __grid_constant
 // samples, spacing per edge point.
 __device__ __forceinline__ void quad_diffusion_edge(const QuadStageArgs& a, const Physics& ph, long long e) {
     const int nx = a.nx, ny = a.ny, gj0 = a.gj0, gny = a.gny;
-    const double* __restrict__ H = a.H;
-    const double* __restrict__ C = a.C;
+    const double* H = a.H;
+    const double* C = a.C;
     unsigned long long* status = a.status;
     const QuadDev& q = a.q;
-    const double* __restrict__ rec = a.rec;
-    double* __restrict__ face = a.face;
+    const double* rec = a.rec;
+    double* face = a.face;
     const long long nE = (long long)nx * (ny + 1) + (long long)(nx + 1) * ny;
     const size_t N = (size_t)nx * ny;
     MP_CHECK_INDEX(status, e, nE);

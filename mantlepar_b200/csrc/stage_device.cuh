@@ -112,22 +112,20 @@ __device__ __forceinline__ void phase_plain(const StageConst& k, double H, doubl
 }
 
 // Row / column coefficients of a Q2 polynomial (coefficient m = j*3 + i of
-// xi^i eta^j): along the row eta = y, p(xi) = a0 + xi*(a1 + xi*a2).
-template <class R>
-__device__ __forceinline__ void q2_row(const R* D, R y, R& a0, R& a1, R& a2) {
-    a0 = D[0] + y * (D[3] + y * D[6]);
-    a1 = D[1] + y * (D[4] + y * D[7]);
-    a2 = D[2] + y * (D[5] + y * D[8]);
+// xi^i eta^j): along the row eta = y, p(xi) = a0 + xi*(a1 + xi*a2). Written
+// as FMAs, so that kernels that split a cell over lanes round alike.
+__device__ __forceinline__ double quad(double c0, double c1, double c2, double s) { return fma(s, fma(s, c2, c1), c0); }
+__device__ __forceinline__ void q2_row(const double* D, double y, double& a0, double& a1, double& a2) {
+    a0 = quad(D[0], D[3], D[6], y);
+    a1 = quad(D[1], D[4], D[7], y);
+    a2 = quad(D[2], D[5], D[8], y);
 }
 // Along the column xi = x, p(eta) = b0 + eta*(b1 + eta*b2).
-template <class R>
-__device__ __forceinline__ void q2_col(const R* D, R x, R& b0, R& b1, R& b2) {
-    b0 = D[0] + x * (D[1] + x * D[2]);
-    b1 = D[3] + x * (D[4] + x * D[5]);
-    b2 = D[6] + x * (D[7] + x * D[8]);
+__device__ __forceinline__ void q2_col(const double* D, double x, double& b0, double& b1, double& b2) {
+    b0 = quad(D[0], D[1], D[2], x);
+    b1 = quad(D[3], D[4], D[5], x);
+    b2 = quad(D[6], D[7], D[8], x);
 }
-template <class R>
-__device__ __forceinline__ R quad(R c0, R c1, R c2, R s) { return c0 + s * (c1 + s * c2); }
 
 // Nonlinear weights alpha_k = (sigma_k + epsA)^-(s*r_k + eta(r_k)): exponent
 // 7 for the 3x3 order-2 candidate, 5 for the 2x2 order-1 candidates
@@ -165,13 +163,14 @@ __device__ __forceinline__ int weno_weights(const double (&s)[5], unsigned on, d
         for (int k = 0; k < 5; ++k) w[k] = wc[k];
         return st;
     }
-    auto p5 = [](double x) { const double x2 = x * x; return x2 * x2 * x; };
+    auto p5 = [](double x) { const double x2 = x * x; return __dmul_rn(x2 * x2, x); };
     const double f = (on & 1u ? epsA2 : 1.0) * (s02 * s02 * (s02 * s[0]));
     w[0] = p5(P);
-    w[1] = f * p5(s[2] * s34);
-    w[2] = f * p5(s[1] * s34);
-    w[3] = f * p5(s12 * s[4]);
-    w[4] = f * p5(s12 * s[3]);
+    // Rounded products: the sum below adds the weights themselves.
+    w[1] = __dmul_rn(f, p5(s[2] * s34));
+    w[2] = __dmul_rn(f, p5(s[1] * s34));
+    w[3] = __dmul_rn(f, p5(s12 * s[4]));
+    w[4] = __dmul_rn(f, p5(s12 * s[3]));
     if (on != 31u) {
 #pragma unroll
         for (int k = 0; k < 5; ++k) w[k] = (on >> k) & 1u ? w[k] : 0.0;
@@ -235,7 +234,7 @@ __device__ __forceinline__ int reconstruct(const StageHot& t, unsigned on, const
     const double bSE = (dSE - dE) - dS, bNE = (dNE - dE) - dN, bSW = (dSW - dW) - dS, bNW = (dNW - dW) - dN;
     {
         const double e = fma(t.gx2 * dE, dE, 1.0), w = fma(t.gx2 * dW, dW, 1.0);
-        const double n = (t.gy2 * dN) * dN, o = (t.gy2 * dS) * dS;
+        const double n = __dmul_rn(t.gy2 * dN, dN), o = __dmul_rn(t.gy2 * dS, dS);
         s[1] = fma(t.gb * bSE, bSE, e + o);
         s[2] = fma(t.gb * bNE, bNE, e + n);
         s[3] = fma(t.gb * bSW, bSW, w + o);

@@ -15,6 +15,13 @@
 #include "stage_device.cuh"
 #include "tables.hpp"
 
+// Load of an array that some phase of a stage writes: through the read-only
+// path in kernels of one phase each, a plain load where one kernel runs every
+// phase (small_steps.cu).
+#ifndef MP_LD
+#define MP_LD(p) __ldg(p)
+#endif
+
 namespace mp {
 namespace {
 
@@ -29,13 +36,20 @@ __device__ __forceinline__ size_t rec_at(long long cell) {
 }
 constexpr int kRedBlock = 256;
 // The accumulation and axpy kernels give each thread kSumPer cells (strided
-// by the block size, so loads stay coalesced) before one block reduction.
+// by the block size, so loads stay coalesced) before one block reduction; on
+// a mesh of at most kSmallCells cells (whose steps one cluster of 16 blocks
+// runs, small_steps.cu) one, so that every block of the cluster has a share.
+// A function of the mesh alone: the grouping fixes the order of the sums.
 constexpr int kSumPer = 4;
-constexpr int kSumCells = kRedBlock * kSumPer;
+constexpr long long kSmallCells = 1536, kSmallQuadCells = 1024;
+__host__ __device__ __forceinline__ int sum_per(long long cells) { return cells <= kSmallCells ? 1 : kSumPer; }
+__host__ __device__ __forceinline__ int sum_cells_per_block(long long cells) { return kRedBlock * sum_per(cells); }
 
 enum : int {
     E_OUTOFRANGE = MP_ERR_ARG_OUTOFRANGE, E_FP = MP_ERR_FP, E_WRONG = MP_ERR_ARG_WRONG
 };
+
+}  // namespace
 
 struct Physics {
     PhaseConst k;
@@ -62,6 +76,8 @@ struct Physics {
     double cooling;
 };
 
+namespace {
+
 // Pressure-corrected eutectic temperature at height y (one FMA for the
 // lithostatic model; the constant model returns the stored value exactly).
 __device__ __forceinline__ double tep_at(const Physics& ph, double y) {
@@ -73,6 +89,8 @@ __device__ __forceinline__ double height(const StageHot& t, int gj, double eta) 
     return t.y0 + (gj + 0.5) * t.dy + eta * t.hn;
 }
 
+}  // namespace
+
 // Block partials of one stage (sum_kernel) or state check (axpy_kernel).
 struct Partial {
     double maxRate, divergence, bH, bC, HI, CI, Hmin, Cmin, Cmax;
@@ -80,15 +98,21 @@ struct Partial {
     double sH;             // adiabatic source integral
 };
 
+namespace {
+
 __device__ __forceinline__ Partial partial_identity() {
     return Partial{-INFINITY, 0.0, 0.0, 0.0, 0.0, 0.0, INFINITY, INFINITY, -INFINITY, 0.0, 0.0};
 }
+
+}  // namespace
 
 struct Totals {
     double maxRate, divergence, bH, bC, HI, CI, Hmin, Cmin, Cmax;
     double nonfinite;
     double sH;
 };
+
+namespace {
 
 // Fold one block partial into a running partial (fixed field rules).
 __device__ __forceinline__ void fold_partial(Partial& v, const Partial& p) {
@@ -280,7 +304,7 @@ __device__ __forceinline__ void recon_field(const StageHot& t, const double* __r
 #pragma unroll
     for (int dj = 0; dj < 3; ++dj)
 #pragma unroll
-        for (int di = 0; di < 3; ++di) u[dj][di] = __ldg(F + at[dj][di]);
+        for (int di = 0; di < 3; ++di) u[dj][di] = MP_LD(F + at[dj][di]);
     // 3x3 neighbour bounds (state_reconstruction.cpp:189-196); the clamped
     // gather repeats in-domain values, which leaves min/max unchanged.
     mean = lo = hi = u[1][1];
@@ -391,8 +415,8 @@ __device__ __forceinline__ void load_rec(const double* rec, long long cell, doub
     const double* r = rec + rec_at(cell);
 #pragma unroll
     for (int m = 0; m < 9; ++m) {
-        DH[m] = __ldg(r + m * kRecStride);
-        DC[m] = __ldg(r + (m + 9) * kRecStride);
+        DH[m] = MP_LD(r + m * kRecStride);
+        DC[m] = MP_LD(r + (m + 9) * kRecStride);
     }
 }
 
@@ -407,7 +431,7 @@ __device__ __noinline__ void cellphase_general(const StageHot& t, const CellPhas
     const long long N = (long long)a.nx * a.ny;
     if (cell >= N) return;
     MP_CHECK_INDEX(a.status, cell, N);
-    const double mH = __ldg(a.H + cell), mC = __ldg(a.C + cell);
+    const double mH = MP_LD(a.H + cell), mC = MP_LD(a.C + cell);
     double DH[9], DC[9];
     load_rec(a.rec, cell, DH, DC);
     int st_por = 0, st_cell = 0, st_face = 0;
@@ -514,8 +538,8 @@ __device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhas
     double DH[9], DC[9];
     if (fl & FLAG_PLAIN) {
         load_rec(a.rec, cell, DH, DC);
-        DH[0] += __ldg(a.H + cell);
-        DC[0] += __ldg(a.C + cell);
+        DH[0] += MP_LD(a.H + cell);
+        DC[0] += MP_LD(a.C + cell);
     }
     if (kExt && ph.source) {
         __pipeline_wait_prior(0);
@@ -533,14 +557,15 @@ __device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhas
         q2_row(DH, y, h0, h1, h2);
         q2_row(DC, y, c0, c1, c2);
         const double tep = (kExt && ph.litho) ? tep_at(ph, height(t, gj, y)) : ph.Tep;
+        double Trow = 0.0, Prow = 0.0;   // by row, as the split form adds them
 #pragma unroll
         for (int q = 0; q < kNQ; ++q) {
             const double x = t.g[q];
             PhaseLean pl;
             phase_plain<false>(ph.sk, quad(h0, h1, h2, x), quad(c0, c1, c2, x), tep, pl);
             const double w = t.cw[b * kNQ + q];
-            Tsum = fma(w, pl.T, Tsum);
-            Psum = fma(w, pl.phil, Psum);
+            Trow = fma(w, pl.T, Trow);
+            Prow = fma(w, pl.phil, Prow);
             if (kExt && ph.source) {
                 const int at = (int)(threadIdx.x & 31) * kCellPoints + b * kNQ + q;
                 const double factor = pl.phil == 0.0 ? 0.0 : (ph.theta == 0.0 ? pl.phil : pow(pl.phil, 1.0 + ph.theta));
@@ -550,6 +575,8 @@ __device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhas
                 Rsum += fabs(wv);
             }
         }
+        Tsum += Trow;
+        Psum += Prow;
     }
     // Porosities are not negative: the cell is wet where their mean is not 0.
     a.flags[cell] = (unsigned char)(fl | (Psum > 0.0 ? FLAG_WET : 0));
@@ -589,8 +616,8 @@ __device__ __forceinline__ void side_line(const FaceArgs& a, long long cell, boo
                                           SideLine& s) {
     double DH[9], DC[9];
     load_rec(a.rec, cell, DH, DC);
-    s.mH = __ldg(a.H + cell);
-    s.mC = __ldg(a.C + cell);
+    s.mH = MP_LD(a.H + cell);
+    s.mC = MP_LD(a.C + cell);
     if (row) { q2_row(DH, fixed, s.h0, s.h1, s.h2); q2_row(DC, fixed, s.c0, s.c1, s.c2); }
     else { q2_col(DH, fixed, s.h0, s.h1, s.h2); q2_col(DC, fixed, s.c0, s.c1, s.c2); }
 }
@@ -705,9 +732,9 @@ __device__ __forceinline__ void plain_velocities(const Physics& ph, const PhaseL
         const double bulk = ephi * cl + (1.0 - ephi) * cs;
         clb = bulk > 0.0 ? cl / bulk : 0.0;
     }
-    const double flux = (ph.theta == 0.0 || ephi == 0.0 ? ephi : pow(ephi, 1.0 + ph.theta)) * ud;
-    vn = vs + flux;
-    ve = fma(clb, flux, vs);
+    const double factor = ph.theta == 0.0 || ephi == 0.0 ? ephi : pow(ephi, 1.0 + ph.theta);
+    vn = fma(factor, ud, vs);
+    ve = fma(clb, __dmul_rn(factor, ud), vs);
 }
 
 // face_point of an interior edge between two plain cells. With local speeds
@@ -780,6 +807,10 @@ __device__ __forceinline__ EdgeAt edge_by_kind(int nx, int ny, long long kk) {
     if (k < 2u * (unsigned)nx) return EdgeAt{true, (int)(k < (unsigned)nx ? k : k - nx), k < (unsigned)nx ? 0 : ny};
     k -= 2u * (unsigned)nx;
     return EdgeAt{false, k < (unsigned)ny ? 0 : nx, (int)(k < (unsigned)ny ? k : k - ny)};
+}
+
+__device__ __forceinline__ long long edge_id(int nx, int ny, const EdgeAt& g) {
+    return g.horizontal ? (long long)g.j * nx + g.i : (long long)nx * (ny + 1) + (long long)g.j * (nx + 1) + g.i;
 }
 
 // Left/right cells and orientation as the reference's Build (evolve.cpp:230-251).
@@ -864,8 +895,8 @@ __device__ __forceinline__ void edge_line(const FaceArgs& a, long long cell, boo
                                           double (&h)[3], double (&c)[3]) {
     double DH[9], DC[9];
     load_rec(a.rec, cell, DH, DC);
-    DH[0] += __ldg(a.H + cell);
-    DC[0] += __ldg(a.C + cell);
+    DH[0] += MP_LD(a.H + cell);
+    DC[0] += MP_LD(a.C + cell);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         if (horizontal) {
@@ -887,6 +918,15 @@ __device__ __forceinline__ void store_face(const FaceArgs& a, long long e, doubl
     a.face[3 * nE + e] = half * fluxMix;
 }
 
+// The Gauss point taken l-th: the centre, then the two pairs.
+__device__ __forceinline__ int face_point_at(int l) { return l == 0 ? 2 : (l & 1 ? 2 + ((l + 1) >> 1) : 2 - (l >> 1)); }
+// Eutectic temperature at the point s of an edge.
+template <bool kExt>
+__device__ __forceinline__ double face_tep(const StageHot& t, const FaceArgs& a, const Physics& ph, const EdgeAt& at, double s) {
+    if (!(kExt && ph.litho)) return ph.Tep;
+    return tep_at(ph, at.horizontal ? t.y0 + (a.gj0 + at.j) * t.dy : height(t, a.gj0 + at.j, s));
+}
+
 // A wall edge of a plain cell (in warps of their own, edge_by_kind). Out of
 // line: its branches in the interior edges' loop cost that loop registers
 // (147 us against 130 at 640x1280).
@@ -900,14 +940,14 @@ __device__ __noinline__ void face_wall(const StageHot& t, const FaceArgs& a, con
     const double sgn = g.reverse ? -1.0 : 1.0;
     double fluxH = 0.0, fluxC = 0.0, fluxMix = 0.0, rate = 0.0;
     int st = 0;
-    for (int q = 0; q < kNQ; ++q) {
-        const double x = t.g[q], w = t.gw[q];
+    for (int l = 0; l < kNQ; ++l) {
+        const int q = face_point_at(l);
+        const double x = t.g[q], x2 = x * x, w = t.gw[q];
         const double vs = sgn * __ldg(a.vsn + e * kNQ + q), ud = sgn * __ldg(a.udn + e * kNQ + q);
-        const double tep = !(kExt && ph.litho) ? ph.Tep
-                         : tep_at(ph, at.horizontal ? t.y0 + (a.gj0 + at.j) * t.dy : height(t, a.gj0 + at.j, x));
-        const double cx = quad(c[0], c[1], c[2], x);
+        const double tep = face_tep<kExt>(t, a, ph, at, x);
+        const double cx = fma(c[1], x, fma(c[2], x2, c[0]));
         PhaseLean A;
-        phase_plain<true>(ph.sk, quad(h[0], h[1], h[2], x), cx, tep, A);
+        phase_plain<true>(ph.sk, fma(h[1], x, fma(h[2], x2, h[0])), cx, tep, A);
         const PointFlux pf = wall_point_plain(ph, A, cx, wet, vs, ud, tep, st);
         fluxH = fma(w, pf.fh, fluxH);
         fluxC = fma(w, pf.fc, fluxC);
@@ -951,8 +991,7 @@ __device__ __forceinline__ void face_edge(const StageHot& t, const FaceArgs& a, 
             const double s = m ? -x : x;
             const long long v = g.e * kNQ + (m ? 2 - p : 2 + p);
             const double vs = __ldg(a.vsn + v), ud = __ldg(a.udn + v);
-            const double tep = !(kExt && ph.litho) ? ph.Tep
-                             : tep_at(ph, at.horizontal ? t.y0 + (a.gj0 + at.j) * t.dy : height(t, a.gj0 + at.j, s));
+            const double tep = face_tep<kExt>(t, a, ph, at, s);
             const double cl = fma(cL[1], s, eCL), cr = fma(cR[1], s, eCR);
             PhaseLean A, B;
             phase_plain<true>(ph.sk, fma(hL[1], s, eHL), cl, tep, A);
@@ -1016,10 +1055,10 @@ __device__ __noinline__ void diffusion_general(const StageHot& t, const FaceArgs
     double mHL = 0, mCL = 0, mHR = 0, mCR = 0;
     if (type == 1) {
         load_rec(a.rec, L, DL, CL);
-        mHL = __ldg(a.H + L); mCL = __ldg(a.C + L);
+        mHL = MP_LD(a.H + L); mCL = MP_LD(a.C + L);
         if (!boundary) {
             load_rec(a.rec, Rc, DR, CR);
-            mHR = __ldg(a.H + Rc); mCR = __ldg(a.C + Rc);
+            mHR = MP_LD(a.H + Rc); mCR = MP_LD(a.C + Rc);
         }
     }
     double integral = 0.0, rate = a.face[2 * nE + e];
@@ -1095,8 +1134,8 @@ __device__ __forceinline__ void diffusion_plain(const StageHot& t, const FaceArg
         const long long cell = n ? g.R : g.L;
         double DH[9], DC[9];
         load_rec(a.rec, cell, DH, DC);
-        DH[0] += __ldg(a.H + cell);
-        DC[0] += __ldg(a.C + cell);
+        DH[0] += MP_LD(a.H + cell);
+        DC[0] += MP_LD(a.C + cell);
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
@@ -1173,6 +1212,15 @@ __device__ __forceinline__ void diffusion_edge(const StageHot& t, const FaceArgs
 
 // ----------------------------------------------------------------- sum kernel
 
+// Where a block of the accumulation (or axpy) kernels leaves its share, and
+// who adds the shares up: the block that finishes last, in share order.
+struct Shares {
+    Partial* partial;      // `count` shares
+    Totals* totals;
+    unsigned* ticket;      // blocks finished; 0 between launches
+    int count;
+};
+
 enum SumMode : int { SUM_STORE_L = 0, SUM_RK = 1 };
 
 struct SumArgs {
@@ -1189,7 +1237,7 @@ struct SumArgs {
     double* rate;          // optional per-cell rate
     int mode;
     double a0, a1, dt;     // next = a0*U^n + a1*(U + dt*L)
-    Partial* partial;
+    Shares shares;
     const double* dtp;     // when set, dt is read from device memory (batched instances)
     int gj0 = 0, gny = 0;  // slab: global row of local row 0, global rows
     long long cbeg = 0;    // cells [cbeg, cend) are accumulated (cend < 0: all)
@@ -1222,28 +1270,63 @@ __device__ __forceinline__ double warp_min(double v) {
     return v;
 }
 
-// Deterministic block reduction of a Partial (fixed shuffle tree per block).
-__device__ void block_reduce_write(Partial v, Partial* out) {
-    __shared__ double sh[32][11];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double r[11] = {v.maxRate, v.divergence, v.bH, v.bC, v.HI, v.CI, v.Hmin, v.Cmin, v.Cmax, v.nonfinite, v.sH};
-    r[0] = warp_max(r[0]); r[1] = warp_max(r[1]);
-    r[2] = warp_sum(r[2]); r[3] = warp_sum(r[3]); r[4] = warp_sum(r[4]); r[5] = warp_sum(r[5]);
-    r[6] = warp_min(r[6]); r[7] = warp_min(r[7]); r[8] = warp_max(r[8]); r[9] = warp_max(r[9]);
-    r[10] = warp_sum(r[10]);
-    if (lane == 0)
-        for (int k = 0; k < 11; ++k) sh[warp][k] = r[k];
+// Deterministic reduction of one Partial per thread over the first kRedBlock
+// threads of a block (every thread of the block calls; valid in thread 0).
+// The 11 fields lie in shared memory as rows: a warp folds whole rows, lane l
+// the entries l, l + 32, ... in order, then its shuffle tree. Reducing all
+// fields in every warp and again over the warps took two thirds of a small
+// block's time (55 dependent shuffle steps twice).
+constexpr int kFields = 11;
+__device__ __forceinline__ Partial block_reduce(const Partial& v) {
+    __shared__ double sh[kFields][kRedBlock];
+    __shared__ double out[kFields];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     __syncthreads();
-    if (warp == 0) {
-        const int nw = (blockDim.x + 31) >> 5;
-        const Partial id = partial_identity();
-        double s[11] = {id.maxRate, id.divergence, 0, 0, 0, 0, id.Hmin, id.Cmin, id.Cmax, 0, 0};
-        if (lane < nw) for (int k = 0; k < 11; ++k) s[k] = sh[lane][k];
-        s[0] = warp_max(s[0]); s[1] = warp_max(s[1]);
-        s[2] = warp_sum(s[2]); s[3] = warp_sum(s[3]); s[4] = warp_sum(s[4]); s[5] = warp_sum(s[5]);
-        s[6] = warp_min(s[6]); s[7] = warp_min(s[7]); s[8] = warp_max(s[8]); s[9] = warp_max(s[9]);
-        s[10] = warp_sum(s[10]);
-        if (lane == 0) *out = Partial{s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], s[8], s[9], s[10]};
+    if (tid < kRedBlock) {
+        const double r[kFields] = {v.maxRate, v.divergence, v.Cmax, v.nonfinite, v.Hmin, v.Cmin, v.bH, v.bC, v.HI, v.CI, v.sH};
+#pragma unroll
+        for (int k = 0; k < kFields; ++k) sh[k][tid] = r[k];
+    }
+    __syncthreads();
+    // Rows 0-3: maxima, 4-5: minima, 6-10: sums.
+    for (int k = warp; k < kFields; k += (int)(blockDim.x >> 5)) {
+        double x = sh[k][lane];
+        auto fold = [&](double y) { x = k < 4 ? fmax(x, y) : k < 6 ? fmin(x, y) : x + y; };
+#pragma unroll
+        for (int n = 32; n < kRedBlock; n += 32) fold(sh[k][lane + n]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) fold(__shfl_down_sync(0xffffffffu, x, o));
+        if (lane == 0) out[k] = x;
+    }
+    __syncthreads();
+    return Partial{out[0], out[1], out[6], out[7], out[8], out[9], out[4], out[5], out[2], out[3], out[10]};
+}
+
+// This block's share, and by the last block the totals.
+__device__ __forceinline__ void finish_block(const Partial& v, const Shares& s, int index) {
+    __shared__ bool last;
+    const Partial b = block_reduce(v);
+    if (threadIdx.x == 0) {
+        s.partial[index] = b;
+        __threadfence();
+        last = atomicAdd(s.ticket, 1u) == (unsigned)s.count - 1u;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    Partial w = partial_identity();
+    for (int k = threadIdx.x; k < s.count; k += kRedBlock) {
+        const double* f = reinterpret_cast<const double*>(s.partial + k);
+        Partial q;
+        double* d = reinterpret_cast<double*>(&q);
+#pragma unroll
+        for (int n = 0; n < kFields; ++n) d[n] = __ldcg(f + n);
+        fold_partial(w, q);
+    }
+    w = block_reduce(w);
+    if (threadIdx.x == 0) {
+        *s.totals = Totals{w.maxRate, w.divergence, w.bH, w.bC, w.HI, w.CI, w.Hmin, w.Cmin, w.Cmax, w.nonfinite, w.sH};
+        *s.ticket = 0;
     }
 }
 
@@ -1251,7 +1334,7 @@ __device__ void block_reduce_write(Partial v, Partial* out) {
 // the stage reductions into v.
 // kSrc: the adiabatic source terms are added. kArea: per-cell areas.
 template <bool kSrc = false, bool kArea = false>
-__device__ __forceinline__ void sum_cell(const SumArgs& a, unsigned cell, Partial& v) {
+__device__ __forceinline__ void sum_cell(const SumArgs& a, unsigned cell, const double* dtp, Partial& v) {
     const int nx = a.nx, ny = a.ny;
     const long long nI = (long long)nx * (ny + 1);
     const long long nE = nI + (long long)(nx + 1) * ny;
@@ -1273,8 +1356,8 @@ __device__ __forceinline__ void sum_cell(const SumArgs& a, unsigned cell, Partia
     double rH = 0.0, rC = 0.0, rr = 0.0, dv = 0.0, bH = 0.0, bC = 0.0;
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
-        const double FH = __ldg(a.face + ids[f]), FC = __ldg(a.face + nE + ids[f]);
-        const double FR = __ldg(a.face + 2 * nE + ids[f]), FM = __ldg(a.face + 3 * nE + ids[f]);
+        const double FH = MP_LD(a.face + ids[f]), FC = MP_LD(a.face + nE + ids[f]);
+        const double FR = MP_LD(a.face + 2 * nE + ids[f]), FM = MP_LD(a.face + 3 * nE + ids[f]);
         rH += sg[f] * FH;
         rC += sg[f] * FC;
         rr += FR;
@@ -1284,22 +1367,22 @@ __device__ __forceinline__ void sum_cell(const SumArgs& a, unsigned cell, Partia
     double sH = 0.0;
     if (kSrc) {
         // The source terms follow the face terms, as the reference adds them.
-        rH += __ldg(a.srcH + cell); rr += __ldg(a.srcR + cell); sH = __ldg(a.srcS + cell);
+        rH += MP_LD(a.srcH + cell); rr += MP_LD(a.srcR + cell); sH = MP_LD(a.srcS + cell);
     }
-    if (gj == 0) { bH += __ldg(a.face + eb); bC += __ldg(a.face + nE + eb); }
-    if (gj == gny - 1) { bH += __ldg(a.face + et); bC += __ldg(a.face + nE + et); }
-    if (i == 0) { bH += __ldg(a.face + el); bC += __ldg(a.face + nE + el); }
-    if (i == nx - 1) { bH += __ldg(a.face + er); bC += __ldg(a.face + nE + er); }
+    if (gj == 0) { bH += MP_LD(a.face + eb); bC += MP_LD(a.face + nE + eb); }
+    if (gj == gny - 1) { bH += MP_LD(a.face + et); bC += MP_LD(a.face + nE + et); }
+    if (i == 0) { bH += MP_LD(a.face + el); bC += MP_LD(a.face + nE + el); }
+    if (i == nx - 1) { bH += MP_LD(a.face + er); bC += MP_LD(a.face + nE + er); }
     double nh, nc;
     if (a.mode == SUM_RK) {
-        const double dt_ = a.dtp ? *a.dtp : a.dt;
-        const double h = __ldg(a.H + cell), c = __ldg(a.C + cell);
+        const double dt_ = dtp ? *dtp : a.dt;
+        const double h = MP_LD(a.H + cell), c = MP_LD(a.C + cell);
         const double sh_ = __dadd_rn(h, __dmul_rn(dt_, rH));
         const double sc_ = __dadd_rn(c, __dmul_rn(dt_, rC));
-        nh = __dadd_rn(__dmul_rn(a.a0, __ldg(a.H0 + cell)), __dmul_rn(a.a1, sh_));
-        nc = __dadd_rn(__dmul_rn(a.a0, __ldg(a.C0 + cell)), __dmul_rn(a.a1, sc_));
+        nh = __dadd_rn(__dmul_rn(a.a0, MP_LD(a.H0 + cell)), __dmul_rn(a.a1, sh_));
+        nc = __dadd_rn(__dmul_rn(a.a0, MP_LD(a.C0 + cell)), __dmul_rn(a.a1, sc_));
     } else {
-        nh = __ldg(a.H + cell); nc = __ldg(a.C + cell);
+        nh = MP_LD(a.H + cell); nc = MP_LD(a.C + cell);
     }
     a.outH[cell] = a.mode == SUM_RK ? nh : rH;
     a.outC[cell] = a.mode == SUM_RK ? nc : rC;
@@ -1314,15 +1397,18 @@ __device__ __forceinline__ void sum_cell(const SumArgs& a, unsigned cell, Partia
 }
 
 // The kSumPer cells of this thread in the sum block starting at first.
-// `first` counts from the start of the accumulated range [cbeg, cend).
+// `first` counts from the start of the accumulated range [cbeg, cend); dtp:
+// where the step size is (null: in the arguments).
 template <bool kSrc = false, bool kArea = false>
-__device__ __forceinline__ Partial sum_cells(const SumArgs& a, long long first) {
+__device__ __forceinline__ Partial sum_cells(const SumArgs& a, long long first, const double* dtp) {
     const long long end = a.cend >= 0 ? a.cend : (long long)a.nx * a.ny;
+    const int per = sum_per(end - a.cbeg);
     Partial v = partial_identity();
 #pragma unroll
     for (int k = 0; k < kSumPer; ++k) {
+        if (k >= per) break;
         const long long c = a.cbeg + first + k * kRedBlock + threadIdx.x;
-        if (c < end) sum_cell<kSrc, kArea>(a, (unsigned)c, v);
+        if (c < end) sum_cell<kSrc, kArea>(a, (unsigned)c, dtp, v);
     }
     return v;
 }
@@ -1333,9 +1419,11 @@ __device__ __forceinline__ Partial sum_cells(const SumArgs& a, long long first) 
 __device__ __forceinline__ Partial axpy_cells(long long n, const double* H0, const double* C0, const double* LH,
                                               const double* LC, double dt, double area, double* H1, double* C1,
                                               long long first, const double* cell_area = nullptr) {
+    const int per = sum_per(n);
     Partial v = partial_identity();
 #pragma unroll
     for (int q = 0; q < kSumPer; ++q) {
+        if (q >= per) break;
         const long long k = first + q * kRedBlock + threadIdx.x;
         if (k >= n) continue;
         const double h = __dadd_rn(H0[k], __dmul_rn(dt, LH[k]));

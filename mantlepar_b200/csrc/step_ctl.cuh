@@ -25,10 +25,6 @@
 #include "stage_kernels.cuh"
 
 namespace mp {
-namespace {
-
-constexpr int kMaxAttempts = 41;     // the first attempt and 40 retries
-constexpr int kCtlThreads = 256;
 
 // Options of the step rule (per run, identical for every instance).
 struct StepOpts {
@@ -39,12 +35,6 @@ struct StepOpts {
     int snap_end;       // after a step within 32 eps of t_end, time = t_end (batched engine)
     int end_reports;    // a step not taken at the end time reports time = t_end (single instance)
     int restore_time;   // a failure after commit restores the step's start time (single instance)
-};
-
-// Why an instance's step failed, for the host's message.
-enum : int {
-    FAIL_NONE = 0, FAIL_STAGE = 1, FAIL_RATE = 2, FAIL_RETRIES = 3, FAIL_FIXED_LIMIT = 4, FAIL_FIXED_STAGE = 5,
-    FAIL_BALANCE = 6
 };
 
 struct InstCtl {
@@ -66,6 +56,17 @@ struct CtlHeader {
     int attempts;                     // attempts of the current step
     int total_attempts;               // over the launch (kernel count)
     int stop;                         // a single instance failed: no further steps
+};
+
+namespace {
+
+constexpr int kMaxAttempts = 41;     // the first attempt and 40 retries
+constexpr int kCtlThreads = 256;
+
+// Why an instance's step failed, for the host's message.
+enum : int {
+    FAIL_NONE = 0, FAIL_STAGE = 1, FAIL_RATE = 2, FAIL_RETRIES = 3, FAIL_FIXED_LIMIT = 4, FAIL_FIXED_STAGE = 5,
+    FAIL_BALANCE = 6
 };
 
 // Explicitly rounded FP64 (the host loops compile without contraction).
@@ -96,35 +97,128 @@ __device__ __forceinline__ void fail_inst(InstCtl& c, int status, int fail) {
 // Block-wide "any" of a per-thread flag (one block of kCtlThreads).
 __device__ __forceinline__ int block_any(int v) { return __syncthreads_or(v); }
 
+// ------------------------------------------------ the rule for one instance
+
+// Start of a step: its dt. r: the step's report; stop: a run has ended.
+__device__ __forceinline__ void begin_one(InstCtl& c, mp_step_report& r, const StepOpts& so, bool stop) {
+    r = mp_step_report{};
+    c.pending = c.valid = c.done = 0;
+    if (!c.used || c.status || stop) { r.status = c.status; return; }
+    if (at_end(c.time, c.t_end)) {
+        c.time = c.t_end;
+        if (so.end_reports) r.time = c.t_end;
+        return;
+    }
+    c.first = c.cur;
+    c.remaining = sb(c.t_end, c.time);
+    const double cap = so.fixed ? so.dt_initial : (c.accepted == 0 ? so.dt_initial : so.dt_max);
+    const double limit = c.cur.maxRate > 0 ? dv(so.cfl, c.cur.maxRate) : so.dt_max;
+    double dt = mn(c.remaining, cap);
+    if (so.fixed && !(dt <= ml(limit, 1 + 1e-12))) { fail_inst(c, MP_ERR_ARG_OUTOFRANGE, FAIL_FIXED_LIMIT); r.status = c.status; return; }
+    if (!so.fixed) dt = mn(dt, limit);
+    c.dt = dt;
+    c.start = c.time;
+    c.retries = 0;
+    c.courant = 0.0;
+    c.pending = 1;
+}
+
+// Start of an attempt: the retry bounds.
+__device__ __forceinline__ void attempt_one(InstCtl& c, const StepOpts& so) {
+    if (c.pending && !(c.dt >= mn(c.remaining, so.dt_min) && c.retries < 40))
+        fail_inst(c, MP_ERR_NOT_CONVERGED, FAIL_RETRIES);
+}
+
+// After stage `which` (2 or 3) of an attempt, with its status word and
+// totals. `last`: the attempt ends here (accept, fail, or halve dt).
+__device__ __forceinline__ void after_stage_one(InstCtl& c, const StepOpts& so, unsigned long long w, const Totals& t,
+                                                int which, int last) {
+    if (c.valid) {
+        if (w != ~0ULL) {
+            fail_inst(c, word_code(w), FAIL_STAGE);
+            c.word = w; c.fail_stage = which;
+        } else if (!isfinite(t.maxRate)) {
+            fail_inst(c, MP_ERR_FP, FAIL_RATE);
+            c.fail_stage = which;
+        } else {
+            double rate = mx(c.first.maxRate, t.maxRate);
+            if (which == 2) c.second = t;
+            else { c.third = t; rate = mx(mx(c.first.maxRate, c.second.maxRate), t.maxRate); }
+            c.courant = ml(c.dt, rate);
+            c.valid = c.courant <= ml(so.cfl, 1 + 1e-12) && admissible_dev(t, so.Xe);
+        }
+    }
+    if (last && c.pending) {
+        if (c.valid) { c.done = 1; c.pending = 0; }
+        else if (so.fixed) fail_inst(c, MP_ERR_ARG_OUTOFRANGE, FAIL_FIXED_STAGE);
+        else { c.dt = ml(c.dt, 0.5); c.retries += 1; }
+    }
+}
+
+// Balance check (evolve.cpp:486-490), commit bookkeeping and the report.
+__device__ __forceinline__ void commit_one(InstCtl& c, mp_step_report& r, const StepOpts& so) {
+    if (!c.done) return;
+    const Totals& f = c.first;
+    const Totals& s = c.second;
+    const Totals& fin = so.rk3 ? c.third : c.second;
+    double repH, repC, repS, bH, bC;
+    if (so.rk3) {
+        const double two3 = 2.0 / 3.0;
+        repH = ad(dv(ad(f.bH, s.bH), 6.0), ml(c.third.bH, two3));
+        repC = ad(dv(ad(f.bC, s.bC), 6.0), ml(c.third.bC, two3));
+        repS = ad(dv(ad(f.sH, s.sH), 6.0), ml(c.third.sH, two3));
+        bH = ad(sb(fin.HI, f.HI), ml(c.dt, sb(repH, repS)));
+        bC = ad(sb(fin.CI, f.CI), ml(c.dt, repC));
+    } else {
+        repH = ml(.5, ad(f.bH, s.bH));
+        repC = ml(.5, ad(f.bC, s.bC));
+        repS = ml(.5, ad(f.sH, s.sH));
+        bH = ad(sb(fin.HI, f.HI), ml(ml(.5, c.dt), sb(sb(ad(f.bH, s.bH), f.sH), s.sH)));
+        bC = ad(sb(fin.CI, f.CI), ml(ml(.5, c.dt), ad(f.bC, s.bC)));
+    }
+    if (!(fabs(bH) < ml(1e-10, mx(1.0, fabs(f.HI))) && fabs(bC) < 1e-10)) {
+        fail_inst(c, MP_ERR_PLIB, FAIL_BALANCE);
+        c.bal_H = bH; c.bal_C = bC;
+        return;
+    }
+    c.time = ad(c.start, c.dt);
+    if (so.snap_end && at_end(c.time, c.t_end)) c.time = c.t_end;
+    c.have_L = 0;
+    r.retries = c.retries; r.dt = c.dt; r.time = c.time; r.courant = c.courant;
+    r.boundaryH = repH; r.boundaryC = repC; r.sourceH = repS;
+    r.balanceH = bH; r.balanceC = bC; r.H_integral = fin.HI; r.C_integral = fin.CI;
+}
+
+// After L(U^{n+1}): the new L's totals and the report.
+__device__ __forceinline__ void after_rhs_one(InstCtl& c, mp_step_report& r, const StepOpts& so, unsigned long long w,
+                                              const Totals& t) {
+    if (c.done) {
+        if (w != ~0ULL) { fail_inst(c, word_code(w), FAIL_STAGE); c.word = w; c.fail_stage = 4; }
+        else if (!isfinite(t.maxRate)) { fail_inst(c, MP_ERR_FP, FAIL_RATE); c.fail_stage = 4; }
+        if (c.status) {
+            if (so.restore_time) c.time = c.start;
+        } else {
+            c.cur = t;
+            c.have_L = 1;
+            c.accepted += 1;
+            r.maxRate = c.cur.maxRate;
+            r.divergence = c.cur.divergence;
+        }
+    }
+    if (c.used) r.status = c.status;
+    c.done = 0;
+}
+
+// ------------------------------------------------------- the graphs' kernels
+
 // Start of a step: dt of every healthy instance; the attempt loop's
 // condition. reps: this step's report row.
 __global__ void __launch_bounds__(kCtlThreads) ctl_begin_kernel(InstCtl* ctl, int n, StepOpts so, CtlHeader* hdr,
                                                                 mp_step_report* reps, cudaGraphConditionalHandle attempt) {
     int any = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        InstCtl& c = ctl[i];
-        mp_step_report& r = reps[(size_t)hdr->step * n + i];
-        r = mp_step_report{};
-        c.pending = c.valid = c.done = 0;
-        if (!c.used || c.status || hdr->stop) { r.status = c.status; continue; }
-        if (at_end(c.time, c.t_end)) {
-            c.time = c.t_end;
-            if (so.end_reports) r.time = c.t_end;
-            continue;
-        }
-        c.first = c.cur;
-        c.remaining = sb(c.t_end, c.time);
-        const double cap = so.fixed ? so.dt_initial : (c.accepted == 0 ? so.dt_initial : so.dt_max);
-        const double limit = c.cur.maxRate > 0 ? dv(so.cfl, c.cur.maxRate) : so.dt_max;
-        double dt = mn(c.remaining, cap);
-        if (so.fixed && !(dt <= ml(limit, 1 + 1e-12))) { fail_inst(c, MP_ERR_ARG_OUTOFRANGE, FAIL_FIXED_LIMIT); r.status = c.status; continue; }
-        if (!so.fixed) dt = mn(dt, limit);
-        c.dt = dt;
-        c.start = c.time;
-        c.retries = 0;
-        c.courant = 0.0;
-        c.pending = 1;
-        any = 1;
+        begin_one(ctl[i], reps[(size_t)hdr->step * n + i], so, hdr->stop != 0);
+        any |= ctl[i].pending;
     }
     any = block_any(any);
     if (threadIdx.x == 0) {
@@ -138,8 +232,7 @@ __global__ void __launch_bounds__(kCtlThreads) ctl_attempt_kernel(InstCtl* ctl, 
                                                                   int* active, double* dt_dev) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         InstCtl& c = ctl[i];
-        if (c.pending && !(c.dt >= mn(c.remaining, so.dt_min) && c.retries < 40))
-            fail_inst(c, MP_ERR_NOT_CONVERGED, FAIL_RETRIES);
+        attempt_one(c, so);
         active[i] = c.pending;
         if (c.pending) dt_dev[i] = c.dt;
     }
@@ -166,29 +259,8 @@ __global__ void __launch_bounds__(kCtlThreads) ctl_after_stage_kernel(InstCtl* c
     int any = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         InstCtl& c = ctl[i];
-        if (c.valid) {
-            const unsigned long long w = words[i];
-            if (w != ~0ULL) {
-                fail_inst(c, word_code(w), FAIL_STAGE);
-                c.word = w; c.fail_stage = which;
-            } else if (!isfinite(tot[i].maxRate)) {
-                fail_inst(c, MP_ERR_FP, FAIL_RATE);
-                c.fail_stage = which;
-            } else {
-                const Totals& t = tot[i];
-                double rate = mx(c.first.maxRate, t.maxRate);
-                if (which == 2) c.second = t;
-                else { c.third = t; rate = mx(mx(c.first.maxRate, c.second.maxRate), t.maxRate); }
-                c.courant = ml(c.dt, rate);
-                c.valid = c.courant <= ml(so.cfl, 1 + 1e-12) && admissible_dev(t, so.Xe);
-            }
-        }
+        after_stage_one(c, so, words[i], tot[i], which, last);
         words[i] = ~0ULL;
-        if (last && c.pending) {
-            if (c.valid) { c.done = 1; c.pending = 0; }
-            else if (so.fixed) fail_inst(c, MP_ERR_ARG_OUTOFRANGE, FAIL_FIXED_STAGE);
-            else { c.dt = ml(c.dt, 0.5); c.retries += 1; }
-        }
         active[i] = c.valid;
         any |= c.pending;
     }
@@ -205,52 +277,20 @@ __global__ void __launch_bounds__(kCtlThreads) ctl_after_stage_kernel(InstCtl* c
     }
 }
 
-// Balance check (evolve.cpp:486-490), commit bookkeeping and the report;
-// `active` gates the state copy and the evaluation of L(U^{n+1}).
+// Balance check and commit; `active` gates the state copy and the evaluation
+// of L(U^{n+1}).
 __global__ void __launch_bounds__(kCtlThreads) ctl_commit_kernel(InstCtl* ctl, int n, StepOpts so, CtlHeader* hdr,
                                                                  mp_step_report* reps, unsigned long long* words,
                                                                  int* active) {
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        InstCtl& c = ctl[i];
         words[i] = ~0ULL;
-        if (c.done) {
-            const Totals& f = c.first;
-            const Totals& s = c.second;
-            const Totals& fin = so.rk3 ? c.third : c.second;
-            double repH, repC, repS, bH, bC;
-            if (so.rk3) {
-                const double two3 = 2.0 / 3.0;
-                repH = ad(dv(ad(f.bH, s.bH), 6.0), ml(c.third.bH, two3));
-                repC = ad(dv(ad(f.bC, s.bC), 6.0), ml(c.third.bC, two3));
-                repS = ad(dv(ad(f.sH, s.sH), 6.0), ml(c.third.sH, two3));
-                bH = ad(sb(fin.HI, f.HI), ml(c.dt, sb(repH, repS)));
-                bC = ad(sb(fin.CI, f.CI), ml(c.dt, repC));
-            } else {
-                repH = ml(.5, ad(f.bH, s.bH));
-                repC = ml(.5, ad(f.bC, s.bC));
-                repS = ml(.5, ad(f.sH, s.sH));
-                bH = ad(sb(fin.HI, f.HI), ml(ml(.5, c.dt), sb(sb(ad(f.bH, s.bH), f.sH), s.sH)));
-                bC = ad(sb(fin.CI, f.CI), ml(ml(.5, c.dt), ad(f.bC, s.bC)));
-            }
-            if (!(fabs(bH) < ml(1e-10, mx(1.0, fabs(f.HI))) && fabs(bC) < 1e-10)) {
-                fail_inst(c, MP_ERR_PLIB, FAIL_BALANCE);
-                c.bal_H = bH; c.bal_C = bC;
-            } else {
-                c.time = ad(c.start, c.dt);
-                if (so.snap_end && at_end(c.time, c.t_end)) c.time = c.t_end;
-                c.have_L = 0;
-                mp_step_report& r = reps[(size_t)hdr->step * n + i];
-                r.retries = c.retries; r.dt = c.dt; r.time = c.time; r.courant = c.courant;
-                r.boundaryH = repH; r.boundaryC = repC; r.sourceH = repS;
-                r.balanceH = bH; r.balanceC = bC; r.H_integral = fin.HI; r.C_integral = fin.CI;
-            }
-        }
-        active[i] = c.done;
+        commit_one(ctl[i], reps[(size_t)hdr->step * n + i], so);
+        active[i] = ctl[i].done;
     }
 }
 
-// After L(U^{n+1}): the new L's totals, the step count and the run's loop
-// condition (bounded by the requested step count).
+// After L(U^{n+1}): the step count and the run's loop condition (bounded by
+// the requested step count).
 __global__ void __launch_bounds__(kCtlThreads) ctl_after_rhs_kernel(InstCtl* ctl, int n, StepOpts so, const Totals* tot,
                                                                     unsigned long long* words, mp_step_report* reps,
                                                                     CtlHeader* hdr, int stop_on_fail,
@@ -258,25 +298,9 @@ __global__ void __launch_bounds__(kCtlThreads) ctl_after_rhs_kernel(InstCtl* ctl
     int failed = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         InstCtl& c = ctl[i];
-        mp_step_report& r = reps[(size_t)hdr->step * n + i];
-        if (c.done) {
-            const unsigned long long w = words[i];
-            if (w != ~0ULL) { fail_inst(c, word_code(w), FAIL_STAGE); c.word = w; c.fail_stage = 4; }
-            else if (!isfinite(tot[i].maxRate)) { fail_inst(c, MP_ERR_FP, FAIL_RATE); c.fail_stage = 4; }
-            if (c.status) {
-                if (so.restore_time) c.time = c.start;
-            } else {
-                c.cur = tot[i];
-                c.have_L = 1;
-                c.accepted += 1;
-                r.maxRate = c.cur.maxRate;
-                r.divergence = c.cur.divergence;
-            }
-        }
+        after_rhs_one(c, reps[(size_t)hdr->step * n + i], so, words[i], tot[i]);
         words[i] = ~0ULL;
-        if (c.used) r.status = c.status;
         failed |= c.used && c.status != 0;
-        c.done = 0;
     }
     failed = block_any(failed);
     if (threadIdx.x == 0) {

@@ -1,8 +1,8 @@
 // Coupled H/C transport on B200: FP64 stage kernels, the SSPRK2/SSPRK3 time
 // loop and the mp_transport_* entry points.
 //
-// One stage L(U) (RHS, src/couple/evolve.cpp:279-384) is four kernels and a
-// fixed-order reduction:
+// One stage L(U) (RHS, src/couple/evolve.cpp:279-384) is four kernels, the
+// last of which also reduces its totals in a fixed order:
 //   recon_kernel      per cell: candidate smoothness + weights, limiter theta,
 //                     limited deviation polynomials;
 //   cellphase_kernel  per cell: 5x5 cell quadrature of the phase (T, phi, wet
@@ -25,6 +25,7 @@
 #include "tables.hpp"
 #include "quad_kernels.cuh"
 #include "quad_tables.hpp"
+#include "small_steps.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -119,20 +120,20 @@ __global__ void __launch_bounds__(128, 4) diffusion_kernel(const __grid_constant
 template <bool kSrc, bool kArea = false>
 __global__ void __launch_bounds__(kRedBlock) sum_kernel(SumArgs a) {
     if (gated_off(a.gate)) return;
-    const Partial v = sum_cells<kSrc, kArea>(a, (long long)blockIdx.x * kSumCells);
-    block_reduce_write(v, a.partial + blockIdx.x);
+    const Partial v = sum_cells<kSrc, kArea>(a, (long long)blockIdx.x * sum_cells_per_block(a.cend - a.cbeg), a.dtp);
+    finish_block(v, a.shares, (int)blockIdx.x);
 }
 
 // U1 = U^n + dt*L^n with the admissibility/integral partials of U1 (dtp:
 // dt read from device memory; gate: see ReconArgs).
 __global__ void __launch_bounds__(kRedBlock) axpy_kernel(int n, const double* H0, const double* C0, const double* LH,
                                                          const double* LC, double dt, double area, double* H1,
-                                                         double* C1, Partial* partial, const double* cell_area,
+                                                         double* C1, Shares shares, const double* cell_area,
                                                          const double* dtp = nullptr, const int* gate = nullptr) {
     if (gated_off(gate)) return;
-    const Partial v = axpy_cells(n, H0, C0, LH, LC, dtp ? *dtp : dt, area, H1, C1, (long long)blockIdx.x * kSumCells,
+    const Partial v = axpy_cells(n, H0, C0, LH, LC, dtp ? *dtp : dt, area, H1, C1, (long long)blockIdx.x * sum_cells_per_block(n),
                                  cell_area);
-    block_reduce_write(v, partial + blockIdx.x);
+    finish_block(v, shares, (int)blockIdx.x);
 }
 
 // Commit of an accepted step on the device: U^{n+1} (a stage buffer) into U^n.
@@ -142,21 +143,6 @@ __global__ void __launch_bounds__(kRedBlock) commit_kernel(long long n, const do
     for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
         H[k] = sH[k];
         C[k] = sC[k];
-    }
-}
-
-// Fixed-order reduction of the block partials into one Totals.
-__global__ void __launch_bounds__(1024) reduce_kernel(const Partial* partial, int nblocks, Totals* out,
-                                                      const int* gate = nullptr) {
-    if (gated_off(gate)) return;
-    Partial v = partial_identity();
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) fold_partial(v, partial[b]);
-    __shared__ Partial result;
-    block_reduce_write(v, &result);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        *out = Totals{result.maxRate, result.divergence, result.bH, result.bC, result.HI, result.CI,
-                      result.Hmin, result.Cmin, result.Cmax, result.nonfinite, result.sH};
     }
 }
 
@@ -188,6 +174,7 @@ struct mp_transport {
     double* rate = nullptr;
     mp::Partial* partial = nullptr;
     mp::Totals* d_tot = nullptr;
+    unsigned* d_ticket = nullptr;          // finished blocks of the running reduction
     mp::Totals* h_tot = nullptr;           // pinned, several slots
     unsigned long long* d_status = nullptr;
     unsigned long long* h_status = nullptr;
@@ -222,7 +209,8 @@ struct mp_transport {
     // graph launch, decisions by the step controller; the graph is captured
     // again when a setter changes what it captured (gen).
     bool use_graph = true;
-    unsigned long long gen = 1, graph_gen = 0;
+    unsigned long long gen = 1, graph_gen = 0, small_gen = 0;
+    int small_blocks = 0;                  // steps in one kernel of so many blocks (small_steps.cu), or 0: the graph
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     mp::InstCtl *d_ctl = nullptr, *h_ctl = nullptr;
@@ -282,7 +270,7 @@ void free_all(mp_transport* t) {
     for (void* p : {(void*)t->h_ctl, (void*)t->h_hdr, (void*)t->h_rep}) if (p) cudaFreeHost(p);
     for (cudaEvent_t e : t->ev_pool) cudaEventDestroy(e);
     void* bufs[] = {t->H, t->C, t->S1H, t->S1C, t->S2H, t->S2C, t->LH, t->LC, t->T, t->phi,
-                    t->rec, t->flags, t->vsn, t->udn, t->face, t->rate, t->partial, t->d_tot, t->d_status,
+                    t->rec, t->flags, t->vsn, t->udn, t->face, t->rate, t->partial, t->d_tot, t->d_ticket, t->d_status,
                     t->cvs_y, t->cud_y, t->srcH, t->srcR, t->srcS};
     for (void* b : bufs) if (b) cudaFree(b);
     if (t->qbuf) cudaFree(t->qbuf);
@@ -348,6 +336,9 @@ void launch_stage_kernels(int nx, int ny, const StageRange& rg, const ParamTable
     }
 }
 
+// The shares of a launch of `count` blocks of the accumulation or axpy kernel.
+Shares shares_of(const mp_transport* t, int count) { return Shares{t->partial, t->d_tot, t->d_ticket, count}; }
+
 // Launch one stage evaluation of state (H, C). mode SUM_STORE_L writes L to
 // (outH, outC); SUM_RK writes a0*U^n + a1*(U + dt*L). Totals land in *d_tot.
 // gate / dtp (device-resident steps): a device flag that switches the whole
@@ -390,7 +381,7 @@ mp_status launch_stage(mp_transport* t, const double* H, const double* C, int mo
     }
     {
         SumArgs a{t->nx, t->ny, t->host_tab.area, 1.0 / t->host_tab.area, t->face, H, C, t->H, t->C, outH, outC, t->rate, mode, a0, a1, dt,
-                  t->partial, dtp, t->range.gj0, t->range.gny, (long long)t->range.own0 * t->nx,
+                  shares_of(t, t->sum_blocks), dtp, t->range.gj0, t->range.gny, (long long)t->range.own0 * t->nx,
                   (long long)t->range.own1 * t->nx, sb.srcH, sb.srcR, sb.srcS, t->cell_area, gate, t->d_status};
         if (t->quad) {
             if (sb.srcH) timed(t, 3, [&] { sum_kernel<true, true><<<t->sum_blocks, kRedBlock, 0, s>>>(a); });
@@ -400,8 +391,7 @@ mp_status launch_stage(mp_transport* t, const double* H, const double* C, int mo
             else timed(t, 3, [&] { sum_kernel<false><<<t->sum_blocks, kRedBlock, 0, s>>>(a); });
         }
     }
-    timed(t, 4, [&] { reduce_kernel<<<1, 1024, 0, s>>>(t->partial, t->sum_blocks, t->d_tot, gate); });
-    count_launch(t->quad ? 2 : 5);
+    count_launch(t->quad ? 1 : 4);
     if (!t->quad && t->ph.diffusion) count_launch();
     MP_CUDA(cudaGetLastError());
     return MP_OK;
@@ -475,7 +465,7 @@ mp_status do_step(mp_transport* t, mp_step_report& rep) {
     double courant = 0.0;
     Totals second{}, third{}, fin{};
     const size_t o0 = own_begin(t), on = own_count(t);
-    const int nblk_axpy = (int)((on + kSumCells - 1) / kSumCells);
+    const int per_block = sum_cells_per_block((long long)on), nblk_axpy = (int)((on + per_block - 1) / per_block);
     for (;;) {
         if (!(dt >= std::min(remaining, o.dt_min) && retries < 40)) {
             set_error("Coupled step cannot satisfy admissibility/CFL above minimum step");
@@ -486,11 +476,10 @@ mp_status do_step(mp_transport* t, mp_step_report& rep) {
         timed(t, 4, [&] {
             axpy_kernel<<<nblk_axpy, kRedBlock, 0, s>>>((int)on, t->H + o0, t->C + o0, t->LH + o0, t->LC + o0, dt,
                                                          t->host_tab.area,
-                                                         t->S1H + o0, t->S1C + o0, t->partial,
+                                                         t->S1H + o0, t->S1C + o0, shares_of(t, nblk_axpy),
                                                          t->cell_area ? t->cell_area + o0 : nullptr);
         });
-        timed(t, 4, [&] { reduce_kernel<<<1, 1024, 0, s>>>(t->partial, nblk_axpy, t->d_tot); });
-        count_launch(2);
+        count_launch();
         MP_CUDA(cudaGetLastError());
         MP_TRY(read_totals(t, adm, failed, "stage 1"));
         valid = admissible(adm, Xe);
@@ -627,13 +616,12 @@ mp_status capture_steps(mp_transport* t, cudaGraph_t g) {
     MP_CUDA(cudaStreamEndCapture(s, &tmp));
     MP_TRY(add_while(step_body, leaves, attempt, &attempt_node, &attempt_body));
     const size_t o0 = own_begin(t), on = own_count(t);
-    const int nblk_axpy = (int)((on + kSumCells - 1) / kSumCells);
+    const int per_block = sum_cells_per_block((long long)on), nblk_axpy = (int)((on + per_block - 1) / per_block);
     MP_CUDA(cudaStreamBeginCaptureToGraph(s, attempt_body, nullptr, nullptr, 0, mode));
     ctl_attempt_kernel<<<1, kCtlThreads, 0, s>>>(t->d_ctl, 1, so, t->d_hdr, t->d_gate, t->d_dt);
     axpy_kernel<<<nblk_axpy, kRedBlock, 0, s>>>((int)on, t->H + o0, t->C + o0, t->LH + o0, t->LC + o0, 0.0,
-                                                 t->host_tab.area, t->S1H + o0, t->S1C + o0, t->partial,
+                                                 t->host_tab.area, t->S1H + o0, t->S1C + o0, shares_of(t, nblk_axpy),
                                                  t->cell_area ? t->cell_area + o0 : nullptr, t->d_dt, t->d_gate);
-    reduce_kernel<<<1, 1024, 0, s>>>(t->partial, nblk_axpy, t->d_tot, t->d_gate);
     ctl_after_axpy_kernel<<<1, kCtlThreads, 0, s>>>(t->d_ctl, 1, so, t->d_tot, t->d_status, t->d_gate);
     MP_TRY(launch_stage(t, t->S1H, t->S1C, SUM_RK, rk3 ? 0.75 : 0.5, rk3 ? 0.25 : 0.5, 0.0, t->S2H, t->S2C, nullptr,
                         t->d_gate, t->d_dt));
@@ -666,7 +654,8 @@ void release_graph(mp_transport* t) {
     t->graph_gen = 0;
 }
 
-mp_status ensure_graph(mp_transport* t) {
+// Control records of the device-resident steps.
+mp_status ensure_ctl(mp_transport* t) {
     if (!t->d_ctl) {
         MP_CUDA(cudaMalloc((void**)&t->d_ctl, sizeof(InstCtl)));
         MP_CUDA(cudaMalloc((void**)&t->d_hdr, sizeof(CtlHeader)));
@@ -677,6 +666,22 @@ mp_status ensure_graph(mp_transport* t) {
         MP_CUDA(cudaMallocHost((void**)&t->h_hdr, sizeof(CtlHeader)));
         MP_CUDA(cudaMallocHost((void**)&t->h_rep, kGraphSteps * sizeof(mp_step_report)));
     }
+    return MP_OK;
+}
+
+// The handle as the one-kernel form of the steps takes it.
+SmallMesh small_mesh(mp_transport* t) {
+    SmallMesh m{};
+    m.nx = t->nx; m.ny = t->ny; m.tab = &t->host_tab; m.ph = &t->ph; m.quad = t->quad; m.q = t->qdev;
+    m.cell_area = t->cell_area;
+    m.H = t->H; m.C = t->C; m.S1H = t->S1H; m.S1C = t->S1C; m.S2H = t->S2H; m.S2C = t->S2C; m.LH = t->LH; m.LC = t->LC;
+    m.T = t->T; m.phi = t->phi; m.rec = static_cast<double*>(t->rec); m.face = t->face; m.rate = t->rate;
+    m.flags = t->flags; m.vsn = t->vsn; m.udn = t->udn; m.partial = t->partial; m.status = t->d_status;
+    m.ctl = t->d_ctl; m.hdr = t->d_hdr; m.reports = t->d_rep; m.opts = single_step_opts(t);
+    return m;
+}
+
+mp_status ensure_graph(mp_transport* t) {
     if (t->graph_exec && t->graph_gen == t->gen) return MP_OK;
     release_graph(t);
     MP_CUDA(cudaGraphCreate(&t->graph, 0));
@@ -728,11 +733,18 @@ mp_status graph_failure(mp_transport* t, const InstCtl& c) {
 mp_status graph_steps(mp_transport* t, int nsteps, mp_step_report* reports) {
     NvtxRange range("mp_transport steps (device-resident graph)");
     if (!t->have_L) MP_TRY(eval_current(t));
-    MP_TRY(ensure_graph(t));
+    MP_TRY(ensure_ctl(t));
+    const SmallMesh sm = small_mesh(t);
+    if (t->small_gen != t->gen) {
+        t->small_blocks = t->range.gny == 0 ? small_steps_blocks(sm) : 0;
+        t->small_gen = t->gen;
+    }
+    const bool small = t->small_blocks > 0;
+    if (!small) MP_TRY(ensure_graph(t));
     cudaStream_t s = t->stream;
     // Kernels of one stage evaluation: reconstruction, cell phase, faces,
-    // sums, reduction (a quad mesh: WENO and limiter apart, one more).
-    const int sk = (t->quad ? 6 : 5) + (t->ph.diffusion ? 1 : 0);
+    // sums (a quad mesh: WENO and limiter apart, one more).
+    const int sk = (t->quad ? 5 : 4) + (t->ph.diffusion ? 1 : 0);
     const bool rk3 = t->opts.integrator == MP_SSPRK3;
     for (int done = 0; done < nsteps; done += kGraphSteps) {
         const int chunk = std::min(kGraphSteps, nsteps - done);
@@ -742,14 +754,16 @@ mp_status graph_steps(mp_transport* t, int nsteps, mp_step_report* reports) {
         *t->h_hdr = CtlHeader{0, chunk, 0, 0, 0};
         MP_CUDA(cudaMemcpyAsync(t->d_ctl, t->h_ctl, sizeof(InstCtl), cudaMemcpyHostToDevice, s));
         MP_CUDA(cudaMemcpyAsync(t->d_hdr, t->h_hdr, sizeof(CtlHeader), cudaMemcpyHostToDevice, s));
-        MP_CUDA(cudaGraphLaunch(t->graph_exec, s));
+        if (small) MP_TRY(launch_small_steps(sm, t->small_blocks, s));
+        else MP_CUDA(cudaGraphLaunch(t->graph_exec, s));
         MP_CUDA(cudaMemcpyAsync(t->h_ctl, t->d_ctl, sizeof(InstCtl), cudaMemcpyDeviceToHost, s));
         MP_CUDA(cudaMemcpyAsync(t->h_hdr, t->d_hdr, sizeof(CtlHeader), cudaMemcpyDeviceToHost, s));
         MP_CUDA(cudaMemcpyAsync(t->h_rep, t->d_rep, (size_t)chunk * sizeof(mp_step_report), cudaMemcpyDeviceToHost, s));
         MP_CUDA(cudaStreamSynchronize(s));
         t->host_syncs += 1;
         const CtlHeader h = *t->h_hdr;
-        count_launch((unsigned long long)h.step * (4 + sk) + (unsigned long long)h.total_attempts * (4 + (sk + 1) * (rk3 ? 2 : 1)));
+        if (small) count_launch();
+        else count_launch((unsigned long long)h.step * (4 + sk) + (unsigned long long)h.total_attempts * (3 + (sk + 1) * (rk3 ? 2 : 1)));
         t->time = c.time;
         t->accepted = c.accepted;
         t->curTot = c.cur;
@@ -860,7 +874,8 @@ mp_status create_impl(const mp_mesh_desc* mesh, bool slab, int row_begin, int ro
     const int tb = build_stage_tables(mesh->nx, mesh->ny, mesh->x0, mesh->x1, mesh->y0, mesh->y1, t->host_tab);
     if (tb) { delete t; set_error("stencil table construction failed"); return (mp_status)tb; }
     make_param_tables(t->host_tab, t->ptab);
-    t->sum_blocks = (int)((own_count(t) + kSumCells - 1) / kSumCells);
+    const int per_block = sum_cells_per_block((long long)own_count(t));
+    t->sum_blocks = (int)((own_count(t) + per_block - 1) / per_block);
     const size_t N = t->N, NE = t->NE;
     cudaError_t e = cudaSuccess;
     if (t->ph.source)
@@ -875,6 +890,8 @@ mp_status create_impl(const mp_mesh_desc* mesh, bool slab, int row_begin, int ro
     alloc((void**)&t->face, 4 * NE * sizeof(double));
     alloc((void**)&t->partial, (size_t)std::max(t->sum_blocks, 1) * sizeof(Partial));
     alloc((void**)&t->d_tot, sizeof(Totals));
+    alloc((void**)&t->d_ticket, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemsetAsync(t->d_ticket, 0, sizeof(unsigned), t->stream);
     alloc((void**)&t->d_status, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&t->h_tot, sizeof(Totals));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&t->h_status, sizeof(unsigned long long));
@@ -924,7 +941,7 @@ extern "C" size_t mp_transport_instance_bytes(const mp_mesh_desc* mesh, int quad
     size_t b = 11 * pages(N * sizeof(double))                   // state, stage buffers, L, T, phi, rate
              + pages(rec_doubles(N) * sizeof(double)) + pages(N)   // records, flags
              + 2 * pages(NE * kNQ * sizeof(double)) + pages(4 * NE * sizeof(double))   // velocities, face values
-             + pages(((N + kSumCells - 1) / kSumCells) * sizeof(Partial)) + page;
+             + pages((N / sum_cells_per_block((long long)N) + 1) * sizeof(Partial)) + page;
     if (quads) {
         const size_t V = 2 * (nx + 1) * (ny + 1);
         // Per-cell tables and geometry, vertices and edge spacing in one
@@ -1233,8 +1250,11 @@ extern "C" mp_status mp_probe_fp64_peak(mp_stream_t stream, double* tflops) {
 
 namespace mp {
 
-size_t raw_partial_bytes(size_t ncell) { return ((ncell + kSumCells - 1) / kSumCells) * sizeof(Partial); }
-size_t raw_totals_bytes() { return sizeof(Totals); }
+size_t raw_partial_bytes(size_t ncell) {
+    const size_t per = (size_t)sum_cells_per_block((long long)ncell);
+    return (ncell + per - 1) / per * sizeof(Partial);
+}
+size_t raw_totals_bytes() { return sizeof(Totals) + sizeof(unsigned); }
 
 // One stage evaluation L(U) (STORE_L mode) on buffers the caller provides:
 // tab (host StageTables, passed to the kernels by value), rec (18 doubles per
@@ -1259,9 +1279,11 @@ mp_status stage_rhs_raw(int nx, int ny, const mp_transport_opts& o, const double
     for (int w = 0; w < 4; ++w) { ph.wall_type[w] = 0; ph.wall_value[w] = 0.0; }
     const size_t N = (size_t)nx * ny;
     const size_t NE = (size_t)nx * (ny + 1) + (size_t)(nx + 1) * ny;
-    const int sum_blocks = (int)((N + kSumCells - 1) / kSumCells);
+    const int per_block = sum_cells_per_block((long long)N), sum_blocks = (int)((N + per_block - 1) / per_block);
     Partial* part = static_cast<Partial*>(partial);
     Totals* tot = static_cast<Totals*>(totals);
+    unsigned* ticket = reinterpret_cast<unsigned*>(tot + 1);
+    MP_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned), s));
     MP_CUDA(cudaMemsetAsync(status, 0xff, sizeof(unsigned long long), s));
     (void)NE;
     ParamTables pt;
@@ -1269,11 +1291,11 @@ mp_status stage_rhs_raw(int nx, int ny, const mp_transport_opts& o, const double
     launch_stage_kernels(nx, ny, whole(ny), pt, ph, H, C, rec, wet, T, phi, vsn, udn, face, status, nullptr, s,
                                  nullptr);
     {
-        SumArgs a{nx, ny, tab.area, 1.0 / tab.area, face, H, C, H, C, rhsH, rhsC, rate, SUM_STORE_L, 0.0, 0.0, 0.0, part};
+        SumArgs a{nx, ny, tab.area, 1.0 / tab.area, face, H, C, H, C, rhsH, rhsC, rate, SUM_STORE_L, 0.0, 0.0, 0.0,
+                  Shares{part, tot, ticket, sum_blocks}, nullptr, 0, 0, 0, (long long)N};
         sum_kernel<false><<<sum_blocks, kRedBlock, 0, s>>>(a);
     }
-    reduce_kernel<<<1, 1024, 0, s>>>(part, sum_blocks, tot);
-    count_launch(5);
+    count_launch(4);
     MP_CUDA(cudaGetLastError());
     Totals host_tot;
     unsigned long long host_status = 0;

@@ -155,3 +155,35 @@ def test_diffusion_and_source(nx, ny, patchy, types, values):
     assert per_cell(got["phi"], ref["phi"]) <= 1e-12
     for k in ("rhsH", "rhsC", "rate"):
         assert np.max(np.abs(got[k] - ref[k])) <= 1e-12 * np.max(np.abs(ref[k]))
+
+
+@pytest.mark.parametrize("mesh", ["uniform", "lithostatic", "perturbed"])
+@pytest.mark.parametrize("nx,ny", [(2, 2), (9, 3), (16, 16), (17, 31), (32, 32), (31, 33), (32, 48), (41, 38)])
+def test_small_meshes_step_as_the_host_loop(nx, ny, mesh):
+    # Steps in one cluster kernel (up to 1536 cells, quads 1024) and in the
+    # graph beyond, both against the host-driven loop: bit for bit, with
+    # plain and other cells, retries and an end time inside the run.
+    from mantlepar_b200.transport import Transport, TransportConfig
+    w = sy.Workload(nx=nx, ny=ny, seed=nx)
+    xy = sy.quad_vertices(w, 1, 0.2, 11) if mesh == "perturbed" else None
+    vs, ud = sy.face_velocity(w) if xy is None else sy.face_velocity_quads(w, xy)
+    H, C = patchy_state(w) if nx > 8 else sy.initial_state(w)
+    got = []
+    for device in (True, False):
+        t = Transport(w, TransportConfig(cfl=0.4, integrator=3 if nx % 2 else 2), vertices=xy)
+        t.set_device_steps(device)
+        if mesh == "lithostatic":
+            t.set_pressure_model(t.LITHOSTATIC, 1.02)
+        t.set_face_velocity(vs, ud)
+        t.set_state(H, C)
+        code, reps = t.step(3, raise_on_error=False)
+        if code == 0:
+            t.set_time_control(t.CFL, reps[-1]["time"] + 1.5 * reps[-1]["dt"])
+            code, more = t.step(4, raise_on_error=False)
+            reps += more
+        got.append((code, reps, t.get_time(), t.get_state()))
+        t.close()
+    a, b = got
+    assert a[:3] == b[:3]
+    for x, y in zip(a[3], b[3]):
+        assert np.array_equal(x, y)
