@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(128) batch_recon_kernel(const InstArgs* args, 
 // kExt: the adiabatic source (alpha0 != 0) is compiled in.
 template <bool kExt>
 __global__ void __launch_bounds__(128, kExt ? 4 : 6) batch_phase_kernel(const InstArgs* args, const Work* work, const int* active,
-                                                          const __grid_constant__ Physics ph) {
+                                                          const __grid_constant__ Physics ph, int averages) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const CellPhaseArgs& a = args[w.inst].phase;
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(128, kExt ? 4 : 6) batch_phase_kernel(const In
     double* vy = kExt ? source_buf + (threadIdx.x >> 5) * (2 * 32 * kCellPoints) : nullptr;
     const long long N = (long long)a.nx * a.ny, cell = (long long)w.a + threadIdx.x, first = cell - (threadIdx.x & 31);
     if (kExt && ph.source && first < N) stage_source(a, first, N, vy);
-    cellphase_cell<kExt>(*a.tab, a, ph, cell, N, vy);
+    cellphase_cell<kExt>(*a.tab, a, ph, cell, N, averages != 0, vy);
 }
 
 __global__ void __launch_bounds__(128, 5) batch_face_kernel(const InstArgs* args, const Work* work, const int* active,
@@ -136,12 +136,13 @@ __global__ void __launch_bounds__(128, 4) batch_quad_limit_kernel(const QuadStag
 }
 
 __global__ void __launch_bounds__(128, 4) batch_quad_phase_kernel(const QuadStageArgs* args, const Work* work,
-                                                                  const int* active, const __grid_constant__ Physics ph) {
+                                                                  const int* active, const __grid_constant__ Physics ph,
+                                                                  int averages) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const QuadStageArgs& a = args[w.inst];
     const long long cell = (long long)w.a + threadIdx.x;
-    if (cell < (long long)a.nx * a.ny) quad_cellphase_cell(a, ph, cell);
+    if (cell < (long long)a.nx * a.ny) quad_cellphase_cell(a, ph, cell, averages != 0);
 }
 
 __global__ void __launch_bounds__(128, 5) batch_quad_face_kernel(const QuadStageArgs* args, const Work* work,
@@ -621,14 +622,26 @@ mp_status set_active(mp_batch* b, const std::vector<int>& act) {
     return MP_OK;
 }
 
-void launch_kind(mp_batch* b, int kind) {
+// T and phi of one stage kind on the active instances (averages: of every
+// cell; otherwise the cells whose checks, wet flag or source need them).
+void launch_phases(mp_batch* b, int kind, bool averages) {
+    cudaStream_t s = b->stream;
+    const InstArgs* args = static_cast<const InstArgs*>(b->d_args[kind]);
+    if (b->ph.source) timed(b, 1, [&] { batch_phase_kernel<true><<<b->cap_wphase, 128, kSourceBufBytes, s>>>(args, b->d_wphase, b->d_active, b->ph, averages); });
+    else timed(b, 1, [&] { batch_phase_kernel<false><<<b->cap_wphase, 128, 0, s>>>(args, b->d_wphase, b->d_active, b->ph, averages); });
+}
+void launch_quad_phases(mp_batch* b, int kind, bool averages) {
+    const QuadStageArgs* qa = static_cast<const QuadStageArgs*>(b->d_qargs[kind]);
+    timed(b, 1, [&] { batch_quad_phase_kernel<<<b->cap_wqphase, 128, 0, b->stream>>>(qa, b->d_wqphase, b->d_active, b->ph, averages); });
+}
+
+void launch_kind(mp_batch* b, int kind, bool averages = true) {
     cudaStream_t s = b->stream;
     const InstArgs* args = static_cast<const InstArgs*>(b->d_args[kind]);
     const Tuning tu = b->tune;
     // Grids cover the work lists' capacities (padded items exit at once).
     timed(b, 0, [&] { batch_recon_kernel<<<b->cap_wrecon, dim3(tu.bx, tu.by), 0, s>>>(args, b->d_wrecon, b->d_active, b->ph, tu.cpt); });
-    if (b->ph.source) timed(b, 1, [&] { batch_phase_kernel<true><<<b->cap_wphase, 128, kSourceBufBytes, s>>>(args, b->d_wphase, b->d_active, b->ph); });
-    else timed(b, 1, [&] { batch_phase_kernel<false><<<b->cap_wphase, 128, 0, s>>>(args, b->d_wphase, b->d_active, b->ph); });
+    launch_phases(b, kind, averages);
     timed(b, 2, [&] { batch_face_kernel<<<b->cap_wface, 128, 0, s>>>(args, b->d_wface, b->d_active, b->ph); });
     if (b->ph.diffusion)
         timed(b, 2, [&] { batch_diffusion_kernel<<<b->cap_wface, 128, 0, s>>>(args, b->d_wface, b->d_active, b->ph); });
@@ -638,7 +651,7 @@ void launch_kind(mp_batch* b, int kind) {
         const QuadStageArgs* qa = static_cast<const QuadStageArgs*>(b->d_qargs[kind]);
         timed(b, 0, [&] { batch_quad_weno_kernel<<<b->cap_wqrec, dim3(32, 4), 0, s>>>(qa, b->d_wqrec, b->d_active); });
         timed(b, 0, [&] { batch_quad_limit_kernel<<<b->cap_wqrec, dim3(32, 4), 0, s>>>(qa, b->d_wqrec, b->d_active, b->ph); });
-        timed(b, 1, [&] { batch_quad_phase_kernel<<<b->cap_wqphase, 128, 0, s>>>(qa, b->d_wqphase, b->d_active, b->ph); });
+        launch_quad_phases(b, kind, averages);
         timed(b, 2, [&] { batch_quad_face_kernel<<<b->cap_wqface, 128, 0, s>>>(qa, b->d_wqface, b->d_active, b->ph); });
         if (b->ph.diffusion)
             timed(b, 2, [&] { batch_quad_diffusion_kernel<<<b->cap_wqface, 128, 0, s>>>(qa, b->d_wqface, b->d_active, b->ph); });
@@ -946,11 +959,11 @@ mp_status capture_graph(mp_batch* b, cudaGraph_t* out) {
     ctl_attempt_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_hdr, b->d_active, b->d_dt);
     batch_axpy_kernel<<<b->cap_wsum, kRedBlock, 0, s>>>(b->d_axpy, b->d_wsum, b->d_active);
     ctl_after_axpy_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_tot, b->d_status, b->d_active);
-    launch_kind(b, KIND_B);
+    launch_kind(b, KIND_B, false);
     ctl_after_stage_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_tot, b->d_status, b->d_active, 2,
                                                       rk3 ? 0 : 1, b->d_hdr, attempt);
     if (rk3) {
-        launch_kind(b, KIND_C);
+        launch_kind(b, KIND_C, false);
         ctl_after_stage_kernel<<<1, kCtlThreads, 0, s>>>(b->d_ctl, slots, so, b->d_tot, b->d_status, b->d_active, 3, 1,
                                                           b->d_hdr, attempt);
     }
@@ -1055,6 +1068,24 @@ mp_status graph_steps(mp_batch* b, int nsteps, mp_step_report* reports) {
         const int per_attempt = 4 + (b->stage_kernels + 1) * (b->opts.integrator == MP_SSPRK3 ? 2 : 1);
         count_launch((unsigned long long)h.step * (3 + b->stage_kernels + 1) +
                      (unsigned long long)h.total_attempts * per_attempt);
+        // T and phi of the stage that an instance failed after: the latest
+        // evaluation, whose averages the step left out.
+        for (int kind : {KIND_B, KIND_C}) {
+            std::vector<int> act(slots, 0);
+            bool any = false;
+            for (int i = 0; i < slots; ++i) {
+                const InstCtl& c = b->h_ctl[i];
+                act[i] = c.used && c.status && !b->inst[i].status && c.evaluated == (kind == KIND_B ? 2 : 3);
+                any = any || act[i];
+            }
+            if (!any) continue;
+            MP_TRY(set_active(b, act));
+            launch_phases(b, kind, true);
+            if (b->has_quads) launch_quad_phases(b, kind, true);
+            count_launch(b->has_quads ? 2 : 1);
+            MP_CUDA(cudaMemsetAsync(b->d_status, 0xff, slots * sizeof(unsigned long long), s));
+            MP_CUDA(cudaStreamSynchronize(s));   // h_active is written again
+        }
         for (int i = 0; i < slots; ++i) {
             MPInstance& in = b->inst[i];
             if (!in.used) continue;

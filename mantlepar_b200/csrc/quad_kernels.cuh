@@ -131,14 +131,16 @@ __device__ __noinline__ void quad_scan_exact(const QuadStageArgs& a, long long c
 
 // Extremes of both deviation polynomials over the cell's limiter points
 // (state_reconstruction.cpp:152-168): centre, 5x5 Gauss points, 5 points per
-// edge, the normal-line samples on this side. The points are formed in the
+// edge, the normal-line samples on this side; mq: the largest H value at the
+// centre and the Gauss points. The points are formed in the
 // cell's frame from its normalised corners (two FMAs each), so that a point
 // costs little beside its two Q2 values (16 FMAs): 2438 FP64 instructions per
 // warp and 225 us at 640x1280, against 3135 and 310 us with the points mapped
 // in physical coordinates and every value tested. Bound by the FP64 pipe; 3
 // resident blocks instead of 4 took 248 us, 5 (96 registers) 231.
 __device__ __forceinline__ void quad_scan(const QuadStageArgs& a, int i, int j, const NormalCell& k, double inv_h,
-                                          const double (&DH)[9], const double (&DC)[9], Extremes& eh, Extremes& ec) {
+                                          const double (&DH)[9], const double (&DC)[9], Extremes& eh, Extremes& ec,
+                                          double& mq) {
     const QuadDev& q = a.q;
     auto visit = [&](double x, double y) {
         const double vh = q2v(DH, x, y), vc = q2v(DC, x, y);
@@ -155,6 +157,7 @@ __device__ __forceinline__ void quad_scan(const QuadStageArgs& a, int i, int j, 
 #pragma unroll
         for (int r = 0; r < kNQ; ++r) visit(fma(x1, q.gq[r], x0), fma(y1, q.gq[r], y0));
     }
+    mq = eh.mx;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         long long id;
@@ -222,11 +225,11 @@ __device__ __forceinline__ void quad_limit_cell(const QuadStageArgs& a, const Ph
     int st_lim = 0;
     if (!(isfinite(mH) && mH >= 0.0 && isfinite(mC) && mC >= 0.0 && mC <= ph.k.Xe)) st_lim = E_OUTOFRANGE;
     Extremes eh, ec;
-    double size = 0.0;
+    double size = 0.0, mq;
 #pragma unroll
     for (int k = 0; k < 9; ++k) size += fabs(DH[k]) + fabs(DC[k]);
     if (size < kQuadGuard) {
-        quad_scan(a, i, j, normal_cell(f), f.inv_h, DH, DC, eh, ec);
+        quad_scan(a, i, j, normal_cell(f), f.inv_h, DH, DC, eh, ec, mq);
     } else {
         double D0[9], D1[9], ext[4];
         bool bad;
@@ -234,6 +237,7 @@ __device__ __forceinline__ void quad_limit_cell(const QuadStageArgs& a, const Ph
         for (int k = 0; k < 9; ++k) { D0[k] = DH[k]; D1[k] = DC[k]; }
         quad_scan_exact(a, cell, D0, D1, ext, &bad);
         eh = Extremes{ext[0], ext[1]};
+        mq = ext[0];
         ec = Extremes{ext[2], ext[3]};
         if (bad) st_lim = st_lim ? st_lim : E_FP;
     }
@@ -252,7 +256,7 @@ __device__ __forceinline__ void quad_limit_cell(const QuadStageArgs& a, const Ph
         r[(k + 9) * kRecStride] = DC[k] * thC;
     }
     flags[cell] = st_lim ? (unsigned char)FLAG_CHECK
-                         : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), loH, hiH, loC, hiC);
+                         : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), loH, hiH, loC, hiC, fma(thH, mq, mH));
     if (st_lim) record_error(status, PART_LIMIT, cell + (long long)gj0 * nx, st_lim);
 }
 __global__ void __launch_bounds__(128, 4) quad_limit_kernel(const __grid_constant__ QuadStageArgs a, const __grid_constant__ Physics ph, int jlo,
@@ -334,15 +338,18 @@ __device__ __noinline__ void quad_cellphase_general(const QuadStageArgs& a, cons
 }
 
 // The same quadrature of a plain cell (phase_plain): the points in the
-// cell's frame, and the Jacobian, which is linear in (r, s), per unit area.
+// cell's frame, and the Jacobian, which is linear in (r, s), per unit area;
+// averages as for cellphase_cell.
 // 93 us at 640x1280 (217 with every point tested and mapped in physical
 // coordinates); 5 and 6 resident blocks took 106 and 131 us.
-__device__ __forceinline__ void quad_cellphase_cell(const QuadStageArgs& a, const Physics& ph, long long cell) {
+__device__ __forceinline__ void quad_cellphase_cell(const QuadStageArgs& a, const Physics& ph, long long cell,
+                                                    bool averages) {
     const int nx = a.nx;
     const size_t N = (size_t)nx * a.ny;
     MP_CHECK_INDEX(a.status, cell, N);
     const unsigned char fl = a.flags[cell];
     if (!(fl & FLAG_PLAIN)) { quad_cellphase_general(a, ph, cell); return; }
+    if (!averages && !ph.litho && !ph.source) return;
     const QuadDev& q = a.q;
     const CellFrame f = cell_frame(q, nx, N, cell);
     const NormalCell k = normal_cell(f);
@@ -379,17 +386,18 @@ __device__ __forceinline__ void quad_cellphase_cell(const QuadStageArgs& a, cons
         Psum += Prow;
     }
     // Porosities are not negative: the cell is wet where their mean is not 0.
-    a.flags[cell] = (unsigned char)(fl | (Psum > 0.0 ? FLAG_WET : 0));
+    if (ph.litho) a.flags[cell] = (unsigned char)(fl | (Psum > 0.0 ? FLAG_WET : 0));
     a.T[cell] = Tsum;
     a.phi[cell] = Psum;
     if (ph.source) { a.src.srcH[cell] = Ssum; a.src.srcR[cell] = Rsum; a.src.srcS[cell] = Ssum * f.area; }
 }
 __global__ void __launch_bounds__(128, 4) quad_cellphase_kernel(const __grid_constant__ QuadStageArgs a, const __grid_constant__ Physics ph,
-                                                             long long c0, long long c1, const int* gate) {
+                                                             long long c0, long long c1, int averages,
+                                                             const int* gate) {
     if (gated_off(gate)) return;
     const long long cell = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (cell >= c1) return;
-    quad_cellphase_cell(a, ph, cell);
+    quad_cellphase_cell(a, ph, cell, averages != 0);
 }
 
 
@@ -650,13 +658,13 @@ __global__ void __launch_bounds__(128) quad_diffusion_kernel(const __grid_consta
 // on a general quad mesh; the accumulation is the shared sum kernel. Local
 // rows [rec0, rec1) are reconstructed, the edges [h0, h0+nh) and [v0, v0+nv)
 // (those of the advanced rows) get fluxes; local row 0 is global row gj0 of
-// gny (a whole mesh: gj0 = 0, gny = ny). gate: device flag, every kernel
+// gny (a whole mesh: gj0 = 0, gny = ny). averages: see cellphase_cell. gate: device flag, every kernel
 // returns at once while it is 0 (the device-resident step graph).
 void launch_quad_stage(const QuadDev& q, int nx, int ny, int gj0, int gny, int rec0, int rec1, long long h0,
                        long long nh, long long v0, long long nv, const Physics& ph, const double* H, const double* C,
                        double* rec, unsigned char* flags, double* T, double* phi, const double* vsn, const double* udn,
                        double* face, unsigned long long* status, double* theta, const SourcePtrs& src,
-                       cudaStream_t s, const int* gate = nullptr) {
+                       bool averages, cudaStream_t s, const int* gate = nullptr) {
     QuadStageArgs a;
     a.nx = nx; a.ny = ny; a.gj0 = gj0; a.gny = gny;
     a.H = H; a.C = C; a.rec = rec; a.flags = flags; a.T = T; a.phi = phi;
@@ -666,7 +674,7 @@ void launch_quad_stage(const QuadDev& q, int nx, int ny, int gj0, int gny, int r
     quad_weno_kernel<<<grd, blk, 0, s>>>(a, rec0, rec1, gate);
     quad_limit_kernel<<<grd, blk, 0, s>>>(a, ph, rec0, rec1, gate);
     const long long c0 = (long long)rec0 * nx, c1 = (long long)rec1 * nx;
-    quad_cellphase_kernel<<<(unsigned)((c1 - c0 + 127) / 128), 128, 0, s>>>(a, ph, c0, c1, gate);
+    quad_cellphase_kernel<<<(unsigned)((c1 - c0 + 127) / 128), 128, 0, s>>>(a, ph, c0, c1, averages, gate);
     const unsigned ge = (unsigned)((nh + nv + 127) / 128);
     quad_face_kernel<<<ge, 128, 0, s>>>(a, ph, h0, nh, v0, nv, gate);
     count_launch(4);

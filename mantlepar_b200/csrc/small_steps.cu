@@ -94,16 +94,19 @@ __device__ __forceinline__ double points_sum(const double (&w)[kNQ], double v) {
 }
 
 // Limiter factors, records and flag byte of the group's cell from each field's
-// extremes (lanes 0-3 field H, 4-7 field C, quarter `part` of its scan).
+// extremes (lanes 0-3 field H, 4-7 field C, quarter `part` of its scan; mq:
+// the largest value of its share of the cell quadrature points).
 template <class TepRange>
 __device__ __forceinline__ void small_limit(const Physics& ph, bool active, int part, int f, long long cell, double mean,
-                                            double lo, double hi, Extremes x, int st, bool bad, const double (&D)[9],
-                                            double* rec, unsigned char* flags, unsigned long long* status,
+                                            double lo, double hi, Extremes x, double mq, int st, bool bad,
+                                            const double (&D)[9], double* rec, unsigned char* flags, unsigned long long* status,
                                             TepRange&& tep_range) {
 #pragma unroll
     for (int o = 1; o <= 2; o <<= 1) {
         x.up(__shfl_xor_sync(kAll, x.mx, o));
         x.down(__shfl_xor_sync(kAll, x.mn, o));
+        const double y = __shfl_xor_sync(kAll, mq, o);
+        mq = y > mq ? y : mq;
     }
     const double th = theta_of(mean, lo, hi, x.mx, x.mn);
     const bool mean_ok = isfinite(mean) && mean >= 0.0 && (f == 0 || mean <= ph.k.Xe);
@@ -122,15 +125,17 @@ __device__ __forceinline__ void small_limit(const Physics& ph, bool active, int 
         double t0, t1;
         tep_range(t0, t1);
         flags[cell] = st_all || st_lim ? (unsigned char)FLAG_CHECK
-                                       : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), lo, hi, loC, hiC);
+                                       : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), lo, hi, loC, hiC, fma(th, mq, mean));
         if (st_all) record_error(status, PART_UPDATE, cell, st_all);
         if (st_lim) record_error(status, PART_LIMIT, cell, st_lim);
     }
 }
 
-// Reconstruction and limiter of a uniform mesh. Each lane of a field scans
+// Reconstruction and limiter of a uniform mesh, and the whole cell phase of
+// the cells that are not plain. Each lane of a field scans
 // two of the symmetric line pairs of scan_cell and one of the lines that
 // depend on the walls (the centre row as a pair at 0).
+template <bool kLitho>
 __device__ __noinline__ void small_recon(const SmallArgs& m, int kind, int group, int groups) {
     const StageHot& t = m.tab;
     const ReconArgs& a = m.recon[kind];
@@ -166,6 +171,7 @@ __device__ __noinline__ void small_recon(const SmallArgs& m, int kind, int group
         double D[9];
         const int st = reconstruct(t, candidate_mask(ci, cj), u, D);
         Extremes x{D[0], D[0]};
+        double mq;
         bool bad = false;
         if (small) {
             // Pairs: rows 0, g1 | g2, 0.8 | row 1, column 0.8 | column 1 (twice).
@@ -176,8 +182,11 @@ __device__ __noinline__ void small_recon(const SmallArgs& m, int kind, int group
                 const double p2[3] = {col ? D[2] : D[6], col ? D[5] : D[7], D[8]};
                 x.line_pair(c, p0, p1, p2);
             };
+            mq = D[0];
             pair(part == 3, ca);
+            if (part == 1) mq = x.mx;
             pair(part >= 2, cb);
+            if (part == 0) mq = x.mx;
             // The 0.3-size line of one side (parts 0, 1: bottom and top rows,
             // 2, 3: left and right columns), or the wall's three.
             const bool col = part >= 2;
@@ -197,8 +206,9 @@ __device__ __noinline__ void small_recon(const SmallArgs& m, int kind, int group
             for (int k = 0; k < 9; ++k) Dc[k] = D[k];
             scan_lines_exact(t, t.line_off[cj * 3 + ci], t.line_off[cj * 3 + ci + 1], Dc, mx, mn, bad);
             x = Extremes{mx, mn};
+            mq = mx;
         }
-        small_limit(m.ph, active, part, f, cell, mean, lo, hi, x, st, bad, D, a.rec, a.flags, a.status,
+        small_limit(m.ph, active, part, f, cell, mean, lo, hi, x, mq, st, bad, D, a.rec, a.flags, a.status,
                     [&](double& t0, double& t1) {
                         t0 = t1 = m.ph.Tep;
                         if (m.ph.litho) {
@@ -206,6 +216,9 @@ __device__ __noinline__ void small_recon(const SmallArgs& m, int kind, int group
                             t1 = tep_at(m.ph, t.y0 + (j + 1) * t.dy);
                         }
                     });
+        __syncwarp();
+        if (active && l == 0 && !(a.flags[cell] & FLAG_PLAIN)) cellphase_general<kLitho>(t, m.phase[kind], m.ph, cell);
+        __syncwarp();
     }
 }
 
@@ -244,6 +257,7 @@ __device__ __noinline__ void small_quad_recon(const SmallArgs& m, int kind, int 
 #pragma unroll
         for (int k = 0; k < 9; ++k) size += fabs(D[0][k]);
         Extremes x;
+        double mq;
         bool bad = false;
         if (size < 0.5 * kQuadGuard) {
             const NormalCell k = normal_cell(fr);
@@ -256,6 +270,7 @@ __device__ __noinline__ void small_quad_recon(const SmallArgs& m, int kind, int 
                 const double s = q.gq[n / kNQ], r = q.gq[n % kNQ];
                 visit(fma(fma(k.d.x, s, k.b.x), r, fma(k.c.x, s, k.m.x)), fma(fma(k.d.y, s, k.b.y), r, fma(k.c.y, s, k.m.y)));
             }
+            mq = x.mx;
             long long id;
             bool wall, rev;
             cell_edge(nx, ny, i, j, 0, ny, part, id, wall, rev);
@@ -283,8 +298,9 @@ __device__ __noinline__ void small_quad_recon(const SmallArgs& m, int kind, int 
             for (int k = 0; k < 9; ++k) Dc[k] = D[0][k];
             quad_scan_exact(a, cell, Dc, Dc, ext, &bad);
             x = Extremes{ext[0], ext[1]};
+            mq = ext[0];
         }
-        small_limit(m.ph, active, part, f, cell, mean, lo, hi, x, st, bad, D[0], a.rec, a.flags, a.status,
+        small_limit(m.ph, active, part, f, cell, mean, lo, hi, x, mq, st, bad, D[0], a.rec, a.flags, a.status,
                     [&](double& t0, double& t1) {
                         t0 = t1 = m.ph.Tep;
                         if (m.ph.litho) {
@@ -295,10 +311,13 @@ __device__ __noinline__ void small_quad_recon(const SmallArgs& m, int kind, int 
                             t1 = tep_at(m.ph, yhi);
                         }
                     });
+        __syncwarp();
+        if (active && l == 0 && !(a.flags[cell] & FLAG_PLAIN)) quad_cellphase_general(a, m.ph, cell);
+        __syncwarp();
     }
 }
 
-// Cell quadrature: lane b < 5 takes row b.
+// Cell quadrature of the plain cells: lane b < 5 takes row b.
 template <bool kQuad, bool kLitho>
 __device__ __noinline__ void small_phase(const SmallArgs& m, int kind, int group, int groups) {
     const int nx = m.nx, N = nx * m.ny, l = threadIdx.x & 7, b = min(l, kNQ - 1);
@@ -351,16 +370,10 @@ __device__ __noinline__ void small_phase(const SmallArgs& m, int kind, int group
             }
         }
         const double T = rows_sum(Trow), P = rows_sum(Prow);
-        if (active && l == 0) {
-            if (fl & FLAG_PLAIN) {
-                a.flags[cell] = (unsigned char)(fl | (P > 0.0 ? FLAG_WET : 0));
-                a.T[cell] = T;
-                a.phi[cell] = P;
-            } else if (kQuad) {
-                quad_cellphase_general(m.quad[kind], m.ph, cell);
-            } else {
-                cellphase_general<kLitho>(m.tab, a, m.ph, cell);
-            }
+        if (active && l == 0 && (fl & FLAG_PLAIN)) {
+            if (m.ph.litho) a.flags[cell] = (unsigned char)(fl | (P > 0.0 ? FLAG_WET : 0));
+            a.T[cell] = T;
+            a.phi[cell] = P;
         }
     }
 }
@@ -509,10 +522,12 @@ __global__ void __launch_bounds__(kSmallThreads, 1) small_steps_kernel(const __g
     // One stage evaluation; dt scales the Runge-Kutta combination.
     auto stage = [&](int kind, double dt) {
         if (kQuad) small_quad_recon(m, kind, group, groups);
-        else small_recon(m, kind, group, groups);
+        else small_recon<kLitho>(m, kind, group, groups);
         cluster.sync();
-        small_phase<kQuad, kLitho>(m, kind, group, groups);
-        cluster.sync();
+        // T and phi of the accepted state; with a lithostatic pressure every
+        // stage's wet flags, which the faces read.
+        if (kind == KIND_P || m.ph.litho) small_phase<kQuad, kLitho>(m, kind, group, groups);
+        if (m.ph.litho) cluster.sync();
         small_faces<kQuad, kLitho>(m, kind, group, groups);
         cluster.sync();
         small_sums<kQuad>(m, kind, rank, blocks, dt);

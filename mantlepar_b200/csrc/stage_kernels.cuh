@@ -170,14 +170,19 @@ enum : unsigned char { FLAG_WET = 1, FLAG_CHECK = 2, FLAG_PLAIN = 4 };
 // samples) within [lo, hi] up to roundoff, and Hliq at (hi_C, lowest tep) is
 // the lowest liquidus, so bounds that keep a margin of 1e-12 prove each
 // point's admissibility: the samples' (cell flagged otherwise: they are
-// checked one by one), and for a plain cell all of them.
+// checked one by one), and for a plain cell all of them. Melt begins where H
+// passes Tep, so with a constant pressure a plain cell is wet when topH, its
+// largest limited enthalpy at the quadrature points, does (with a
+// lithostatic pressure the quadrature decides).
 __device__ __forceinline__ unsigned char cell_flags(const Physics& ph, double tep_lo, double tep_hi, double loH, double hiH,
-                                                    double loC, double hiC) {
+                                                    double loC, double hiC, double topH) {
     const double Hliq = tep_lo + (1.0 - hiC * ph.sk.invXe) + ph.k.LD;
     const double slack = 1e-12 * (1.0 + fabs(hiH));
     if (!(tep_lo >= 0.0 && hiH + slack < Hliq)) return FLAG_CHECK;
-    return ph.sk.ordinary && tep_lo >= 1e-9 && tep_hi <= 1e100 && loH >= slack && loC >= 1e-90 &&
-           hiC <= ph.k.Xe * (1.0 - 1e-12) ? FLAG_PLAIN : 0;
+    if (!(ph.sk.ordinary && tep_lo >= 1e-9 && tep_hi <= 1e100 && loH >= slack && loC >= 1e-90 &&
+          hiC <= ph.k.Xe * (1.0 - 1e-12)))
+        return 0;
+    return FLAG_PLAIN | (!ph.litho && topH > ph.Tep ? FLAG_WET : 0);
 }
 
 struct ReconArgs {
@@ -256,12 +261,14 @@ struct Extremes {
 // symmetric pairs and their points as symmetric pairs (85 points in 280 FP64
 // operations, 84 of them comparisons); a wall adds its lines, so that a cell
 // takes the same operations whatever its neighbours in the warp are.
-__device__ __forceinline__ void scan_cell(const double (&D)[9], int ci, int cj, double& mx, double& mn) {
+// mq: the largest value at the 25 points of the cell quadrature.
+__device__ __forceinline__ void scan_cell(const double (&D)[9], int ci, int cj, double& mx, double& mn, double& mq) {
     Extremes x{D[0], D[0]};
     x.pairs(D[0], D[1], D[2]);
     const double r0[3] = {D[0], D[1], D[2]}, r1[3] = {D[3], D[4], D[5]}, r2[3] = {D[6], D[7], D[8]};
     x.line_pair(kG1, r0, r1, r2);
     x.line_pair(kG2, r0, r1, r2);
+    mq = x.mx;
     x.line_pair(0.8, r0, r1, r2);
     x.line_pair(1.0, r0, r1, r2);
     const double c0[3] = {D[0], D[3], D[6]}, c1[3] = {D[1], D[4], D[7]}, c2[3] = {D[2], D[5], D[8]};
@@ -299,7 +306,7 @@ constexpr double kScanGuard = 1e30;
 // composition).
 __device__ __forceinline__ void recon_field(const StageHot& t, const double* __restrict__ F, const unsigned (&at)[3][3],
                                             int ci, int cj, double top, double (&D)[9], double& mean, double& lo,
-                                            double& hi, double& th, int& st, bool& bad) {
+                                            double& hi, double& th, double& mq, int& st, bool& bad) {
     double u[3][3];
 #pragma unroll
     for (int dj = 0; dj < 3; ++dj)
@@ -329,10 +336,10 @@ __device__ __forceinline__ void recon_field(const StageHot& t, const double* __r
 #pragma unroll
         for (int m = 0; m < 9; ++m) Dc[m] = D[m];
         scan_lines_exact(t, t.line_off[cj * 3 + ci], t.line_off[cj * 3 + ci + 1], Dc, x, n, b);
-        mx = x; mn = n;
+        mx = mq = x; mn = n;
         bad = bad || b;
     } else {
-        scan_cell(D, ci, cj, mx, mn);
+        scan_cell(D, ci, cj, mx, mn, mq);
     }
     th = theta_of(mean, lo, hi, mx, mn);
 }
@@ -360,15 +367,15 @@ __device__ __forceinline__ void recon_cell(const StageHot& t, const ReconArgs& a
         }
     int st = 0;
     bool bad = false, means = true;
-    double loH = 0, hiH = 0, loC = 0, hiC = 0;
+    double loH = 0, hiH = 0, loC = 0, hiC = 0, topH = 0;
 #pragma unroll 1
     for (int f = 0; f < 2; ++f) {
-        double D[9], mean, lo, hi, th;
-        recon_field(t, f ? a.C : a.H, at, ci, cj, f ? ph.k.Xe : INFINITY, D, mean, lo, hi, th, st, bad);
+        double D[9], mean, lo, hi, th, mq;
+        recon_field(t, f ? a.C : a.H, at, ci, cj, f ? ph.k.Xe : INFINITY, D, mean, lo, hi, th, mq, st, bad);
         // state_reconstruction.cpp:187-188: admissible means.
         means = means && isfinite(mean) && mean >= 0.0 && (f == 0 || mean <= ph.k.Xe);
         if (f) { loC = lo; hiC = hi; }
-        else { loH = lo; hiH = hi; }
+        else { loH = lo; hiH = hi; topH = fma(th, mq, mean); }
         if (a.theta) a.theta[f * N + cell] = th;
         double* r = a.rec + rec_at(cell) + f * 9 * kRecStride;
 #pragma unroll
@@ -382,7 +389,7 @@ __device__ __forceinline__ void recon_cell(const StageHot& t, const ReconArgs& a
         t1 = tep_at(ph, t.y0 + (gj + 1) * t.dy);
     }
     a.flags[cell] = st || st_lim ? (unsigned char)FLAG_CHECK
-                                 : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), loH, hiH, loC, hiC);
+                                 : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), loH, hiH, loC, hiC, topH);
     if (st) record_error(a.status, PART_UPDATE, key, st);
     if (st_lim) record_error(a.status, PART_LIMIT, key, st_lim);
 }
@@ -529,12 +536,15 @@ __device__ __forceinline__ void stage_source(const CellPhaseArgs& a, long long f
     }
     __pipeline_commit();
 }
-// The cell of this lane, [0, end) (every lane of a warp calls).
+// The cell of this lane, [0, end) (every lane of a warp calls). averages: T
+// and phi are wanted; the stages inside a step, whose averages nothing reads,
+// leave out a plain cell unless its wet flag or source needs the quadrature.
 template <bool kExt>
 __device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhaseArgs& a, const Physics& ph, long long cell,
-                                               long long end, const double* vy = nullptr) {
+                                               long long end, bool averages, const double* vy = nullptr) {
     const bool valid = cell < end;
     const unsigned char fl = valid ? a.flags[cell] : 0;
+    if (!averages && !(kExt && (ph.litho || ph.source)) && (fl & FLAG_PLAIN)) return;
     double DH[9], DC[9];
     if (fl & FLAG_PLAIN) {
         load_rec(a.rec, cell, DH, DC);
@@ -579,7 +589,7 @@ __device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhas
         Psum += Prow;
     }
     // Porosities are not negative: the cell is wet where their mean is not 0.
-    a.flags[cell] = (unsigned char)(fl | (Psum > 0.0 ? FLAG_WET : 0));
+    if (kExt && ph.litho) a.flags[cell] = (unsigned char)(fl | (Psum > 0.0 ? FLAG_WET : 0));
     a.T[cell] = Tsum;
     a.phi[cell] = Psum;
     if (kExt && ph.source) {

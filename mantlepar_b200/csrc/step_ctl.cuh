@@ -48,6 +48,7 @@ struct InstCtl {
     // The step in progress.
     double dt, start, remaining, courant;
     int retries, pending, valid, done;
+    int evaluated;                    // stage (2, 3) evaluated last without its T and phi; 0: none since L(U^n)
     Totals first, second, third;
 };
 
@@ -134,6 +135,7 @@ __device__ __forceinline__ void attempt_one(InstCtl& c, const StepOpts& so) {
 __device__ __forceinline__ void after_stage_one(InstCtl& c, const StepOpts& so, unsigned long long w, const Totals& t,
                                                 int which, int last) {
     if (c.valid) {
+        c.evaluated = which;
         if (w != ~0ULL) {
             fail_inst(c, word_code(w), FAIL_STAGE);
             c.word = w; c.fail_stage = which;
@@ -193,6 +195,7 @@ __device__ __forceinline__ void commit_one(InstCtl& c, mp_step_report& r, const 
 __device__ __forceinline__ void after_rhs_one(InstCtl& c, mp_step_report& r, const StepOpts& so, unsigned long long w,
                                               const Totals& t) {
     if (c.done) {
+        c.evaluated = 0;
         if (w != ~0ULL) { fail_inst(c, word_code(w), FAIL_STAGE); c.word = w; c.fail_stage = 4; }
         else if (!isfinite(t.maxRate)) { fail_inst(c, MP_ERR_FP, FAIL_RATE); c.fail_stage = 4; }
         if (c.status) {

@@ -79,14 +79,14 @@ template <bool kExt>
 __global__ void __launch_bounds__(128, kExt ? 4 : 6) cellphase_kernel(const __grid_constant__ CellPhaseArgs a,
                                                            const __grid_constant__ Physics ph,
                                                            const __grid_constant__ ParamTables p, long long c0,
-                                                           long long c1) {
+                                                           long long c1, int averages) {
     if (gated_off(a.gate)) return;
     const long long cell = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x;
     extern __shared__ double source_buf[];
     double* vy = kExt ? source_buf + (threadIdx.x >> 5) * (2 * 32 * kCellPoints) : nullptr;
     const long long first = cell - (threadIdx.x & 31);
     if (kExt && ph.source && first < c1) stage_source(a, first, c1, vy);
-    cellphase_cell<kExt>(p.d, a, ph, cell, c1, vy);
+    cellphase_cell<kExt>(p.d, a, ph, cell, c1, averages != 0, vy);
 }
 // Edges [h0, h0 + nh) (horizontal) then [v0, v0 + nv) (vertical): every edge
 // of the mesh, or of a slab's owned cells.
@@ -299,7 +299,7 @@ mp_status check_status(mp_transport* t, const char* where) {
 // Launch the stage kernels of state (H, C).
 void launch_stage_kernels(int nx, int ny, const StageRange& rg, const ParamTables& pt, const Physics& ph, const double* H, const double* C, double* rec,
                           unsigned char* flags, double* T, double* phi, const double* vsn, const double* udn,
-                          double* face, unsigned long long* status, double* theta, cudaStream_t s,
+                          double* face, unsigned long long* status, double* theta, bool averages, cudaStream_t s,
                           mp_transport* prof, const SourceBufs& src = SourceBufs{}, const int* gate = nullptr) {
     const size_t NE = (size_t)nx * (ny + 1) + (size_t)(nx + 1) * ny;
     auto run = [&](int kind, auto&& f) { if (prof) timed(prof, kind, f); else f(); };
@@ -313,8 +313,8 @@ void launch_stage_kernels(int nx, int ny, const StageRange& rg, const ParamTable
                            src.cvs_y, src.cud_y, src.srcH, src.srcR, src.srcS, gate};
         const long long c0 = (long long)rg.rec0 * nx, c1 = (long long)rg.rec1 * nx;
         const unsigned g = (unsigned)((c1 - c0 + 127) / 128);
-        if (ph.litho || ph.source) run(1, [&] { cellphase_kernel<true><<<g, 128, ph.source ? kSourceBufBytes : 0, s>>>(a, ph, pt, c0, c1); });
-        else run(1, [&] { cellphase_kernel<false><<<g, 128, 0, s>>>(a, ph, pt, c0, c1); });
+        if (ph.litho || ph.source) run(1, [&] { cellphase_kernel<true><<<g, 128, ph.source ? kSourceBufBytes : 0, s>>>(a, ph, pt, c0, c1, averages); });
+        else run(1, [&] { cellphase_kernel<false><<<g, 128, 0, s>>>(a, ph, pt, c0, c1, averages); });
     }
     {
         FaceArgs a{nx, ny, nullptr, H, C, rec, flags, vsn, udn, face, status, rg.gj0, rg.gny, gate};
@@ -355,6 +355,10 @@ mp_status launch_stage(mp_transport* t, const double* H, const double* C, int mo
         if (rc) { set_error("halo exchange failed (%d)", rc); return rc > 0 ? (mp_status)rc : MP_ERR_CUDA; }
     }
     mp_transport* prof = t->profile ? t : nullptr;
+    // The averages T and phi that get_state returns are those of the latest
+    // evaluation: in a device-resident step that is L(U^{n+1}), or after a
+    // failure the stage that complete_averages then finishes.
+    const bool averages = mode == SUM_STORE_L || !gate;
     SourceBufs sb;
     if (t->ph.source) {
         if (!t->cvs_y) {
@@ -373,11 +377,11 @@ mp_status launch_stage(mp_transport* t, const double* H, const double* C, int mo
         timed(t, 0, [&] {
             launch_quad_stage(t->qdev, t->nx, t->ny, rg.gj0, gny, rg.rec0, rg.rec1, h0, nh, v0, nv, t->ph, H, C,
                               static_cast<double*>(t->rec), t->flags, t->T, t->phi, t->vsn, t->udn, t->face,
-                              t->d_status, theta, SourcePtrs{sb.cvs_y, sb.cud_y, sb.srcH, sb.srcR, sb.srcS}, s, gate);
+                              t->d_status, theta, SourcePtrs{sb.cvs_y, sb.cud_y, sb.srcH, sb.srcR, sb.srcS}, averages, s, gate);
         });
     } else {
         launch_stage_kernels(t->nx, t->ny, t->range, t->ptab, t->ph, H, C, static_cast<double*>(t->rec), t->flags, t->T,
-                                     t->phi, t->vsn, t->udn, t->face, t->d_status, theta, s, prof, sb, gate);
+                                     t->phi, t->vsn, t->udn, t->face, t->d_status, theta, averages, s, prof, sb, gate);
     }
     {
         SumArgs a{t->nx, t->ny, t->host_tab.area, 1.0 / t->host_tab.area, t->face, H, C, t->H, t->C, outH, outC, t->rate, mode, a0, a1, dt,
@@ -710,6 +714,33 @@ mp_status ensure_graph(mp_transport* t) {
     return MP_OK;
 }
 
+// T and phi of stage `which` (2, 3) of a failed step, from the records that
+// the stage left: the latest evaluation, whose averages the step left out.
+mp_status complete_averages(mp_transport* t, int which) {
+    const double* H = which == 2 ? t->S1H : t->S2H;
+    const double* C = which == 2 ? t->S1C : t->S2C;
+    const long long N = (long long)t->N;
+    const unsigned g = (unsigned)((N + 127) / 128);
+    if (t->quad) {
+        QuadStageArgs a;
+        a.nx = t->nx; a.ny = t->ny; a.gj0 = 0; a.gny = t->ny;
+        a.H = H; a.C = C; a.rec = static_cast<double*>(t->rec); a.flags = t->flags; a.T = t->T; a.phi = t->phi;
+        a.status = t->d_status; a.q = t->qdev;
+        a.src = SourcePtrs{t->cvs_y, t->cud_y, t->srcH, t->srcR, t->srcS};
+        quad_cellphase_kernel<<<g, 128, 0, t->stream>>>(a, t->ph, 0, N, 1, nullptr);
+    } else {
+        CellPhaseArgs a{t->nx, t->ny, nullptr, H, C, static_cast<double*>(t->rec), t->flags, t->T, t->phi, t->d_status, 0, 0,
+                        t->cvs_y, t->cud_y, t->srcH, t->srcR, t->srcS};
+        if (t->ph.litho || t->ph.source)
+            cellphase_kernel<true><<<g, 128, t->ph.source ? kSourceBufBytes : 0, t->stream>>>(a, t->ph, t->ptab, 0, N, 1);
+        else
+            cellphase_kernel<false><<<g, 128, 0, t->stream>>>(a, t->ph, t->ptab, 0, N, 1);
+    }
+    count_launch();
+    MP_CUDA(cudaGetLastError());
+    return reset_status(t);
+}
+
 // The host loop's message for the failure the controller recorded.
 mp_status graph_failure(mp_transport* t, const InstCtl& c) {
     switch (c.fail) {
@@ -777,6 +808,7 @@ mp_status graph_steps(mp_transport* t, int nsteps, mp_step_report* reports) {
                 reports[done + k].status = c.status;
             }
             t->have_L = false;
+            if (c.evaluated) MP_TRY(complete_averages(t, c.evaluated));
             return graph_failure(t, c);
         }
         if (reports) std::memcpy(reports + done, t->h_rep, (size_t)chunk * sizeof(mp_step_report));
@@ -1288,7 +1320,7 @@ mp_status stage_rhs_raw(int nx, int ny, const mp_transport_opts& o, const double
     (void)NE;
     ParamTables pt;
     make_param_tables(tab, pt);
-    launch_stage_kernels(nx, ny, whole(ny), pt, ph, H, C, rec, wet, T, phi, vsn, udn, face, status, nullptr, s,
+    launch_stage_kernels(nx, ny, whole(ny), pt, ph, H, C, rec, wet, T, phi, vsn, udn, face, status, nullptr, true, s,
                                  nullptr);
     {
         SumArgs a{nx, ny, tab.area, 1.0 / tab.area, face, H, C, H, C, rhsH, rhsC, rate, SUM_STORE_L, 0.0, 0.0, 0.0,
