@@ -67,10 +67,18 @@ struct CommitArgs {
 };
 
 // Work items: block -> instance and the first element of its tile (faces:
-// edges [a, b); reconstruction: columns from a, row b).
+// edges [a, b); reconstruction: columns from a, row b, or with b < 0 cells
+// from a in id order).
 struct Work { int inst, a, b, part; };
 
-struct Tuning { int bx = 32, by = 4, cpt = 1; };
+// Tile shape of the reconstruction: bx x by threads, cpt cells per thread
+// along x. {128, 1, 1}, the default, is a run of 128 cells in id order: a mesh
+// whose width is no multiple of 32 leaves no lane idle (24 uneven meshes, 20
+// to 400 cells wide: 32x4 tiles launched 1.6 threads per cell).
+struct Tuning {
+    int bx = 128, by = 1, cpt = 1;
+    bool run() const { return bx == 128 && by == 1 && cpt == 1; }
+};
 
 // ------------------------------------------------------------ batched kernels
 
@@ -79,6 +87,11 @@ __global__ void __launch_bounds__(128) batch_recon_kernel(const InstArgs* args, 
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const ReconArgs& a = args[w.inst].recon;
+    if (w.b < 0) {
+        const unsigned cell = (unsigned)w.a + threadIdx.x, nx = (unsigned)a.nx;
+        if (cell < nx * (unsigned)a.ny) recon_cell(*a.tab, a, ph, (int)(cell % nx), (int)(cell / nx));
+        return;
+    }
     const int j = w.b + threadIdx.y;
     for (int c = 0; c < cpt; ++c) recon_cell(*a.tab, a, ph, w.a + c * blockDim.x + threadIdx.x, j);
 }
@@ -122,8 +135,8 @@ __global__ void __launch_bounds__(128, 2) batch_quad_weno_kernel(const QuadStage
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const QuadStageArgs& a = args[w.inst];
-    const int i = w.a + threadIdx.x, j = w.b + threadIdx.y;
-    if (i < a.nx && j < a.ny) quad_weno_cell(a, i, j);
+    const unsigned cell = (unsigned)w.a + threadIdx.x, nx = (unsigned)a.nx;
+    if (cell < nx * (unsigned)a.ny) quad_weno_cell(a, (int)(cell % nx), (int)(cell / nx));
 }
 
 __global__ void __launch_bounds__(128, 4) batch_quad_limit_kernel(const QuadStageArgs* args, const Work* work,
@@ -131,8 +144,8 @@ __global__ void __launch_bounds__(128, 4) batch_quad_limit_kernel(const QuadStag
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const QuadStageArgs& a = args[w.inst];
-    const int i = w.a + threadIdx.x, j = w.b + threadIdx.y;
-    if (i < a.nx && j < a.ny) quad_limit_cell(a, ph, i, j);
+    const unsigned cell = (unsigned)w.a + threadIdx.x, nx = (unsigned)a.nx;
+    if (cell < nx * (unsigned)a.ny) quad_limit_cell(a, ph, (int)(cell % nx), (int)(cell / nx));
 }
 
 __global__ void __launch_bounds__(128, 4) batch_quad_phase_kernel(const QuadStageArgs* args, const Work* work,
@@ -262,9 +275,9 @@ struct mp_batch {
     // accumulation, axpy and commit lists cover every instance).
     bool has_quads = false;            // launch the quad kernels (set by the first quad instance)
     void* d_qargs[mp::NKIND] = {nullptr, nullptr, nullptr};
-    mp::Work *d_wqrec = nullptr, *d_wqphase = nullptr, *d_wqface = nullptr;
-    int n_wqrec = 0, n_wqphase = 0, n_wqface = 0;
-    int cap_wqrec = 0, cap_wqphase = 0, cap_wqface = 0;
+    mp::Work *d_wqcell = nullptr, *d_wqface = nullptr;
+    int n_wqcell = 0, n_wqface = 0;
+    int cap_wqcell = 0, cap_wqface = 0;
     int* d_active = nullptr;
     unsigned* d_ticket = nullptr;      // finished blocks of each slot's running reduction
     mp::Partial* d_partial = nullptr;
@@ -467,7 +480,7 @@ mp_status rebuild_args(mp_batch* b, int slots) {
     for (int k = 0; k < NKIND; ++k) args[k].resize(slots);
     std::vector<QuadStageArgs> qargs[NKIND];
     for (int k = 0; k < NKIND; ++k) qargs[k].resize(slots);
-    std::vector<Work> wqr, wqp, wqf;
+    std::vector<Work> wqc, wqf;
     std::vector<AxpyArgs> ax(slots);
     std::vector<CommitArgs> cm(slots);
     std::vector<Work> wr, wp, wf, ws;
@@ -509,13 +522,12 @@ mp_status rebuild_args(mp_batch* b, int slots) {
         const bool rk3 = b->opts.integrator == MP_SSPRK3;
         cm[i] = CommitArgs{(int)in.N, rk3 ? in.S1H : in.S2H, rk3 ? in.S1C : in.S2C, in.H, in.C};
         if (in.quad) {
-            // The quad kernels' tiles: 32x4 cells, 128 cells, 128 edges.
-            for (int ty = 0; ty < in.ny; ty += 4)
-                for (int tx = 0; tx < in.nx; tx += 32) wqr.push_back(Work{i, tx, ty, 0});
-            for (size_t c = 0; c < in.N; c += 128) wqp.push_back(Work{i, (int)c, 0, 0});
+            // The quad kernels' blocks: 128 cells, 128 edges.
+            for (size_t c = 0; c < in.N; c += 128) wqc.push_back(Work{i, (int)c, 0, 0});
             for (size_t e = 0; e < in.NE; e += 128) wqf.push_back(Work{i, (int)e, (int)std::min(in.NE, e + 128), 0});
         } else {
-            for (int ty = 0; ty < in.ny; ty += tu.by)
+            for (size_t c = 0; tu.run() && c < in.N; c += 128) wr.push_back(Work{i, (int)c, -1, 0});
+            for (int ty = 0; !tu.run() && ty < in.ny; ty += tu.by)
                 for (int tx = 0; tx < in.nx; tx += tu.bx * tu.cpt) wr.push_back(Work{i, tx, ty, 0});
             for (size_t c = 0; c < in.N; c += 128) wp.push_back(Work{i, (int)c, 0, 0});
             for (size_t e = 0; e < in.NE; e += 128) wf.push_back(Work{i, (int)e, (int)std::min(in.NE, e + 128), 0});
@@ -551,13 +563,11 @@ mp_status rebuild_args(mp_batch* b, int slots) {
     MP_CUDA(cudaMemcpyAsync(b->d_wface, wf.data(), wf.size() * sizeof(Work), cudaMemcpyHostToDevice, s));
     MP_CUDA(cudaMemcpyAsync(b->d_wsum, ws.data(), ws.size() * sizeof(Work), cudaMemcpyHostToDevice, s));
     if (b->has_quads) {
-        b->n_wqrec = (int)wqr.size(); b->n_wqphase = (int)wqp.size(); b->n_wqface = (int)wqf.size();
-        MP_TRY(grow(&b->d_wqrec, b->cap_wqrec, b->n_wqrec, s, &grown));
-        MP_TRY(grow(&b->d_wqphase, b->cap_wqphase, b->n_wqphase, s, &grown));
+        b->n_wqcell = (int)wqc.size(); b->n_wqface = (int)wqf.size();
+        MP_TRY(grow(&b->d_wqcell, b->cap_wqcell, b->n_wqcell, s, &grown));
         MP_TRY(grow(&b->d_wqface, b->cap_wqface, b->n_wqface, s, &grown));
-        wqr.resize(b->cap_wqrec, pad); wqp.resize(b->cap_wqphase, pad); wqf.resize(b->cap_wqface, pad);
-        MP_CUDA(cudaMemcpyAsync(b->d_wqrec, wqr.data(), wqr.size() * sizeof(Work), cudaMemcpyHostToDevice, s));
-        MP_CUDA(cudaMemcpyAsync(b->d_wqphase, wqp.data(), wqp.size() * sizeof(Work), cudaMemcpyHostToDevice, s));
+        wqc.resize(b->cap_wqcell, pad); wqf.resize(b->cap_wqface, pad);
+        MP_CUDA(cudaMemcpyAsync(b->d_wqcell, wqc.data(), wqc.size() * sizeof(Work), cudaMemcpyHostToDevice, s));
         MP_CUDA(cudaMemcpyAsync(b->d_wqface, wqf.data(), wqf.size() * sizeof(Work), cudaMemcpyHostToDevice, s));
     }
     if (grown) b->gen += 1;
@@ -632,7 +642,7 @@ void launch_phases(mp_batch* b, int kind, bool averages) {
 }
 void launch_quad_phases(mp_batch* b, int kind, bool averages) {
     const QuadStageArgs* qa = static_cast<const QuadStageArgs*>(b->d_qargs[kind]);
-    timed(b, 1, [&] { batch_quad_phase_kernel<<<b->cap_wqphase, 128, 0, b->stream>>>(qa, b->d_wqphase, b->d_active, b->ph, averages); });
+    timed(b, 1, [&] { batch_quad_phase_kernel<<<b->cap_wqcell, 128, 0, b->stream>>>(qa, b->d_wqcell, b->d_active, b->ph, averages); });
 }
 
 void launch_kind(mp_batch* b, int kind, bool averages = true) {
@@ -649,8 +659,8 @@ void launch_kind(mp_batch* b, int kind, bool averages = true) {
         // General quad meshes: reconstruction, limiter, cell phase (the wet
         // flags the faces read), faces; the sums below cover every instance.
         const QuadStageArgs* qa = static_cast<const QuadStageArgs*>(b->d_qargs[kind]);
-        timed(b, 0, [&] { batch_quad_weno_kernel<<<b->cap_wqrec, dim3(32, 4), 0, s>>>(qa, b->d_wqrec, b->d_active); });
-        timed(b, 0, [&] { batch_quad_limit_kernel<<<b->cap_wqrec, dim3(32, 4), 0, s>>>(qa, b->d_wqrec, b->d_active, b->ph); });
+        timed(b, 0, [&] { batch_quad_weno_kernel<<<b->cap_wqcell, 128, 0, s>>>(qa, b->d_wqcell, b->d_active); });
+        timed(b, 0, [&] { batch_quad_limit_kernel<<<b->cap_wqcell, 128, 0, s>>>(qa, b->d_wqcell, b->d_active, b->ph); });
         launch_quad_phases(b, kind, averages);
         timed(b, 2, [&] { batch_quad_face_kernel<<<b->cap_wqface, 128, 0, s>>>(qa, b->d_wqface, b->d_active, b->ph); });
         if (b->ph.diffusion)
@@ -1155,7 +1165,7 @@ extern "C" void mp_batch_destroy(mp_batch* b) {
     }
     for (int k = 0; k < mp::NKIND; ++k) if (b->d_args[k]) cudaFreeAsync(b->d_args[k], b->stream);
     for (int k = 0; k < mp::NKIND; ++k) if (b->d_qargs[k]) cudaFreeAsync(b->d_qargs[k], b->stream);
-    for (void* p : {(void*)b->d_wqrec, (void*)b->d_wqphase, (void*)b->d_wqface}) if (p) cudaFreeAsync(p, b->stream);
+    for (void* p : {(void*)b->d_wqcell, (void*)b->d_wqface}) if (p) cudaFreeAsync(p, b->stream);
     for (void* p : {(void*)b->d_axpy, (void*)b->d_wrecon, (void*)b->d_wphase, (void*)b->d_wface, (void*)b->d_wsum,
                     (void*)b->d_active, (void*)b->d_ticket, (void*)b->d_partial,
                     (void*)b->d_tot, (void*)b->d_status, (void*)b->d_dt})

@@ -94,12 +94,11 @@ __device__ __forceinline__ void quad_weno_cell(const QuadStageArgs& a, int i, in
     }
     if (st) record_error(status, PART_UPDATE, cell + (long long)gj0 * nx, st);
 }
-__global__ void __launch_bounds__(128, 2) quad_weno_kernel(const __grid_constant__ QuadStageArgs a, int jlo, int jhi,
+__global__ void __launch_bounds__(128, 2) quad_weno_kernel(const __grid_constant__ QuadStageArgs a, unsigned c0, unsigned c1,
                                                            const int* gate) {
     if (gated_off(gate)) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = jlo + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    if (i >= a.nx || j >= jhi) return;
-    quad_weno_cell(a, i, j);
+    const unsigned cell = c0 + blockIdx.x * blockDim.x + threadIdx.x, nx = (unsigned)a.nx;
+    if (cell < c1) quad_weno_cell(a, (int)(cell % nx), (int)(cell / nx));
 }
 
 // Extremes of both deviation polynomials over the cell's limiter points, in
@@ -259,12 +258,12 @@ __device__ __forceinline__ void quad_limit_cell(const QuadStageArgs& a, const Ph
                          : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), loH, hiH, loC, hiC, fma(thH, mq, mH));
     if (st_lim) record_error(status, PART_LIMIT, cell + (long long)gj0 * nx, st_lim);
 }
-__global__ void __launch_bounds__(128, 4) quad_limit_kernel(const __grid_constant__ QuadStageArgs a, const __grid_constant__ Physics ph, int jlo,
-                                                         int jhi, const int* gate) {
+__global__ void __launch_bounds__(128, 4) quad_limit_kernel(const __grid_constant__ QuadStageArgs a,
+                                                            const __grid_constant__ Physics ph, unsigned c0, unsigned c1,
+                                                            const int* gate) {
     if (gated_off(gate)) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = jlo + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    if (i >= a.nx || j >= jhi) return;
-    quad_limit_cell(a, ph, i, j);
+    const unsigned cell = c0 + blockIdx.x * blockDim.x + threadIdx.x, nx = (unsigned)a.nx;
+    if (cell < c1) quad_limit_cell(a, ph, (int)(cell % nx), (int)(cell / nx));
 }
 
 
@@ -670,9 +669,9 @@ void launch_quad_stage(const QuadDev& q, int nx, int ny, int gj0, int gny, int r
     a.H = H; a.C = C; a.rec = rec; a.flags = flags; a.T = T; a.phi = phi;
     a.vsn = vsn; a.udn = udn; a.face = face; a.status = status; a.theta = theta;
     a.q = q; a.src = src;
-    dim3 blk(32, 4), grd((nx + 31) / 32, (rec1 - rec0 + 3) / 4);
-    quad_weno_kernel<<<grd, blk, 0, s>>>(a, rec0, rec1, gate);
-    quad_limit_kernel<<<grd, blk, 0, s>>>(a, ph, rec0, rec1, gate);
+    const unsigned u0 = (unsigned)rec0 * nx, u1 = (unsigned)rec1 * nx, gc = (u1 - u0 + 127) / 128;
+    quad_weno_kernel<<<gc, 128, 0, s>>>(a, u0, u1, gate);
+    quad_limit_kernel<<<gc, 128, 0, s>>>(a, ph, u0, u1, gate);
     const long long c0 = (long long)rec0 * nx, c1 = (long long)rec1 * nx;
     quad_cellphase_kernel<<<(unsigned)((c1 - c0 + 127) / 128), 128, 0, s>>>(a, ph, c0, c1, averages, gate);
     const unsigned ge = (unsigned)((nh + nv + 127) / 128);

@@ -67,13 +67,14 @@ struct SourceBufs {
 // 6: 139),
 // faces 5 (127; 4: 133, 6: 129); the reconstruction keeps its natural register
 // count (87 us; 5 and 6 blocks the same).
-// Rows [jlo, jhi) are reconstructed (all rows, or a slab's owned rows +- 1).
+// Cells [c0, c1) are reconstructed (all rows, or a slab's owned rows +- 1), in
+// id order: with 32x4 tiles a mesh of 321 columns idles a tenth of the lanes.
 __global__ void __launch_bounds__(128) recon_kernel(const __grid_constant__ ReconArgs a,
                                                     const __grid_constant__ Physics ph,
-                                                    const __grid_constant__ ParamTables p, int jlo, int jhi) {
+                                                    const __grid_constant__ ParamTables p, unsigned c0, unsigned c1) {
     if (gated_off(a.gate)) return;
-    const int j = jlo + (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    if (j < jhi) recon_cell(p.d, a, ph, blockIdx.x * blockDim.x + threadIdx.x, j);
+    const unsigned cell = c0 + blockIdx.x * blockDim.x + threadIdx.x, nx = (unsigned)a.nx;
+    if (cell < c1) recon_cell(p.d, a, ph, (int)(cell % nx), (int)(cell / nx));
 }
 template <bool kExt>
 __global__ void __launch_bounds__(128, kExt ? 4 : 6) cellphase_kernel(const __grid_constant__ CellPhaseArgs a,
@@ -305,8 +306,8 @@ void launch_stage_kernels(int nx, int ny, const StageRange& rg, const ParamTable
     auto run = [&](int kind, auto&& f) { if (prof) timed(prof, kind, f); else f(); };
     {
         ReconArgs a{nx, ny, nullptr, H, C, rec, flags, status, theta, rg.gj0, rg.gny, gate};
-        dim3 blk(32, 4), grd((nx + 31) / 32, (rg.rec1 - rg.rec0 + 3) / 4);
-        run(0, [&] { recon_kernel<<<grd, blk, 0, s>>>(a, ph, pt, rg.rec0, rg.rec1); });
+        const unsigned c0 = (unsigned)rg.rec0 * nx, c1 = (unsigned)rg.rec1 * nx;
+        run(0, [&] { recon_kernel<<<(c1 - c0 + 127) / 128, 128, 0, s>>>(a, ph, pt, c0, c1); });
     }
     {
         CellPhaseArgs a{nx, ny, nullptr, H, C, rec, flags, T, phi, status, rg.gj0, rg.gny,
