@@ -2,26 +2,22 @@
 // src/couple/preheat.cpp:65-287): H_t + div(us H - kappa grad H) = 0 with C
 // fixed and the Stokes velocity frozen, forward Euler.
 //
-// One step is three kernels:
-//   pre_recon_kernel   per cell: the unlimited deviation polynomial of H
-//                      (StateReconstruction::Update(s, false): limiter 1);
-//   pre_face_kernel    per edge: traces of both sides at the 5 Gauss points,
-//                      linear-law Lax-Friedrichs flux or the boundary policy,
-//                      plus the diffusion of the cell averages;
-//   pre_update_kernel  per cell: the face fluxes summed in the reference's
-//                      face order, H + dt*rhs into the other state buffer,
-//                      block partials; the last block to finish folds them in
-//                      a fixed order and applies the step's checks (finite
-//                      candidate, heat balance), accepting or stopping.
-// The step sizes do not depend on the state (the rate is fixed at Build), so
+// One step is one kernel (pre_step_kernel): per cell the unlimited deviation
+// polynomial of H (StateReconstruction::Update(s, false): limiter 1), per edge
+// the traces of both sides at the 5 Gauss points, the linear-law Lax-Friedrichs
+// flux or the boundary policy and the diffusion of the cell averages, then the
+// face fluxes summed in the reference's face order and H + dt*rhs into the
+// other state buffer, with block partials; the last block to finish folds them
+// in a fixed order and applies the step's checks (finite candidate, heat
+// balance), accepting or stopping. The step sizes do not depend on the state (the rate is fixed at Build), so
 // the host plans a batch of steps and issues them without waiting; a failed
-// step sets the status word and every kernel queued after it returns at once.
+// step sets the status word and every kernel queued after it does no work.
 //
 // On a general quad mesh (mp_preheat_create_quads; the reference's preheat
-// runs on any mesh family, preheat.cpp:86-117) the reconstruction, face,
-// rate and diagnostics kernels have quad forms that read the per-cell
-// tables, map every point from the cell's corners and use physical edge
-// lengths, normal-line spacing per edge point and per-cell areas.
+// runs on any mesh family, preheat.cpp:86-117) the step, rate and diagnostics
+// kernels have quad forms that read the per-cell tables, map every point from
+// the cell's corners and use physical edge lengths, normal-line spacing per
+// edge point and per-cell areas.
 #include "common.hpp"
 #include "phase_math.cuh"
 #include "stage_device.cuh"
@@ -34,6 +30,8 @@
 #include <cmath>
 #include <limits>
 #include <vector>
+
+#include <cuda_pipeline.h>
 
 namespace mp {
 
@@ -52,6 +50,13 @@ struct PreheatPhys {
     double inflowH;
     int lf_global;
     double lf_speed;
+    // Diffusion of constant samples (preheat.cpp:183-194 with
+    // diffusiveflux.cpp:105-200): interior samples [L, L, R, R], wall samples
+    // [L, L, L, L, wall value], gradient sum_k c_k (v_k - v_last) / ds, so the
+    // flux is -kappa times these sums of c_k times (v_L - v_last) / ds.
+    double c_int, c_bnd;
+    double dif[2][2];      // uniform mesh: -kappa times these, integrated over a [horizontal, vertical] [interior, wall] edge
+    double inv_area;
 };
 
 // Block partial of the preheat reductions.
@@ -73,10 +78,10 @@ struct PreCtl {
     PrePartial last;           // totals of the latest rhs / measure / rate launch
 };
 
-enum PreMode : int { PRE_STEP = 0, PRE_RHS = 1, PRE_MEASURE = 2 };
+enum PreMode : int { PRE_STEP = 0, PRE_RHS = 1 };
 
 constexpr int kPreBlock = 256;
-constexpr int kPrePer = 4;                      // cells per thread in the update kernel
+constexpr int kPrePer = 4;                      // cells per thread in the per-cell kernels
 constexpr int kPreCells = kPreBlock * kPrePer;
 
 __device__ __forceinline__ bool halted(const unsigned long long* status) {
@@ -116,17 +121,18 @@ __device__ __forceinline__ void pre_fold(PrePartial& a, const PrePartial* p) {
 // true in every thread with the totals in `tot` (valid in thread 0).
 __device__ bool pre_finish_blocks(PrePartial v, PrePartial* partial, PreCtl* ctl, PrePartial& tot) {
     __shared__ bool last;
+    const unsigned blocks = gridDim.x * gridDim.y;
     const PrePartial b = pre_block_reduce(v);
     if (threadIdx.x == 0) {
-        partial[blockIdx.x] = b;
+        partial[blockIdx.y * gridDim.x + blockIdx.x] = b;
         __threadfence();
-        last = atomicAdd(&ctl->ticket, 1u) == gridDim.x - 1;
+        last = atomicAdd(&ctl->ticket, 1u) == blocks - 1;
     }
     __syncthreads();
     if (!last) return false;
     __threadfence();
     PrePartial a = pre_identity();
-    for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) pre_fold(a, partial + k);
+    for (unsigned k = threadIdx.x; k < blocks; k += blockDim.x) pre_fold(a, partial + k);
     tot = pre_block_reduce(a);
     if (threadIdx.x == 0) ctl->ticket = 0;
     return true;
@@ -181,177 +187,324 @@ __device__ __forceinline__ bool speed_bounds(double bound, double required) {
 
 // ------------------------------------------------------------------ kernels
 
-// H-only reconstruction without the limiter.
-__global__ void __launch_bounds__(128) pre_recon_kernel(int nx, int ny, const double* __restrict__ H,
-                                                        double* __restrict__ rec, unsigned long long* status,
-                                                        const __grid_constant__ ParamTables p) {
-    if (halted(status)) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= nx || j >= ny) return;
-    const StageHot& t = p.d;
-    const long long cell = (long long)j * nx + i;
-    const size_t N = (size_t)nx * ny;
-    double u[3][3];
-#pragma unroll
-    for (int dj = 0; dj < 3; ++dj)
-#pragma unroll
-        for (int di = 0; di < 3; ++di) {
-            const int ii = min(max(i + di - 1, 0), nx - 1), jj = min(max(j + dj - 1, 0), ny - 1);
-            u[dj][di] = __ldg(H + (size_t)jj * nx + ii);
-        }
-    const int ci = i == 0 ? 0 : (i == nx - 1 ? 2 : 1), cj = j == 0 ? 0 : (j == ny - 1 ? 2 : 1);
-    double D[9];
-    const int st = reconstruct(t, candidate_mask(ci, cj), u, D);
-#pragma unroll
-    for (int m = 0; m < 9; ++m) rec[(size_t)m * N + cell] = D[m];
-    if (st) record_error(status, PART_UPDATE, cell, st);
-}
+// Arguments of one step (or RHS evaluation).
+struct PreStepArgs {
+    int nx, ny, passes, mode, row;
+    double dt;
+    const double* H;
+    const double* vn;
+    const double* edge;        // quad mesh: pre_quad_edge_kernel's table
+    double* Hout;
+    double* rhs;
+    PreRow* rows;
+    PrePartial* partial;
+    PreCtl* ctl;
+    unsigned long long* status;
+};
 
-// Edge flux of preheat.cpp:166-196: advection + diffusion of H.
-__global__ void __launch_bounds__(128, 8) pre_face_kernel(int nx, int ny, const double* __restrict__ H,
-                                                       const double* __restrict__ rec, const double* __restrict__ vn,
-                                                       double* __restrict__ flux, unsigned long long* status,
-                                                       const __grid_constant__ PreheatPhys pp,
-                                                       const __grid_constant__ ParamTables p) {
-    if (halted(status)) return;
-    const long long nE = (long long)nx * (ny + 1) + (long long)(nx + 1) * ny;
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nE) return;
-    const StageHot& t = p.d;
-    const size_t N = (size_t)nx * ny;
-    const EdgeGeo g = edge_geo(t, nx, ny, e);
-    const int o = g.horizontal ? 0 : 1;
-    double DL[9], DR[9];
-#pragma unroll
-    for (int m = 0; m < 9; ++m) {
-        DL[m] = __ldg(rec + (size_t)m * N + g.L);
-        DR[m] = g.boundary ? 0.0 : __ldg(rec + (size_t)m * N + g.R);
-    }
-    const double mL = __ldg(H + g.L), mR = g.boundary ? mL : __ldg(H + g.R);
-    double l0, l1, l2, r0, r1, r2;
-    if (g.horizontal) { q2_row(DL, g.lfix, l0, l1, l2); q2_row(DR, g.rfix, r0, r1, r2); }
-    else { q2_col(DL, g.lfix, l0, l1, l2); q2_col(DR, g.rfix, r0, r1, r2); }
-    const double sgn = g.reverse ? -1.0 : 1.0;
-    int st = 0;
+constexpr int kStepBlock = 128;
+constexpr int kStepRows = kStepBlock / 32;      // rows a block advances at a time, one per warp
+constexpr int kStepCols = 30;                   // columns a warp owns; its outer lanes are the neighbours'
+constexpr int kStepPasses = 32;
+
+// What the flux of one edge needs besides the traces.
+struct PreEdge {
+    bool boundary;
+    bool right;                // the wall cell is the right argument
+    int wall;
+    double sgn;                // -1: the canonical normal points into the wall cell
+    double half;               // half its length
+    double dif_int, dif_bnd;   // d flux / d (v_L - v_last)
+};
+
+// Edge flux of preheat.cpp:166-196: advection and diffusion of H out of the
+// left (wall) cell. The traces and the velocity are finite exactly when every
+// Lax-Friedrichs flux is or overflows, and the sum of them shows both, so the
+// interior's points are tested one by one only when it is not finite.
+__device__ __forceinline__ double pre_flux(const PreheatPhys& pp, const PreEdge& g, const double* gw, const double* v,
+                                           const double (&uL)[kNQ], const double (&uR)[kNQ], double mL, double mR,
+                                           int& st) {
     double sum = 0.0;
+    if (!g.boundary) {
+        bool low = false;
+#pragma unroll
+        for (int q = 0; q < kNQ; ++q) {
+            const double vq = v[q];
+            const double a = pp.lf_global ? pp.lf_speed : fabs(vq);
+            if (pp.lf_global) low |= !(a >= fabs(vq));
+            sum = fma(gw[q], fma(vq, uL[q] + uR[q], -(a * (uR[q] - uL[q]))), sum);
+        }
+        sum *= 0.5 * g.half;
+        const double flux = pp.diffusion ? fma(g.dif_int, mL - mR, sum) : sum;
+        if (low || !isfinite(flux)) {
+#pragma unroll
+            for (int q = 0; q < kNQ; ++q) {
+                const double vq = v[q], a = pp.lf_global ? pp.lf_speed : fabs(vq);
+                if (!isfinite(vq) || !isfinite(uL[q]) || !isfinite(uR[q]) || !speed_bounds(a, fabs(vq)))
+                    st = st ? st : E_OUTOFRANGE;
+                if (!isfinite(0.5 * (vq * uL[q] + vq * uR[q] - a * (uR[q] - uL[q])))) st = st ? st : E_FP;
+            }
+            if (pp.diffusion && !isfinite(g.dif_int * (mL - mR))) st = st ? st : E_FP;
+        }
+        return flux;
+    }
+    // EvaluateAdvectionBoundary (initialization.cpp:469-489) and the physical
+    // boundary flux (advectiveflux.cpp:229-271).
 #pragma unroll
     for (int q = 0; q < kNQ; ++q) {
-        const int cq = g.reverse ? kNQ - 1 - q : q;
-        const double at = t.g[cq];
-        const double v = sgn * __ldg(vn + e * kNQ + cq);
-        const double uL = mL + quad(l0, l1, l2, at);
-        if (!isfinite(v) || !isfinite(uL)) st = st ? st : E_OUTOFRANGE;
+        const double vq = g.sgn * v[q], u = g.right ? uR[q] : uL[q];
+        if (!isfinite(vq) || !isfinite(u)) st = st ? st : E_OUTOFRANGE;
         double f;
-        if (g.boundary) {
-            // EvaluateAdvectionBoundary (initialization.cpp:469-489) and the
-            // physical boundary flux (advectiveflux.cpp:229-271).
-            if (pp.Hpol == MP_BC_ZERO_FLUX || v == 0.0) f = 0.0;
-            else if (v < 0.0) {
-                if (pp.Hpol != MP_BC_INFLOW_OUTFLOW) st = st ? st : E_OUTOFRANGE;
-                f = v * pp.inflowH;
-            } else f = v * uL;
-        } else {
-            const double uR = mR + quad(r0, r1, r2, at);
-            if (!isfinite(uR)) st = st ? st : E_OUTOFRANGE;
-            const double a = pp.lf_global ? pp.lf_speed : fabs(v);
-            if (!speed_bounds(a, fabs(v))) st = st ? st : E_OUTOFRANGE;
-            f = 0.5 * (v * uL + v * uR - a * (uR - uL));
-        }
+        if (pp.Hpol == MP_BC_ZERO_FLUX || vq == 0.0) f = 0.0;
+        else if (vq < 0.0) {
+            if (pp.Hpol != MP_BC_INFLOW_OUTFLOW) st = st ? st : E_OUTOFRANGE;
+            f = vq * pp.inflowH;
+        } else f = vq * u;
         if (!isfinite(f)) st = st ? st : E_FP;
-        sum += t.dif_w[o][q] * f;
+        sum = fma(gw[q], f, sum);
     }
+    sum *= g.half;
     if (pp.diffusion) {
-        // Diffusion of H on constant cell-average samples (preheat.cpp:183-194
-        // with diffusiveflux.cpp:105-200): interior samples [L, L, R, R],
-        // wall samples [L, L, L, L, wall value]; gradient sum_k c_k (v_k -
-        // v_last) / ds.
-        const int type = g.boundary ? pp.wall_type[g.wall] : MP_THERMAL_TEMPERATURE;
-        const double wv = g.boundary ? pp.wall_value[g.wall] : 0.0;
-        if (type == MP_THERMAL_FLUX) {
+        const double wv = pp.wall_value[g.wall];
+        if (pp.wall_type[g.wall] == MP_THERMAL_FLUX) {
+            double w = 0.0;
 #pragma unroll
-            for (int q = 0; q < kNQ; ++q) sum += t.dif_w[o][q] * wv;
-        } else if (type == MP_THERMAL_TEMPERATURE) {
-            double grad = 0.0;
-            if (g.boundary) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) grad += t.dif_c_bnd[k] * (mL - wv);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) grad += t.dif_c_int[k] * ((k < 2 ? mL : mR) - mR);
-            }
-            grad /= t.dif_ds[o][g.boundary ? 1 : 0];
-            if (!isfinite(grad)) st = st ? st : E_FP;
-            double integral = 0.0;
-#pragma unroll
-            for (int q = 0; q < kNQ; ++q) integral -= t.dif_w[o][q] * pp.kappa * grad;
-            sum += integral;
+            for (int q = 0; q < kNQ; ++q) w += gw[q];
+            sum = fma(w * g.half, wv, sum);
+        } else if (pp.wall_type[g.wall] == MP_THERMAL_TEMPERATURE) {
+            const double d = g.dif_bnd * ((g.right ? mR : mL) - wv);
+            if (!isfinite(d)) st = st ? st : E_FP;
+            sum += d;
         }
     }
-    flux[e] = sum;
-    if (st) record_error(status, PART_FACES, e, st);
+    return sum;
 }
 
-// Per-cell sum of the face fluxes (faces bottom, top, left, right in id order,
-// each with its side's sign, preheat.cpp:195-197), the forward-Euler
-// candidate and the step's checks (preheat.cpp:267-273).
-// kQuad: per-cell areas (general quad mesh) instead of the uniform one.
-template <bool kQuad>
-__global__ void __launch_bounds__(kPreBlock) pre_update_kernel(int nx, int ny, double area, double inv_area,
-                                                                const double* __restrict__ cell_area,
-                                                                const double* __restrict__ H, const double* __restrict__ flux,
-                                                                double* __restrict__ Hout, double* __restrict__ rhs,
-                                                                int mode, double dt, int row, PreRow* rows,
-                                                                PrePartial* partial, PreCtl* ctl,
-                                                                unsigned long long* status) {
-    if (halted(status)) return;
-    const long long N = (long long)nx * ny;
+// One forward-Euler step (or the RHS) in one pass over memory. A block owns 30
+// columns and walks up its rows four at a time, a row per warp and a column per
+// lane. Each thread reconstructs its cell, hands its right trace to the next
+// lane and its top trace to the next row (shared memory; the last row of a
+// group stays for the next group), forms the fluxes of its cell's left and
+// bottom edges, and finishes the cell below, whose four fluxes are then known.
+// The outer lanes and the first and last row are the neighbours' cells,
+// reconstructed again. Edge velocities come through shared memory in whole rows
+// while the cells are reconstructed.
+// Bound by instruction issue and FP64 latency on a uniform mesh, whose 96 bytes
+// per cell take a third of the time, and by the cells' tables on a quad mesh.
+// Separate kernels for the reconstruction, the faces and the update moved 280
+// bytes per cell and waited for each other: 19 + 48 + 16 us at 640x1280 and
+// 135 + 118 + 19 on a quad mesh, now 53 and 205. 16 steps at 1280x2560 take
+// 2.63 ms at five blocks per SM (four 2.77, six 2.63 but 3 % more below); the
+// quad form spills above four.
+template <bool kQuad, class Tab>
+__global__ void __launch_bounds__(kStepBlock, kQuad ? 4 : 5) pre_step_kernel(const __grid_constant__ PreStepArgs a,
+                                                                 const __grid_constant__ PreheatPhys pp,
+                                                                 const __grid_constant__ Tab tab) {
+    constexpr int kTr = kQuad ? kNQ : 3;        // a trace: its values at the edge's points, or its coefficients
+    __shared__ double top[2][kStepRows][kTr + 1][32];
+    __shared__ double low[2][kStepRows][3][32];
+    __shared__ double vbuf[kStepRows][2][32 * kNQ];
+    const int lane = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int nx = a.nx, ny = a.ny;
     const long long nI = (long long)nx * (ny + 1);
+    const size_t N = (size_t)nx * ny;
+    PrePartial acc = pre_identity();
+    if (!__syncthreads_or(halted(a.status))) {
+        const int rows = a.passes * kStepRows - 2;
+        const int y0 = blockIdx.y * rows, y1 = min(y0 + rows, ny);
+        const int x0 = blockIdx.x * kStepCols, i = x0 - 1 + lane, x1 = min(x0 + kStepCols, nx);
+        const bool mine = lane >= 1 && lane <= kStepCols && i < nx;
+        const double* gw;
+        if constexpr (kQuad) gw = tab.gw; else gw = tab.d.gw;
+        auto point_values = [&](const double (&tr)[kTr], double (&u)[kNQ]) {
+#pragma unroll
+            for (int q = 0; q < kNQ; ++q) {
+                if constexpr (kQuad) u[q] = tr[q];
+                else u[q] = quad(tr[0], tr[1], tr[2], tab.d.g[q]);
+            }
+        };
+        for (int pass = 0; pass < a.passes; ++pass) {
+            const int base = y0 - 1 + pass * kStepRows, j = base + ty, par = pass & 1;
+            if (base > y1) break;
+            const bool vrow = j >= y0 && j < y1;        // its vertical edges count
+            const bool hrow = j >= y0 && j <= y1;       // the edges below it count
+            double* vv = vbuf[ty][0];
+            double* vh = vbuf[ty][1];
+            if (vrow) {
+                const double* src = a.vn + (nI + (long long)j * (nx + 1) + x0) * kNQ;
+                for (int k = lane; k < (x1 - x0 + 1) * kNQ; k += 32) __pipeline_memcpy_async(vv + k, src + k, sizeof(double));
+            }
+            if (hrow) {
+                const double* src = a.vn + ((long long)j * nx + x0) * kNQ;
+                for (int k = lane; k < (x1 - x0) * kNQ; k += 32) __pipeline_memcpy_async(vh + k, src + k, sizeof(double));
+            }
+            __pipeline_commit();
+            const bool cell_in = j >= 0 && j < ny && j <= y1 && i >= 0 && i < nx;
+            const long long cell = (long long)j * nx + i;
+            double m = 0.0, tl[kTr] = {}, tr[kTr] = {}, tb[kTr] = {}, tt[kTr] = {};
+            if (cell_in) {
+                double u[1][3][3];
+                const int ci = i == 0 ? 0 : (i == nx - 1 ? 2 : 1), cj = j == 0 ? 0 : (j == ny - 1 ? 2 : 1);
+                const double* Hc = a.H + cell;
+                const int west = ci == 0 ? 0 : -1, east = ci == 2 ? 0 : 1, rows3[3] = {cj == 0 ? 0 : -nx, 0, cj == 2 ? 0 : nx};
+#pragma unroll
+                for (int dj = 0; dj < 3; ++dj) {
+                    const double* r = Hc + rows3[dj];
+                    u[0][dj][0] = __ldg(r + west);
+                    u[0][dj][1] = __ldg(r);
+                    u[0][dj][2] = __ldg(r + east);
+                }
+                m = u[0][1][1];
+                double D[1][9];
+                int st;
+                if constexpr (kQuad) st = reconstruct_quad<1>(tab, N, cell, ci, cj, 1e-2 * __ldg(tab.geo + 3 * N + cell), u, D);
+                else st = reconstruct(tab.d, candidate_mask(ci, cj), u[0], D[0]);
+                if (st) record_error(a.status, PART_UPDATE, cell, st);
+                D[0][0] += m;
+                if constexpr (kQuad) {
+                    const double cx = __ldg(tab.geo + cell), cy = __ldg(tab.geo + N + cell);
+                    const double inv_h = 1.0 / __ldg(tab.geo + 2 * N + cell);
+                    const P2 c0 = normalised(vtx(tab, nx, i, j), cx, cy, inv_h),
+                             c1 = normalised(vtx(tab, nx, i + 1, j), cx, cy, inv_h),
+                             c2 = normalised(vtx(tab, nx, i + 1, j + 1), cx, cy, inv_h),
+                             c3 = normalised(vtx(tab, nx, i, j + 1), cx, cy, inv_h);
+                    auto along = [&](P2 s, P2 e, double (&v)[kTr]) {
+                        const P2 mid = P2{0.5 * (s.x + e.x), 0.5 * (s.y + e.y)}, half = P2{0.5 * (e.x - s.x), 0.5 * (e.y - s.y)};
+#pragma unroll
+                        for (int q = 0; q < kNQ; ++q)
+                            v[q] = q2v(D[0], fma(half.x, tab.gq[q], mid.x), fma(half.y, tab.gq[q], mid.y));
+                    };
+                    along(c0, c3, tl); along(c1, c2, tr); along(c0, c1, tb); along(c3, c2, tt);
+                } else {
+                    q2_col(D[0], -1.0, tl[0], tl[1], tl[2]); q2_col(D[0], 1.0, tr[0], tr[1], tr[2]);
+                    q2_row(D[0], -1.0, tb[0], tb[1], tb[2]); q2_row(D[0], 1.0, tt[0], tt[1], tt[2]);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < kTr; ++k) {
+                tr[k] = __shfl_up_sync(~0u, tr[k], 1);
+                top[par][ty][k][lane] = tt[k];
+            }
+            top[par][ty][kTr][lane] = m;
+            const double mw = __shfl_up_sync(~0u, m, 1);
+            __pipeline_wait_prior(0);
+            __syncthreads();
+            // Left edge: the cells (i-1, j) and (i, j).
+            double fl = 0.0, fb = 0.0, ms = 0.0;
+            if (vrow && lane >= 1 && i <= x1) {
+                const long long e = nI + (long long)j * (nx + 1) + i;
+                double uw[kNQ], uo[kNQ];
+                point_values(tr, uw);
+                point_values(tl, uo);
+                PreEdge g;
+                g.boundary = i == 0 || i == nx;
+                g.right = i == 0;
+                g.wall = i == 0 ? 2 : 3;
+                g.sgn = i == 0 ? -1.0 : 1.0;
+                if constexpr (kQuad) {
+                    const double2 w = __ldg(reinterpret_cast<const double2*>(a.edge) + e);
+                    g.half = w.x; g.dif_int = -pp.kappa * pp.c_int * w.y; g.dif_bnd = -pp.kappa * pp.c_bnd * w.y;
+                } else {
+                    g.half = 0.5 * tab.d.len_v; g.dif_int = pp.dif[1][0]; g.dif_bnd = pp.dif[1][1];
+                }
+                int st = 0;
+                fl = pre_flux(pp, g, gw, vv + (lane - 1) * kNQ, uw, uo, mw, m, st);
+                if (st) record_error(a.status, PART_FACES, e, st);
+            }
+            // Bottom edge: the cells (i, j) and (i, j-1).
+            if (hrow && mine) {
+                const int sp = ty > 0 ? par : par ^ 1, sr = ty > 0 ? ty - 1 : kStepRows - 1;
+                const long long e = (long long)j * nx + i;
+                double ts[kTr], us[kNQ], uo[kNQ];
+#pragma unroll
+                for (int k = 0; k < kTr; ++k) ts[k] = top[sp][sr][k][lane];
+                ms = top[sp][sr][kTr][lane];
+                point_values(ts, us);
+                point_values(tb, uo);
+                PreEdge g;
+                g.boundary = j == 0 || j == ny;
+                g.right = j == ny;
+                g.wall = j == 0 ? 0 : 1;
+                g.sgn = j == ny ? -1.0 : 1.0;
+                if constexpr (kQuad) {
+                    const double2 w = __ldg(reinterpret_cast<const double2*>(a.edge) + e);
+                    g.half = w.x; g.dif_int = -pp.kappa * pp.c_int * w.y; g.dif_bnd = -pp.kappa * pp.c_bnd * w.y;
+                } else {
+                    g.half = 0.5 * tab.d.len_h; g.dif_int = pp.dif[0][0]; g.dif_bnd = pp.dif[0][1];
+                }
+                int st = 0;
+                fb = pre_flux(pp, g, gw, vh + (lane - 1) * kNQ, uo, us, m, ms, st);
+                if (st) record_error(a.status, PART_FACES, e, st);
+            }
+            low[par][ty][0][lane] = fb;
+            low[par][ty][1][lane] = fl;
+            low[par][ty][2][lane] = __shfl_down_sync(~0u, fl, 1);
+            __syncthreads();
+            // The cell below: its fluxes in id order with each side's sign
+            // (preheat.cpp:195-197), the candidate and the partials.
+            if (hrow && j > y0 && mine) {
+                const int sp = ty > 0 ? par : par ^ 1, sr = ty > 0 ? ty - 1 : kStepRows - 1;
+                const double b = low[sp][sr][0][lane], l = low[sp][sr][1][lane], r = low[sp][sr][2][lane];
+                const double sum = ((-b) + (j == ny ? -fb : fb)) + (i == 0 ? -l : l) - r;
+                const long long done = cell - nx;
+                double area, rate;
+                if constexpr (kQuad) {
+                    area = __ldg(tab.geo + 3 * N + done);
+                    rate = sum / area;
+                } else {
+                    area = tab.d.area;
+                    rate = sum * pp.inv_area;
+                }
+                if (j == 1) acc.bflux += b;
+                if (j == ny) acc.bflux += fb;
+                if (i == 0) acc.bflux += l;
+                if (i == nx - 1) acc.bflux += r;
+                double cand = ms;
+                if (a.mode == PRE_RHS) a.rhs[done] = rate;
+                else {
+                    cand = __dadd_rn(ms, __dmul_rn(a.dt, rate));
+                    a.Hout[done] = cand;
+                }
+                acc.integral = fma(cand, area, acc.integral);
+                acc.minimum = fmin(acc.minimum, cand);
+                acc.maximum = fmax(acc.maximum, cand);
+                if (!isfinite(cand)) acc.nonfinite = 1.0;
+            }
+        }
+    }
+    PrePartial tot;
+    if (!pre_finish_blocks(acc, a.partial, a.ctl, tot) || threadIdx.x != 0) return;
+    if (a.mode != PRE_STEP) { a.ctl->last = tot; return; }
+    // The step's checks (preheat.cpp:267-273), unless a cell or an edge failed.
+    if (halted(a.status)) return;
+    if (tot.nonfinite != 0.0) { record_error(a.status, PART_CELLS, 0, E_FP); return; }
+    const double prev = a.ctl->prev_integral;
+    const double bal = tot.integral - prev + a.dt * tot.bflux;
+    const double tol = 1e-10 * (1.0 + fabs(tot.integral) + fabs(prev) + fabs(a.dt * tot.bflux));
+    if (!(fabs(bal) <= tol)) { record_error(a.status, PART_CELLS, 0, MP_ERR_PLIB); return; }
+    a.rows[a.row] = PreRow{tot.integral, tot.minimum, tot.maximum, tot.bflux, bal};
+    a.ctl->prev_integral = tot.integral;
+    a.ctl->accepted += 1;
+}
+
+// Integral, minimum and maximum of a state.
+__global__ void __launch_bounds__(kPreBlock) pre_measure_kernel(long long N, double area,
+                                                                const double* __restrict__ cell_area,
+                                                                const double* __restrict__ H, PrePartial* partial,
+                                                                PreCtl* ctl) {
     PrePartial v = pre_identity();
 #pragma unroll
     for (int k = 0; k < kPrePer; ++k) {
         const long long cell = (long long)blockIdx.x * kPreCells + k * kPreBlock + threadIdx.x;
         if (cell >= N) continue;
         const double h = __ldg(H + cell);
-        double cand = h;
-        double a = area;
-        if constexpr (kQuad) a = __ldg(cell_area + cell);
-        if (mode != PRE_MEASURE) {
-            const int i = (int)(cell % nx), j = (int)(cell / nx);
-            const long long eb = (long long)j * nx + i, et = eb + nx;
-            const long long el = nI + (long long)j * (nx + 1) + i, er = el + 1;
-            const double fb = __ldg(flux + eb), ft = __ldg(flux + et), fl = __ldg(flux + el), fr = __ldg(flux + er);
-            const double sum = ((-fb) + (j == ny - 1 ? -ft : ft)) + (i == 0 ? -fl : fl) - fr;
-            double r;
-            if constexpr (kQuad) r = sum / a;
-            else r = sum * inv_area;
-            double b = 0.0;
-            if (j == 0) b += fb;
-            if (j == ny - 1) b += ft;
-            if (i == 0) b += fl;
-            if (i == nx - 1) b += fr;
-            v.bflux += b;
-            if (mode == PRE_RHS) rhs[cell] = r;
-            else {
-                cand = __dadd_rn(h, __dmul_rn(dt, r));
-                Hout[cell] = cand;
-            }
-        }
-        v.integral += cand * a;
-        v.minimum = fmin(v.minimum, cand);
-        v.maximum = fmax(v.maximum, cand);
-        v.nonfinite = fmax(v.nonfinite, isfinite(cand) ? 0.0 : 1.0);
+        v.integral += h * (cell_area ? __ldg(cell_area + cell) : area);
+        v.minimum = fmin(v.minimum, h);
+        v.maximum = fmax(v.maximum, h);
+        v.nonfinite = fmax(v.nonfinite, isfinite(h) ? 0.0 : 1.0);
     }
     PrePartial tot;
-    if (!pre_finish_blocks(v, partial, ctl, tot) || threadIdx.x != 0) return;
-    if (mode != PRE_STEP) { ctl->last = tot; return; }
-    if (tot.nonfinite != 0.0) { record_error(status, PART_CELLS, 0, E_FP); return; }
-    const double prev = ctl->prev_integral;
-    const double bal = tot.integral - prev + dt * tot.bflux;
-    const double tol = 1e-10 * (1.0 + fabs(tot.integral) + fabs(prev) + fabs(dt * tot.bflux));
-    if (!(fabs(bal) <= tol)) { record_error(status, PART_CELLS, 0, MP_ERR_PLIB); return; }
-    rows[row] = PreRow{tot.integral, tot.minimum, tot.maximum, tot.bflux, bal};
-    ctl->prev_integral = tot.integral;
-    ctl->accepted += 1;
+    if (pre_finish_blocks(v, partial, ctl, tot) && threadIdx.x == 0) ctl->last = tot;
 }
 
 // Build (preheat.cpp:130-156), per edge: LF speed sum_q L w_q alpha / 2 and
@@ -490,130 +643,20 @@ __global__ void __launch_bounds__(128) pre_diag_kernel(int nx, int ny, const dou
 
 // ------------------------------------------------- general quad mesh forms
 
-// H-only reconstruction with the cell's own tables, without the limiter.
-__global__ void __launch_bounds__(128, 4) pre_quad_recon_kernel(int nx, int ny, const double* __restrict__ H,
-                                                                double* __restrict__ rec, unsigned long long* status,
-                                                                QuadDev q) {
-    if (halted(status)) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= nx || j >= ny) return;
-    const long long cell = (long long)j * nx + i;
-    const size_t N = (size_t)nx * ny;
-    const int ci = i == 0 ? 0 : (i == nx - 1 ? 2 : 1), cj = j == 0 ? 0 : (j == ny - 1 ? 2 : 1);
-    const double eA = 1e-2 * __ldg(q.geo + 3 * N + cell);
-    double u[1][3][3];
-#pragma unroll
-    for (int dj = 0; dj < 3; ++dj)
-#pragma unroll
-        for (int di = 0; di < 3; ++di) {
-            const int ii = min(max(i + di - 1, 0), nx - 1), jj = min(max(j + dj - 1, 0), ny - 1);
-            u[0][dj][di] = __ldg(H + (size_t)jj * nx + ii);
-        }
-    double D[1][9];
-    const int st = reconstruct_quad<1>(q, N, cell, ci, cj, eA, u, D);
-#pragma unroll
-    for (int m = 0; m < 9; ++m) rec[(size_t)m * N + cell] = D[0][m];
-    if (st) record_error(status, PART_UPDATE, cell, st);
-}
-
-// One side of an edge: the cell's frame and its H polynomial.
-struct PreSide {
-    double cx, cy, inv_h, m;
-    double D[9];
-};
-__device__ __forceinline__ void pre_side(const QuadDev& q, size_t N, const double* H, const double* rec, long long cell,
-                                         PreSide& s) {
-    s.cx = __ldg(q.geo + cell);
-    s.cy = __ldg(q.geo + N + cell);
-    s.inv_h = 1.0 / __ldg(q.geo + 2 * N + cell);
-    s.m = __ldg(H + cell);
-#pragma unroll
-    for (int k = 0; k < 9; ++k) s.D[k] = __ldg(rec + (size_t)k * N + cell);
-}
-__device__ __forceinline__ double pre_trace(const PreSide& s, P2 p) {
-    return s.m + q2v(s.D, (p.x - s.cx) * s.inv_h, (p.y - s.cy) * s.inv_h);
-}
-
-// Edge flux of preheat.cpp:166-196 on a general quad mesh: the traces at the
-// edge's Gauss points in each side's frame, the linear-law Lax-Friedrichs
-// flux or the boundary policy with weights L w_q / 2, and the diffusion of
-// the cell averages with the normal-line spacing of each edge point.
-__global__ void __launch_bounds__(128) pre_quad_face_kernel(int nx, int ny, const double* __restrict__ H,
-                                                            const double* __restrict__ rec,
-                                                            const double* __restrict__ vn, double* __restrict__ flux,
-                                                            unsigned long long* status,
-                                                            const __grid_constant__ PreheatPhys pp, QuadDev q) {
-    if (halted(status)) return;
+// Per edge of a quad mesh, half its length and that times sum_q w_q / ds_q
+// (ds: the normal-line spacing of each edge point), for pre_step_kernel.
+__global__ void __launch_bounds__(128) pre_quad_edge_kernel(int nx, int ny, double* __restrict__ edge, QuadDev q) {
     const long long nE = (long long)nx * (ny + 1) + (long long)(nx + 1) * ny;
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nE) return;
-    const size_t N = (size_t)nx * ny;
     const QuadEdge g = quad_edge(q, nx, ny, 0, ny, e);
     double len;
     P2 nrm;
     edge_geometry(g.a, g.b, len, nrm);
-    PreSide sl, sr;
-    pre_side(q, N, H, rec, g.L, sl);
-    if (!g.boundary) pre_side(q, N, H, rec, g.R, sr);
-    const double mL = sl.m, mR = g.boundary ? mL : sr.m;
-    const double sgn = g.reverse ? -1.0 : 1.0;
-    int st = 0;
     double sum = 0.0;
-#pragma unroll
-    for (int k = 0; k < kNQ; ++k) {
-        const int cq = g.reverse ? kNQ - 1 - k : k;
-        const P2 p = lerp_edge(q.gq[k], g.a, g.b);
-        const double v = sgn * __ldg(vn + e * kNQ + cq);
-        const double uL = pre_trace(sl, p);
-        if (!isfinite(v) || !isfinite(uL)) st = st ? st : E_OUTOFRANGE;
-        double f;
-        if (g.boundary) {
-            if (pp.Hpol == MP_BC_ZERO_FLUX || v == 0.0) f = 0.0;
-            else if (v < 0.0) {
-                if (pp.Hpol != MP_BC_INFLOW_OUTFLOW) st = st ? st : E_OUTOFRANGE;
-                f = v * pp.inflowH;
-            } else f = v * uL;
-        } else {
-            const double uR = pre_trace(sr, p);
-            if (!isfinite(uR)) st = st ? st : E_OUTOFRANGE;
-            const double a = pp.lf_global ? pp.lf_speed : fabs(v);
-            if (!speed_bounds(a, fabs(v))) st = st ? st : E_OUTOFRANGE;
-            f = 0.5 * (v * uL + v * uR - a * (uR - uL));
-        }
-        if (!isfinite(f)) st = st ? st : E_FP;
-        sum += 0.5 * len * q.gw[k] * f;
-    }
-    if (pp.diffusion) {
-        // Interior samples [L, L, R, R], wall samples [L, L, L, L, wall
-        // value]; gradient sum_k c_k (v_k - v_last) / spacing at each point.
-        const int type = g.boundary ? pp.wall_type[g.wall] : MP_THERMAL_TEMPERATURE;
-        const double wv = g.boundary ? pp.wall_value[g.wall] : 0.0;
-        if (type == MP_THERMAL_FLUX) {
-#pragma unroll
-            for (int k = 0; k < kNQ; ++k) sum += len * q.gw[k] / 2 * wv;
-        } else if (type == MP_THERMAL_TEMPERATURE) {
-            double integral = 0.0;
-#pragma unroll
-            for (int k = 0; k < kNQ; ++k) {
-                const int cq = g.reverse ? kNQ - 1 - k : k;
-                const double sp = __ldg(q.sp + e * kNQ + cq);
-                double grad = 0.0;
-                if (g.boundary) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) grad += q.dif_c_bnd[c] * (mL - wv);
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) grad += q.dif_c_int[c] * ((c < 2 ? mL : mR) - mR);
-                }
-                grad /= sp;
-                if (!isfinite(grad)) st = st ? st : E_FP;
-                integral -= len * q.gw[k] / 2 * pp.kappa * grad;
-            }
-            sum += integral;
-        }
-    }
-    flux[e] = sum;
-    if (st) record_error(status, PART_FACES, e, st);
+    for (int k = 0; k < kNQ; ++k) sum += q.gw[k] / __ldg(q.sp + e * kNQ + k);
+    edge[2 * e] = 0.5 * len;
+    edge[2 * e + 1] = 0.5 * len * sum;
 }
 
 // Build (preheat.cpp:130-156) on a general quad mesh: per edge the LF speed
@@ -731,7 +774,7 @@ struct mp_preheat {
     mp::ParamTables ptab;
     double* Hb[2] = {nullptr, nullptr};   // state ping-pong; Hb[cur] is accepted
     int cur = 0;
-    double *C = nullptr, *rec = nullptr, *vn = nullptr, *flux = nullptr, *rr = nullptr, *rate = nullptr;
+    double *C = nullptr, *vn = nullptr, *edge = nullptr, *rr = nullptr, *rate = nullptr;
     double *rhs = nullptr, *T = nullptr, *phi = nullptr;
     mp::PrePartial* partial = nullptr;
     mp::PreCtl* ctl = nullptr;
@@ -740,7 +783,8 @@ struct mp_preheat {
     mp::PreRow* h_rows = nullptr;
     unsigned long long* d_status = nullptr;
     unsigned long long* h_status = nullptr;
-    int blocks = 0;
+    int blocks = 0;                 // of the per-cell kernels
+    int passes = 1;                 // row groups per block of pre_step_kernel
     double time = 0.0;
     long long accepted = 0;
     long long steps = 0;            // steps of the current run
@@ -759,7 +803,7 @@ namespace {
 constexpr int kBatch = 512;         // steps issued per host round trip
 
 void pre_free(mp_preheat* p) {
-    void* bufs[] = {p->Hb[0], p->Hb[1], p->C, p->rec, p->vn, p->flux, p->rr, p->rate, p->rhs, p->T, p->phi,
+    void* bufs[] = {p->Hb[0], p->Hb[1], p->C, p->vn, p->edge, p->rr, p->rate, p->rhs, p->T, p->phi,
                     p->partial, p->ctl, p->rows, p->d_status, p->qbuf};
     for (void* b : bufs) if (b) cudaFree(b);
     if (p->h_ctl) cudaFreeHost(p->h_ctl);
@@ -795,36 +839,45 @@ mp_status read_status(mp_preheat* p) {
     return MP_OK;
 }
 
-// The three kernels of one RHS evaluation / step on state Hb[src].
-void launch_rhs_kernels(mp_preheat* p, const double* H) {
-    const int nx = p->nx, ny = p->ny;
-    if (p->quad) {
-        dim3 blk(32, 4), grd((nx + 31) / 32, (ny + 3) / 4);
-        pre_quad_recon_kernel<<<grd, blk, 0, p->stream>>>(nx, ny, H, p->rec, p->d_status, p->qdev);
-        pre_quad_face_kernel<<<(unsigned)((p->NE + 127) / 128), 128, 0, p->stream>>>(nx, ny, H, p->rec, p->vn, p->flux,
-                                                                                     p->d_status, p->pp, p->qdev);
-        count_launch(2);
-        return;
-    }
-    {
-        dim3 blk(32, 4), grd((nx + 31) / 32, (ny + 3) / 4);
-        pre_recon_kernel<<<grd, blk, 0, p->stream>>>(nx, ny, H, p->rec, p->d_status, p->ptab);
-    }
-    pre_face_kernel<<<(unsigned)((p->NE + 127) / 128), 128, 0, p->stream>>>(nx, ny, H, p->rec, p->vn, p->flux,
-                                                                            p->d_status, p->pp, p->ptab);
-    count_launch(2);
+// Blocks of one pre_step_kernel launch.
+dim3 step_grid(int nx, int ny, int passes) {
+    const int rows = passes * kStepRows - 2;
+    return dim3((nx + kStepCols - 1) / kStepCols, (ny + rows - 1) / rows);
 }
 
-void launch_update(mp_preheat* p, const double* H, double* Hout, int mode, double dt, int row) {
-    if (p->quad)
-        pre_update_kernel<true><<<p->blocks, kPreBlock, 0, p->stream>>>(p->nx, p->ny, 0.0, 0.0, p->qdev.geo + 3 * p->N,
-                                                                       H, p->flux, Hout, p->rhs, mode, dt, row,
-                                                                       p->rows, p->partial, p->ctl, p->d_status);
-    else
-        pre_update_kernel<false><<<p->blocks, kPreBlock, 0, p->stream>>>(p->nx, p->ny, p->host_tab.area,
-                                                                        1.0 / p->host_tab.area, nullptr, H, p->flux,
-                                                                        Hout, p->rhs, mode, dt, row, p->rows,
-                                                                        p->partial, p->ctl, p->d_status);
+// Row groups per block: each block repeats two rows of its neighbours, so long
+// blocks waste less, but they have to fill the GPU. Waves of resident blocks
+// times the groups of each (and one for a block's start and end) is the time of
+// a launch; the smallest is taken, the shorter blocks of two that are equal.
+mp_status choose_passes(mp_preheat* p) {
+    int sms = 0, resident = 0, dev = 0;
+    MP_CUDA(cudaGetDevice(&dev));
+    MP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    MP_CUDA(p->quad ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pre_step_kernel<true, QuadDev>, kStepBlock, 0)
+                    : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, pre_step_kernel<false, ParamTables>,
+                                                                    kStepBlock, 0));
+    const long long slots = (long long)sms * std::max(resident, 1);
+    long long best = -1;
+    for (int n = 1; n <= kStepPasses; ++n) {
+        const dim3 g = step_grid(p->nx, p->ny, n);
+        if (g.y > 65535) continue;
+        const long long cost = ((long long)g.x * g.y + slots - 1) / slots * (n + 1);
+        if (best < 0 || cost < best) { best = cost; p->passes = n; }
+    }
+    return MP_OK;
+}
+
+// One RHS evaluation / step on the state H.
+void launch_step(mp_preheat* p, const double* H, double* Hout, int mode, double dt, int row) {
+    PreStepArgs a{};
+    a.nx = p->nx; a.ny = p->ny; a.passes = p->passes; a.mode = mode; a.row = row;
+    a.dt = dt;
+    a.H = H; a.vn = p->vn; a.edge = p->edge;
+    a.Hout = Hout; a.rhs = p->rhs;
+    a.rows = p->rows; a.partial = p->partial; a.ctl = p->ctl; a.status = p->d_status;
+    const dim3 grid = step_grid(p->nx, p->ny, p->passes);
+    if (p->quad) pre_step_kernel<true><<<grid, kStepBlock, 0, p->stream>>>(a, p->pp, p->qdev);
+    else pre_step_kernel<false><<<grid, kStepBlock, 0, p->stream>>>(a, p->pp, p->ptab);
     count_launch();
 }
 
@@ -936,15 +989,30 @@ mp_status preheat_create_impl(const mp_mesh_desc* mesh, const double* xy, const 
         make_param_tables(p->host_tab, p->ptab);
     }
     p->blocks = (int)((p->N + kPreCells - 1) / kPreCells);
-    const size_t N = p->N, NE = p->NE;
+    p->quad = xy != nullptr;
+    const double* ci = xy ? qt.dif_c_int : p->host_tab.dif_c_int;
+    const double* cb = xy ? qt.dif_c_bnd : p->host_tab.dif_c_bnd;
+    pp.c_int = ci[0] + ci[1];
+    pp.c_bnd = cb[0] + cb[1] + cb[2] + cb[3];
+    if (!xy)
+        for (int o = 0; o < 2; ++o) {
+            double w = 0.0;
+            for (int q = 0; q < kNQ; ++q) w += p->host_tab.dif_w[o][q];
+            pp.dif[o][0] = -pp.kappa * pp.c_int * w / p->host_tab.dif_ds[o][0];
+            pp.dif[o][1] = -pp.kappa * pp.c_bnd * w / p->host_tab.dif_ds[o][1];
+        }
+    pp.inv_area = xy ? 0.0 : 1.0 / p->host_tab.area;
+    const mp_status ps = choose_passes(p);
+    if (ps != MP_OK) { delete p; return ps; }
+    const dim3 grid = step_grid(p->nx, p->ny, p->passes);
+    const size_t N = p->N, NE = p->NE, blocks = std::max((size_t)p->blocks, (size_t)grid.x * grid.y);
     cudaError_t e = cudaSuccess;
     auto alloc = [&](void** q, size_t bytes) { if (e == cudaSuccess) e = cudaMalloc(q, bytes); };
     for (double** q : {&p->Hb[0], &p->Hb[1], &p->C, &p->rate, &p->rhs, &p->T, &p->phi}) alloc((void**)q, N * sizeof(double));
-    alloc((void**)&p->rec, 9 * N * sizeof(double));
     alloc((void**)&p->vn, NE * kNQ * sizeof(double));
-    alloc((void**)&p->flux, NE * sizeof(double));
+    if (xy) alloc((void**)&p->edge, 2 * NE * sizeof(double));
     alloc((void**)&p->rr, 2 * NE * sizeof(double));
-    alloc((void**)&p->partial, (size_t)p->blocks * sizeof(PrePartial));
+    alloc((void**)&p->partial, blocks * sizeof(PrePartial));
     alloc((void**)&p->ctl, sizeof(PreCtl));
     alloc((void**)&p->rows, kBatch * sizeof(PreRow));
     alloc((void**)&p->d_status, sizeof(unsigned long long));
@@ -956,11 +1024,15 @@ mp_status preheat_create_impl(const mp_mesh_desc* mesh, const double* xy, const 
     if (e == cudaSuccess) e = cudaMemsetAsync(p->d_status, 0xff, sizeof(unsigned long long), p->stream);
     if (xy && e == cudaSuccess) {
         const int gs = upload_quad_tables(p->nx, p->ny, xy, qt, 0, p->ny, p->stream, &p->qbuf, p->qdev, &e);
-        p->quad = true;
         if (gs == MP_ERR_ARG_WRONG) {
             pre_free(p); delete p;
             set_error("per-cell stencil table construction failed (singular stencil or degenerate cell)");
             return (mp_status)gs;
+        }
+        if (e == cudaSuccess) {
+            pre_quad_edge_kernel<<<(unsigned)((NE + 127) / 128), 128, 0, p->stream>>>(p->nx, p->ny, p->edge, p->qdev);
+            count_launch();
+            e = cudaGetLastError();
         }
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
@@ -1045,7 +1117,10 @@ extern "C" mp_status mp_preheat_begin(mp_preheat* p, double* rate, double* limit
     p->rate_max = rt.maximum;
     p->limit = p->rate_max > 0 ? p->opts.cfl / p->rate_max : p->opts.dt_max;
     // Integral, minimum and maximum of the initial H (preheat.cpp:245-249).
-    launch_update(p, p->Hb[p->cur], nullptr, PRE_MEASURE, 0.0, 0);
+    pre_measure_kernel<<<p->blocks, kPreBlock, 0, p->stream>>>((long long)p->N, p->quad ? 0.0 : p->host_tab.area,
+                                                               p->quad ? p->qdev.geo + 3 * p->N : nullptr,
+                                                               p->Hb[p->cur], p->partial, p->ctl);
+    count_launch();
     MP_CUDA(cudaGetLastError());
     MP_TRY(read_status(p));
     const PrePartial m = p->h_ctl->last;
@@ -1069,8 +1144,7 @@ extern "C" mp_status mp_preheat_rhs(mp_preheat* p, double* rhs, double* boundary
     if (!p) { set_error("null argument"); return MP_ERR_ARG_WRONG; }
     MP_TRY(reset_status(p));
     const double* H = p->Hb[p->cur];
-    launch_rhs_kernels(p, H);
-    launch_update(p, H, nullptr, PRE_RHS, 0.0, 0);
+    launch_step(p, H, nullptr, PRE_RHS, 0.0, 0);
     MP_CUDA(cudaGetLastError());
     MP_TRY(read_status(p));
     MP_TRY(pre_status(p, "mp_preheat_rhs"));
@@ -1106,8 +1180,7 @@ extern "C" mp_status mp_preheat_advance(mp_preheat* p, long long nsteps, mp_preh
             for (int k = 0; k < n; ++k) {
                 const double* H = p->Hb[(p->cur + k) & 1];
                 double* Hn = p->Hb[(p->cur + k + 1) & 1];
-                launch_rhs_kernels(p, H);
-                launch_update(p, H, Hn, PRE_STEP, dts[k], k);
+                launch_step(p, H, Hn, PRE_STEP, dts[k], k);
             }
             MP_CUDA(cudaGetLastError());
             MP_CUDA(cudaMemcpyAsync(p->h_rows, p->rows, (size_t)n * sizeof(PreRow), cudaMemcpyDeviceToHost, p->stream));

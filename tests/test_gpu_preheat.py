@@ -8,6 +8,7 @@ face fluxes, against its infinity norm (1e-12); step sizes, integrals and
 extrema of every history row 1e-12 relative (the boundary flux 1e-12 of
 max(1, |ref|)); failure statuses equal.
 """
+import dataclasses
 import os
 
 import numpy as np
@@ -320,3 +321,31 @@ def test_linear_field_gives_the_exact_rhs(cuda_lib, nx, ny, families):
             code, ref, _ = t.preheat_rhs()
             assert code == 0 and rel_inf(rhs, ref) <= RTOL, family
         p.close()
+
+
+# The step kernel's blocks own 30 columns and 4 n - 2 rows: one column more and
+# less, one row more and less, one column in the last block, and a mesh of
+# three row groups per block (the rule takes n = 1 below ~36 000 cells).
+@pytest.mark.parametrize("nx,ny", [(2, 3), (29, 4), (30, 2), (31, 5), (60, 3), (61, 7), (361, 301)])
+@pytest.mark.parametrize("name", ["through_diffusion", "global_fixed", "quad_through", "quad_outflow"])
+def test_preheat_step_blocks(cuda_lib, name, nx, ny):
+    case = pc.CASES[name]
+    if nx > 100 and name in ("global_fixed", "quad_outflow"):
+        pytest.skip("the large mesh runs once per mesh family")
+    # Steps of a tenth of the limit of these meshes' cells, for every case.
+    h = min(0.5 / nx, 1.0 / ny)
+    dt = 0.1 * min(h / 4.0, h * h / (8.0 * case.kappa))
+    case = dataclasses.replace(case, w=dataclasses.replace(case.w, nx=nx, ny=ny), control=1, dt_initial=dt,
+                               dt_max=dt, dt_min=0.0, end=2 * dt)
+    ref = pc.oracle_run(case)
+    p = pc.gpu_instance(case)
+    p.begin()
+    rhs, bflux = p.rhs()
+    assert rel_inf(rhs, ref["rhs"]) <= RTOL
+    assert abs(bflux - ref["bflux"]) <= RTOL * max(1.0, abs(ref["bflux"]))
+    code, rows = p.advance(2)
+    assert code == 0 and len(rows) == len(ref["rows"])
+    for row, want in zip(rows, ref["rows"]):
+        for k in ["integral", "minimum", "maximum"]:
+            assert abs(row[k] - want[k]) <= RTOL * max(abs(want[k]), 1e-300), k
+    assert rel(p.get_state()[0], ref["H"]) <= RTOL
