@@ -173,3 +173,46 @@ def test_scalar_helpers_and_classify(models):
     assert m.classify(math.nextafter(b.Tep, math.inf), 0.4 * p.Xe, 0.0) == 3
     with pytest.raises(ValueError):
         m.classify(0.5, 2.0, 0.0)
+
+
+def test_interval_ends_and_range_limits(models):
+    """Points on, one double beside and far from the interval ends of each
+    region, and scales on both sides of the limits of the division-free
+    evaluation. Regions as the host's FP64 boundaries select them; where the
+    oracle's 80-bit ends select the same one and the state does not sit on the
+    pure melting point (there T - Tmp is one rounding), its fields to RTOL."""
+    from oracle import pyoracle as po
+    m, p = models[0], ka.parameter_sets()[0]
+    ref = po.PhaseOracle(p)
+    H, C, region = [], [], []
+    for c in [0.0, 5e-324, 1e-300, 0.9e-200, 1e-200, 1e-12, 0.3 * p.Xe, np.nextafter(p.Xe, 0.0), p.Xe]:
+        b = m.boundaries(c, 0.0)
+        for end in (b.Tep, b.Tmp, b.H_eutectic_end, b.H_liquidus, 0.0, 0.7, 1e99, -1e99, 1.1e100, -1.1e100):
+            for h in (np.nextafter(end, -np.inf), end, np.nextafter(end, np.inf)):
+                H.append(h)
+                C.append(c)
+                if c == 0.0:
+                    region.append(1 if h <= b.Tmp else 6 if h < b.H_liquidus else 5)
+                else:
+                    region.append(2 if h <= b.Tep else 5 if h >= b.H_liquidus else 3 if h <= b.H_eutectic_end else 4)
+    out, code, bad = m.evaluate_batch(np.array(H), np.array(C), None, 0.0, raise_on_error=False)
+    got = {k: v.cpu().numpy() for k, v in out.items()}
+    assert np.array_equal(got["region"], region)
+    # The one refused state: the smallest composition one double above Tep,
+    # whose melt fraction underflows.
+    above = np.nextafter(m.boundaries(0.0, 0.0).Tep, np.inf)
+    refused = (np.array(C) == 5e-324) & (np.array(H) == above)
+    assert code == 103 and bad == np.nonzero(refused)[0][0] and np.array_equal(np.isnan(got["TDp"]), refused)
+    checked = 0
+    for i, (h, c) in enumerate(zip(H, C)):
+        st, want = ref.evaluate(h, c, 0.0)
+        tmp = m.boundaries(0.0, 0.0).Tmp
+        if st or refused[i] or want["region"] != region[i] or (c < 1e-3 and abs(h - tmp) < 1e-3):
+            continue
+        checked += 1
+        for f in FIELDS:
+            if f == "cs" and want["phi1"] + want["phi2"] <= 1e-12:
+                continue
+            w, g = want[f], got[f][i]
+            assert g == w or abs(g - w) <= RTOL * max(abs(w), 1e-3), (f, h, c, g, w)
+    assert checked > 150
