@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(128) batch_quad_diffusion_kernel(const QuadSta
 // kSrc: the adiabatic source terms are added. An instance with per-cell
 // areas (a general quad mesh) takes them.
 template <bool kSrc>
-__global__ void __launch_bounds__(kRedBlock) batch_sum_kernel(const InstArgs* args, const Work* work, const int* active) {
+__global__ void __launch_bounds__(kRedBlock, 4) batch_sum_kernel(const InstArgs* args, const Work* work, const int* active) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;
     const SumArgs& a = args[w.inst].sum;
@@ -202,9 +202,8 @@ __global__ void __launch_bounds__(kRedBlock) batch_commit_kernel(const CommitArg
     if (!active[w.inst]) return;
     const CommitArgs& a = args[w.inst];
     const int per = sum_per(a.n);
-#pragma unroll
-    for (int q = 0; q < kSumPer; ++q) {
-        if (q >= per) break;
+#pragma unroll 4
+    for (int q = 0; q < per; ++q) {
         const long long k = (long long)w.a + q * kRedBlock + threadIdx.x;
         if (k < a.n) { a.dstH[k] = a.srcH[k]; a.dstC[k] = a.srcC[k]; }
     }

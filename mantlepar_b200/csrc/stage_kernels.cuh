@@ -35,14 +35,21 @@ __device__ __forceinline__ size_t rec_at(long long cell) {
     return (size_t)((unsigned)cell >> 5) * (32 * kRec) + ((unsigned)cell & 31u);
 }
 constexpr int kRedBlock = 256;
-// The accumulation and axpy kernels give each thread kSumPer cells (strided
-// by the block size, so loads stay coalesced) before one block reduction; on
-// a mesh of at most kSmallCells cells (whose steps one cluster of 16 blocks
-// runs, small_steps.cu) one, so that every block of the cluster has a share.
-// A function of the mesh alone: the grouping fixes the order of the sums.
+// The accumulation and axpy kernels give each thread several cells (strided by
+// the block size, so loads stay coalesced) before one block reduction: as many
+// as make one wave of 592 resident blocks (at 640x1280 27 us; four cells and
+// 1.35 waves 35), at least four, and one below kSumOne, where few blocks leave
+// most of the GPU idle (61x127, one step with transfers: 311 us, four 323; a
+// 40x80 quad mesh, four steps: 818, 863; a batch of 24 uneven meshes the
+// same). A function of the mesh alone: the grouping fixes the order of the
+// sums.
 constexpr int kSumPer = 4;
-constexpr long long kSmallCells = 1536, kSmallQuadCells = 1024;
-__host__ __device__ __forceinline__ int sum_per(long long cells) { return cells <= kSmallCells ? 1 : kSumPer; }
+constexpr long long kSumOne = 16384, kSmallCells = 1536, kSmallQuadCells = 1024;
+static_assert(kSmallCells <= kSumOne, "the cluster's sums take one cell per thread");
+__host__ __device__ __forceinline__ int sum_per(long long cells) {
+    const long long wave = 592LL * kRedBlock, per = (cells + wave - 1) / wave;
+    return cells <= kSumOne ? 1 : (int)(per > kSumPer ? per : kSumPer);
+}
 __host__ __device__ __forceinline__ int sum_cells_per_block(long long cells) { return kRedBlock * sum_per(cells); }
 
 enum : int {
@@ -1353,21 +1360,21 @@ __device__ __forceinline__ void sum_cell(const SumArgs& a, unsigned cell, const 
     const double A = kArea ? __ldg(a.cell_area + cell) : a.area, invA = kArea ? 1.0 / A : a.inv_area;
     // Faces of this cell in the reference's id order: bottom, top, left, right,
     // each with the sign of its side (evolve.cpp:350-354).
-    const long long eb = (long long)j * nx + i, et = (long long)(j + 1) * nx + i;
-    const long long el = nI + (long long)j * (nx + 1) + i, er = el + 1;
+    const unsigned eb = cell, et = cell + (unsigned)nx;
+    const unsigned el = (unsigned)nI + cell + (unsigned)j, er = el + 1u;    // below 2^31 (mesh_too_large)
     MP_CHECK_INDEX(a.status, et, nI);
     MP_CHECK_INDEX(a.status, er, nE);
     const int gj = a.gj0 + j, gny = global_ny(a);
     const double sb = -1.0, stp = (gj == gny - 1) ? -1.0 : 1.0, sl = (i == 0) ? -1.0 : 1.0, sr = -1.0;
-    const long long ids[4] = {eb, et, el, er};
+    const unsigned ids[4] = {eb, et, el, er};
     const double sg[4] = {sb, stp, sl, sr};
+    const double *fH = a.face, *fC = fH + nE, *fR = fC + nE, *fM = fR + nE;
     // The reference divides each face term by the area; here the signed sums
     // are scaled once by 1/A (a few ulp apart).
     double rH = 0.0, rC = 0.0, rr = 0.0, dv = 0.0, bH = 0.0, bC = 0.0;
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
-        const double FH = MP_LD(a.face + ids[f]), FC = MP_LD(a.face + nE + ids[f]);
-        const double FR = MP_LD(a.face + 2 * nE + ids[f]), FM = MP_LD(a.face + 3 * nE + ids[f]);
+        const double FH = MP_LD(fH + ids[f]), FC = MP_LD(fC + ids[f]), FR = MP_LD(fR + ids[f]), FM = MP_LD(fM + ids[f]);
         rH += sg[f] * FH;
         rC += sg[f] * FC;
         rr += FR;
@@ -1379,10 +1386,10 @@ __device__ __forceinline__ void sum_cell(const SumArgs& a, unsigned cell, const 
         // The source terms follow the face terms, as the reference adds them.
         rH += MP_LD(a.srcH + cell); rr += MP_LD(a.srcR + cell); sH = MP_LD(a.srcS + cell);
     }
-    if (gj == 0) { bH += MP_LD(a.face + eb); bC += MP_LD(a.face + nE + eb); }
-    if (gj == gny - 1) { bH += MP_LD(a.face + et); bC += MP_LD(a.face + nE + et); }
-    if (i == 0) { bH += MP_LD(a.face + el); bC += MP_LD(a.face + nE + el); }
-    if (i == nx - 1) { bH += MP_LD(a.face + er); bC += MP_LD(a.face + nE + er); }
+    if (gj == 0) { bH += MP_LD(fH + eb); bC += MP_LD(fC + eb); }
+    if (gj == gny - 1) { bH += MP_LD(fH + et); bC += MP_LD(fC + et); }
+    if (i == 0) { bH += MP_LD(fH + el); bC += MP_LD(fC + el); }
+    if (i == nx - 1) { bH += MP_LD(fH + er); bC += MP_LD(fC + er); }
     double nh, nc;
     if (a.mode == SUM_RK) {
         const double dt_ = dtp ? *dtp : a.dt;
@@ -1406,7 +1413,7 @@ __device__ __forceinline__ void sum_cell(const SumArgs& a, unsigned cell, const 
     v.sH += sH;
 }
 
-// The kSumPer cells of this thread in the sum block starting at first.
+// This thread's cells in the sum block starting at first.
 // `first` counts from the start of the accumulated range [cbeg, cend); dtp:
 // where the step size is (null: in the arguments).
 template <bool kSrc = false, bool kArea = false>
@@ -1414,16 +1421,25 @@ __device__ __forceinline__ Partial sum_cells(const SumArgs& a, long long first, 
     const long long end = a.cend >= 0 ? a.cend : (long long)a.nx * a.ny;
     const int per = sum_per(end - a.cbeg);
     Partial v = partial_identity();
-#pragma unroll
-    for (int k = 0; k < kSumPer; ++k) {
-        if (k >= per) break;
+    auto add = [&](int k) {
         const long long c = a.cbeg + first + k * kRedBlock + threadIdx.x;
         if (c < end) sum_cell<kSrc, kArea>(a, (unsigned)c, dtp, v);
+    };
+    // A known count lets the cells' loads overlap (1 - 2 % of a step at 321x643).
+    if (per <= kSumPer) {
+#pragma unroll
+        for (int k = 0; k < kSumPer; ++k) {
+            if (k >= per) break;
+            add(k);
+        }
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < per; ++k) add(k);
     }
     return v;
 }
 
-// U1 = U^n + dt*L^n over the kSumPer cells of this thread, with the
+// U1 = U^n + dt*L^n over this thread's cells, with the
 // admissibility/integral partials of U1 (cell_area: per-cell areas, or null
 // for `area` everywhere).
 __device__ __forceinline__ Partial axpy_cells(long long n, const double* H0, const double* C0, const double* LH,
@@ -1431,9 +1447,8 @@ __device__ __forceinline__ Partial axpy_cells(long long n, const double* H0, con
                                               long long first, const double* cell_area = nullptr) {
     const int per = sum_per(n);
     Partial v = partial_identity();
-#pragma unroll
-    for (int q = 0; q < kSumPer; ++q) {
-        if (q >= per) break;
+#pragma unroll 4
+    for (int q = 0; q < per; ++q) {
         const long long k = first + q * kRedBlock + threadIdx.x;
         if (k >= n) continue;
         const double h = __dadd_rn(H0[k], __dmul_rn(dt, LH[k]));

@@ -118,8 +118,10 @@ __global__ void __launch_bounds__(128, 4) diffusion_kernel(const __grid_constant
     diffusion_edge(p.d, a, ph, all ? edge_by_kind(a.nx, a.ny, k) : edge_by_id(a.nx, a.ny, k < nh ? h0 + k : v0 + (k - nh)));
 }
 
+// Four resident blocks; with the source three (of 84 registers: a step of the
+// product physics at 256x512 takes 2 % less).
 template <bool kSrc, bool kArea = false>
-__global__ void __launch_bounds__(kRedBlock) sum_kernel(SumArgs a) {
+__global__ void __launch_bounds__(kRedBlock, kSrc ? 3 : 4) sum_kernel(SumArgs a) {
     if (gated_off(a.gate)) return;
     const Partial v = sum_cells<kSrc, kArea>(a, (long long)blockIdx.x * sum_cells_per_block(a.cend - a.cbeg), a.dtp);
     finish_block(v, a.shares, (int)blockIdx.x);
@@ -127,7 +129,7 @@ __global__ void __launch_bounds__(kRedBlock) sum_kernel(SumArgs a) {
 
 // U1 = U^n + dt*L^n with the admissibility/integral partials of U1 (dtp:
 // dt read from device memory; gate: see ReconArgs).
-__global__ void __launch_bounds__(kRedBlock) axpy_kernel(int n, const double* H0, const double* C0, const double* LH,
+__global__ void __launch_bounds__(kRedBlock, 4) axpy_kernel(int n, const double* H0, const double* C0, const double* LH,
                                                          const double* LC, double dt, double area, double* H1,
                                                          double* C1, Shares shares, const double* cell_area,
                                                          const double* dtp = nullptr, const int* gate = nullptr) {
