@@ -2,7 +2,7 @@
 // together, each with its own dt, CFL retries, balance check and status.
 //
 // Every stage is one launch per kernel over ALL active instances: a device
-// work map sends each thread block to (instance, tile) and the block's
+// work map sends each thread block to (instance, cells) and the block's
 // instance record holds that instance's buffers and tables. The per-element
 // arithmetic is the single-instance path's (stage_kernels.cuh; for general
 // quad meshes quad_kernels.cuh, over the quad instances' own work lists), and

@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(128, 4) diffusion_kernel(const __grid_constant
     diffusion_edge(p.d, a, ph, all ? edge_by_kind(a.nx, a.ny, k) : edge_by_id(a.nx, a.ny, k < nh ? h0 + k : v0 + (k - nh)));
 }
 
-// Four resident blocks; with the source three (of 84 registers: a step of the
+// Four resident blocks; with the source three (of 79 registers: a step of the
 // product physics at 256x512 takes 2 % less).
 template <bool kSrc, bool kArea = false>
 __global__ void __launch_bounds__(kRedBlock, kSrc ? 3 : 4) sum_kernel(SumArgs a) {
@@ -981,8 +981,10 @@ extern "C" size_t mp_transport_instance_bytes(const mp_mesh_desc* mesh, int quad
         const size_t V = 2 * (nx + 1) * (ny + 1);
         // Per-cell tables and geometry, vertices and edge spacing in one
         // allocation; the builder's copy of the vertices is held while the
-        // tables are built.
-        b += pages(((size_t)(kQG0 + kQT4 + kQMom + kQGeo) * N + V + NE * kNQ) * sizeof(double)) +
+        // tables are built. The budget counts a cell's folded smoothness
+        // forms (kQS9 + kQS4), which the device keeps only kQMom moments of:
+        // requests are admitted by the same figure as with them resident.
+        b += pages(((size_t)(kQG0 + kQS9 + kQT4 + kQS4 + kQGeo) * N + V + NE * kNQ) * sizeof(double)) +
              pages(V * sizeof(double) + sizeof(int));
     }
     return b;
