@@ -80,6 +80,14 @@ struct NormalCell {
     P2 m, b, c, d;
     // Jacobian j0 + jr r + js s of the map (d x d vanishes).
     __device__ __forceinline__ static double cross(P2 u, P2 v) { return fma(u.x, v.y, -__dmul_rn(u.y, v.x)); }
+    // The same over four times j0, the map's area: Gauss weights times it add
+    // up to one, whatever the corners' roundings.
+    __device__ __forceinline__ void mean_jacobian(double& j0, double& jr, double& js) const {
+        const double g = __dmul_rn(0.25, rcp(cross(b, c)));
+        j0 = 0.25;
+        jr = __dmul_rn(cross(b, d), g);
+        js = __dmul_rn(cross(d, c), g);
+    }
 };
 __device__ __forceinline__ NormalCell normal_cell(const CellFrame& f) {
     NormalCell k;

@@ -356,7 +356,8 @@ __device__ __forceinline__ void quad_cellphase_cell(const QuadStageArgs& a, cons
     load_rec(a.rec, cell, DH, DC);
     DH[0] += MP_LD(a.H + cell);
     DC[0] += MP_LD(a.C + cell);
-    const double j0 = k.cross(k.b, k.c), jr = k.cross(k.b, k.d), js = k.cross(k.d, k.c);
+    double j0, jr, js;
+    k.mean_jacobian(j0, jr, js);
     double Tsum = 0.0, Psum = 0.0, Ssum = 0.0, Rsum = 0.0;
 #pragma unroll 1
     for (int b = 0; b < kNQ; ++b) {

@@ -337,7 +337,8 @@ __device__ __noinline__ void small_phase(const SmallArgs& m, int kind, int group
                 const QuadDev& q = m.quad[kind].q;
                 const CellFrame f = cell_frame(q, nx, (size_t)N, cell);
                 const NormalCell k = normal_cell(f);
-                const double j0 = k.cross(k.b, k.c), jr = k.cross(k.b, k.d), js = k.cross(k.d, k.c);
+                double j0, jr, js;
+                k.mean_jacobian(j0, jr, js);
                 const double s = q.gq[b], ws = q.gw[b], js0 = fma(js, s, j0);
                 const double x0 = fma(k.c.x, s, k.m.x), y0 = fma(k.c.y, s, k.m.y);
                 const double x1 = fma(k.d.x, s, k.b.x), y1 = fma(k.d.y, s, k.b.y);

@@ -981,10 +981,9 @@ extern "C" size_t mp_transport_instance_bytes(const mp_mesh_desc* mesh, int quad
         const size_t V = 2 * (nx + 1) * (ny + 1);
         // Per-cell tables and geometry, vertices and edge spacing in one
         // allocation; the builder's copy of the vertices is held while the
-        // tables are built. The budget counts a cell's folded smoothness
-        // forms (kQS9 + kQS4), which the device keeps only kQMom moments of:
-        // requests are admitted by the same figure as with them resident.
-        b += pages(((size_t)(kQG0 + kQS9 + kQT4 + kQS4 + kQGeo) * N + V + NE * kNQ) * sizeof(double)) +
+        // tables are built. The budget takes kQBudget doubles of tables per
+        // cell (quad_tables.hpp).
+        b += pages(((size_t)kQBudget * N + V + NE * kNQ) * sizeof(double)) +
              pages(V * sizeof(double) + sizeof(int));
     }
     return b;
