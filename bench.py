@@ -48,12 +48,12 @@ WORKLOAD = dict(nx=1280, ny=2560)
 ALG_BYTES_PER_CELL_STAGE = 224
 # Executed FP64 operations per cell per stage (DFMA counted as 2, DADD/DMUL
 # as 1) of the stage kernels, from an ncu capture of a 640x1280 stage:
-# reconstruction 2073, cell phase 1188, faces 1703, accumulation ~48
+# reconstruction 1156, cell phase 796, faces 1080, accumulation 43
 # (per-cell figures are size-independent).
-FP64_FLOPS_PER_CELL_STAGE = 5012
+FP64_FLOPS_PER_CELL_STAGE = 3075
 # DRAM bytes per cell per stage of the four stage kernels from the same capture
 # (640x1280 keeps every stage array above L2 size; traffic scales with cells).
-DRAM_BYTES_PER_CELL_STAGE = 924
+DRAM_BYTES_PER_CELL_STAGE = 903
 # B200 FP64 (vector and tensor) datasheet figure per GPU of an HGX B200
 # (296 TFLOP/s for 8 GPUs); the driver measures no FP64 peak.
 FP64_DATASHEET_TFLOPS = 37.0
@@ -288,12 +288,9 @@ def timed_steps(obj, steps, stream):
     return e0.elapsed_time(e1), out
 
 
-# Legacy dry preheat (src/couple/preheat.cpp) per cell-step: unlimited H
-# reconstruction (read H, write 9 coefficients), edge fluxes (read both
-# sides' coefficients and averages, 2 edges x 5 normal velocities, write 2
-# fluxes), update (read H and 4 fluxes, write H): 8 + 72 + 72 + 8 + 80 + 16 +
-# 8 + 16 + 8 bytes.
-PREHEAT_BYTES_PER_CELL_STEP = 288
+# Legacy dry preheat (src/couple/preheat.cpp) per cell-step, one kernel: read
+# H and the normal velocities of 2 edges x 5 points, write H: 8 + 80 + 8 bytes.
+PREHEAT_BYTES_PER_CELL_STEP = 96
 
 
 def preheat_form(steps, stream, nx=None, ny=None, perturbed=False):
@@ -345,13 +342,13 @@ def preheat_form(steps, stream, nx=None, ny=None, perturbed=False):
                       f"host round trip every 512 steps"}
 
 
-# Per-cell tables a stage of the general-quad path streams (G0 72, S9 36,
-# T4 48, S4 24, geometry 4 doubles).
-QUAD_TABLE_BYTES_PER_CELL = 184 * 8
+# Per-cell tables a stage of the general-quad path streams (G0 72, T4 36 of 48
+# (the constants are not read), moments 6, geometry 4 doubles).
+QUAD_TABLE_BYTES_PER_CELL = 118 * 8
 # What a preheat step on a general quad mesh reads beyond the uniform one:
-# the per-cell tables, the normal-line spacing of the 2 owned edges x 5
-# points, and one vertex (x, y) per cell.
-PREHEAT_QUAD_EXTRA_BYTES = QUAD_TABLE_BYTES_PER_CELL + 2 * 5 * 8 + 16
+# the per-cell tables, two numbers for each of the 2 owned edges, and one
+# vertex (x, y) per cell.
+PREHEAT_QUAD_EXTRA_BYTES = QUAD_TABLE_BYTES_PER_CELL + 2 * 2 * 8 + 16
 
 
 def quads_form(steps, stream, nx=None, ny=None):
