@@ -703,7 +703,8 @@ mp_status launch_small_steps(const SmallMesh& s, int blocks, cudaStream_t stream
     m.partial = s.partial; m.status = s.status; m.ctl = s.ctl; m.hdr = s.hdr; m.reports = s.reports;
     const void* f = small_kernel(s.quad, s.ph->litho != 0);
     cudaLaunchAttribute attr[1];
-    const cudaLaunchConfig_t cfg = small_config(blocks, attr);
+    cudaLaunchConfig_t cfg = small_config(blocks, attr);
+    cfg.stream = stream;
     void* args[] = {&m};
     MP_CUDA(cudaLaunchKernelExC(&cfg, f, args));
     return MP_OK;
