@@ -437,11 +437,15 @@ __device__ __forceinline__ void load_rec(const double* rec, long long cell, doub
 // Cell quadrature of T and phi (evolve.cpp:359-376) and the wet flag of the
 // porosity sampling (initial_flow.cpp:56-67) on the same 5x5 points, with
 // every point's admissibility test and the exact check of the diffusion
-// samples. Out of line: cells that are not plain.
+// samples: cells that are not plain. Inlined, as the other tested forms are: a
+// function of its own reads the tables and constants through generic pointers
+// into the kernel's parameters. Where no cell is plain (pure composition,
+// 640x1280) the cell phase takes 60 us so and took 90 that way, the faces 185
+// and 222, the diffusion 250 and 313; plain cells are as fast either way.
 // kExt: the lithostatic pressure and the adiabatic source are compiled in
 // (a launch picks the variant; the default path carries none of their code).
 template <bool kExt>
-__device__ __noinline__ void cellphase_general(const StageHot& t, const CellPhaseArgs& a, const Physics& ph, long long cell) {
+__device__ __forceinline__ void cellphase_general(const StageHot& t, const CellPhaseArgs& a, const Physics& ph, long long cell) {
     const long long N = (long long)a.nx * a.ny;
     if (cell >= N) return;
     MP_CHECK_INDEX(a.status, cell, N);
@@ -804,7 +808,7 @@ struct EdgeAt {
     bool horizontal;
     int i, j;
 };
-// Edge k in id order (slabs, and the out-of-line forms below).
+// Edge k in id order (slabs, and the tested forms below).
 __device__ __forceinline__ EdgeAt edge_by_id(int nx, int ny, long long e) {
     const long long nI = (long long)nx * (ny + 1);
     if (e < nI) return EdgeAt{true, (int)((unsigned)e % (unsigned)nx), (int)((unsigned)e / (unsigned)nx)};
@@ -856,11 +860,11 @@ __device__ __forceinline__ EdgeCells edge_cells(const FaceArgs& a, const EdgeAt&
     return c;
 }
 
-// An edge of any cells, every point with its admissibility tests. Out of
-// line: edges with a cell that is not plain.
+// An edge of any cells, every point with its admissibility tests: edges with
+// a cell that is not plain.
 // kExt: the lithostatic pressure is compiled in.
 template <bool kExt>
-__device__ __noinline__ void face_general(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
+__device__ __forceinline__ void face_general(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
     const long long nE = (long long)a.nx * (a.ny + 1) + (long long)(a.nx + 1) * a.ny;
     const size_t N = (size_t)a.nx * a.ny;
     const EdgeAt at_ = edge_by_id(a.nx, a.ny, e);
@@ -1033,8 +1037,8 @@ __device__ __forceinline__ void face_edge(const StageHot& t, const FaceArgs& a, 
 // wall value), gradient sum_k c_k (T_k - T_last) / ds, flux -= w kappa grad,
 // and |d flux / d T_k| added to the rate sample by sample. Added to the face
 // results after the advective part, as the reference adds them.
-// Out of line: edges with a cell that is not plain.
-__device__ __noinline__ void diffusion_general(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
+// Edges with a cell that is not plain.
+__device__ __forceinline__ void diffusion_general(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
     const int nx = a.nx, ny = a.ny;
     const long long nI = (long long)nx * (ny + 1);
     const long long nE = nI + (long long)(nx + 1) * ny;

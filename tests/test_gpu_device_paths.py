@@ -45,3 +45,61 @@ def test_steps_run_on_the_handles_stream(cuda_lib, nx, ny, quad):
     assert got[0][:2] == got[1][:2]
     for x, y in zip(got[0][2], got[1][2]):
         assert np.array_equal(x, y)
+
+
+def untidy_state(w, kind):
+    """States whose cells are not plain: pure component, eutectic composition,
+    or a band of C = 0 beside a ramp."""
+    n = np.arange(w.cells)
+    x, y = (n % w.nx + 0.5) / w.nx, (n // w.nx + 0.5) / w.ny
+    H = 0.05 + 0.6 * y + 0.02 * sy.unit_noise(w.seed, 0, n.astype(np.uint64))
+    C = {"pure": 0.0 * x, "eutectic": 0.5 + 0.0 * x, "ramp": 0.3 * np.clip(x - 0.4, 0.0, 1.0)}[kind]
+    return H, C
+
+
+@pytest.mark.parametrize("kind", ["pure", "eutectic", "ramp"])
+@pytest.mark.parametrize("nx,ny,quad", [(9, 7, False), (25, 33, False), (48, 40, False), (9, 7, True), (19, 25, True),
+                                        (36, 40, True)])
+def test_cells_that_are_not_plain_agree_on_every_path(cuda_lib, nx, ny, quad, kind):
+    """The tested forms of the cell phase, faces and diffusion are compiled
+    into the stage kernels, the batch's kernels and the cluster kernel: device
+    steps, the host-driven loop and a batch give the same doubles."""
+    from mantlepar_b200.batch import Batch
+    from mantlepar_b200.transport import Transport, TransportConfig
+    w = sy.Workload(nx=nx, ny=ny, seed=5)
+    xy = sy.quad_vertices(w, sy.MESH_PERTURBED, 0.2, seed=11) if quad else None
+    cfg = TransportConfig(cfl=0.4, integrator=3, diffusivity=1e-3)
+    types, values = (1, 2, 0, 1), (0.9, -0.02, 0.0, 0.4)
+    velocity = sy.face_velocity_quads(w, xy) if quad else sy.face_velocity(w)
+    state = untidy_state(w, kind)
+    got = []
+    for device in (True, False):
+        t = Transport(w, cfg, vertices=xy)
+        t.set_device_steps(device)
+        t.set_thermal_bc(types, values)
+        t.set_face_velocity(*velocity)
+        t.set_state(*state)
+        code, reps = t.step(5, raise_on_error=False)
+        got.append((code, reps, t.get_time(), t.get_state()))
+        t.close()
+    b = Batch([w] if not quad else [sy.Workload(nx=4, ny=4)], cfg)
+    k = b.add_quads(w, xy) if quad else 0
+    b.set_thermal_bc(types, values)
+    if quad:
+        b.set_face_velocity(0, *sy.face_velocity(sy.Workload(nx=4, ny=4)))
+        b.set_state(0, *sy.initial_state(sy.Workload(nx=4, ny=4)))
+    b.set_face_velocity(k, *velocity)
+    b.set_state(k, *state)
+    b.step(5)
+    s = b.get_state(k)
+    b.close()
+    a, h = got
+    assert a[:3] == h[:3]
+    for x, y in zip(a[3], h[3]):
+        assert np.array_equal(x, y)
+    if kind != "ramp":
+        assert a[0] == 0
+    if a[0] == 0:
+        assert s["status"] == 0
+        for x, name in zip(a[3], ("H", "C", "T", "phi")):
+            assert np.array_equal(x, s[name]), name
