@@ -585,21 +585,75 @@ __global__ void __launch_bounds__(128, 5) quad_face_kernel(const __grid_constant
 
 // Diffusive H flux and rate of one edge (diffusiveflux.cpp:105-200 through
 // evolve.cpp:330-347): temperatures of the limited states at the normal-line
-// samples, spacing per edge point.
+// samples, spacing per edge point. By Gauss point, so that the lanes of
+// small_steps.cu share an edge: quad_diffusion_gradient is the temperature
+// gradient at point k of an interior edge or a wall of prescribed temperature,
+// quad_diffusion_add the sums over the points in their order.
+__device__ __forceinline__ double quad_diffusion_gradient(const QuadDev& q, const Physics& ph, const QuadEdge& g,
+                                                          const P2& nrm, const Side& sl, const Side& sr, int k, int& st) {
+    const int cq = g.reverse ? kNQ - 1 - k : k;
+    const P2 p = lerp_edge(q.gq[k], g.a, g.b);
+    const double sp = __ldg(q.sp + g.e * kNQ + cq);
+    const int count = g.boundary ? 5 : 4;
+    double v[5];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const bool left = g.boundary || s < 2;
+        const double d = (g.boundary ? (double)(s - 4) : (double)s - 1.5) * sp;
+        const P2 x = P2{p.x + d * nrm.x, p.y + d * nrm.y};
+        double h, c;
+        side_values(left ? sl : sr, x, h, c);
+        const double tep = ph.litho ? tep_at(ph, x.y) : ph.Tep;
+        PhaseLean pl;
+        int s1 = phase_stage_lean(ph.sk, h, c, tep, pl);
+        if (!s1 && !(pl.T >= 0.0 && pl.phil < 1.0)) s1 = E_OUTOFRANGE;
+        if (s1) st = st ? st : s1;
+        v[s] = s1 ? 0.0 : pl.T;
+    }
+    v[4] = g.boundary ? ph.wall_value[g.wall] : 0.0;
+    const double* c = g.boundary ? q.dif_c_bnd : q.dif_c_int;
+    const double last = v[count - 1];
+    double grad = 0.0;
+    for (int s = 0; s + 1 < count; ++s) grad += c[s] * (v[s] - last);
+    grad /= sp;
+    if (!isfinite(grad)) st = st ? st : E_FP;
+    return grad;
+}
+// Adds the diffusive part to the edge's H flux and rate; gradient(k): the
+// gradient at point k (called for them in order).
+template <class Gradient>
+__device__ __forceinline__ void quad_diffusion_add(const QuadStageArgs& a, const Physics& ph, const QuadEdge& g, int type,
+                                                   double len, Gradient&& gradient) {
+    const QuadDev& q = a.q;
+    const long long nE = (long long)a.nx * (a.ny + 1) + (long long)(a.nx + 1) * a.ny;
+    const int count = g.boundary ? 5 : 4;
+    const double* c = g.boundary ? q.dif_c_bnd : q.dif_c_int;
+    double integral = 0.0, rate = a.face[2 * nE + g.e];
+    for (int k = 0; k < kNQ; ++k) {
+        const double w = len * q.gw[k] / 2;
+        if (g.boundary && type == 2) { integral += w * ph.wall_value[g.wall]; continue; }
+        const double sp = __ldg(q.sp + g.e * kNQ + (g.reverse ? kNQ - 1 - k : k));
+        integral = fma(-(w * ph.kappa), gradient(k), integral);
+        double clast = 0.0;
+        for (int s = 0; s + 1 < count; ++s) clast -= c[s];
+        const double scale = -w * ph.kappa / sp;
+        for (int s = 0; s < count; ++s) {
+            if (g.boundary && s + 1 == count) continue;
+            rate += fabs(scale * (s + 1 == count ? clast : c[s]));
+        }
+    }
+    a.face[g.e] += integral;
+    a.face[2 * nE + g.e] = rate;
+}
 __device__ __forceinline__ void quad_diffusion_edge(const QuadStageArgs& a, const Physics& ph, long long e) {
     const int nx = a.nx, ny = a.ny, gj0 = a.gj0, gny = a.gny;
-    const double* H = a.H;
-    const double* C = a.C;
-    unsigned long long* status = a.status;
     const QuadDev& q = a.q;
-    const double* rec = a.rec;
-    double* face = a.face;
     const long long nE = (long long)nx * (ny + 1) + (long long)(nx + 1) * ny;
     const size_t N = (size_t)nx * ny;
-    MP_CHECK_INDEX(status, e, nE);
+    MP_CHECK_INDEX(a.status, e, nE);
     const QuadEdge g = quad_edge(q, nx, ny, gj0, gny, e);
-    MP_CHECK_INDEX(status, g.L, N);
-    if (!g.boundary) MP_CHECK_INDEX(status, g.R, N);
+    MP_CHECK_INDEX(a.status, g.L, N);
+    if (!g.boundary) MP_CHECK_INDEX(a.status, g.R, N);
     const int type = g.boundary ? ph.wall_type[g.wall] : 1;
     if (g.boundary && type == 0) return;
     double len;
@@ -607,51 +661,12 @@ __device__ __forceinline__ void quad_diffusion_edge(const QuadStageArgs& a, cons
     edge_geometry(g.a, g.b, len, nrm);
     Side sl, sr;
     if (type == 1) {
-        load_side(q, N, H, C, rec, g.L, sl);
-        if (!g.boundary) load_side(q, N, H, C, rec, g.R, sr);
+        load_side(q, N, a.H, a.C, a.rec, g.L, sl);
+        if (!g.boundary) load_side(q, N, a.H, a.C, a.rec, g.R, sr);
     }
-    double integral = 0.0, rate = face[2 * nE + e];
-    const double kappa = ph.kappa;
     int st = 0;
-    for (int k = 0; k < kNQ; ++k) {
-        const double w = len * q.gw[k] / 2;
-        if (g.boundary && type == 2) { integral += w * ph.wall_value[g.wall]; continue; }
-        const int cq = g.reverse ? kNQ - 1 - k : k;
-        const P2 p = lerp_edge(q.gq[k], g.a, g.b);
-        const double sp = __ldg(q.sp + e * kNQ + cq);
-        const int count = g.boundary ? 5 : 4;
-        double v[5];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const bool left = g.boundary || s < 2;
-            const double d = (g.boundary ? (double)(s - 4) : (double)s - 1.5) * sp;
-            const P2 x = P2{p.x + d * nrm.x, p.y + d * nrm.y};
-            double h, c;
-            side_values(left ? sl : sr, x, h, c);
-            const double tep = ph.litho ? tep_at(ph, x.y) : ph.Tep;
-            PhaseLean pl;
-            int s1 = phase_stage_lean(ph.sk, h, c, tep, pl);
-            if (!s1 && !(pl.T >= 0.0 && pl.phil < 1.0)) s1 = E_OUTOFRANGE;
-            if (s1) st = st ? st : s1;
-            v[s] = s1 ? 0.0 : pl.T;
-        }
-        v[4] = g.boundary ? ph.wall_value[g.wall] : 0.0;
-        const double* c = g.boundary ? q.dif_c_bnd : q.dif_c_int;
-        const double last = v[count - 1];
-        double grad = 0.0, clast = 0.0;
-        for (int s = 0; s + 1 < count; ++s) { grad += c[s] * (v[s] - last); clast -= c[s]; }
-        grad /= sp;
-        if (!isfinite(grad)) st = st ? st : E_FP;
-        integral -= w * kappa * grad;
-        const double scale = -w * kappa / sp;
-        for (int s = 0; s < count; ++s) {
-            if (g.boundary && s + 1 == count) continue;
-            rate += fabs(scale * (s + 1 == count ? clast : c[s]));
-        }
-    }
-    if (st) record_error(status, PART_FACES, g.L + (long long)gj0 * nx, st);
-    face[e] += integral;
-    face[2 * nE + e] = rate;
+    quad_diffusion_add(a, ph, g, type, len, [&](int k) { return quad_diffusion_gradient(q, ph, g, nrm, sl, sr, k, st); });
+    if (st) record_error(a.status, PART_FACES, g.L + (long long)gj0 * nx, st);
 }
 __global__ void __launch_bounds__(128) quad_diffusion_kernel(const __grid_constant__ QuadStageArgs a, const __grid_constant__ Physics ph,
                                                              long long h0, long long nh, long long v0, long long nv,

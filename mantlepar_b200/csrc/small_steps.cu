@@ -66,13 +66,17 @@ struct Board {
 
 constexpr int kSmallThreads = 512;
 
+// Largest meshes (small_steps_blocks); kSmallCells is in stage_kernels.cuh.
+constexpr long long kSmallCellsMore = 1024, kSmallQuadCells = 1024, kSmallQuadDiffusion = 640;
+
 // A mesh this small leaves a cell's chain of dependent FP64 instructions as
 // the length of a phase, so a group of eight lanes shares each element:
 // reconstruction and limiter by field and quarter of the limiter's lines or
 // points, the cell quadrature by row, a face by Gauss point. Extremes combine
 // in any order and sums are added by one lane in the kernels' order, so the
 // values are those of one thread per element. Cells and edges that are not
-// plain fall to the group's first lane and the kernels' own forms.
+// plain, and the diffusion of a uniform mesh, take the kernels' own forms
+// (each_of_warp).
 constexpr int kGroup = 8;
 constexpr unsigned kAll = 0xffffffffu;
 
@@ -95,9 +99,10 @@ __device__ __forceinline__ double points_sum(const double (&w)[kNQ], double v) {
 
 // Limiter factors, records and flag byte of the group's cell from each field's
 // extremes (lanes 0-3 field H, 4-7 field C, quarter `part` of its scan; mq:
-// the largest value of its share of the cell quadrature points).
+// the largest value of its share of the cell quadrature points). True in the
+// group's first lane when the cell is not plain.
 template <class TepRange>
-__device__ __forceinline__ void small_limit(const Physics& ph, bool active, int part, int f, long long cell, double mean,
+__device__ __forceinline__ bool small_limit(const Physics& ph, bool active, int part, int f, long long cell, double mean,
                                             double lo, double hi, Extremes x, double mq, int st, bool bad,
                                             const double (&D)[9], double* rec, unsigned char* flags, unsigned long long* status,
                                             TepRange&& tep_range) {
@@ -114,20 +119,98 @@ __device__ __forceinline__ void small_limit(const Physics& ph, bool active, int 
     const int stH = __shfl_sync(kAll, st, 0, kGroup), stC = __shfl_sync(kAll, st, 4, kGroup);
     const int okH = __shfl_sync(kAll, (int)mean_ok, 0, kGroup), okC = __shfl_sync(kAll, (int)mean_ok, 4, kGroup);
     const int badH = __shfl_sync(kAll, (int)bad, 0, kGroup), badC = __shfl_sync(kAll, (int)bad, 4, kGroup);
-    if (!active) return;
+    if (!active) return false;
     double* r = rec + rec_at(cell) + f * 9 * kRecStride;
 #pragma unroll
     for (int m = 0; m < 9; ++m)
         if ((m & 3) == part) r[m * kRecStride] = D[m] * th;
-    if (part == 0 && f == 0) {
-        const int st_all = stH ? stH : stC;
-        const int st_lim = !(okH && okC) ? (int)E_OUTOFRANGE : (badH || badC ? (int)E_FP : 0);
-        double t0, t1;
-        tep_range(t0, t1);
-        flags[cell] = st_all || st_lim ? (unsigned char)FLAG_CHECK
-                                       : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), lo, hi, loC, hiC, fma(th, mq, mean));
-        if (st_all) record_error(status, PART_UPDATE, cell, st_all);
-        if (st_lim) record_error(status, PART_LIMIT, cell, st_lim);
+    if (part != 0 || f != 0) return false;
+    const int st_all = stH ? stH : stC;
+    const int st_lim = !(okH && okC) ? (int)E_OUTOFRANGE : (badH || badC ? (int)E_FP : 0);
+    double t0, t1;
+    tep_range(t0, t1);
+    const unsigned char fl = st_all || st_lim ? (unsigned char)FLAG_CHECK
+                                              : cell_flags(ph, fmin(t0, t1), fmax(t0, t1), lo, hi, loC, hiC, fma(th, mq, mean));
+    flags[cell] = fl;
+    if (st_all) record_error(status, PART_UPDATE, cell, st_all);
+    if (st_lim) record_error(status, PART_LIMIT, cell, st_lim);
+    return !(fl & FLAG_PLAIN);
+}
+
+// What takes a whole element in one lane runs after the warp's rounds of four
+// elements, each element in a lane of its own, and out of line. Done in every
+// round by the first lane of each group, four steps of a 32x48 mesh of pure
+// component took 980 us, with diffusion 1597; so 618 and 857 (the graph 537
+// and 677).
+template <class F>
+__device__ __forceinline__ void each_of_warp(int group, int groups, int count, F&& f) {
+    const int lane = threadIdx.x & 31, base = group - (lane >> 3);
+    __syncwarp();
+    for (int k = lane;; k += 32) {
+        const int at = base + (k >> 2) * groups + (k & 3);
+        if (at >= count) break;
+        f(at);
+    }
+}
+template <bool kQuad, bool kLitho>
+__device__ __noinline__ void small_cells_rest(const SmallArgs& m, int kind, int group, int groups) {
+    const CellPhaseArgs& a = m.phase[kind];
+    each_of_warp(group, groups, m.nx * m.ny, [&](int cell) {
+        if (a.flags[cell] & FLAG_PLAIN) return;
+        if (kQuad) quad_cellphase_general(m.quad[kind], m.ph, cell);
+        else cellphase_general<kLitho>(m.tab, a, m.ph, cell);
+    });
+}
+template <bool kQuad, bool kLitho>
+__device__ __noinline__ void small_edges_rest(const SmallArgs& m, int kind, int group, int groups) {
+    const int nx = m.nx, ny = m.ny;
+    const FaceArgs& a = m.face[kind];
+    each_of_warp(group, groups, nx * (ny + 1) + (nx + 1) * ny, [&](int k) {
+        const EdgeAt at = edge_by_kind(nx, ny, k);
+        const EdgeCells g = edge_cells(a, at);
+        if (!(a.flags[g.L] & (g.boundary ? 0xff : a.flags[g.R]) & FLAG_PLAIN)) {
+            if (kQuad) quad_face_general(m.quad[kind], m.ph, g.e);
+            else face_general<kLitho>(m.tab, a, m.ph, g.e);
+        }
+        if (!kQuad && m.ph.diffusion) diffusion_edge(m.tab, a, m.ph, at);
+    });
+}
+
+// Diffusion on a general quad mesh: lane p < 5 takes the p-th Gauss point's
+// gradient, the first lane adds them up (four steps of a 20x24 mesh 807 us;
+// with an edge per lane 1111, the graph 1240).
+__device__ __noinline__ void small_quad_diffusion(const SmallArgs& m, int kind, int group, int groups) {
+    const QuadStageArgs& a = m.quad[kind];
+    const Physics& ph = m.ph;
+    const int nx = m.nx, ny = m.ny, edges = nx * (ny + 1) + (nx + 1) * ny;
+    const int l = threadIdx.x & 7, p = min(l, kNQ - 1);
+    const size_t N = (size_t)nx * ny;
+    __syncwarp();
+    for (int base = group - ((threadIdx.x & 31) >> 3); base < edges; base += groups) {
+        const int k0 = base + (int)((threadIdx.x & 31) >> 3);
+        const EdgeAt at = edge_by_kind(nx, ny, k0 < edges ? k0 : edges - 1);
+        const QuadEdge g = quad_edge(a.q, nx, ny, 0, ny, at.horizontal, at.i, at.j);
+        const int type = g.boundary ? ph.wall_type[g.wall] : 1;
+        double len, grad = 0.0, all[kNQ];
+        P2 nrm;
+        edge_geometry(g.a, g.b, len, nrm);
+        int st = 0;
+        if (type == 1) {
+            Side sl, sr;
+            load_side(a.q, N, a.H, a.C, a.rec, g.L, sl);
+            if (!g.boundary) load_side(a.q, N, a.H, a.C, a.rec, g.R, sr);
+            grad = quad_diffusion_gradient(a.q, ph, g, nrm, sl, sr, p, st);
+        }
+        int first = 0;                      // failure of the first point that has one
+#pragma unroll
+        for (int n = 0; n < kNQ; ++n) {
+            all[n] = group_get(grad, n);
+            const int s = __shfl_sync(kAll, st, n, kGroup);
+            first = first ? first : s;
+        }
+        if (k0 >= edges || l != 0 || type == 0) continue;
+        quad_diffusion_add(a, ph, g, type, len, [&](int k) { return all[k]; });
+        if (first) record_error(a.status, PART_FACES, g.L, first);
     }
 }
 
@@ -141,6 +224,7 @@ __device__ __noinline__ void small_recon(const SmallArgs& m, int kind, int group
     const ReconArgs& a = m.recon[kind];
     const int nx = m.nx, ny = m.ny, N = nx * ny;
     const int l = threadIdx.x & 7, f = l >> 2, part = l & 3;
+    bool rest = false;
     for (int base = group - ((threadIdx.x & 31) >> 3); base < N; base += groups) {
         const int c0 = base + (int)((threadIdx.x & 31) >> 3);
         const bool active = c0 < N;
@@ -208,7 +292,7 @@ __device__ __noinline__ void small_recon(const SmallArgs& m, int kind, int group
             x = Extremes{mx, mn};
             mq = mx;
         }
-        small_limit(m.ph, active, part, f, cell, mean, lo, hi, x, mq, st, bad, D, a.rec, a.flags, a.status,
+        rest |= small_limit(m.ph, active, part, f, cell, mean, lo, hi, x, mq, st, bad, D, a.rec, a.flags, a.status,
                     [&](double& t0, double& t1) {
                         t0 = t1 = m.ph.Tep;
                         if (m.ph.litho) {
@@ -216,10 +300,8 @@ __device__ __noinline__ void small_recon(const SmallArgs& m, int kind, int group
                             t1 = tep_at(m.ph, t.y0 + (j + 1) * t.dy);
                         }
                     });
-        __syncwarp();
-        if (active && l == 0 && !(a.flags[cell] & FLAG_PLAIN)) cellphase_general<kLitho>(t, m.phase[kind], m.ph, cell);
-        __syncwarp();
     }
+    if (__any_sync(kAll, rest)) small_cells_rest<false, kLitho>(m, kind, group, groups);
 }
 
 // The same on a general quad mesh: each lane of a field scans one edge's
@@ -229,6 +311,7 @@ __device__ __noinline__ void small_quad_recon(const SmallArgs& m, int kind, int 
     const QuadDev& q = a.q;
     const int nx = m.nx, ny = m.ny, N = nx * ny;
     const int l = threadIdx.x & 7, f = l >> 2, part = l & 3;
+    bool rest = false;
     for (int base = group - ((threadIdx.x & 31) >> 3); base < N; base += groups) {
         const int c0 = base + (int)((threadIdx.x & 31) >> 3);
         const bool active = c0 < N;
@@ -300,7 +383,7 @@ __device__ __noinline__ void small_quad_recon(const SmallArgs& m, int kind, int 
             x = Extremes{ext[0], ext[1]};
             mq = ext[0];
         }
-        small_limit(m.ph, active, part, f, cell, mean, lo, hi, x, mq, st, bad, D[0], a.rec, a.flags, a.status,
+        rest |= small_limit(m.ph, active, part, f, cell, mean, lo, hi, x, mq, st, bad, D[0], a.rec, a.flags, a.status,
                     [&](double& t0, double& t1) {
                         t0 = t1 = m.ph.Tep;
                         if (m.ph.litho) {
@@ -311,10 +394,8 @@ __device__ __noinline__ void small_quad_recon(const SmallArgs& m, int kind, int 
                             t1 = tep_at(m.ph, yhi);
                         }
                     });
-        __syncwarp();
-        if (active && l == 0 && !(a.flags[cell] & FLAG_PLAIN)) quad_cellphase_general(a, m.ph, cell);
-        __syncwarp();
     }
+    if (__any_sync(kAll, rest)) small_cells_rest<true, false>(m, kind, group, groups);
 }
 
 // Cell quadrature of the plain cells: lane b < 5 takes row b.
@@ -386,6 +467,7 @@ __device__ __noinline__ void small_faces(const SmallArgs& m, int kind, int group
     const int l = threadIdx.x & 7, p = min(l, kNQ - 1);
     const FaceArgs& a = m.face[kind];
     const Physics& ph = m.ph;
+    bool rest = false;
     for (int base = group - ((threadIdx.x & 31) >> 3); base < edges; base += groups) {
         const int k0 = base + (int)((threadIdx.x & 31) >> 3);
         const bool active = k0 < edges;
@@ -459,20 +541,14 @@ __device__ __noinline__ void small_faces(const SmallArgs& m, int kind, int group
             const int s = __shfl_sync(kAll, st, n, kGroup);
             st = st ? st : s;
         }
-        if (active && l == 0) {
-            if (!plain) {
-                if (kQuad) quad_face_general(m.quad[kind], ph, g.e);
-                else face_general<kLitho>(m.tab, a, ph, g.e);
-            } else {
-                if (st) record_error(a.status, PART_FACES, g.L, st);
-                store_face(a, g.e, half, fluxH, fluxC, rate, fluxMix);
-            }
-            if (ph.diffusion) {
-                if (kQuad) quad_diffusion_edge(m.quad[kind], ph, g.e);
-                else diffusion_edge(m.tab, a, ph, at);
-            }
+        rest = rest || (active && (!plain || (!kQuad && ph.diffusion)));
+        if (active && l == 0 && plain) {
+            if (st) record_error(a.status, PART_FACES, g.L, st);
+            store_face(a, g.e, half, fluxH, fluxC, rate, fluxMix);
         }
     }
+    if (__any_sync(kAll, rest)) small_edges_rest<kQuad, kLitho>(m, kind, group, groups);
+    if (kQuad && ph.diffusion) small_quad_diffusion(m, kind, group, groups);
 }
 
 template <bool kQuad>
@@ -656,14 +732,26 @@ int small_blocks(const void* f) {
 
 }  // namespace
 
-// One SSPRK3 step, this kernel against the graph (us): uniform meshes 20x20
-// 101 / 173, 25x40 124 / 167, 32x48 162 / 172, 32x64 157 / 143, 40x80 203 /
-// 146; perturbed meshes 10x20 143 / 235, 25x32 140 / 173, 25x40 171 / 202,
-// 32x48 216 / 176. Beyond the limits 16 SMs lack the throughput.
+// Four SSPRK3 steps, this kernel / the graph (us; retries differ from mesh to
+// mesh). Uniform: 20x20 338 / 523, 25x40 509 / 647, 32x48 521 / 574, 32x64 and
+// beyond slower; with a lithostatic pressure, whose wet flags need the
+// quadrature in every stage, 25x40 440 / 474, 32x40 496 / 486; with diffusion
+// 25x40 688 / 835, 32x40 636 / 637. Perturbed: 20x24 601 / 955, 25x40 603 / 735,
+// 32x48 slower, lithostatic 25x40 634 / 724; with diffusion 20x24 807 / 1240,
+// 25x40 882 / 951. Where no cell is plain the tested forms have a lane per
+// element in both and the graph has more of the GPU: pure component 20x20
+// 514 / 526, 32x48 617 / 537, with diffusion 20x20 696 / 665, 25x40 1019 / 847;
+// perturbed 25x40 886 / 790, with diffusion 20x24 878 / 927, 20x32 998 / 943,
+// 25x40 1111 / 919. The limits are where the ordinary cells gain and those do
+// not lose more. A cluster of 8 blocks has half the throughput: 20x20 384,
+// 24x32 597 / 652, 25x40 670 / 647, perturbed 20x24 717 / 955, 25x32 802 / 746.
 int small_steps_blocks(const SmallMesh& m) {
     const long long cells = (long long)m.nx * m.ny;
-    if (cells > (m.quad ? kSmallQuadCells : kSmallCells) || m.ph->source) return 0;
-    return small_blocks(small_kernel(m.quad, m.ph->litho != 0));
+    const long long limit = m.quad ? (m.ph->diffusion ? kSmallQuadDiffusion : kSmallQuadCells)
+                                   : (m.ph->diffusion || m.ph->litho ? kSmallCellsMore : kSmallCells);
+    if (cells > limit || m.ph->source) return 0;
+    const int blocks = small_blocks(small_kernel(m.quad, m.ph->litho != 0));
+    return 16 * cells <= limit * blocks ? blocks : 0;
 }
 
 mp_status launch_small_steps(const SmallMesh& s, int blocks, cudaStream_t stream) {

@@ -44,7 +44,7 @@ constexpr int kRedBlock = 256;
 // same). A function of the mesh alone: the grouping fixes the order of the
 // sums.
 constexpr int kSumPer = 4;
-constexpr long long kSumOne = 16384, kSmallCells = 1536, kSmallQuadCells = 1024;
+constexpr long long kSumOne = 16384, kSmallCells = 1536;   // kSmallCells: steps in one cluster (small_steps.cu)
 static_assert(kSmallCells <= kSumOne, "the cluster's sums take one cell per thread");
 __host__ __device__ __forceinline__ int sum_per(long long cells) {
     const long long wave = 592LL * kRedBlock, per = (cells + wave - 1) / wave;

@@ -103,3 +103,28 @@ def test_cells_that_are_not_plain_agree_on_every_path(cuda_lib, nx, ny, quad, ki
         assert s["status"] == 0
         for x, name in zip(a[3], ("H", "C", "T", "phi")):
             assert np.array_equal(x, s[name]), name
+
+
+@pytest.mark.parametrize("nx,ny,quad,diffusion,lithostatic", [
+    (32, 48, False, 0.0, False), (32, 32, False, 1e-3, False), (25, 41, False, 1e-3, False), (32, 32, False, 0.0, True),
+    (25, 41, False, 0.0, True), (32, 32, True, 0.0, False), (20, 32, True, 1e-3, False), (27, 24, True, 1e-3, False)])
+def test_both_sides_of_the_cluster_kernels_limits(cuda_lib, nx, ny, quad, diffusion, lithostatic):
+    """Meshes at the limits of the cluster kernel (1536 cells, 1024 with
+    diffusion or a lithostatic pressure; quads 1024 and 640) and just beyond:
+    the host-driven loop's states and reports."""
+    from mantlepar_b200.transport import TransportConfig
+    cfg = TransportConfig(cfl=0.4, integrator=3, diffusivity=diffusion)
+    got = []
+    for device in (True, False):
+        t = transport(nx, ny, cfg, quad)
+        t.set_device_steps(device)
+        if diffusion:
+            t.set_thermal_bc((1, 2, 0, 1), (0.9, -0.02, 0.0, 0.4))
+        if lithostatic:
+            t.set_pressure_model(t.LITHOSTATIC, 1.1)
+        code, reps = t.step(5)
+        got.append((code, reps, t.get_time(), t.get_state()))
+        t.close()
+    assert got[0][:3] == got[1][:3]
+    for x, y in zip(got[0][3], got[1][3]):
+        assert np.array_equal(x, y)
