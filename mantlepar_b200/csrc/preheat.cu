@@ -11,7 +11,7 @@
 // in a fixed order and applies the step's checks (finite candidate, heat
 // balance), accepting or stopping. The step sizes do not depend on the state (the rate is fixed at Build), so
 // the host plans a batch of steps and issues them without waiting; a failed
-// step sets the status word and every kernel queued after it does no work.
+// step sets the status words and every kernel queued after it does no work.
 //
 // On a general quad mesh (mp_preheat_create_quads; the reference's preheat
 // runs on any mesh family, preheat.cpp:86-117) the step, rate and diagnostics
@@ -84,8 +84,13 @@ constexpr int kPreBlock = 256;
 constexpr int kPrePer = 4;                      // cells per thread in the per-cell kernels
 constexpr int kPreCells = kPreBlock * kPrePer;
 
+// The status words: [0] the first failure, which every block of a launch may
+// lower while the others still run, and [1] set by a launch's last block once
+// the step has failed. Launches queued after it go by [1], so that every block
+// of the failing launch does its work and the failure reported is the first by
+// part and key, whichever block met one first.
 __device__ __forceinline__ bool halted(const unsigned long long* status) {
-    return *(volatile const unsigned long long*)status != ~0ULL;
+    return *(volatile const unsigned long long*)(status + 1) != ~0ULL;
 }
 
 // Fixed-tree block reduction; the result is valid in thread 0.
@@ -476,15 +481,20 @@ __global__ void __launch_bounds__(kStepBlock, kQuad ? 4 : 5) pre_step_kernel(con
     if (!pre_finish_blocks(acc, a.partial, a.ctl, tot) || threadIdx.x != 0) return;
     if (a.mode != PRE_STEP) { a.ctl->last = tot; return; }
     // The step's checks (preheat.cpp:267-273), unless a cell or an edge failed.
-    if (halted(a.status)) return;
-    if (tot.nonfinite != 0.0) { record_error(a.status, PART_CELLS, 0, E_FP); return; }
     const double prev = a.ctl->prev_integral;
     const double bal = tot.integral - prev + a.dt * tot.bflux;
     const double tol = 1e-10 * (1.0 + fabs(tot.integral) + fabs(prev) + fabs(a.dt * tot.bflux));
-    if (!(fabs(bal) <= tol)) { record_error(a.status, PART_CELLS, 0, MP_ERR_PLIB); return; }
-    a.rows[a.row] = PreRow{tot.integral, tot.minimum, tot.maximum, tot.bflux, bal};
-    a.ctl->prev_integral = tot.integral;
-    a.ctl->accepted += 1;
+    if (*(volatile unsigned long long*)a.status == ~0ULL) {
+        if (tot.nonfinite != 0.0) record_error(a.status, PART_CELLS, 0, E_FP);
+        else if (!(fabs(bal) <= tol)) record_error(a.status, PART_CELLS, 0, MP_ERR_PLIB);
+        else {
+            a.rows[a.row] = PreRow{tot.integral, tot.minimum, tot.maximum, tot.bflux, bal};
+            a.ctl->prev_integral = tot.integral;
+            a.ctl->accepted += 1;
+            return;
+        }
+    }
+    a.status[1] = 0;
 }
 
 // Integral, minimum and maximum of a state.
@@ -781,7 +791,7 @@ struct mp_preheat {
     mp::PreRow* rows = nullptr;     // kBatch rows
     mp::PreCtl* h_ctl = nullptr;    // pinned mirrors
     mp::PreRow* h_rows = nullptr;
-    unsigned long long* d_status = nullptr;
+    unsigned long long* d_status = nullptr;   // two words (halted)
     unsigned long long* h_status = nullptr;
     int blocks = 0;                 // of the per-cell kernels
     int passes = 1;                 // row groups per block of pre_step_kernel
@@ -828,7 +838,7 @@ mp_status pre_status(mp_preheat* p, const char* where) {
 }
 
 mp_status reset_status(mp_preheat* p) {
-    MP_CUDA(cudaMemsetAsync(p->d_status, 0xff, sizeof(unsigned long long), p->stream));
+    MP_CUDA(cudaMemsetAsync(p->d_status, 0xff, 2 * sizeof(unsigned long long), p->stream));
     return MP_OK;
 }
 
@@ -1015,13 +1025,13 @@ mp_status preheat_create_impl(const mp_mesh_desc* mesh, const double* xy, const 
     alloc((void**)&p->partial, blocks * sizeof(PrePartial));
     alloc((void**)&p->ctl, sizeof(PreCtl));
     alloc((void**)&p->rows, kBatch * sizeof(PreRow));
-    alloc((void**)&p->d_status, sizeof(unsigned long long));
+    alloc((void**)&p->d_status, 2 * sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&p->h_ctl, sizeof(PreCtl));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&p->h_rows, kBatch * sizeof(PreRow));
     if (e == cudaSuccess) e = cudaMallocHost((void**)&p->h_status, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaMemsetAsync(p->vn, 0, NE * kNQ * sizeof(double), p->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(p->ctl, 0, sizeof(PreCtl), p->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p->d_status, 0xff, sizeof(unsigned long long), p->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p->d_status, 0xff, 2 * sizeof(unsigned long long), p->stream);
     if (xy && e == cudaSuccess) {
         const int gs = upload_quad_tables(p->nx, p->ny, xy, qt, 0, p->ny, p->stream, &p->qbuf, p->qdev, &e);
         if (gs == MP_ERR_ARG_WRONG) {
