@@ -175,8 +175,8 @@ enum : unsigned char { FLAG_WET = 1, FLAG_CHECK = 2, FLAG_PLAIN = 4 };
 // The flag byte of a cell from its neighbour bounds: the limiter keeps every
 // limited value at the cell's points (cell and edge Gauss points, diffusion
 // samples) within [lo, hi] up to roundoff, and Hliq at (hi_C, lowest tep) is
-// the lowest liquidus, so bounds that keep a margin of 1e-12 prove each
-// point's admissibility: the samples' (cell flagged otherwise: they are
+// the lowest liquidus, so bounds that keep a margin of 1e-12 of the field's
+// largest value from the ends of the ranges prove each point's admissibility: the samples' (cell flagged otherwise: they are
 // checked one by one), and for a plain cell all of them. Melt begins where H
 // passes Tep, so with a constant pressure a plain cell is wet when topH, its
 // largest limited enthalpy at the quadrature points, does (with a
@@ -186,7 +186,7 @@ __device__ __forceinline__ unsigned char cell_flags(const Physics& ph, double te
     const double Hliq = tep_lo + (1.0 - hiC * ph.sk.invXe) + ph.k.LD;
     const double slack = 1e-12 * (1.0 + fabs(hiH));
     if (!(tep_lo >= 0.0 && hiH + slack < Hliq)) return FLAG_CHECK;
-    if (!(ph.sk.ordinary && tep_lo >= 1e-9 && tep_hi <= 1e100 && loH >= slack && loC >= 1e-90 &&
+    if (!(ph.sk.ordinary && tep_lo >= 1e-9 && tep_hi <= 1e100 && loH >= slack && loC >= 1e-90 + 1e-12 * hiC &&
           hiC <= ph.k.Xe * (1.0 - 1e-12)))
         return 0;
     return FLAG_PLAIN | (!ph.litho && topH > ph.Tep ? FLAG_WET : 0);
