@@ -128,3 +128,133 @@ def test_both_sides_of_the_cluster_kernels_limits(cuda_lib, nx, ny, quad, diffus
     assert got[0][:3] == got[1][:3]
     for x, y in zip(got[0][3], got[1][3]):
         assert np.array_equal(x, y)
+
+
+def failing_minimum(nx, ny, cfg_of, quad):
+    """A minimum step for which a run gives up at its first retry, after a
+    stage of the rejected attempt was evaluated; and that step's index."""
+    t = transport(nx, ny, cfg_of(1e-14), quad)
+    reps = t.step(200)[1]
+    t.close()
+    k = next(i for i, r in enumerate(reps) if r["retries"])
+    attempted = reps[k]["dt"] * 2 ** reps[k]["retries"]
+    assert all(r["dt"] > 0.75 * attempted for r in reps[:k])
+    return 0.75 * attempted, k
+
+
+@pytest.mark.parametrize("integrator", [2, 3])
+@pytest.mark.parametrize("nx,ny,quad", [(20, 20, False), (48, 40, False), (20, 24, True), (36, 40, True)])
+def test_state_after_a_step_that_fails_in_a_stage(cuda_lib, nx, ny, quad, integrator):
+    """A step given up after a stage was evaluated leaves that stage's T and
+    phi, as the host-driven loop does: single mesh and batch."""
+    from mantlepar_b200.batch import Batch
+    from mantlepar_b200.transport import TransportConfig
+
+    def cfg(dt_min):
+        return TransportConfig(cfl=0.4, integrator=integrator, dt_min=dt_min)
+
+    dt_min, k = failing_minimum(nx, ny, cfg, quad)
+    got = []
+    for device in (True, False):
+        t = transport(nx, ny, cfg(dt_min), quad)
+        t.set_device_steps(device)
+        if k:
+            t.step(k)
+        accepted = t.get_state()
+        code, reps = t.step(70, raise_on_error=False)
+        assert code == 91
+        state = t.get_state()
+        assert np.array_equal(state[0], accepted[0]) and not np.array_equal(state[2], accepted[2])
+        got.append((reps, t.get_time(), state))
+        t.close()
+    assert got[0][:2] == got[1][:2]
+    for x, y in zip(got[0][2], got[1][2]):
+        assert np.array_equal(x, y)
+
+    # The same mesh in a batch, beside one that runs on.
+    w, other = sy.Workload(nx=nx, ny=ny, seed=5), sy.Workload(nx=4, ny=3)
+    states = []
+    for device in (True, False):
+        b = Batch([other], cfg(dt_min))
+        b.set_device_steps(device)
+        xy = sy.quad_vertices(w, sy.MESH_PERTURBED, 0.2, seed=11) if quad else None
+        i = b.add_quads(w, xy) if quad else b.add(w)
+        b.set_face_velocity(0, *sy.face_velocity(other))
+        b.set_state(0, *sy.initial_state(other))
+        b.set_face_velocity(i, *(sy.face_velocity_quads(w, xy) if quad else sy.face_velocity(w)))
+        b.set_state(i, *sy.initial_state(w))
+        reps = b.step(k + 3)
+        s = b.get_state(i)
+        assert s["status"] == 91
+        states.append((reps, s))
+        b.close()
+    assert states[0][0] == states[1][0]
+    for name in ("H", "C", "T", "phi"):
+        assert np.array_equal(states[0][1][name], states[1][1][name]), name
+    for x, name in zip(got[0][2], ("H", "C", "T", "phi")):
+        assert np.array_equal(x, states[0][1][name]), name
+
+
+FORMS = [(20, 20, False), (48, 40, False), (20, 24, True), (36, 40, True)]
+
+
+def run_both(make, steps):
+    got = []
+    for device in (True, False):
+        t = make(device)
+        code, reps = t.step(steps, raise_on_error=False)
+        got.append(dict(code=code, reps=reps, time=t.get_time(), state=t.get_state(), syncs=t.host_syncs(),
+                        message=t._lib.mp_last_error_string() if code else b""))
+        t.close()
+    a, b = got
+    for key in ("code", "reps", "time", "message"):
+        assert a[key] == b[key], key
+    for x, y in zip(a["state"], b["state"]):
+        assert np.array_equal(x, y)
+    return a, b
+
+
+@pytest.mark.parametrize("integrator", [2, 3])
+@pytest.mark.parametrize("nx,ny,quad", FORMS)
+def test_long_runs_with_retries(cuda_lib, nx, ny, quad, integrator):
+    """Several chunks of 64 steps with CFL retries among them."""
+    from mantlepar_b200.transport import TransportConfig
+
+    def make(device):
+        t = transport(nx, ny, TransportConfig(cfl=0.4, integrator=integrator), quad)
+        t.set_device_steps(device)
+        return t
+
+    a, b = run_both(make, 200)
+    assert a["code"] == 0 and sum(r["retries"] for r in a["reps"]) > 0
+    assert a["syncs"] <= 1 + 4 and b["syncs"] >= 3 * 200
+
+
+@pytest.mark.parametrize("nx,ny,quad", FORMS)
+@pytest.mark.parametrize("control", ["end", "fixed", "fixed too large", "minimum", "setters"])
+def test_time_controls_and_setters(cuda_lib, nx, ny, quad, control):
+    """An end time inside the run, the fixed control below and above the CFL
+    bound, a minimum step that no attempt meets, and setters between runs."""
+    from mantlepar_b200.transport import Transport, TransportConfig
+    options = {"fixed": dict(dt_initial=2e-5), "fixed too large": dict(dt_initial=1.0), "minimum": dict(dt_min=10.0),
+               "setters": dict(diffusivity=1e-4)}.get(control, {})
+
+    def make(device):
+        t = transport(nx, ny, TransportConfig(cfl=0.4, integrator=3, **options), quad)
+        t.set_device_steps(device)
+        if control == "end":
+            dt = t.step(3)[1][-1]["dt"]
+            t.set_time_control(Transport.CFL, t.get_time()[0] + 10.5 * dt)
+        elif control.startswith("fixed"):
+            t.set_time_control(Transport.FIXED)
+        elif control == "setters":
+            t.step(10)
+            t.set_thermal_bc((1, 1, 0, 0), (0.9, 0.2, 0.0, 0.0))
+            t.step(10)
+            t.set_state(*sy.initial_state(sy.Workload(nx=nx, ny=ny, seed=9)))
+        return t
+
+    a, _ = run_both(make, 20)
+    assert a["code"] == {"fixed too large": 63, "minimum": 91}.get(control, 0)
+    if control == "end":
+        assert a["reps"][-1]["dt"] == 0.0
