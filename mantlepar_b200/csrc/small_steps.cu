@@ -168,6 +168,8 @@ __device__ __noinline__ void small_edges_rest(const SmallArgs& m, int kind, int 
     each_of_warp(group, groups, nx * (ny + 1) + (nx + 1) * ny, [&](int k) {
         const EdgeAt at = edge_by_kind(nx, ny, k);
         const EdgeCells g = edge_cells(a, at);
+        MP_CHECK_INDEX(a.status, g.L, nx * ny);
+        if (!g.boundary) MP_CHECK_INDEX(a.status, g.R, nx * ny);
         if (!(a.flags[g.L] & (g.boundary ? 0xff : a.flags[g.R]) & FLAG_PLAIN)) {
             if (kQuad) quad_face_general(m.quad[kind], m.ph, g.e);
             else face_general<kLitho>(m.tab, a, m.ph, g.e);
@@ -188,8 +190,12 @@ __device__ __noinline__ void small_quad_diffusion(const SmallArgs& m, int kind, 
     __syncwarp();
     for (int base = group - ((threadIdx.x & 31) >> 3); base < edges; base += groups) {
         const int k0 = base + (int)((threadIdx.x & 31) >> 3);
-        const EdgeAt at = edge_by_kind(nx, ny, k0 < edges ? k0 : edges - 1);
-        const QuadEdge g = quad_edge(a.q, nx, ny, 0, ny, at.horizontal, at.i, at.j);
+        bool active = k0 < edges;
+        const EdgeAt at = edge_by_kind(nx, ny, active ? k0 : edges - 1);
+        QuadEdge g = quad_edge(a.q, nx, ny, 0, ny, at.horizontal, at.i, at.j);
+        g.e = checked_index(a.status, g.e, edges, active);
+        g.L = checked_index(a.status, g.L, N, active);
+        if (!g.boundary) g.R = checked_index(a.status, g.R, N, active);
         const int type = g.boundary ? ph.wall_type[g.wall] : 1;
         double len, grad = 0.0, all[kNQ];
         P2 nrm;
@@ -208,7 +214,7 @@ __device__ __noinline__ void small_quad_diffusion(const SmallArgs& m, int kind, 
             const int s = __shfl_sync(kAll, st, n, kGroup);
             first = first ? first : s;
         }
-        if (k0 >= edges || l != 0 || type == 0) continue;
+        if (!active || l != 0 || type == 0) continue;
         quad_diffusion_add(a, ph, g, type, len, [&](int k) { return all[k]; });
         if (first) record_error(a.status, PART_FACES, g.L, first);
     }
@@ -227,8 +233,9 @@ __device__ __noinline__ void small_recon(const SmallArgs& m, int kind, int group
     bool rest = false;
     for (int base = group - ((threadIdx.x & 31) >> 3); base < N; base += groups) {
         const int c0 = base + (int)((threadIdx.x & 31) >> 3);
-        const bool active = c0 < N;
-        const int cell = active ? c0 : N - 1;   // idle groups repeat the last cell and write nothing
+        bool active = c0 < N;
+        // Idle groups repeat the last cell and write nothing.
+        const int cell = checked_index(a.status, active ? c0 : N - 1, N, active);
         const int i = cell % nx, j = cell / nx;
         const int ci = i == 0 ? 0 : (i == nx - 1 ? 2 : 1), cj = j == 0 ? 0 : (j == ny - 1 ? 2 : 1);
         const double* F = f ? a.C : a.H;
@@ -237,7 +244,7 @@ __device__ __noinline__ void small_recon(const SmallArgs& m, int kind, int group
         for (int dj = 0; dj < 3; ++dj)
 #pragma unroll
             for (int di = 0; di < 3; ++di)
-                u[dj][di] = MP_LD(F + min(max(j + dj - 1, 0), ny - 1) * nx + min(max(i + di - 1, 0), nx - 1));
+                u[dj][di] = MP_LD(F + checked_index(a.status, min(max(j + dj - 1, 0), ny - 1) * nx + min(max(i + di - 1, 0), nx - 1), N, active));
         double lo = u[1][1], hi = u[1][1];
         const double mean = u[1][1];
 #pragma unroll
@@ -314,8 +321,8 @@ __device__ __noinline__ void small_quad_recon(const SmallArgs& m, int kind, int 
     bool rest = false;
     for (int base = group - ((threadIdx.x & 31) >> 3); base < N; base += groups) {
         const int c0 = base + (int)((threadIdx.x & 31) >> 3);
-        const bool active = c0 < N;
-        const int cell = active ? c0 : N - 1;
+        bool active = c0 < N;
+        const int cell = checked_index(a.status, active ? c0 : N - 1, N, active);
         const int i = cell % nx, j = cell / nx;
         const int ci = i == 0 ? 0 : (i == nx - 1 ? 2 : 1), cj = j == 0 ? 0 : (j == ny - 1 ? 2 : 1);
         const double* F = f ? a.C : a.H;
@@ -324,7 +331,7 @@ __device__ __noinline__ void small_quad_recon(const SmallArgs& m, int kind, int 
         for (int dj = 0; dj < 3; ++dj)
 #pragma unroll
             for (int di = 0; di < 3; ++di)
-                u[0][dj][di] = MP_LD(F + min(max(j + dj - 1, 0), ny - 1) * nx + min(max(i + di - 1, 0), nx - 1));
+                u[0][dj][di] = MP_LD(F + checked_index(a.status, min(max(j + dj - 1, 0), ny - 1) * nx + min(max(i + di - 1, 0), nx - 1), N, active));
         const double mean = u[0][1][1];
         double lo = mean, hi = mean;
 #pragma unroll
@@ -357,6 +364,7 @@ __device__ __noinline__ void small_quad_recon(const SmallArgs& m, int kind, int 
             long long id;
             bool wall, rev;
             cell_edge(nx, ny, i, j, 0, ny, part, id, wall, rev);
+            id = checked_index(a.status, id, nx * (ny + 1) + (nx + 1) * ny, active);
             const P2 p = part == 0 ? k.n[0] : part == 1 ? k.n[1] : part == 2 ? k.n[2] : k.n[3];
             const P2 v = part == 0 ? k.n[1] : part == 1 ? k.n[2] : part == 2 ? k.n[3] : k.n[0];
             const P2 mid = P2{0.5 * (p.x + v.x), 0.5 * (p.y + v.y)}, half = P2{0.5 * (v.x - p.x), 0.5 * (v.y - p.y)};
@@ -405,8 +413,8 @@ __device__ __noinline__ void small_phase(const SmallArgs& m, int kind, int group
     const CellPhaseArgs& a = m.phase[kind];
     for (int base = group - ((threadIdx.x & 31) >> 3); base < N; base += groups) {
         const int c0 = base + (int)((threadIdx.x & 31) >> 3);
-        const bool active = c0 < N;
-        const int cell = active ? c0 : N - 1;
+        bool active = c0 < N;
+        const int cell = checked_index(a.status, active ? c0 : N - 1, N, active);
         const unsigned char fl = a.flags[cell];
         double Trow = 0.0, Prow = 0.0;
         if (fl & FLAG_PLAIN) {
@@ -470,9 +478,12 @@ __device__ __noinline__ void small_faces(const SmallArgs& m, int kind, int group
     bool rest = false;
     for (int base = group - ((threadIdx.x & 31) >> 3); base < edges; base += groups) {
         const int k0 = base + (int)((threadIdx.x & 31) >> 3);
-        const bool active = k0 < edges;
+        bool active = k0 < edges;
         const EdgeAt at = edge_by_kind(nx, ny, active ? k0 : edges - 1);
-        const EdgeCells g = edge_cells(a, at);
+        EdgeCells g = edge_cells(a, at);
+        g.e = checked_index(a.status, g.e, edges, active);
+        g.L = checked_index(a.status, g.L, N, active);
+        if (!g.boundary) g.R = checked_index(a.status, g.R, N, active);
         const unsigned char fl = a.flags[g.L] & (g.boundary ? 0xff : a.flags[g.R]);
         const bool plain = (fl & FLAG_PLAIN) != 0, wet = (fl & FLAG_WET) != 0;
         PointFlux pf{0.0, 0.0, 0.0, 0.0};

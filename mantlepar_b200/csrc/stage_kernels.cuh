@@ -163,6 +163,20 @@ __device__ __forceinline__ void record_error(unsigned long long* status, int par
     do {                               \
     } while (0)
 #endif
+// The same where the element may not return, as its warp shuffles or meets a
+// barrier further on: an index outside [0, n) is recorded, `active` cleared and
+// 0 taken in its place.
+template <class T>
+__device__ __forceinline__ T checked_index(unsigned long long* status, T idx, long long n, bool& active) {
+#ifdef MP_CHECKED
+    if (!(idx >= 0 && idx < n)) {
+        if (status) record_error(status, PART_CHECK, idx < 0 ? 0 : idx, MP_ERR_ARG_OUTOFRANGE);
+        active = false;
+        return 0;
+    }
+#endif
+    return idx;
+}
 
 
 // ------------------------------------------------------- reconstruction kernel
@@ -553,7 +567,8 @@ __device__ __forceinline__ void stage_source(const CellPhaseArgs& a, long long f
 template <bool kExt>
 __device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhaseArgs& a, const Physics& ph, long long cell,
                                                long long end, bool averages, const double* vy = nullptr) {
-    const bool valid = cell < end;
+    bool valid = cell < end;
+    if (valid) cell = checked_index(a.status, cell, (long long)a.nx * a.ny, valid);
     const unsigned char fl = valid ? a.flags[cell] : 0;
     if (!averages && !(kExt && (ph.litho || ph.source)) && (fl & FLAG_PLAIN)) return;
     double DH[9], DC[9];
@@ -567,7 +582,6 @@ __device__ __forceinline__ void cellphase_cell(const StageHot& t, const CellPhas
         __syncwarp();
     }
     if (!valid) return;
-    MP_CHECK_INDEX(a.status, cell, (long long)a.nx * a.ny);
     if (!(fl & FLAG_PLAIN)) { cellphase_general<kExt>(t, a, ph, cell); return; }
     const int gj = a.gj0 + (int)((unsigned)cell / (unsigned)a.nx);
     double Tsum = 0.0, Psum = 0.0, Ssum = 0.0, Rsum = 0.0;
