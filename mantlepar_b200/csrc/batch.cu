@@ -937,7 +937,7 @@ mp_status add_while(cudaGraph_t g, const std::vector<cudaGraphNode_t>& deps, cud
 }
 
 // The graph of up to kGraphChunk steps of every instance:
-//   WHILE run:  begin -> WHILE attempt: {attempt, axpy, reduce, gate,
+//   WHILE run:  begin -> WHILE attempt: {attempt, axpy, gate,
 //               stage B, control [, stage C, control]} -> commit, copy,
 //               stage P (L(U^{n+1})), control (run condition).
 mp_status capture_graph(mp_batch* b, cudaGraph_t* out) {
@@ -1074,7 +1074,7 @@ mp_status graph_steps(mp_batch* b, int nsteps, mp_step_report* reports) {
         const CtlHeader h = *b->h_hdr;
         // Kernels the graph ran: per step 5 control/copy kernels and one
         // stage; per attempt 4 control/axpy kernels and one or two stages.
-        const int per_attempt = 4 + (b->stage_kernels + 1) * (b->opts.integrator == MP_SSPRK3 ? 2 : 1);
+        const int per_attempt = 3 + (b->stage_kernels + 1) * (b->opts.integrator == MP_SSPRK3 ? 2 : 1);
         count_launch((unsigned long long)h.step * (3 + b->stage_kernels + 1) +
                      (unsigned long long)h.total_attempts * per_attempt);
         // T and phi of the stage that an instance failed after: the latest

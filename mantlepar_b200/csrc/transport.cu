@@ -602,7 +602,7 @@ mp_status add_while(cudaGraph_t g, const std::vector<cudaGraphNode_t>& deps, cud
 }
 
 // The graph of up to kGraphSteps steps, the same kernels as do_step:
-//   WHILE run:  begin -> WHILE attempt: {attempt, axpy, reduce, gate, stage 2,
+//   WHILE run:  begin -> WHILE attempt: {attempt, axpy, gate, stage 2,
 //               control [, stage 3, control]} -> commit, copy, L(U^{n+1}),
 //               control (run condition).
 mp_status capture_steps(mp_transport* t, cudaGraph_t g) {

@@ -258,3 +258,24 @@ def test_time_controls_and_setters(cuda_lib, nx, ny, quad, control):
     assert a["code"] == {"fixed too large": 63, "minimum": 91}.get(control, 0)
     if control == "end":
         assert a["reps"][-1]["dt"] == 0.0
+
+
+def test_a_batch_counts_the_launches_of_its_graph(cuda_lib):
+    """A batch of one mesh runs the kernels of the single mesh's step graph:
+    the same launches for the same steps and attempts."""
+    from mantlepar_b200._capi import kernel_launches
+    from mantlepar_b200.batch import Batch
+    from mantlepar_b200.transport import TransportConfig
+    cfg = TransportConfig(cfl=0.4, integrator=3)
+    w = sy.Workload(nx=48, ny=40, seed=5)
+    t, b = transport(48, 40, cfg), Batch([w], cfg)
+    b.set_face_velocity(0, *sy.face_velocity(w))
+    b.set_state(0, *sy.initial_state(w))
+    counts = []
+    for x in (t, b):
+        x.step(2)
+        before = kernel_launches()
+        x.step(60)
+        counts.append(kernel_launches() - before)
+        x.close()
+    assert counts[0] == counts[1]
