@@ -1240,7 +1240,11 @@ __device__ __forceinline__ void diffusion_edge(const StageHot& t, const FaceArgs
     MP_CHECK_INDEX(a.status, g.L, N);
     if (!g.boundary) MP_CHECK_INDEX(a.status, g.R, N);
     const unsigned char fl = a.flags[g.L] & (g.boundary ? 0xff : a.flags[g.R]);
-    if (!(fl & FLAG_PLAIN) || (g.boundary && ph.wall_type[wall] == MP_THERMAL_FLUX)) diffusion_general(t, a, ph, g.e);
+    // A wall temperature beyond 1e100 takes the form that tests the gradient
+    // for overflow; a plain cell's temperatures stay below.
+    const bool tested = !(fl & FLAG_PLAIN) ||
+                        (g.boundary && (ph.wall_type[wall] == MP_THERMAL_FLUX || !(fabs(ph.wall_value[wall]) <= 1e100)));
+    if (tested) diffusion_general(t, a, ph, g.e);
     else if (g.boundary) diffusion_wall(t, a, ph, g.e, wall);
     else diffusion_plain<false>(t, a, ph, at, g, 0);
 }
