@@ -222,6 +222,13 @@ struct PreEdge {
     double dif_int, dif_bnd;   // d flux / d (v_L - v_last)
 };
 
+// Whether the gradient at a wall of prescribed temperature, sum_k c_k x / ds in
+// the order of its samples (c = 1/4, -4/3, 3, -4), overflows although the flux d,
+// in which kappa scales it, may not. Out of line: |x| beyond 1e280.
+__device__ __noinline__ bool wall_gradient_overflows(double kappa, double half, double x, double d) {
+    return !isfinite(4.0 * x) || (kappa > 0.0 && !isfinite(d / (2.0 * half * kappa)));
+}
+
 // Edge flux of preheat.cpp:166-196: advection and diffusion of H out of the
 // left (wall) cell. The traces and the velocity are finite exactly when every
 // Lax-Friedrichs flux is or overflows, and the sum of them shows both, so the
@@ -277,8 +284,8 @@ __device__ __forceinline__ double pre_flux(const PreheatPhys& pp, const PreEdge&
             for (int q = 0; q < kNQ; ++q) w += gw[q];
             sum = fma(w * g.half, wv, sum);
         } else if (pp.wall_type[g.wall] == MP_THERMAL_TEMPERATURE) {
-            const double d = g.dif_bnd * ((g.right ? mR : mL) - wv);
-            if (!isfinite(d)) st = st ? st : E_FP;
+            const double x = (g.right ? mR : mL) - wv, d = g.dif_bnd * x;
+            if (!isfinite(d) || (!(fabs(x) < 1e280) && wall_gradient_overflows(pp.kappa, g.half, x, d))) st = st ? st : E_FP;
             sum += d;
         }
     }

@@ -27,3 +27,17 @@ def test_transport(cuda_lib, nx, ny, quad, pure):
     code, _ = t.step(2, raise_on_error=False)
     assert code == 72
     t.close()
+
+
+@pytest.mark.parametrize("quad", [False, True])
+def test_preheat(cuda_lib, quad):
+    from mantlepar_b200.preheat import Preheat, PreheatConfig
+    w = sy.Workload(nx=12, ny=10, seed=5)
+    xy = sy.quad_vertices(w, sy.MESH_PERTURBED, 0.2, seed=11) if quad else None
+    p = Preheat(w, PreheatConfig(end=1.0, cfl=0.5, diffusivity=1e-4, thermal_type=TYPES, thermal_value=VALUES), vertices=xy)
+    p.set_velocity((sy.face_velocity_quads(w, xy) if quad else sy.face_velocity(w))[0])
+    p.set_state(*sy.initial_state(w))
+    p.begin()
+    code, rows = p.advance(2, raise_on_error=False)
+    p.close()
+    assert code == 72 and rows == []
