@@ -155,7 +155,8 @@ static __device__ __noinline__ int weights_general(const double* s, unsigned on,
         sum += w[k];
     }
     for (int k = 0; k < 5; ++k) w[k] /= sum;
-    if (!isfinite(w[0] + w[1] + w[2] + w[3] + w[4])) st = MP_ERR_FP;
+    // A sum so small that its reciprocal overflows cannot be normalised.
+    if (!isfinite(w[0] + w[1] + w[2] + w[3] + w[4]) || !isfinite(1.0 / sum)) st = MP_ERR_FP;
     return st;
 }
 __device__ __forceinline__ int weno_weights(const double (&s)[5], unsigned on, double epsA2, double (&w)[5]) {
