@@ -201,10 +201,10 @@ void mp_transport_destroy(mp_transport* t);
 enum { MP_MESH_RECTANGULAR = 0, MP_MESH_PERTURBED = 1, MP_MESH_SINE_STRETCHED = 2 };
 mp_status mp_transport_create_quads(const mp_mesh_desc* mesh, const double* xy, const mp_transport_opts* opts,
                                     mp_stream_t stream, mp_transport** out);
-/* Device bytes a whole-mesh transport of this mesh allocates (quads != 0:
- * a general quad mesh, its per-cell tables and the builder's transient copy
- * of the vertices included), in whole 2 MiB allocation pages; 0 for an
- * invalid mesh. Not included: the first quad-mesh transport of a process
+/* Device bytes a whole-mesh transport of this mesh allocates (quads != 0: an
+ * upper bound for a general quad mesh, its per-cell tables at 172 doubles a
+ * cell, of which 130 are kept, and the builder's transient copy of the
+ * vertices included), in whole 2 MiB allocation pages; 0 for an invalid mesh. Not included: the first quad-mesh transport of a process
  * raises the CUDA runtime's per-thread stack reservation to the per-cell
  * table builder's 2.7 KB (about 0.5 GB more on a B200), once, for the rest
  * of the process. No counterpart in the reference (host memory there). */

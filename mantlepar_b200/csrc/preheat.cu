@@ -143,44 +143,28 @@ __device__ bool pre_finish_blocks(PrePartial v, PrePartial* partial, PreCtl* ctl
     return true;
 }
 
-// Orientation of edge e as the reference's Build (preheat.cpp:86-95):
-// left cell L (the wall cell on a boundary, whose edge is then reversed when
-// the canonical normal points into it), right cell R, the edge's fixed
-// normalised coordinate in each cell's frame, and the wall.
+// Edge e of a uniform mesh (preheat.cpp:86-95): its direction, whether it is a
+// wall and which, and whether the canonical normal points into the wall cell.
 struct EdgeGeo {
     bool horizontal, boundary, reverse;
-    long long L, R;
-    double lfix, rfix;
     int wall;
 };
 
-__device__ __forceinline__ EdgeGeo edge_geo(const StageHot& t, int nx, int ny, long long e) {
+__device__ __forceinline__ EdgeGeo edge_geo(int nx, int ny, long long e) {
     const long long nI = (long long)nx * (ny + 1);
     EdgeGeo g;
-    g.R = -1;
     g.wall = -1;
-    if (e < nI) {
-        const unsigned ue = (unsigned)e;
-        const int i = (int)(ue % (unsigned)nx), j = (int)(ue / (unsigned)nx);
-        g.horizontal = true;
+    g.horizontal = e < nI;
+    if (g.horizontal) {
+        const int j = (int)((unsigned)e / (unsigned)nx);
         g.boundary = j == 0 || j == ny;
         g.reverse = j == ny;
-        g.L = g.reverse ? (long long)(j - 1) * nx + i : (long long)j * nx + i;
-        if (!g.boundary) g.R = (long long)(j - 1) * nx + i;
-        else g.wall = j == 0 ? 0 : 1;
-        g.lfix = g.reverse ? 1.0 : -1.0;
-        g.rfix = 1.0;
+        if (g.boundary) g.wall = j == 0 ? 0 : 1;
     } else {
-        const unsigned k = (unsigned)(e - nI);
-        const int i = (int)(k % (unsigned)(nx + 1)), j = (int)(k / (unsigned)(nx + 1));
-        g.horizontal = false;
+        const int i = (int)((unsigned)(e - nI) % (unsigned)(nx + 1));
         g.boundary = i == 0 || i == nx;
         g.reverse = i == 0;
-        g.L = g.reverse ? (long long)j * nx : (long long)j * nx + (i - 1);
-        if (!g.boundary) g.R = (long long)j * nx + i;
-        else g.wall = i == 0 ? 2 : 3;
-        g.lfix = g.reverse ? -1.0 : 1.0;
-        g.rfix = -1.0;
+        if (g.boundary) g.wall = i == 0 ? 2 : 3;
     }
     return g;
 }
@@ -535,7 +519,7 @@ __global__ void __launch_bounds__(128) pre_rate_edge_kernel(int nx, int ny, doub
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nE) return;
     const StageHot& t = p.d;
-    const EdgeGeo g = edge_geo(t, nx, ny, e);
+    const EdgeGeo g = edge_geo(nx, ny, e);
     const int o = g.horizontal ? 0 : 1;
     const double len = g.horizontal ? t.len_h : t.len_v;
     int st = 0;

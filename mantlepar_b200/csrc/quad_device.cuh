@@ -157,8 +157,8 @@ __device__ __forceinline__ void visit_samples(const QuadDev& q, int nx, int ny, 
 // candidate's constant from its zero mean over the target; reading the folded
 // smoothness matrices and the constants as well (181 doubles) took 278 us at
 // 640x1280, so it takes 155 (two resident blocks of 255 registers, every
-// table load of a cell in flight; three blocks 176, four 228). Tables of candidates that are off are zero. Returns the first
-// failure in field order.
+// table load of a cell in flight; three blocks 176, four 228). Tables of
+// candidates that are off are zero. Returns the first failure in field order.
 template <int F>
 __device__ __forceinline__ int reconstruct_quad(const QuadDev& q, size_t N, long long cell, int ci, int cj,
                                                 double eA, const double (&u)[F][3][3], double (&D)[F][9]) {

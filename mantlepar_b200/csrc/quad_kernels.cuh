@@ -133,7 +133,7 @@ __device__ __noinline__ void quad_scan_exact(const QuadStageArgs& a, long long c
 // edge, the normal-line samples on this side; mq: the largest H value at the
 // centre and the Gauss points. The points are formed in the
 // cell's frame from its normalised corners (two FMAs each), so that a point
-// costs little beside its two Q2 values (16 FMAs): 2438 FP64 instructions per
+// costs little beside its two Q2 values (16 FMAs): 2461 FP64 instructions per
 // warp and 225 us at 640x1280, against 3135 and 310 us with the points mapped
 // in physical coordinates and every value tested. Bound by the FP64 pipe; 3
 // resident blocks instead of 4 took 248 us, 5 (96 registers) 231.
@@ -341,8 +341,8 @@ __device__ __forceinline__ void quad_cellphase_general(const QuadStageArgs& a, c
 // The same quadrature of a plain cell (phase_plain): the points in the
 // cell's frame, and the Jacobian, which is linear in (r, s), per unit area;
 // averages as for cellphase_cell.
-// 93 us at 640x1280 (217 with every point tested and mapped in physical
-// coordinates); 5 and 6 resident blocks took 106 and 131 us.
+// 101 us at 640x1280 (217 with every point tested and mapped in physical
+// coordinates); 5 and 6 resident blocks took an eighth and two fifths more.
 __device__ __forceinline__ void quad_cellphase_cell(const QuadStageArgs& a, const Physics& ph, long long cell,
                                                     bool averages) {
     const int nx = a.nx;
@@ -513,9 +513,9 @@ __device__ __forceinline__ void quad_edge_values(const QuadStageArgs& a, size_t 
 
 // The same edge between plain cells, or (kWall) at the wall of one: both
 // sides' values first, so that only one side's coefficients are held at a
-// time, then the points without tests or divisions. 167 us at 640x1280 (349
+// time, then the points without tests or divisions. 152 us at 640x1280 (349
 // with both sides' coefficients held and every point tested); 4 and 3
-// resident blocks instead of 5 took 172 and 204 us.
+// resident blocks instead of 5 took 3 and 22 % more.
 template <bool kWall>
 __device__ __forceinline__ void quad_face_plain(const QuadStageArgs& a, const Physics& ph, const QuadEdge& g, bool wet) {
     const QuadDev& q = a.q;

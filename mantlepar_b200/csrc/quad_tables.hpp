@@ -35,11 +35,12 @@ constexpr int kQT4 = 48;   // 4 candidates x 3 differences x 4 monomials
 constexpr int kQS4 = 24;   // 4 candidates x folded 3x3
 constexpr int kQGeo = 4;   // c_x, c_y, h, area
 constexpr int kQMom = 6;   // stencil-frame centre (2), means of x, y, xy, variance sum
-// Table doubles per cell in the memory budget of a request. The device keeps
-// kQG0 + kQT4 + kQMom + kQGeo = 130; with the folded smoothness forms in place
-// of the moments it kept 184. The budget stays above 184 doubles a cell when
-// vertices, spacings and the builder's copy (14 more) are counted, so requests
-// are admitted nearly as they were, and within a fifth of what is taken.
+// Table doubles per cell that mp_transport_instance_bytes counts. The device
+// keeps kQG0 + kQT4 + kQMom + kQGeo = 130; with the folded smoothness forms in
+// place of the moments it kept 184, and callers' budgets were drawn up on that
+// figure. The count is an upper bound that stays near it (more than 184 doubles
+// a cell with vertices, spacings and the builder's copy) and within a fifth of
+// what a whole transport takes.
 constexpr int kQBudget = 172;
 static_assert(kQBudget >= kQG0 + kQT4 + kQMom + kQGeo, "the budget covers the tables");
 

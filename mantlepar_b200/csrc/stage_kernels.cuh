@@ -37,12 +37,12 @@ __device__ __forceinline__ size_t rec_at(long long cell) {
 constexpr int kRedBlock = 256;
 // The accumulation and axpy kernels give each thread several cells (strided by
 // the block size, so loads stay coalesced) before one block reduction: as many
-// as make one wave of 592 resident blocks (at 640x1280 27 us; four cells and
-// 1.35 waves 35), at least four, and one below kSumOne, where few blocks leave
+// as make one wave of 592 blocks, four on each of a B200's 148 SMs (at
+// 640x1280 27 us; four cells and 1.35 waves 35), at least four, and one below kSumOne, where few blocks leave
 // most of the GPU idle (61x127, one step with transfers: 311 us, four 323; a
 // 40x80 quad mesh, four steps: 818, 863; a batch of 24 uneven meshes the
-// same). A function of the mesh alone: the grouping fixes the order of the
-// sums.
+// same). A constant, so that the grouping, which fixes the order of the sums,
+// is a function of the mesh alone.
 constexpr int kSumPer = 4;
 constexpr long long kSumOne = 16384, kSmallCells = 1536;   // kSmallCells: steps in one cluster (small_steps.cu)
 static_assert(kSmallCells <= kSumOne, "the cluster's sums take one cell per thread");
@@ -540,7 +540,7 @@ __device__ __forceinline__ void cellphase_general(const StageHot& t, const CellP
 // The same quadrature of a plain cell: no tests, no failure. Bound by the
 // FP64 pipe; with the tests, clips and library divisions of every point
 // (1239 FP64 and 3187 instructions per warp) it took 100 us at 640x1280, so
-// (641 and 1223) 54 us.
+// (545 and 987) 46 us.
 //
 // The adiabatic source's two velocities at 25 points lie cell by cell (200
 // bytes apart from lane to lane): a warp first copies its cells' stretch to
@@ -964,7 +964,7 @@ __device__ __forceinline__ double face_tep(const StageHot& t, const FaceArgs& a,
 
 // A wall edge of a plain cell (in warps of their own, edge_by_kind). Out of
 // line: its branches in the interior edges' loop cost that loop registers
-// (147 us against 130 at 640x1280).
+// (147 us for them all against 130 when it was taken out).
 template <bool kExt>
 __device__ __noinline__ void face_wall(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
     const EdgeAt at = edge_by_id(a.nx, a.ny, e);
@@ -997,9 +997,9 @@ __device__ __noinline__ void face_wall(const StageHot& t, const FaceArgs& a, con
 // two symmetric pairs, whose values share their even part. With every point
 // tested, clipped and divided through the library, in a loop that carried the
 // boundary policy, the kernel issued 2909 instructions per warp, 969 of them
-// FP64, and took 219 us at 640x1280; so 1201, 474 and 125 us. Bound by the
+// FP64, and took 219 us at 640x1280; so 1135, 482 and 121 us. Bound by the
 // latency of the phase evaluation's chain and the records' loads together
-// (issue 48 %, FP64 pipe 38 %, DRAM 3.6 TB/s).
+// (issue 47 %, FP64 pipe 40 %, DRAM 3.7 TB/s).
 template <bool kExt>
 __device__ __forceinline__ void face_edge(const StageHot& t, const FaceArgs& a, const Physics& ph, const EdgeAt& at) {
     const EdgeCells g = edge_cells(a, at);
@@ -1154,10 +1154,9 @@ __device__ __forceinline__ void diffusion_general(const StageHot& t, const FaceA
 // cell at a wall of prescribed temperature: on each Gauss point's normal line
 // the limited states are one quadratic per side, whose coefficients are taken
 // for the centre and the two symmetric pairs of points. The rate's share is a
-// constant of the edge. 1204 instructions and 151 us at 640x1280; with every
+// constant of the edge. 1100 instructions and 140 us at 640x1280; with every
 // sample tested and its derivative added to the rate one by one 4591 and 441.
-// The derivative
-// weights are [1/24, -9/8, 9/8, -1/24] and [1/4, -4/3, 3, -4, 25/12].
+// The derivative weights are [1/24, -9/8, 9/8, -1/24] and [1/4, -4/3, 3, -4, 25/12].
 template <bool kWall>
 __device__ __forceinline__ void diffusion_plain(const StageHot& t, const FaceArgs& a, const Physics& ph, const EdgeAt& at,
                                                 const EdgeCells& g, int wall) {

@@ -62,11 +62,11 @@ struct SourceBufs {
 // Single-instance kernels: one thread per cell / edge.
 // The stage tables arrive by value as a __grid_constant__ parameter, so the
 // unrolled table coefficients are constant-bank operands. Minimum resident
-// blocks per SM (register caps) as measured fastest on B200: cell phase 6
-// (48 us at 640x1280; 8: 55, 5: 51; with the source's buffers 4: 118, 5: 135,
-// 6: 139),
-// faces 5 (127; 4: 133, 6: 129); the reconstruction keeps its natural register
-// count (87 us; 5 and 6 blocks the same).
+// blocks per SM (register caps) as measured fastest on B200 at 640x1280, each
+// against its neighbours in one build: cell phase 6 (48 us; 8: 55, 5: 51; with
+// the source's buffers 4: 118, 5: 135, 6: 139), faces 5 (127; 4: 133, 6: 129);
+// the reconstruction keeps its natural register count (5 and 6 blocks the
+// same). As built now they take 46, 121 and 85 us.
 // Cells [c0, c1) are reconstructed (all rows, or a slab's owned rows +- 1), in
 // id order: with 32x4 tiles a mesh of 321 columns idles a tenth of the lanes.
 __global__ void __launch_bounds__(128) recon_kernel(const __grid_constant__ ReconArgs a,
@@ -106,7 +106,8 @@ __global__ void __launch_bounds__(128, 5) face_kernel(const __grid_constant__ Fa
                                        : edge_by_kind(a.nx, a.ny, k));
 }
 // The diffusive part of the same edges (only launched when diffusion is on).
-// 4 resident blocks: 151 us at 640x1280 (5: 152; 3, unbounded: 171).
+// 4 resident blocks: 151 us at 640x1280 against 152 with 5 and 171 with 3
+// (unbounded); as built now 140.
 __global__ void __launch_bounds__(128, 4) diffusion_kernel(const __grid_constant__ FaceArgs a,
                                                         const __grid_constant__ Physics ph,
                                                         const __grid_constant__ ParamTables p, long long h0,
@@ -979,10 +980,9 @@ extern "C" size_t mp_transport_instance_bytes(const mp_mesh_desc* mesh, int quad
              + pages((N / sum_cells_per_block((long long)N) + 1) * sizeof(Partial)) + page;
     if (quads) {
         const size_t V = 2 * (nx + 1) * (ny + 1);
-        // Per-cell tables and geometry, vertices and edge spacing in one
-        // allocation; the builder's copy of the vertices is held while the
-        // tables are built. The budget takes kQBudget doubles of tables per
-        // cell (quad_tables.hpp).
+        // Per-cell tables and geometry (an upper bound, kQBudget), vertices
+        // and edge spacing in one allocation; the builder's copy of the
+        // vertices is held while the tables are built.
         b += pages(((size_t)kQBudget * N + V + NE * kNQ) * sizeof(double)) +
              pages(V * sizeof(double) + sizeof(int));
     }
