@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(128, 5) batch_quad_face_kernel(const QuadStage
     if (k < w.b) quad_face_edge(a, ph, edge_by_kind(a.nx, a.ny, k));
 }
 
-__global__ void __launch_bounds__(128) batch_quad_diffusion_kernel(const QuadStageArgs* args, const Work* work,
+// Three resident blocks (168 registers; of itself it takes 177 and two).
+__global__ void __launch_bounds__(128, 3) batch_quad_diffusion_kernel(const QuadStageArgs* args, const Work* work,
                                                                    const int* active, const __grid_constant__ Physics ph) {
     const Work w = work[blockIdx.x];
     if (!active[w.inst]) return;

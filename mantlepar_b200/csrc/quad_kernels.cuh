@@ -349,7 +349,7 @@ __device__ __forceinline__ void quad_cellphase_cell(const QuadStageArgs& a, cons
     const size_t N = (size_t)nx * a.ny;
     MP_CHECK_INDEX(a.status, cell, N);
     const unsigned char fl = a.flags[cell];
-    if (!(fl & FLAG_PLAIN)) { quad_cellphase_general(a, ph, cell); return; }
+    if (__builtin_expect(!(fl & FLAG_PLAIN), 0)) { quad_cellphase_general(a, ph, cell); return; }
     if (!averages && !ph.litho && !ph.source) return;
     const QuadDev& q = a.q;
     const CellFrame f = cell_frame(q, nx, N, cell);
@@ -587,13 +587,16 @@ __global__ void __launch_bounds__(128, 5) quad_face_kernel(const __grid_constant
 // evolve.cpp:330-347): temperatures of the limited states at the normal-line
 // samples, spacing per edge point. By Gauss point, so that the lanes of
 // small_steps.cu share an edge: quad_diffusion_gradient is the temperature
-// gradient at point k of an interior edge or a wall of prescribed temperature,
-// quad_diffusion_add the sums over the points in their order.
+// gradient at point k (sample spacing sp) of an interior edge or a wall of
+// prescribed temperature, quad_diffusion_add the sums over the points in their
+// order.
+__device__ __forceinline__ double quad_spacing(const QuadDev& q, const QuadEdge& g, int k) {
+    return __ldg(q.sp + g.e * kNQ + (g.reverse ? kNQ - 1 - k : k));
+}
 __device__ __forceinline__ double quad_diffusion_gradient(const QuadDev& q, const Physics& ph, const QuadEdge& g,
-                                                          const P2& nrm, const Side& sl, const Side& sr, int k, int& st) {
-    const int cq = g.reverse ? kNQ - 1 - k : k;
+                                                          const P2& nrm, const Side& sl, const Side& sr, int k, double sp,
+                                                          int& st) {
     const P2 p = lerp_edge(q.gq[k], g.a, g.b);
-    const double sp = __ldg(q.sp + g.e * kNQ + cq);
     const int count = g.boundary ? 5 : 4;
     double v[5];
 #pragma unroll
@@ -619,7 +622,7 @@ __device__ __forceinline__ double quad_diffusion_gradient(const QuadDev& q, cons
     if (!isfinite(grad)) st = st ? st : E_FP;
     return grad;
 }
-// Adds the diffusive part to the edge's H flux and rate; gradient(k): the
+// Adds the diffusive part to the edge's H flux and rate; gradient(k, sp): the
 // gradient at point k (called for them in order).
 template <class Gradient>
 __device__ __forceinline__ void quad_diffusion_add(const QuadStageArgs& a, const Physics& ph, const QuadEdge& g, int type,
@@ -628,14 +631,13 @@ __device__ __forceinline__ void quad_diffusion_add(const QuadStageArgs& a, const
     const long long nE = (long long)a.nx * (a.ny + 1) + (long long)(a.nx + 1) * a.ny;
     const int count = g.boundary ? 5 : 4;
     const double* c = g.boundary ? q.dif_c_bnd : q.dif_c_int;
-    double integral = 0.0, rate = a.face[2 * nE + g.e];
+    double integral = 0.0, rate = a.face[2 * nE + g.e], clast = 0.0;
+    for (int s = 0; s + 1 < count; ++s) clast -= c[s];
     for (int k = 0; k < kNQ; ++k) {
         const double w = len * q.gw[k] / 2;
         if (g.boundary && type == 2) { integral += w * ph.wall_value[g.wall]; continue; }
-        const double sp = __ldg(q.sp + g.e * kNQ + (g.reverse ? kNQ - 1 - k : k));
-        integral = fma(-(w * ph.kappa), gradient(k), integral);
-        double clast = 0.0;
-        for (int s = 0; s + 1 < count; ++s) clast -= c[s];
+        const double sp = quad_spacing(q, g, k);
+        integral = fma(-(w * ph.kappa), gradient(k, sp), integral);
         const double scale = -w * ph.kappa / sp;
         for (int s = 0; s < count; ++s) {
             if (g.boundary && s + 1 == count) continue;
@@ -665,7 +667,8 @@ __device__ __forceinline__ void quad_diffusion_edge(const QuadStageArgs& a, cons
         if (!g.boundary) load_side(q, N, a.H, a.C, a.rec, g.R, sr);
     }
     int st = 0;
-    quad_diffusion_add(a, ph, g, type, len, [&](int k) { return quad_diffusion_gradient(q, ph, g, nrm, sl, sr, k, st); });
+    quad_diffusion_add(a, ph, g, type, len,
+                       [&](int k, double sp) { return quad_diffusion_gradient(q, ph, g, nrm, sl, sr, k, sp, st); });
     if (st) record_error(a.status, PART_FACES, g.L + (long long)gj0 * nx, st);
 }
 __global__ void __launch_bounds__(128) quad_diffusion_kernel(const __grid_constant__ QuadStageArgs a, const __grid_constant__ Physics ph,

@@ -205,7 +205,7 @@ __device__ __noinline__ void small_quad_diffusion(const SmallArgs& m, int kind, 
             Side sl, sr;
             load_side(a.q, N, a.H, a.C, a.rec, g.L, sl);
             if (!g.boundary) load_side(a.q, N, a.H, a.C, a.rec, g.R, sr);
-            grad = quad_diffusion_gradient(a.q, ph, g, nrm, sl, sr, p, st);
+            grad = quad_diffusion_gradient(a.q, ph, g, nrm, sl, sr, p, quad_spacing(a.q, g, p), st);
         }
         int first = 0;                      // failure of the first point that has one
 #pragma unroll
@@ -215,7 +215,7 @@ __device__ __noinline__ void small_quad_diffusion(const SmallArgs& m, int kind, 
             first = first ? first : s;
         }
         if (!active || l != 0 || type == 0) continue;
-        quad_diffusion_add(a, ph, g, type, len, [&](int k) { return all[k]; });
+        quad_diffusion_add(a, ph, g, type, len, [&](int k, double) { return all[k]; });
         if (first) record_error(a.status, PART_FACES, g.L, first);
     }
 }
