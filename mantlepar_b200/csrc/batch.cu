@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(128, 4) batch_diffusion_kernel(const InstArgs*
     if (!active[w.inst]) return;
     const long long k = (long long)w.a + threadIdx.x;
     const FaceArgs& a = args[w.inst].face;
-    if (k < w.b) diffusion_edge(*a.tab, a, ph, edge_by_kind(a.nx, a.ny, k));
+    if (k < w.b) diffusion_edge<false>(*a.tab, a, ph, edge_by_kind(a.nx, a.ny, k));
 }
 
 // General quad meshes: the per-element bodies of the single-mesh quad

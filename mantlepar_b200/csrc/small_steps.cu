@@ -174,7 +174,7 @@ __device__ __noinline__ void small_edges_rest(const SmallArgs& m, int kind, int 
             if (kQuad) quad_face_general(m.quad[kind], m.ph, g.e);
             else face_general<kLitho>(m.tab, a, m.ph, g.e);
         }
-        if (!kQuad && m.ph.diffusion) diffusion_edge(m.tab, a, m.ph, at);
+        if (!kQuad && m.ph.diffusion) diffusion_edge<kLitho>(m.tab, a, m.ph, at);
     });
 }
 

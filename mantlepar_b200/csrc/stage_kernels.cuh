@@ -454,8 +454,8 @@ __device__ __forceinline__ void load_rec(const double* rec, long long cell, doub
 // samples: cells that are not plain. Inlined, as the other tested forms are: a
 // function of its own reads the tables and constants through generic pointers
 // into the kernel's parameters. Where no cell is plain (pure composition,
-// 640x1280) the cell phase takes 60 us so and took 90 that way, the faces 185
-// and 222, the diffusion 250 and 313; plain cells are as fast either way.
+// 640x1280) the cell phase takes 60 us so and took 90 that way, the faces 182
+// and 220, the diffusion 238 and 313; plain cells are as fast either way.
 // kExt: the lithostatic pressure and the adiabatic source are compiled in
 // (a launch picks the variant; the default path carries none of their code).
 template <bool kExt>
@@ -1051,7 +1051,9 @@ __device__ __forceinline__ void face_edge(const StageHot& t, const FaceArgs& a, 
 // wall value), gradient sum_k c_k (T_k - T_last) / ds, flux -= w kappa grad,
 // and |d flux / d T_k| added to the rate sample by sample. Added to the face
 // results after the advective part, as the reference adds them.
-// Edges with a cell that is not plain.
+// Edges with a cell that is not plain. kLitho: the lithostatic pressure is
+// compiled in.
+template <bool kLitho>
 __device__ __forceinline__ void diffusion_general(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
     const int nx = a.nx, ny = a.ny;
     const long long nI = (long long)nx * (ny + 1);
@@ -1122,7 +1124,7 @@ __device__ __forceinline__ void diffusion_general(const StageHot& t, const FaceA
             const double h = left ? mHL + quad(lh0, lh1, lh2, s) : mHR + quad(rh0, rh1, rh2, s);
             const double c = left ? mCL + quad(lc0, lc1, lc2, s) : mCR + quad(rc0, rc1, rc2, s);
             const long long cellk = left ? L : Rc;
-            const double tep = !ph.litho ? ph.Tep
+            const double tep = !(kLitho && ph.litho) ? ph.Tep
                              : tep_at(ph, height(t, a.gj0 + (int)(cellk / nx), horizontal ? s : at));
             PhaseLean pl;
             int s1 = phase_stage_lean(ph.sk, h, c, tep, pl);
@@ -1157,7 +1159,7 @@ __device__ __forceinline__ void diffusion_general(const StageHot& t, const FaceA
 // constant of the edge. 1100 instructions and 140 us at 640x1280; with every
 // sample tested and its derivative added to the rate one by one 4591 and 441.
 // The derivative weights are [1/24, -9/8, 9/8, -1/24] and [1/4, -4/3, 3, -4, 25/12].
-template <bool kWall>
+template <bool kWall, bool kLitho>
 __device__ __forceinline__ void diffusion_plain(const StageHot& t, const FaceArgs& a, const Physics& ph, const EdgeAt& at,
                                                 const EdgeCells& g, int wall) {
     const int o = at.horizontal ? 0 : 1;
@@ -1198,7 +1200,7 @@ __device__ __forceinline__ void diffusion_plain(const StageHot& t, const FaceArg
 #pragma unroll
                 for (int q = 0; q < (kWall ? 4 : 2); ++q) {
                     const double y = kWall ? t.dif_pos_bnd[wall][q] : t.dif_pos_int[o][2 * n + q];
-                    const double tep = !ph.litho ? ph.Tep : tep_at(ph, height(t, row, at.horizontal ? y : xs));
+                    const double tep = !(kLitho && ph.litho) ? ph.Tep : tep_at(ph, height(t, row, at.horizontal ? y : xs));
                     PhaseLean pl;
                     phase_plain<false>(ph.sk, quad(h[0], h[1], h[2], y), quad(c[0], c[1], c[2], y), tep, pl);
                     v[2 * n + q] = pl.T;
@@ -1226,11 +1228,18 @@ __device__ __forceinline__ void diffusion_plain(const StageHot& t, const FaceArg
     a.face[g.e] = fma(-scale, sum, a.face[g.e]);
     a.face[2 * nE + g.e] = fma(2.0 * scale, weights, a.face[2 * nE + g.e]);
 }
+template <bool kLitho>
 __device__ __noinline__ void diffusion_wall(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e, int wall) {
     const EdgeAt at = edge_by_id(a.nx, a.ny, e);
-    diffusion_plain<true>(t, a, ph, at, edge_cells(a, at), wall);
+    diffusion_plain<true, kLitho>(t, a, ph, at, edge_cells(a, at), wall);
+}
+// With the pressure compiled in, the tested form beside the plain one spills
+// (155 us against 151 at 640x1280 with plain cells): out of line there.
+__device__ __noinline__ void diffusion_general_litho(const StageHot& t, const FaceArgs& a, const Physics& ph, long long e) {
+    diffusion_general<true>(t, a, ph, e);
 }
 
+template <bool kLitho>
 __device__ __forceinline__ void diffusion_edge(const StageHot& t, const FaceArgs& a, const Physics& ph, const EdgeAt& at) {
     const EdgeCells g = edge_cells(a, at);
     const size_t N = (size_t)a.nx * a.ny;
@@ -1243,9 +1252,12 @@ __device__ __forceinline__ void diffusion_edge(const StageHot& t, const FaceArgs
     // for overflow; a plain cell's temperatures stay below.
     const bool tested = !(fl & FLAG_PLAIN) ||
                         (g.boundary && (ph.wall_type[wall] == MP_THERMAL_FLUX || !(fabs(ph.wall_value[wall]) <= 1e100)));
-    if (tested) diffusion_general(t, a, ph, g.e);
-    else if (g.boundary) diffusion_wall(t, a, ph, g.e, wall);
-    else diffusion_plain<false>(t, a, ph, at, g, 0);
+    if (tested) {
+        if constexpr (kLitho) diffusion_general_litho(t, a, ph, g.e);
+        else diffusion_general<false>(t, a, ph, g.e);
+    }
+    else if (g.boundary) diffusion_wall<kLitho>(t, a, ph, g.e, wall);
+    else diffusion_plain<false, kLitho>(t, a, ph, at, g, 0);
 }
 
 // ----------------------------------------------------------------- sum kernel

@@ -107,7 +107,8 @@ __global__ void __launch_bounds__(128, 5) face_kernel(const __grid_constant__ Fa
 }
 // The diffusive part of the same edges (only launched when diffusion is on).
 // 4 resident blocks: 151 us at 640x1280 against 152 with 5 and 171 with 3
-// (unbounded); as built now 140.
+// (unbounded); as built now 140. kLitho: the pressure model is compiled in.
+template <bool kLitho>
 __global__ void __launch_bounds__(128, 4) diffusion_kernel(const __grid_constant__ FaceArgs a,
                                                         const __grid_constant__ Physics ph,
                                                         const __grid_constant__ ParamTables p, long long h0,
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(128, 4) diffusion_kernel(const __grid_constant
     const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nh + nv) return;
     const bool all = nh == (long long)a.nx * (a.ny + 1) && nv == (long long)(a.nx + 1) * a.ny;
-    diffusion_edge(p.d, a, ph, all ? edge_by_kind(a.nx, a.ny, k) : edge_by_id(a.nx, a.ny, k < nh ? h0 + k : v0 + (k - nh)));
+    diffusion_edge<kLitho>(p.d, a, ph, all ? edge_by_kind(a.nx, a.ny, k) : edge_by_id(a.nx, a.ny, k < nh ? h0 + k : v0 + (k - nh)));
 }
 
 // Four resident blocks; with the source three (of 79 registers: a step of the
@@ -336,7 +337,10 @@ void launch_stage_kernels(int nx, int ny, const StageRange& rg, const ParamTable
             else run(2, [&] { face_kernel<false, false><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
         }
         if (ph.diffusion)
-            run(2, [&] { diffusion_kernel<<<(unsigned)((nh + nv + 127) / 128), 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv); });
+            run(2, [&] {
+                if (ph.litho) diffusion_kernel<true><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv);
+                else diffusion_kernel<false><<<g, 128, 0, s>>>(a, ph, pt, h0, nh, v0, nv);
+            });
     }
 }
 
