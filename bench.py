@@ -48,12 +48,12 @@ WORKLOAD = dict(nx=1280, ny=2560)
 ALG_BYTES_PER_CELL_STAGE = 224
 # Executed FP64 operations per cell per stage (DFMA counted as 2, DADD/DMUL
 # as 1) of the stage kernels, from an ncu capture of a 640x1280 stage:
-# reconstruction 1156, cell phase 796, faces 1080, accumulation 43
+# reconstruction 1158, cell phase 796, faces 1110, accumulation 33
 # (per-cell figures are size-independent).
-FP64_FLOPS_PER_CELL_STAGE = 3075
+FP64_FLOPS_PER_CELL_STAGE = 3098
 # DRAM bytes per cell per stage of the four stage kernels from the same capture
 # (640x1280 keeps every stage array above L2 size; traffic scales with cells).
-DRAM_BYTES_PER_CELL_STAGE = 903
+DRAM_BYTES_PER_CELL_STAGE = 876
 # B200 FP64 (vector and tensor) datasheet figure per GPU of an HGX B200
 # (296 TFLOP/s for 8 GPUs); the driver measures no FP64 peak.
 FP64_DATASHEET_TFLOPS = 37.0
